@@ -161,6 +161,7 @@ struct tnt_xplan_s {
 struct CplanDevice {
   GemmJob* jobs = nullptr;
   std::map<int64_t, std::pair<GemmTile*, int32_t>> f64_tiles;    // per nbatch
+  std::map<int64_t, std::pair<ThinTile*, int32_t>> thin_tiles;   // per nbatch (plans of thin products)
   std::map<int64_t, std::pair<GemmTile*, int32_t>> split_tiles;  // per nbatch and tile width
   std::map<int64_t, void*> split_jobs;                             // per slice count and tile width
 };
@@ -176,6 +177,7 @@ struct tnt_cplan_s {
       cudaSetDevice(kv.first);
       cudaFree(kv.second.jobs);
       for (auto& t : kv.second.f64_tiles) cudaFree(t.second.first);
+      for (auto& t : kv.second.thin_tiles) cudaFree(t.second.first);
       for (auto& t : kv.second.split_tiles) cudaFree(t.second.first);
       for (auto& t : kv.second.split_jobs) cudaFree(t.second);
       if (prev >= 0) cudaSetDevice(prev);
@@ -1180,6 +1182,18 @@ std::pair<GemmTile*, int32_t> f64_tiles(tnt_cplan_s* plan, const ComposeArgs& x,
   return ins.first->second;
 }
 
+// The streaming tiles of a plan of thin products on the current device.
+std::pair<ThinTile*, int32_t> thin_tiles(tnt_cplan_s* plan, int64_t nbatch) {
+  const int d = current_device();
+  std::lock_guard<std::mutex> g(plan->mu);
+  CplanDevice& c = plan->on_device(d);
+  auto it = c.thin_tiles.find(nbatch);
+  if (it != c.thin_tiles.end()) return it->second;
+  const std::vector<ThinTile> tv = build_thin_tiles(plan->p->tables.jobs, nbatch);
+  need(tv.size() < (size_t)INT32_MAX, "too many output tiles");
+  return c.thin_tiles.emplace(nbatch, std::make_pair(upload(tv), (int32_t)tv.size())).first->second;
+}
+
 // The plan's device-resident split packing table for (slices, width, format).
 void* split_table_on_device(tnt_cplan_s* plan, int slices, int tile_n, bool i8) {
   const GemmTables& t = plan->p->tables;
@@ -1295,7 +1309,12 @@ tnt_status tnt_compose(tnt_ctx* ctx, const tnt_cplan* cplan, int64_t nbatch, dou
       need(stride_dst >= t.c_size && stride_lhs >= t.a_size && stride_rhs >= t.b_size, "batch stride too small");
     cudaStream_t st = (cudaStream_t)stream;
     const ComposeArgs x{nbatch, dst, stride_dst, lhs, stride_lhs, rhs, stride_rhs, alpha, beta};
-    if (precision == TNT_PREC_FP64) {
+    if (precision == TNT_PREC_FP64 && thin_plan(t.jobs)) {
+      auto tiles = thin_tiles(plan, nbatch);
+      cuda_check(launch_gemm_thin(plan->jobs_dev(), tiles.first, tiles.second, dst, stride_dst, lhs, stride_lhs, rhs,
+                                  stride_rhs, alpha, beta, st),
+                 "thin fp64 grouped gemm launch");
+    } else if (precision == TNT_PREC_FP64) {
       auto tiles = f64_tiles(plan, x, st);
       cuda_check(launch_gemm_f64(plan->jobs_dev(), tiles.first, tiles.second, dst, stride_dst, lhs, stride_lhs, rhs,
                                  stride_rhs, alpha, beta, st),

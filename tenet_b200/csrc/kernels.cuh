@@ -50,6 +50,21 @@ cudaError_t launch_gemm_f64(const GemmJob* jobs, const GemmTile* tiles, int32_t 
                             const double* a, int64_t sa, const double* b, int64_t sb, double alpha, double beta,
                             cudaStream_t stream);
 
+// FP64 grouped GEMM of plans whose every K is at most kThinMaxK (gemm_thin.cu):
+// one streaming pass over tiles of kThinRows x kThinCols outputs, or ranges of
+// columns where a job has fewer than kThinWide rows.
+constexpr int kThinMaxK = 8, kThinRows = 512, kThinCols = 32, kThinWide = 32, kThinWideElems = 2048;
+struct ThinTile {
+  int32_t job, batch;
+  int64_t row, col;
+  int32_t nrow, ncol;
+};
+bool thin_plan(const std::vector<GemmJob>& jobs);
+std::vector<ThinTile> build_thin_tiles(const std::vector<GemmJob>& jobs, int64_t nbatch);
+cudaError_t launch_gemm_thin(const GemmJob* jobs, const ThinTile* tiles, int32_t ntiles, double* c, int64_t sc,
+                             const double* a, int64_t sa, const double* b, int64_t sb, double alpha, double beta,
+                             cudaStream_t stream);
+
 // Split-precision grouped GEMM (BF16 slices, tcgen05 FP32 accumulation, FP64 recombination).
 constexpr int kSplitTileM = 128;
 // Output tile width picked from the sector-size histogram (64 or 128), given

@@ -113,7 +113,7 @@ class PlannedNetwork:
         prec = precision or rt.precision
         sl = slices or rt.slices
         if out is None:
-            out = TensorMap(rt, self.output_space)
+            out = TensorMap.uninitialized(rt, self.output_space)
         elif not out.space.same_as(self.output_space):
             raise ValueError("out does not have the network's output space")
         ws = self._workspace(rt, prec, sl)

@@ -17,6 +17,7 @@
 #include "autotune.hpp"
 #include "host.hpp"
 #include "kernels.cuh"
+#include "panel.cuh"
 
 using namespace tnt;
 
@@ -222,13 +223,22 @@ struct FplanChunks {
   int64_t n = 0;
 };
 
+// Consecutive jobs of the largest-first table that run in one launch per stage.
+struct FacRun {
+  int32_t first = 0, count = 0;
+  int64_t max_k = 0, max_rows = 0, max_cols = 0;
+  bool rectangular = false;  // some sector is not square
+};
+
 struct tnt_fplan_s {
   std::shared_ptr<FactorPlan> p;
   std::mutex mu;
   std::map<int, std::pair<SvdJob*, int64_t*>> dev;  // jobs, work offsets (sector order)
   std::map<int, std::pair<SvdJob*, int64_t*>> lpt;  // the same, cluster jobs then largest first
-  int32_t n_cluster = 0;                            // leading jobs of the lpt tables run on clusters
-  int32_t n_wide = 0;                               // ... the first n_wide of them on 16-CTA clusters
+  int32_t n_old = 0;      // leading jobs of the lpt tables beyond the cluster QR and Jacobi kernels
+  int32_t n_cluster = 0;  // ... of which the first n_cluster run their SVD on clusters,
+  int32_t n_wide = 0;     // ... and the first n_wide of these on 16-CTA clusters
+  std::vector<FacRun> runs;  // the other jobs, by falling k
   std::map<int, FplanChunks> chunks;                // weighted-dot chunk tables
   int64_t work_elems = 0;
   std::vector<int64_t> work_off;
@@ -291,29 +301,63 @@ struct tnt_fplan_s {
       const double r = (double)std::max(jobs[i].m, jobs[i].n), k = (double)jobs[i].k;
       return r * k * k;
     };
-    // Sectors whose blocked Jacobi has at least one column block per cluster
-    // CTA run on a thread-block cluster (svd_cluster_kernel); they go first,
-    // those with a block for each of 16 CTAs (where the device allows such
-    // clusters) ahead of the 8-CTA ones.
+    // Sectors too long for the cluster QR and Jacobi kernels (old = true) go
+    // first; of these, the ones whose blocked Jacobi has at least one column block
+    // per cluster CTA run on a thread-block cluster (svd_cluster_kernel), those
+    // with a block for each of 16 CTAs (where the device allows such clusters)
+    // ahead of the 8-CTA ones.  The rest follow by falling k.
     const int wide = svd_wide_cluster_size();
+    auto old = [&](size_t i) { return std::max(jobs[i].m, jobs[i].n) > kQrMaxRows; };
     auto clustered = [&](size_t i) {
       const int64_t rows = std::max(jobs[i].m, jobs[i].n), k = jobs[i].k;
-      if (svd_on_chip(rows, k)) return 0;
+      if (!old(i) || svd_on_chip(rows, k)) return 0;
       const int bw = svd_block_width(rows, k);
       if (bw <= 0) return 0;
       const int64_t nb = (k + bw - 1) / bw;
       return wide > 0 && nb >= wide ? 2 : nb >= svd_cluster_size() ? 1 : 0;
     };
     std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) {
+      if (old(a) != old(b)) return old(a);
+      if (!old(a)) return jobs[a].k > jobs[b].k;
       const int ca = clustered(a), cb = clustered(b);
       if (ca != cb) return ca > cb;
       return cost(a) > cost(b);
     });
+    n_old = 0;
     n_cluster = 0;
     n_wide = 0;
     for (size_t i = 0; i < order.size(); ++i) {
+      n_old += old(order[i]) ? 1 : 0;
       n_cluster += clustered(order[i]) > 0 ? 1 : 0;
       n_wide += clustered(order[i]) == 2 ? 1 : 0;
+    }
+    // One run per cluster width of the Jacobi kernel, each its own launch; a
+    // narrower run joins the one before it while all clusters of the joint
+    // launch fit the GPU's SMs at once (apart they would run one after the other).
+    runs.clear();
+    for (size_t i = (size_t)n_old; i < order.size(); ++i) {
+      const SvdJob& J = jobs[order[i]];
+      const int cl = jacobi_cluster(J.k);
+      if (runs.empty() || jacobi_cluster(runs.back().max_k) != cl) {
+        FacRun r;
+        r.first = (int32_t)i;
+        r.max_k = J.k;
+        runs.push_back(r);
+      }
+      FacRun& r = runs.back();
+      r.count += 1;
+      r.max_rows = std::max({r.max_rows, J.m, J.n});
+      r.max_cols = std::max(r.max_cols, J.n);
+      r.rectangular |= J.m != J.n;
+    }
+    for (size_t i = runs.size(); i-- > 1;) {
+      FacRun &x = runs[i - 1], &y = runs[i];
+      if ((int64_t)(x.count + y.count) * jacobi_cluster(x.max_k) > 128) continue;
+      x.count += y.count;
+      x.max_rows = std::max(x.max_rows, y.max_rows);
+      x.max_cols = std::max(x.max_cols, y.max_cols);
+      x.rectangular |= y.rectangular;
+      runs.erase(runs.begin() + (long)i);
     }
     std::vector<SvdJob> sj(jobs.size());
     std::vector<int64_t> sw(jobs.size());
@@ -930,8 +974,7 @@ tnt_status tnt_factor_plan(const tnt_space* src, tnt_fplan** out) {
     int64_t off = 0;
     for (auto& j : f->p->tables.jobs) {
       f->work_off.push_back(off);
-      int64_t rows = std::max(j.m, j.n);
-      off += rows * j.k + j.k * j.k + 2 * j.k;
+      off += fac_work_elems(std::max(j.m, j.n), j.k);
     }
     f->work_elems = off;
     *out = f;
@@ -1550,6 +1593,39 @@ tnt_status tnt_compose_host(tnt_ctx* ctx, const tnt_cplan* cplan, int64_t nbatch
   return st_code;
 }
 
+}  // extern "C"
+
+namespace {
+
+// The batched SVD of a plan: sectors beyond kQrMaxRows on the general Jacobi
+// kernels; the others reduced to R^T (rectangular ones made square first), swept by
+// the cluster Jacobi engine, their factors taken back through the reflectors.
+cudaError_t svd_launches(tnt_fplan_s* plan, std::pair<SvdJob*, int64_t*> dev, const double* a, double* u, double* s,
+                         double* vh, double* work, int32_t* status, cudaStream_t st) {
+  cudaError_t e = cudaSuccess;
+  if (plan->n_old > 0)
+    e = launch_svd_split(dev.first, plan->n_cluster, plan->n_old, a, u, s, vh, work, dev.second, status, st,
+                         plan->n_wide);
+  for (const FacRun& r : plan->runs) {
+    const SvdJob* j = dev.first + r.first;
+    const int64_t* off = dev.second + r.first;
+    auto then = [&](cudaError_t x) { e = e == cudaSuccess ? x : e; };
+    if (e == cudaSuccess && r.rectangular)
+      then(launch_qr_factor(j, r.count, r.max_rows, r.max_k, kQrSvdFirst, a, u, vh, work, off, st));
+    if (e == cudaSuccess) then(launch_qr_factor(j, r.count, r.max_k, r.max_k, kQrSvdSecond, a, u, vh, work, off, st));
+    if (e == cudaSuccess) then(launch_jacobi(j, r.count, r.max_k, work, off, status, true, st));
+    if (e == cudaSuccess) then(launch_qr_apply(j, r.count, r.max_k, r.max_k, kQrSvdSecond, u, vh, work, off, st));
+    if (e == cudaSuccess && r.rectangular)
+      then(launch_qr_apply(j, r.count, r.max_rows, r.max_k, kQrSvdFirst, u, vh, work, off, st));
+    if (e == cudaSuccess) then(launch_svd_finish(j, r.count, r.max_k, u, s, vh, work, off, st));
+  }
+  return e;
+}
+
+}  // namespace
+
+extern "C" {
+
 tnt_status tnt_svd(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, double* u, double* s, double* vh,
                    void* stream) {
   return guarded([&] {
@@ -1570,8 +1646,7 @@ tnt_status tnt_svd(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, double
     }
     cudaStream_t st = (cudaStream_t)stream;
     cuda_check(cudaMemsetAsync(ctx->status, 0, 2 * sizeof(int32_t), st), "memset status");
-    cuda_check(launch_svd_split(dev.first, plan->n_cluster, (int32_t)t.jobs.size(), a, u, s, vh, ctx->svd_work,
-                                dev.second, ctx->status, st, plan->n_wide),
+    cuda_check(svd_launches(plan, dev, a, u, s, vh, ctx->svd_work, ctx->status, st),
                "svd kernel launch");
     int32_t hs[2] = {0, 0};
     cuda_check(cudaMemcpyAsync(hs, ctx->status, sizeof(hs), cudaMemcpyDeviceToHost, st), "read svd status");
@@ -1593,8 +1668,7 @@ tnt_status tnt_svd_ws_async(tnt_ctx* ctx, const tnt_fplan* fplan, const double* 
     auto dev = plan->lpt_on_device();
     cudaStream_t st = (cudaStream_t)stream;
     cuda_check(cudaMemsetAsync(status, 0, 2 * sizeof(int32_t), st), "memset status");
-    cuda_check(launch_svd_split(dev.first, plan->n_cluster, (int32_t)t.jobs.size(), a, u, s, vh, work, dev.second,
-                                status, st, plan->n_wide),
+    cuda_check(svd_launches(plan, dev, a, u, s, vh, work, status, st),
                "svd kernel launch");
   });
 }
@@ -1619,8 +1693,7 @@ tnt_status tnt_svd_ws(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, dou
     cudaStream_t st = (cudaStream_t)stream;
     std::lock_guard<std::recursive_mutex> g(ctx->mu);  // the status words are the context's
     cuda_check(cudaMemsetAsync(ctx->status, 0, 2 * sizeof(int32_t), st), "memset status");
-    cuda_check(launch_svd_split(dev.first, plan->n_cluster, (int32_t)t.jobs.size(), a, u, s, vh, work, dev.second,
-                                ctx->status, st, plan->n_wide),
+    cuda_check(svd_launches(plan, dev, a, u, s, vh, work, ctx->status, st),
                "svd kernel launch");
     int32_t hs[2] = {0, 0};
     cuda_check(cudaMemcpyAsync(hs, ctx->status, sizeof(hs), cudaMemcpyDeviceToHost, st), "read svd status");
@@ -1657,7 +1730,15 @@ tnt_status tnt_qr(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, double*
     std::lock_guard<std::recursive_mutex> g(ctx->mu);
     double* work = factor_work(ctx, plan);
     cudaStream_t st = (cudaStream_t)stream;
-    cuda_check(launch_qr(dev.first, (int32_t)t.jobs.size(), a, q, r, work, dev.second, st), "qr kernel launch");
+    cuda_check(launch_qr(dev.first, plan->n_old, a, q, r, work, dev.second, st), "qr kernel launch");
+    for (const FacRun& x : plan->runs) {
+      const SvdJob* j = dev.first + x.first;
+      const int64_t* off = dev.second + x.first;
+      cuda_check(launch_qr_factor(j, x.count, x.max_rows, x.max_cols, kQrFactor, a, q, r, work, off, st),
+                 "cluster qr launch");
+      cuda_check(launch_qr_apply(j, x.count, x.max_rows, x.max_k, kQrFactor, q, r, work, off, st),
+                 "qr accumulation launch");
+    }
     cuda_check(cudaStreamSynchronize(st), "stream synchronize");
   });
 }
@@ -1679,9 +1760,11 @@ tnt_status tnt_eigh(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, doubl
     cudaStream_t st = (cudaStream_t)stream;
     int64_t max_n = 0;
     for (const SvdJob& j : t.jobs) max_n = std::max<int64_t>(max_n, j.m);
-    if (!eigh_on_chip(max_n)) {
-      // Sectors beyond the on-chip two-sided Jacobi go through the batched
-      // SVD of the shifted, positive semidefinite A + ||A||_F I.
+    cuda_check(cudaMemsetAsync(ctx->status, 0, 2 * sizeof(int32_t), st), "memset status");
+    int32_t hs[2] = {0, 0};
+    if (plan->n_old > 0) {
+      // Sectors beyond the cluster engine go through the general SVD of the
+      // shifted, positive semidefinite A + ||A||_F I.
       const size_t njobs = t.jobs.size();
       const size_t elems = (size_t)(t.a_size + t.u_size + t.s_size + t.v_size) + njobs + 1;
       if (ctx->eigh_tmp_elems < elems) {
@@ -1697,27 +1780,23 @@ tnt_status tnt_eigh(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, doubl
       double* vh = sv + t.s_size;
       double* shift = vh + t.v_size;
       int32_t* bad = reinterpret_cast<int32_t*>(shift + njobs);
-      cuda_check(cudaMemsetAsync(ctx->status, 0, 2 * sizeof(int32_t), st), "memset status");
       cuda_check(cudaMemsetAsync(bad, 0, sizeof(int32_t), st), "memset eigh flag");
-      cuda_check(launch_eigh_by_svd(dev.first, plan->n_cluster, (int32_t)njobs, max_n, a, b, u, sv, vh, shift, bad,
-                                    vecs, vals, mags, work, dev.second, ctx->status, st, plan->n_wide),
+      cuda_check(launch_eigh_by_svd(dev.first, plan->n_cluster, plan->n_old, max_n, a, b, u, sv, vh, shift, bad, vecs,
+                                    vals, mags, work, dev.second, ctx->status, st, plan->n_wide),
                  "eigh (shifted SVD) launch");
-      int32_t hs[2] = {0, 0};
-      cuda_check(cudaMemcpyAsync(&hs[0], ctx->status, sizeof(int32_t), cudaMemcpyDeviceToHost, st), "read svd status");
       cuda_check(cudaMemcpyAsync(&hs[1], bad, sizeof(int32_t), cudaMemcpyDeviceToHost, st), "read eigh flag");
-      cuda_check(cudaStreamSynchronize(st), "stream synchronize");
-      if (hs[1] != 0) throw std::invalid_argument("eigh requires Hermitian coupled-sector blocks");
-      if (hs[0] != 0) throw Failure(TNT_INTERNAL, "Jacobi SVD did not converge within the sweep limit");
-      return;
     }
-    cuda_check(cudaMemsetAsync(ctx->status, 0, sizeof(int32_t), st), "memset status");
-    cuda_check(launch_eigh(dev.first, (int32_t)t.jobs.size(), a, vecs, vals, mags, work, dev.second, ctx->status, st),
-               "eigh kernel launch");
-    int32_t hs = 0;
-    cuda_check(cudaMemcpyAsync(&hs, ctx->status, sizeof(int32_t), cudaMemcpyDeviceToHost, st), "read eigh status");
+    for (const FacRun& r : plan->runs) {
+      const SvdJob* j = dev.first + r.first;
+      const int64_t* off = dev.second + r.first;
+      cuda_check(launch_eigh_prepare(j, r.count, r.max_k, a, work, off, ctx->status, st), "eigh preparation launch");
+      cuda_check(launch_jacobi(j, r.count, r.max_k, work, off, ctx->status, false, st), "eigh sweeps launch");
+      cuda_check(launch_eigh_finish(j, r.count, r.max_k, a, vecs, vals, mags, work, off, st), "eigh output launch");
+    }
+    cuda_check(cudaMemcpyAsync(&hs[0], ctx->status, sizeof(int32_t), cudaMemcpyDeviceToHost, st), "read eigh status");
     cuda_check(cudaStreamSynchronize(st), "stream synchronize");
-    if (hs & 2) throw std::invalid_argument("eigh requires Hermitian coupled-sector blocks");
-    if (hs != 0) throw Failure(TNT_INTERNAL, "Jacobi eigensolver did not converge within the sweep limit");
+    if (hs[1] != 0 || (hs[0] & 2)) throw std::invalid_argument("eigh requires Hermitian coupled-sector blocks");
+    if (hs[0] != 0) throw Failure(TNT_INTERNAL, "Jacobi eigensolver did not converge within the sweep limit");
   });
 }
 
@@ -1897,7 +1976,7 @@ tnt_status tnt_fplan_concat(int32_t n, const tnt_fplan* const* plans, const int6
       int64_t off = 0;
       for (auto& j : T.jobs) {
         f->work_off.push_back(off);
-        off += std::max(j.m, j.n) * j.k + j.k * j.k + 2 * j.k;
+        off += fac_work_elems(std::max(j.m, j.n), j.k);
       }
       f->work_elems = off;
     }

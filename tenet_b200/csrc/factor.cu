@@ -1,4 +1,5 @@
-// Batched per-sector QR and Hermitian eigendecomposition on the device.
+// QR and Hermitian eigendecomposition of sectors beyond the cluster kernels
+// (qr.cu and jacobi.cu take every sector of at most 1408 rows).
 //
 // Replace the serial sector loops of qr_compact (tenet-matrixalgebra/src/
 // factorize.rs:5158, positive_diagonal_gauge :3789-3830) and eigh_full_dyn
@@ -6,9 +7,8 @@
 // eigenvector_gauge :3902-3913 makes each vector's largest-|.| entry
 // positive), which call a dense factorisation per coupled sector.
 //
-// Both kernels run one CTA per coupled-sector matrix and share the SVD's
-// per-sector scratch layout (rows*k + k*k + 2k doubles), keeping the working
-// panel in shared memory when it fits.
+// One CTA per coupled-sector matrix, in the per-sector scratch of panel.cuh,
+// keeping the working panel in shared memory when it fits.
 //
 // QR: Householder reflections H_j = I - tau_j v_j v_j^T (v_j(j) = 1) reduce
 // the m x n panel to R in place, one warp per trailing column; Q (m x k,
@@ -17,14 +17,8 @@
 // negates column j of Q and row j of R when R_jj < 0 (zero keeps sign +1), so
 // Q R is unchanged and the factorisation of a full-rank block is unique.
 //
-// eigh: cyclic two-sided Jacobi with a round-robin tournament of disjoint
-// (p, q) pairs: per round every pair's rotation is computed from the current
-// 2x2 principal block, then all column rotations A <- A J, V <- V J and all
-// row rotations A <- J^T A are applied in parallel (one warp per pair).  A
-// pair is skipped once |a_pq| is below 4 sqrt(n) eps sqrt(|a_pp a_qq|) or the
-// rounding level eps ||A||_F.  Plans with a sector too large for shared
-// memory run the whole eigendecomposition through the batched SVD instead
-// (eigh_shift_kernel, eigh_from_svd_kernel below).
+// eigh: the general SVD of the shifted sector (eigh_shift_kernel,
+// eigh_from_svd_kernel below).
 #include <cfloat>
 
 #include "kernels.cuh"
@@ -35,7 +29,6 @@ namespace {
 
 constexpr int kFacThreads = 512;
 constexpr size_t kFacSmemBytes = 200 * 1024;
-constexpr int kEighSweeps = 40;
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -56,42 +49,6 @@ __device__ double block_sum(double v, double* red) {
   }
   __syncthreads();
   return red[32];
-}
-
-__device__ __forceinline__ void tournament_pair(int r, int i, int k2, int& p, int& q) {
-  int a, b;
-  if (i == 0) {
-    a = k2 - 1;
-    b = r;
-  } else {
-    a = (r + i) % (k2 - 1);
-    b = (r - i + (k2 - 1)) % (k2 - 1);
-  }
-  p = a < b ? a : b;
-  q = a < b ? b : a;
-}
-
-// Index of the first largest-|.| entry of x[0..len) across one warp.
-__device__ __forceinline__ int64_t warp_argmax_abs(const double* x, int64_t len, int lane) {
-  double best = -1.0;
-  int64_t bidx = 0;
-  for (int64_t i = lane; i < len; i += 32) {
-    const double v = fabs(x[i]);
-    if (v > best) {
-      best = v;
-      bidx = i;
-    }
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    const double ob = __shfl_xor_sync(0xffffffffu, best, off);
-    const int64_t oi = __shfl_xor_sync(0xffffffffu, bidx, off);
-    if (ob > best || (ob == best && oi < bidx)) {
-      best = ob;
-      bidx = oi;
-    }
-  }
-  return bidx;
 }
 
 // ---------------------------------------------------------------------------
@@ -320,174 +277,18 @@ __global__ void __launch_bounds__(kFacThreads) qr_kernel(const SvdJob* __restric
 }
 
 // ---------------------------------------------------------------------------
-// Hermitian (real symmetric) eigendecomposition
-// ---------------------------------------------------------------------------
-
-__global__ void __launch_bounds__(kFacThreads) eigh_kernel(const SvdJob* __restrict__ jobs,
-                                                           const double* __restrict__ A, double* __restrict__ VEC,
-                                                           double* __restrict__ VAL, double* __restrict__ MAG,
-                                                           double* __restrict__ work,
-                                                           const int64_t* __restrict__ work_off,
-                                                           int32_t* __restrict__ status) {
-  const SvdJob J = jobs[blockIdx.x];
-  const int64_t n = J.m;
-  if (n == 0) return;
-  extern __shared__ double smem_fac[];
-  const bool on_chip = (size_t)(2 * n * n + 2 * n) * sizeof(double) <= kFacSmemBytes;
-  double* W = on_chip ? smem_fac : work + work_off[blockIdx.x];  // n x n, column-major
-  double* V = W + n * n;
-  double* lam = V + n * n;
-  double* rk = lam + n;
-  __shared__ double red[33];
-  __shared__ int rotated;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-  // Rotation (c, s) of every pair of the current round.
-  __shared__ double rc[kFacThreads / 32 * 8], rs[kFacThreads / 32 * 8];
-  __shared__ int rp[kFacThreads / 32 * 8], rq[kFacThreads / 32 * 8];
-  const double* a = A + J.a_off;
-  double f2 = 0.0, d2 = 0.0;
-  int finite = 1;
-  for (int64_t i = tid; i < n * n; i += blockDim.x) {
-    const double v = a[i];
-    const int64_t r = i % n, c = i / n;
-    const double d = v - a[c + r * n];
-    W[i] = v;
-    V[i] = r == c ? 1.0 : 0.0;
-    f2 = fma(v, v, f2);
-    d2 = fma(d, d, d2);
-    finite &= isfinite(v) ? 1 : 0;
-  }
-  const double frob = sqrt(block_sum(f2, red));
-  const double asym = sqrt(block_sum(d2, red));
-  const int all_finite = __syncthreads_and(finite);
-  // Hermiticity check of the reference (normwise_hermitian, factorize.rs:5999-6021):
-  // ||A - A^T||_F <= 2 * 64 eps ||A||_F, every entry finite.
-  if (!all_finite || asym > 128.0 * DBL_EPSILON * frob) {
-    if (tid == 0) atomicExch(status, 2);
-    return;
-  }
-  // Off-diagonal entries at the rounding level eps ||A||_F are noise that
-  // every rotation regenerates; rotating them again never settles.
-  const double abs_floor = DBL_EPSILON * frob;
-  const double tol = 4.0 * sqrt((double)n) * DBL_EPSILON;  // rounding level of a length-n rotation
-
-  const int k2 = (int)((n + 1) & ~1LL);
-  const int npairs = k2 / 2;
-  int sweep = 0;
-  for (; sweep < kEighSweeps && n > 1; ++sweep) {
-    if (tid == 0) rotated = 0;
-    __syncthreads();
-    for (int r = 0; r < k2 - 1; ++r) {
-      // Pairs are processed in batches of (warps * 8) so the rotation table stays in shared memory.
-      for (int base = 0; base < npairs; base += nwarps * 8) {
-        const int batch = min(npairs - base, nwarps * 8);
-        for (int b = tid; b < batch; b += blockDim.x) {
-          int p, q;
-          tournament_pair(r, base + b, k2, p, q);
-          double c = 1.0, s = 0.0;
-          if (q < n) {
-            const double apq = W[p + (int64_t)q * n];
-            const double app = W[p + (int64_t)p * n], aqq = W[q + (int64_t)q * n];
-            if (fabs(apq) > tol * sqrt(fabs(app * aqq)) && fabs(apq) > abs_floor && fabs(apq) > DBL_MIN) {
-              const double zeta = (aqq - app) / (2.0 * apq);
-              const double t = (zeta >= 0.0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-              c = 1.0 / sqrt(1.0 + t * t);
-              s = c * t;
-              rotated = 1;
-            }
-          }
-          rc[b] = c;
-          rs[b] = s;
-          rp[b] = p;
-          rq[b] = q;
-        }
-        __syncthreads();
-        // Columns: A <- A J, V <- V J.
-        for (int b = warp; b < batch; b += nwarps) {
-          const double c = rc[b], s = rs[b];
-          if (s == 0.0) continue;
-          int p, q;
-          tournament_pair(r, base + b, k2, p, q);
-          double* wp = W + (int64_t)p * n;
-          double* wq = W + (int64_t)q * n;
-          double* vp = V + (int64_t)p * n;
-          double* vq = V + (int64_t)q * n;
-          for (int64_t x = lane; x < n; x += 32) {
-            const double u = wp[x], v = wq[x];
-            wp[x] = c * u - s * v;
-            wq[x] = s * u + c * v;
-            const double g = vp[x], h = vq[x];
-            vp[x] = c * g - s * h;
-            vq[x] = s * g + c * h;
-          }
-        }
-        __syncthreads();
-        // Rows: A <- J^T A, one warp per column (lanes over the pairs), so a
-        // warp's accesses stay inside one contiguous column instead of
-        // striding by n down a row.  Every element is updated once per batch
-        // with the same arithmetic as a row-by-row pass.
-        for (int64_t x = warp; x < n; x += nwarps) {
-          double* col = W + x * n;
-          for (int b = lane; b < batch; b += 32) {
-            const double c = rc[b], s = rs[b];
-            if (s == 0.0) continue;
-            const int p = rp[b], q = rq[b];
-            const double u = col[p], v = col[q];
-            col[p] = c * u - s * v;
-            col[q] = s * u + c * v;
-          }
-        }
-        __syncthreads();
-      }
-    }
-    const int done = rotated == 0;
-    __syncthreads();
-    if (done) break;
-  }
-  if (tid == 0 && sweep == kEighSweeps) atomicExch(status, 1);
-
-  for (int64_t i = tid; i < n; i += blockDim.x) lam[i] = W[i + i * n];
-  __syncthreads();
-  // Order: descending |lambda|; ties keep LAPACK's ascending-value order, then index.
-  for (int64_t i = tid; i < n; i += blockDim.x) {
-    const double li = lam[i], ai = fabs(li);
-    int64_t pos = 0;
-    for (int64_t o = 0; o < n; ++o) {
-      const double lo = lam[o], ao = fabs(lo);
-      pos += (ao > ai || (ao == ai && (lo < li || (lo == li && o < i)))) ? 1 : 0;
-    }
-    rk[i] = (double)pos;
-  }
-  __syncthreads();
-  double* vec = VEC + J.u_off;
-  double* val = VAL + J.s_off;
-  for (int64_t c = warp; c < n; c += nwarps) {
-    const int64_t pos = (int64_t)rk[c];
-    const double* vc = V + c * n;
-    const int64_t b = warp_argmax_abs(vc, n, lane);
-    const double sgn = vc[b] < 0.0 ? -1.0 : 1.0;
-    for (int64_t x = lane; x < n; x += 32) vec[x + pos * n] = sgn * vc[x];
-    if (lane == 0) {
-      val[pos] = lam[c];
-      if (MAG) MAG[J.s_off + pos] = fabs(lam[c]);
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
 // Eigendecomposition of large sectors through the batched SVD
 // ---------------------------------------------------------------------------
 //
-// A sector too large for the on-chip two-sided Jacobi is shifted to
+// The sector is shifted to
 // B = A + c I with c = ||A||_F, at least the spectral radius, so B is
 // positive semidefinite: its singular values are lambda + c and its right
 // singular vectors are eigenvectors of A (for a repeated singular value they
 // span the eigenspace).  The batched SVD, with thread-block clusters for the
 // largest sectors, does the work; eigh_from_svd_kernel maps sigma back to
 // lambda = sigma - c, orders by descending |lambda| (ties: ascending value,
-// then index) and applies the largest-entry gauge, as eigh_kernel does.
-// Eigenvalue error: about eps (||A||_2 + c) absolute, against eps ||A||_2 for
-// the two-sided Jacobi.
+// then index) and applies the largest-entry gauge.  Eigenvalue error: about
+// eps (||A||_2 + c) absolute.
 
 __global__ void __launch_bounds__(kFacThreads) eigh_shift_kernel(const SvdJob* __restrict__ jobs,
                                                                  const double* __restrict__ A, double* __restrict__ B,
@@ -515,7 +316,7 @@ __global__ void __launch_bounds__(kFacThreads) eigh_shift_kernel(const SvdJob* _
   const double frob = sqrt(block_sum(f2, red));
   const double asym = sqrt(block_sum(d2, red));
   const int all_finite = __syncthreads_and(finite);
-  // The Hermiticity check of eigh_kernel (normwise_hermitian, factorize.rs:5999-6021).
+  // The Hermiticity check of the reference (normwise_hermitian, factorize.rs:5999-6021).
   if ((!all_finite || asym > 128.0 * DBL_EPSILON * frob) && tid == 0) atomicExch(bad, 1);
   const double c = all_finite ? frob : 0.0;
   if (tid == 0) shift[blockIdx.x] = c;
@@ -590,17 +391,6 @@ cudaError_t launch_qr(const SvdJob* jobs, int32_t njobs, const double* a, double
   qr_kernel<<<njobs, kFacThreads, kFacSmemBytes, stream>>>(jobs, a, q, r, work, work_off);
   return cudaGetLastError();
 }
-
-cudaError_t launch_eigh(const SvdJob* jobs, int32_t njobs, const double* a, double* vecs, double* vals, double* mags,
-                        double* work, const int64_t* work_off, int32_t* status, cudaStream_t stream) {
-  if (njobs == 0) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(eigh_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFacSmemBytes);
-  if (e != cudaSuccess) return e;
-  eigh_kernel<<<njobs, kFacThreads, kFacSmemBytes, stream>>>(jobs, a, vecs, vals, mags, work, work_off, status);
-  return cudaGetLastError();
-}
-
-bool eigh_on_chip(int64_t n) { return (size_t)(2 * n * n + 2 * n) * sizeof(double) <= kFacSmemBytes; }
 
 cudaError_t launch_eigh_by_svd(const SvdJob* jobs, int32_t n_cluster, int32_t njobs, int64_t max_n, const double* a,
                                double* b, double* u, double* s, double* vh, double* shift, int32_t* bad,

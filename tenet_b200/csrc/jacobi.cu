@@ -1,0 +1,882 @@
+// One-sided Jacobi on a thread-block cluster per sector: the engine of the
+// batched SVD and of the symmetric eigendecomposition.
+//
+// In: W (k x k, leading dimension ldw) in the sector's scratch, for the SVD the
+// transposed R factor of the sector (qr.cu), for eigh the shifted matrix.  Out:
+// W J = columns orthogonal to 4 sqrt(k) eps, J (SVD only) in the scratch, column
+// norms in sv.
+//
+// Columns are split into nb blocks (nb even, w columns each); a sweep is a
+// round-robin tournament of the blocks, one pair per CTA and round, with the
+// pairs inside each block rotated in the first round.  What bounds a round is
+// the latency of the rotation chain (dot product, reduction, angle, update) and,
+// for the largest sectors, the FP64 units, so:
+//  * the w columns of one block stay in registers (G lanes per column) while the
+//    other block's columns pass by in shared memory: per rotation one column is
+//    read and written there instead of two read twice and written once;
+//  * short columns take few lanes each (G = 8 up to k = 64, 16 up to 128), so the
+//    reduction and the angle are shared by several pairs of a warp;
+//  * squared norms are formed when a block is loaded and updated per rotation,
+//    so a pair needs one dot product;
+//  * tests and the tangent run in single precision (its error only leaves 1e-6 of
+//    the pair's cosine behind), the cosine and sine come from one third-order
+//    step in FP64, so c^2 + s^2 = 1 to FP64 rounding;
+//  * rotations accumulate in 2w x 2w matrices kept below the staged columns, and
+//    J's columns are multiplied by them once per block pair on the FP64 tensor
+//    cores (m8n8k4);
+//  * the sweep that only confirms convergence is left out when the sweep
+//    before it cannot have left a cosine above the tolerance (below).
+// Measured on a B200 against the general kernels of svd.cu and a two-sided
+// Jacobi in shared memory: truncated SVD of the D = 2048 chain (six sectors of
+// 586, two of 293) 94.9 -> 22.4 ms, a whole two-site update at D = 224 (104 x 104)
+// 5.4 -> 1.65 ms, eigh at D = 224 6.4 -> 1.3 ms with eigenvalues to 4e-16 (1.4e-14).
+#include <algorithm>
+
+#include "panel.cuh"
+
+namespace tnt {
+
+namespace {
+
+using namespace panel;
+
+constexpr int kMaxSweeps = 40;
+constexpr size_t kJacobiSmem = 216 * 1024;
+
+// Stride of a staged column: k rounded up to 32, the zr rows of its accumulator,
+// and a pad that keeps the accesses conflict-free (8-lane columns side by side:
+// 8 mod 16; MMA fragments of the accumulator: 4 mod 16).
+__host__ __device__ __forceinline__ int col_stride(int k, int zr, int g) {
+  return (k + 31) / 32 * 32 + zr + (g == 8 ? 8 : 4);
+}
+
+// Block width and (even) block count for k columns on cl CTAs of `owners` column
+// owners each.
+__host__ __device__ __forceinline__ void block_split(int k, int cl, int owners, int zr, int g, int& w, int& nb) {
+  int cap = (int)(kJacobiSmem / 8 / (2 * col_stride(k, zr, g)));
+  if (cap > owners) cap = owners;
+  if (cap > zr / 2) cap = zr / 2;
+  int per = 1;  // block pairs per CTA and round
+  while ((k + 2 * cl * per - 1) / (2 * cl * per) > cap) ++per;
+  w = (k + 2 * cl * per - 1) / (2 * cl * per);
+  nb = (k + w - 1) / w;
+  nb = nb < 2 ? 2 : (nb + 1) & ~1;
+}
+
+struct Thresholds {
+  float tol, noise2, floor;
+};
+
+struct Rotation {
+  double c, s, tg;  // cosine, sine, tangent * gamma (the norms' change)
+};
+
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// The rotation that makes the pair orthogonal (squared norms al, be, dot ga);
+// false when the pair counts as orthogonal already.  The sector is scaled to a
+// largest entry below 1, so every float here is in range: squared norms lie
+// between noise2 (about 1e-30) and k^2, |ga| above floor (about 1e-33).
+__device__ __forceinline__ bool rotation(double al, double be, double ga, const Thresholds& th, Rotation& R,
+                                         float& cosmax, float& fillmax) {
+  const float gf = (float)ga, af = (float)al, bf = (float)be;
+  const float rr = rsqrt_approx(af) * rsqrt_approx(bf), cosine = fabsf(gf) * rr;
+  if (!(cosine > th.tol && fminf(af, bf) > th.noise2 && fabsf(gf) > th.floor)) return false;
+  const float z = 0.5f * (float)(be - al) * rcp_approx(gf), az = fabsf(z);
+  float t = rcp_approx(az < 1e4f ? az + sqrt_approx(fmaf(z, z, 1.0f)) : az + az);
+  t = z < 0.0f ? -t : t;
+  const double td = (double)t, y = (double)rsqrt_approx(fmaf(t, t, 1.0f)), x = fma(td, td, 1.0);
+  const double e = fma(-x * y, y, 1.0);  // y (1 + e/2 + 3 e^2 / 8) = x^{-1/2} up to e^3
+  R.c = fma(y * e, fma(0.375, e, 0.5), y);
+  R.s = R.c * td;
+  R.tg = td * ga;
+  // Cosine of the pair, and the most this rotation can put back between one of
+  // its columns and a third per unit of the other's cosine with it.
+  cosmax = fmaxf(cosmax, cosine);
+  fillmax = fmaxf(fillmax, fabsf(t) * rr * fmaxf(af, bf));
+  return true;
+}
+
+// Sum over the G lanes of a column.
+template <int G>
+__device__ __forceinline__ double group_sum(double v) {
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Both columns in shared memory (pairs inside a block); every lane of the warp calls it.
+template <int G, int ZR>
+__device__ __forceinline__ void rotate_smem(bool live, double* p, double* q, double* np, double* nq, int pw, bool acc_j,
+                                            const Thresholds& th, float& cosmax, float& fillmax) {
+  const int gl = threadIdx.x % G;
+  double ga = 0.0, al = 0.0, be = 0.0;
+  if (live) {
+    al = *np;
+    be = *nq;
+    for (int j = 0; j < pw; ++j) ga = fma(p[gl + G * j], q[gl + G * j], ga);
+  }
+  ga = group_sum<G>(ga);
+  Rotation R;
+  if (live && rotation(al, be, ga, th, R, cosmax, fillmax)) {
+    const int n = acc_j ? pw + ZR / G : pw;
+    for (int j = 0; j < n; ++j) {
+      const double u = p[gl + G * j], v = q[gl + G * j];
+      p[gl + G * j] = R.c * u - R.s * v;
+      q[gl + G * j] = R.s * u + R.c * v;
+    }
+    if (gl == 0) {
+      *np = al - R.tg;
+      *nq = be + R.tg;
+    }
+  }
+  __syncwarp();
+}
+
+// Columns of blocks bi and bj of J times the accumulated rotations: J[:, cols] <-
+// J[:, cols] Z, rows split over the warps in strips of 8 (a strip is read whole
+// before it is written).  Z's column c starts at zs + c * ls, c < w for block bi's
+// columns and w + (index) for block bj's.
+template <int ZR>
+__device__ __forceinline__ void apply_z(double* J, int k, int w, int p0, int np, int q0, int nq, const double* zs,
+                                        int ls) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int g = lane >> 2, t4 = lane & 3;
+  const int kt = (2 * w + 3) / 4, nt = (2 * w + 7) / 8;
+  for (int x0 = warp * 8; x0 < k; x0 += nwarps * 8) {
+    const bool row = x0 + g < k;
+    double a[ZR / 4];
+#pragma unroll
+    for (int i = 0; i < ZR / 4; ++i) {
+      const int z = 4 * i + t4;
+      const bool in = z < w ? z < np : z - w < nq;
+      a[i] = (i < kt && row && in) ? __ldcg(J + (int64_t)(z < w ? p0 + z : q0 + z - w) * k + x0 + g) : 0.0;
+    }
+    for (int n = 0; n < nt; ++n) {
+      double d0 = 0.0, d1 = 0.0;
+      const double* zc = zs + (int64_t)(8 * n + g) * ls;
+      const bool col = 8 * n + g < 2 * w;
+#pragma unroll
+      for (int i = 0; i < ZR / 4; ++i)
+        if (i < kt) dmma(d0, d1, a[i], col ? zc[4 * i + t4] : 0.0);
+      const int c = 8 * n + 2 * t4;  // output columns c, c + 1 of row g
+      if (row) {
+        if (c < w ? c < np : c - w < nq) J[(int64_t)(c < w ? p0 + c : q0 + c - w) * k + x0 + g] = d0;
+        const int c1 = c + 1;
+        if (c1 < w ? c1 < np : c1 - w < nq) J[(int64_t)(c1 < w ? p0 + c1 : q0 + c1 - w) * k + x0 + g] = d1;
+      }
+    }
+  }
+}
+
+// G lanes per column, at most PW elements of W and ZR / G of the accumulator each;
+// NW warps own 32 / G columns each; HOLD: the passing column stays in registers
+// between its dot product and its update.
+template <int G, int PW, int ZR, int NW, bool HOLD>
+__global__ void __launch_bounds__(NW * 32, 1)
+    jacobi_kernel(const SvdJob* __restrict__ jobs, double* __restrict__ work, const int64_t* __restrict__ work_off,
+                  int32_t* __restrict__ status, int cl, int acc) {
+  constexpr int PP = 32 / G, PZ = ZR / G;
+  const int rank = (int)(blockIdx.x % cl);
+  const SvdJob S = jobs[blockIdx.x / cl];
+  const int k = (int)S.k;
+  const int64_t ldw = S.m > S.n ? S.m : S.n;
+  if (k == 0) return;
+  const bool acc_j = acc != 0;
+  const FacWork f = fac_work(work + work_off[blockIdx.x / cl], ldw, k);
+  double* W = f.W;
+  double* J = f.J;
+  int* words = reinterpret_cast<int*>(f.meta + 4);  // per sweep parity: cosine, fill (float bits)
+  extern __shared__ __align__(16) double sm[];
+  __shared__ double nrm[ZR];
+  __shared__ double part[32];
+  __shared__ int s_cos, s_fill;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int gl = lane % G, owner = warp * PP + lane / G;
+  int w, nb;
+  block_split(k, cl, NW * PP, ZR, G, w, nb);
+  const int kp = (k + 31) / 32 * 32, pw = kp / G, ls = col_stride(k, ZR, G);
+  const bool resident = cl == 1 && nb == 2;  // every column stays in shared memory for all sweeps
+  auto bsize = [&](int b) {
+    const int n = k - b * w;
+    return n < 0 ? 0 : n < w ? n : w;
+  };
+
+  // ||W||_F^2 (the same sum in the same order in every CTA) for the thresholds,
+  // J = I, cleared reduction words.
+  for (int c = rank * NW + warp; c < k; c += cl * NW) {
+    double s = 0.0;
+    for (int x = lane; x < k; x += 32) {
+      const double v = __ldcg(W + (int64_t)c * ldw + x);
+      s = fma(v, v, s);
+      if (acc_j && !resident) J[(int64_t)c * k + x] = x == c ? 1.0 : 0.0;
+    }
+    s = warp_sum(s);
+    if (lane == 0) f.sv[c] = s;
+  }
+  if (rank == 0 && tid < 4) words[tid] = 0;
+  cluster_barrier(cl);
+  double fs = 0.0;
+  for (int c = tid; c < k; c += NW * 32) fs += __ldcg(f.sv + c);
+  fs = warp_sum(fs);
+  if (lane == 0) part[warp] = fs;
+  __syncthreads();
+  double frob2 = 0.0;
+  for (int i = 0; i < NW; ++i) frob2 += part[i];
+  // A pair is rotated only while its cosine exceeds the rounding level of a
+  // length-k dot product and both columns stand above the rounding noise
+  // k eps ||A||_F (columns of the null space shrink to that level, and every
+  // rotation refills them with noise whose cosine is O(1)).
+  const double tol = 4.0 * sqrt((double)k) * DBL_EPSILON;
+  Thresholds th;
+  th.tol = (float)tol;
+  th.noise2 = (float)(((double)k * DBL_EPSILON) * ((double)k * DBL_EPSILON) * frob2);
+  th.floor = (float)(1e-33 * frob2);  // below every gamma above the tolerance of two columns above the noise
+
+  int sweep = 0;
+  for (; sweep < kMaxSweeps && k > 1; ++sweep) {
+    float cosmax = 0.0f, fillmax = 0.0f;
+    if (tid == 0) {
+      s_cos = 0;
+      s_fill = 0;
+    }
+    for (int t = 0; t < nb - 1; ++t) {
+      for (int i = rank; i < nb / 2; i += cl) {
+        int bi, bj;
+        tournament_pair(t, i, nb, bi, bj);
+        const int np = bsize(bi), nq = bsize(bj), p0 = bi * w, q0 = bj * w;
+        const bool within = t == 0;
+        double* Q = sm + (int64_t)w * ls;  // block bj's columns; block bi's at sm while within its own pairs
+        // Stage: block bj (and bi in the first round) in shared memory, one warp per column.
+        if (!resident || sweep == 0) {
+          for (int c = within ? warp : w + warp; c < 2 * w; c += NW) {
+            if (c < w ? c >= np : c - w >= nq) continue;
+            const double* src = W + (int64_t)(c < w ? p0 + c : q0 + c - w) * ldw;
+            double* d = sm + (int64_t)c * ls;
+            for (int x = lane; x < kp; x += 32) d[x] = x < k ? __ldcg(src + x) : 0.0;
+            if (acc_j)
+              for (int z = lane; z < ZR; z += 32) d[kp + z] = z == c ? 1.0 : 0.0;
+          }
+          __syncwarp();
+        } else {
+          __syncthreads();  // the last sweep's columns, written by other warps
+        }
+        for (int c = within ? warp : w + warp; c < 2 * w; c += NW) {
+          if (c < w ? c >= np : c - w >= nq) continue;
+          const double* d = sm + (int64_t)c * ls;
+          double s = 0.0;
+          for (int x = lane; x < kp; x += 32) s = fma(d[x], d[x], s);
+          s = warp_sum(s);
+          if (lane == 0) nrm[c] = s;
+        }
+        if (within) {
+          __syncthreads();
+          const int n2 = (w + 1) & ~1, half = n2 / 2;
+          for (int r = 0; r < n2 - 1; ++r) {
+            for (int base = warp * PP; base < n2; base += NW * PP) {
+              const int e = base + lane / G, b = e >= half;
+              int p = 0, q = 0;
+              bool live = e < n2;
+              if (live) {
+                tournament_pair(r, b ? e - half : e, n2, p, q);
+                live = q < (b ? nq : np);
+                p += b ? w : 0;
+                q += b ? w : 0;
+              }
+              rotate_smem<G, ZR>(live, sm + (int64_t)p * ls, sm + (int64_t)q * ls, nrm + p, nrm + q, pw, acc_j, th,
+                                 cosmax, fillmax);
+            }
+            __syncthreads();
+          }
+        }
+        // Cross pairs: G lanes keep column `owner` of block bi in registers.
+        double p[PW], pz[PZ];
+        double al = 0.0;
+        const bool own = owner < np;
+        if (within) {
+          const double* d = sm + (int64_t)(own ? owner : 0) * ls + gl;
+#pragma unroll
+          for (int j = 0; j < PW; ++j) p[j] = (own && j < pw) ? d[G * j] : 0.0;
+#pragma unroll
+          for (int h = 0; h < PZ; ++h) pz[h] = (own && acc_j) ? d[kp + G * h] : 0.0;
+          al = own ? nrm[owner] : 0.0;
+        } else {
+          const double* d = W + (int64_t)(p0 + (own ? owner : 0)) * ldw;
+#pragma unroll
+          for (int j = 0; j < PW; ++j) {
+            p[j] = (own && gl + G * j < k) ? __ldcg(d + gl + G * j) : 0.0;
+            al = fma(p[j], p[j], al);
+          }
+          al = group_sum<G>(al);
+#pragma unroll
+          for (int h = 0; h < PZ; ++h) pz[h] = gl + G * h == owner ? 1.0 : 0.0;  // accumulator row of a block-bi column
+        }
+        __syncthreads();
+        for (int r = 0; r < w; ++r) {
+          int jq = owner + r;
+          if (jq >= w) jq -= w;
+          const bool live = own && jq < nq;
+          double* q = Q + (int64_t)(live ? jq : 0) * ls + gl;
+          double ga = 0.0, gb = 0.0;
+          double qv[HOLD ? PW : 1];
+#pragma unroll
+          for (int j = 0; j < PW; ++j) {
+            const double v = (j < pw && live) ? q[G * j] : 0.0;
+            if constexpr (HOLD) qv[j] = v;
+            if (j & 1) gb = fma(p[j], v, gb);
+            else ga = fma(p[j], v, ga);
+          }
+          const double be = live ? nrm[w + jq] : 0.0;
+          ga = group_sum<G>(ga + gb);
+          Rotation R;
+          if (live && rotation(al, be, ga, th, R, cosmax, fillmax)) {
+            if constexpr (!HOLD) asm volatile("" ::: "memory");  // read q again: holding it would spill
+#pragma unroll
+            for (int j = 0; j < PW; ++j)
+              if (j < pw) {
+                const double u = p[j], v = HOLD ? qv[HOLD ? j : 0] : q[G * j];
+                p[j] = R.c * u - R.s * v;
+                q[G * j] = R.s * u + R.c * v;
+              }
+            if (acc_j) {
+#pragma unroll
+              for (int h = 0; h < PZ; ++h) {
+                const double u = pz[h], v = q[kp + G * h];
+                pz[h] = R.c * u - R.s * v;
+                q[kp + G * h] = R.s * u + R.c * v;
+              }
+            }
+            al -= R.tg;
+            if (gl == 0) nrm[w + jq] = be + R.tg;
+          }
+          __syncthreads();
+        }
+        // Back: block bi from registers, block bj from shared memory.
+        if (own) {
+          double* z = sm + (int64_t)owner * ls + gl;
+          double* d = resident ? z : W + (int64_t)(p0 + owner) * ldw + gl;
+#pragma unroll
+          for (int j = 0; j < PW; ++j)
+            if (gl + G * j < (resident ? kp : k)) d[G * j] = p[j];
+          if (acc_j)
+#pragma unroll
+            for (int h = 0; h < PZ; ++h) z[kp + G * h] = pz[h];
+        }
+        if (!resident) {
+          for (int c = warp; c < nq; c += NW) {
+            const double* d = Q + (int64_t)c * ls;
+            for (int x = lane; x < k; x += 32) W[(int64_t)(q0 + c) * ldw + x] = d[x];
+          }
+          if (acc_j) {
+            __syncthreads();
+            apply_z<ZR>(J, k, w, p0, np, q0, nq, sm + kp, ls);
+          }
+          __syncthreads();  // the staging area is reused by the next pair
+        }
+      }
+      if (cl > 1) cluster_barrier(cl);
+    }
+    // The sweep's largest cosine before rotation and largest fill factor, over the cluster.
+    const int wc = __reduce_max_sync(0xffffffffu, __float_as_int(cosmax));  // non-negative: ordered like their bits
+    const int wf = __reduce_max_sync(0xffffffffu, __float_as_int(fillmax));
+    if (lane == 0) {
+      atomicMax(&s_cos, wc);
+      atomicMax(&s_fill, wf);
+    }
+    __syncthreads();
+    int* wd = words + 2 * (sweep & 1);
+    if (cl > 1) {
+      if (tid == 0) {
+        atomicMax(wd, s_cos);
+        atomicMax(wd + 1, s_fill);
+        if (rank == 0) {  // the other parity's words: last read before the previous barrier
+          words[2 * ((sweep & 1) ^ 1)] = 0;
+          words[2 * ((sweep & 1) ^ 1) + 1] = 0;
+        }
+      }
+      cluster_barrier(cl);
+      cosmax = __int_as_float(__ldcg(wd));
+      fillmax = __int_as_float(__ldcg(wd + 1));
+      cluster_barrier(cl);  // read by all before the next sweep clears or adds
+    } else {
+      cosmax = __int_as_float(s_cos);
+      fillmax = __int_as_float(s_fill);
+      __syncthreads();
+    }
+    // No pair above the tolerance: done.  Otherwise, a cosine zeroed in this
+    // sweep can only come back through later rotations of its two columns (at most
+    // 2 k of them), each adding at most fill * cosine, and the single-precision
+    // tangent leaves at most 2e-6 of a cosine behind: when both stay below the
+    // tolerance, a further sweep would rotate nothing.
+    if (cosmax == 0.0f || (2.0 * k * (double)fillmax * (double)cosmax <= tol && 2e-6 * (double)cosmax <= tol)) {
+      ++sweep;
+      break;
+    }
+  }
+  if (rank == 0 && tid == 0) {
+    if (sweep == kMaxSweeps) atomicOr(status, 1);
+    atomicMax(status + 1, sweep);
+  }
+  if (resident) {
+    for (int c = warp; c < k; c += NW) {
+      const double* d = sm + (int64_t)c * ls;  // column c sits in slot c: bi = 0 fills slots 0 .. w - 1
+      if (k > 1)
+        for (int x = lane; x < k; x += 32) W[(int64_t)c * ldw + x] = d[x];
+      if (acc_j)
+        for (int z = lane; z < k; z += 32) J[(int64_t)c * k + z] = k > 1 ? d[kp + z] : 1.0;
+    }
+    __syncthreads();
+  }
+  for (int c = rank * NW + warp; c < k; c += cl * NW) {
+    double s = 0.0;
+    for (int x = lane; x < k; x += 32) {
+      const double v = __ldcg(W + (int64_t)c * ldw + x);
+      s = fma(v, v, s);
+    }
+    s = sqrt(warp_sum(s));
+    if (lane == 0) f.sv[c] = s;
+    if (!acc_j)  // eigh: the normalised columns
+      for (int x = lane; x < k; x += 32) J[(int64_t)c * k + x] = __ldcg(W + (int64_t)c * ldw + x) / s;
+  }
+}
+
+template <int G, int PW, int ZR, int NW, bool HOLD>
+cudaError_t launch_class(const SvdJob* jobs, int32_t njobs, int64_t max_k, double* work, const int64_t* work_off,
+                         int32_t* status, int cl, int acc, cudaStream_t st) {
+  // Single-CTA sectors take what they need (w and the stride grow with k), so
+  // several fit an SM; clusters take the whole staging area.
+  size_t smem = kJacobiSmem;
+  if (cl == 1) {
+    int w, nb;
+    block_split((int)max_k, cl, NW * (32 / G), ZR, G, w, nb);
+    smem = (size_t)2 * w * col_stride((int)max_k, ZR, G) * sizeof(double);
+  }
+  auto fn = jacobi_kernel<G, PW, ZR, NW, HOLD>;
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kJacobiSmem);
+  if (e != cudaSuccess) return e;
+  if (cl > 8) {
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(njobs * cl));
+  cfg.blockDim = dim3(NW * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)cl;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fn, jobs, work, work_off, status, cl, acc);
+}
+
+// ---------------------------------------------------------------------------
+// Outputs
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ int64_t warp_argmax_abs(const double* x, int64_t len) {
+  const int lane = threadIdx.x & 31;
+  double best = -1.0;
+  int64_t at = 0;
+  for (int64_t i = lane; i < len; i += 32) {
+    const double v = fabs(x[i]);
+    if (v > best) {
+      best = v;
+      at = i;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+    const int64_t oi = __shfl_xor_sync(0xffffffffu, at, o);
+    if (ob > best || (ob == best && oi < at)) {
+      best = ob;
+      at = oi;
+    }
+  }
+  return at;
+}
+
+constexpr int kFinishWarps = 8;
+
+// Singular triplets in descending order, one warp per column: W's column over its
+// norm and J's column, the left vector's largest-|.| entry positive
+// (factorize.rs:3836-3852, 3945-3962; the first maximum wins).
+__global__ void __launch_bounds__(kFinishWarps * 32)
+    svd_finish_kernel(const SvdJob* __restrict__ jobs, double* __restrict__ U, double* __restrict__ SV,
+                      double* __restrict__ VH, double* __restrict__ work, const int64_t* __restrict__ work_off) {
+  const SvdJob S = jobs[blockIdx.x];
+  const int64_t m = S.m, n = S.n, k = S.k;
+  const int lane = threadIdx.x & 31;
+  const int64_t c = (int64_t)blockIdx.y * kFinishWarps + (threadIdx.x >> 5);
+  if (c >= k) return;
+  const bool wide = m < n;
+  const int64_t ldw = wide ? n : m;
+  const FacWork f = fac_work(work + work_off[blockIdx.x], ldw, k);
+  const double sc = f.sv[c];
+  int64_t pos = 0;
+  for (int64_t o = lane; o < k; o += 32) {
+    const double so = f.sv[o];
+    pos += (so > sc || (so == sc && o < c)) ? 1 : 0;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) pos += __shfl_xor_sync(0xffffffffu, pos, o);
+  const double inv = sc > 0.0 ? 1.0 / sc : 0.0;
+  const double* wc = f.W + c * ldw;
+  const double* jc = f.J + c * k;
+  double* u = U + S.u_off + pos * m;
+  double* vh = VH + S.v_off + pos;
+  const double* lv = wide ? jc : wc;
+  const double sign = lv[warp_argmax_abs(lv, wide ? k : m)] < 0.0 ? -1.0 : 1.0;
+  for (int64_t x = lane; x < m; x += 32) u[x] = wide ? sign * jc[x] : sign * wc[x] * inv;
+  for (int64_t x = lane; x < n; x += 32) vh[x * k] = wide ? sign * wc[x] * inv : sign * jc[x];
+  if (lane == 0) SV[S.s_off + pos] = sc / f.meta[0];
+}
+
+// eigh runs on B = A + c I with c above the spectral radius rho: B is positive
+// definite, its columns after the sweeps, divided by their norms lambda + c, are A's
+// eigenvectors, and no rotations need accumulating.  Every error scales with
+// c, so c is min(9/8 ||A||_F, 17/16 ||A^2||_inf^{1/2}): within a small factor of
+// rho, where ||A||_F alone can be sqrt(n) times it.  Condition number of B: at
+// most 33.
+//
+// Scan: scale (a power of two, largest entry below 1) and ||A||_F to meta[0],
+// meta[1].  Sectors that fail the reference's Hermiticity check
+// (normwise_hermitian, factorize.rs:5999-6021: ||A - A^T||_F <= 2 * 64 eps ||A||_F,
+// every entry finite) set bit 1 of *status.
+__global__ void __launch_bounds__(1024) eigh_scan_kernel(const SvdJob* __restrict__ jobs, const double* __restrict__ A,
+                                                         double* __restrict__ work,
+                                                         const int64_t* __restrict__ work_off,
+                                                         int32_t* __restrict__ status) {
+  const SvdJob S = jobs[blockIdx.x];
+  const int64_t n = S.m;
+  if (n == 0) return;
+  const FacWork f = fac_work(work + work_off[blockIdx.x], n, n);
+  const double* a = A + S.a_off;
+  __shared__ double red[2][32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double mx = 0.0;
+  int finite = 1;
+  for (int64_t i = tid; i < n * n; i += blockDim.x) {
+    mx = fmax(mx, fabs(a[i]));
+    finite &= isfinite(a[i]) ? 1 : 0;
+  }
+  finite = __syncthreads_and(finite);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (lane == 0) red[0][warp] = mx;
+  __syncthreads();
+  for (int i = 0; i < 32; ++i) mx = fmax(mx, red[0][i]);
+  __syncthreads();
+  double scale = 1.0;
+  if (finite && mx > 0.0) {
+    int e;
+    frexp(mx, &e);
+    scale = ldexp(1.0, e < -1022 ? 1022 : -e);
+  }
+  double f2 = 0.0, d2 = 0.0;
+  for (int64_t i = tid; i < n * n; i += blockDim.x) {
+    const int64_t c = i / n, r = i - c * n;
+    const double v = a[i] * scale, d = v - a[c + r * n] * scale;
+    f2 = fma(v, v, f2);
+    d2 = fma(d, d, d2);
+  }
+  f2 = warp_sum(f2);
+  d2 = warp_sum(d2);
+  if (lane == 0) {
+    red[0][warp] = f2;
+    red[1][warp] = d2;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    f2 = d2 = 0.0;
+    for (int i = 0; i < 32; ++i) {
+      f2 += red[0][i];
+      d2 += red[1][i];
+    }
+    const double frob = sqrt(f2);
+    if (!finite || sqrt(d2) > 128.0 * DBL_EPSILON * frob) atomicOr(status, 2);
+    f.meta[0] = scale;
+    f.meta[1] = frob;
+    reinterpret_cast<unsigned long long*>(f.meta)[2] = 0ull;  // ||A^2||_inf, by bits
+  }
+}
+
+constexpr int kBoundWarps = 8;
+
+// Row sums of |A^2| for 16 rows per CTA (8 x 8 tiles on the FP64 tensor cores, A's
+// symmetry giving rows as columns); their maximum to meta[2].
+__global__ void __launch_bounds__(kBoundWarps * 32)
+    eigh_bound_kernel(const SvdJob* __restrict__ jobs, const double* __restrict__ A, double* __restrict__ work,
+                      const int64_t* __restrict__ work_off) {
+  const SvdJob S = jobs[blockIdx.x];
+  const int n = (int)S.m, r0 = 16 * (int)blockIdx.y;
+  if (r0 >= n) return;
+  const FacWork f = fac_work(work + work_off[blockIdx.x], n, n);
+  const double scale = f.meta[0];
+  const double* a = A + S.a_off;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
+  __shared__ double rows[kBoundWarps][16];
+  double sum[2] = {0.0, 0.0};
+  for (int c0 = 16 * warp; c0 < n; c0 += 16 * kBoundWarps) {
+    double d[2][2][2] = {};
+#pragma unroll 2
+    for (int x0 = 0; x0 < n; x0 += 4) {
+      const int x = x0 + t4;
+      double u[2], v[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = r0 + 8 * h + g, c = c0 + 8 * h + g;
+        u[h] = (x < n && r < n) ? __ldg(a + x + (int64_t)r * n) * scale : 0.0;
+        v[h] = (x < n && c < n) ? __ldg(a + x + (int64_t)c * n) * scale : 0.0;
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) dmma(d[h][i][0], d[h][i][1], u[h], v[i]);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) sum[h] += fabs(d[h][i][0]) + fabs(d[h][i][1]);
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    sum[h] += __shfl_xor_sync(0xffffffffu, sum[h], 1);
+    sum[h] += __shfl_xor_sync(0xffffffffu, sum[h], 2);
+    if (t4 == 0) rows[warp][8 * h + g] = sum[h];
+  }
+  __syncthreads();
+  if (threadIdx.x < 16) {
+    double t = 0.0;
+    for (int i = 0; i < kBoundWarps; ++i) t += rows[i][threadIdx.x];
+    atomicMax(reinterpret_cast<unsigned long long*>(f.meta) + 2, (unsigned long long)__double_as_longlong(t));
+  }
+}
+
+__device__ __forceinline__ double eigh_shift(const double* meta) {
+  const double c = fmin(1.125 * meta[1], 1.0625 * sqrt(meta[2]));
+  return c > 0.0 ? c : 1.0;  // a zero sector (or one that failed the scan)
+}
+
+__global__ void __launch_bounds__(256) eigh_form_kernel(const SvdJob* __restrict__ jobs, const double* __restrict__ A,
+                                                        double* __restrict__ work,
+                                                        const int64_t* __restrict__ work_off) {
+  const SvdJob S = jobs[blockIdx.x];
+  const int64_t n = S.m;
+  if (n == 0) return;
+  const FacWork f = fac_work(work + work_off[blockIdx.x], n, n);
+  const double scale = f.meta[0], c = eigh_shift(f.meta);
+  const double* a = A + S.a_off;
+  for (int64_t i = (int64_t)blockIdx.y * 256 + threadIdx.x; i < n * n; i += (int64_t)gridDim.y * 256)
+    f.W[i] = fma(a[i], scale, (i % n) == (i / n) ? c : 0.0);
+}
+
+// One refinement step of the eigenvectors V (Ogita and Aishima, "Iterative
+// refinement for symmetric eigenvalue decomposition", 2018): the sweeps' rounding
+// errors, a random walk of about 12 n rotations at the scale of c, are replaced by
+// those of three products.  With S = V^T A V and R = I - V^T V,
+// lambda_i = S_ii / (V^T V)_ii and V <- V + V X,
+// X_ij = (S_ij + lambda_j R_ij) / (lambda_j - lambda_i), written as R_ij / 2 plus an
+// antisymmetric part (S symmetrised, so that its rounding cannot cost
+// orthogonality over a small gap).  Where that part exceeds 1e-8 (a cluster within
+// the errors) it is left out.
+
+// Fragments of an m x 4 slice: rows g of a matrix walked down its columns (TR) or
+// across them.
+__device__ __forceinline__ double frag(const double* a, int64_t ld, int r, int x, int n, bool tr) {
+  return (r < n && x < n) ? __ldg(tr ? a + x + (int64_t)r * ld : a + r + (int64_t)x * ld) : 0.0;
+}
+
+constexpr int kRefineWarps = 4;  // a CTA takes a 32 x 32 tile, a warp 16 x 16 of it
+
+// step 0: W = scale A V.  step 1: X (into VEC).  step 2: W[:, rank] = V + V X.
+__global__ void __launch_bounds__(kRefineWarps * 32)
+    eigh_refine_kernel(const SvdJob* __restrict__ jobs, const double* __restrict__ A, double* __restrict__ VEC,
+                       double* __restrict__ work, const int64_t* __restrict__ work_off, int step) {
+  const SvdJob S = jobs[blockIdx.x];
+  const int n = (int)S.m;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+  const int r0 = 32 * (int)blockIdx.y + 16 * (warp & 1), c0 = 32 * (int)blockIdx.z + 16 * (warp >> 1);
+  if (r0 >= n || c0 >= n) return;
+  const FacWork f = fac_work(work + work_off[blockIdx.x], n, n);
+  const double *V = f.J, *a = A + S.a_off, *X = VEC + S.u_off;
+  const double* lhs = step == 0 ? a : V;
+  const double* rhs = step == 0 ? V : step == 1 ? f.W : X;
+  double d[2][2][2] = {}, e[2][2][2] = {}, t[2][2][2] = {};
+#pragma unroll 2
+  for (int x0 = 0; x0 < n; x0 += 4) {
+    const int x = x0 + t4;
+    double u[2], v[2], w[2], z[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      u[h] = frag(lhs, n, r0 + 8 * h + g, x, n, step == 1);
+      v[h] = frag(rhs, n, c0 + 8 * h + g, x, n, true);
+      w[h] = step == 1 ? frag(V, n, c0 + 8 * h + g, x, n, true) : 0.0;
+      z[h] = step == 1 ? frag(f.W, n, r0 + 8 * h + g, x, n, true) : 0.0;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        dmma(d[h][i][0], d[h][i][1], u[h], v[i]);
+        if (step == 1) {
+          dmma(e[h][i][0], e[h][i][1], u[h], w[i]);
+          dmma(t[h][i][0], t[h][i][1], z[h], w[i]);
+        }
+      }
+  }
+  const double scale = f.meta[0];
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int r = r0 + 8 * h + g, c = c0 + 8 * i + 2 * t4 + q;
+        if (r >= n || c >= n) continue;
+        if (step == 0) {
+          f.W[r + (int64_t)c * n] = scale * d[h][i][q];
+        } else if (step == 1) {
+          const double lr = f.sv[r], lc = f.sv[c], res = (r == c ? 1.0 : 0.0) - e[h][i][q];
+          const double mid = 0.5 * (d[h][i][q] + t[h][i][q] + (lr + lc) * res), gap = lc - lr;
+          double x = 0.5 * res;
+          if (r != c && fabs(mid) < 1e-8 * fabs(gap)) x += mid / gap;
+          VEC[S.u_off + r + (int64_t)c * n] = x;
+        } else {
+          f.W[r + (int64_t)f.rk[c] * n] = V[r + (int64_t)c * n] + d[h][i][q];
+        }
+      }
+}
+
+// lambda_c = (v_c, A v_c) / (v_c, v_c) into sv; ranks by descending |lambda| (ties:
+// ascending value, then index) into rk; the sorted values out.
+__global__ void __launch_bounds__(1024) eigh_values_kernel(const SvdJob* __restrict__ jobs, double* __restrict__ VAL,
+                                                           double* __restrict__ MAG, double* __restrict__ work,
+                                                           const int64_t* __restrict__ work_off) {
+  const SvdJob S = jobs[blockIdx.x];
+  const int n = (int)S.m, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  if (n == 0) return;
+  const FacWork f = fac_work(work + work_off[blockIdx.x], n, n);
+  for (int c = warp; c < n; c += nwarps) {
+    const double *v = f.J + (int64_t)c * n, *w = f.W + (int64_t)c * n;
+    double s = 0.0, q = 0.0;
+    for (int x = lane; x < n; x += 32) {
+      s = fma(v[x], w[x], s);
+      q = fma(v[x], v[x], q);
+    }
+    s = warp_sum(s);
+    q = warp_sum(q);
+    if (lane == 0) f.sv[c] = s / q;
+  }
+  __syncthreads();
+  for (int c = warp; c < n; c += nwarps) {
+    const double lc = f.sv[c], ac = fabs(lc);
+    int pos = 0;
+    for (int o = lane; o < n; o += 32) {
+      const double lo = f.sv[o], ao = fabs(lo);
+      pos += (ao > ac || (ao == ac && (lo < lc || (lo == lc && o < c)))) ? 1 : 0;
+    }
+    pos = __reduce_add_sync(0xffffffffu, pos);
+    if (lane == 0) {
+      f.rk[c] = (double)pos;
+      VAL[S.s_off + pos] = lc / f.meta[0];
+      if (MAG) MAG[S.s_off + pos] = ac / f.meta[0];
+    }
+  }
+}
+
+// Each vector's largest-|.| entry positive (factorize.rs:3902-3913).
+__global__ void __launch_bounds__(kFinishWarps * 32)
+    eigh_finish_kernel(const SvdJob* __restrict__ jobs, double* __restrict__ VEC, double* __restrict__ work,
+                       const int64_t* __restrict__ work_off) {
+  const SvdJob S = jobs[blockIdx.x];
+  const int64_t n = S.m;
+  const int lane = threadIdx.x & 31;
+  const int64_t c = (int64_t)blockIdx.y * kFinishWarps + (threadIdx.x >> 5);
+  if (c >= n) return;
+  const FacWork f = fac_work(work + work_off[blockIdx.x], n, n);
+  const double* wc = f.W + c * n;
+  const double sign = wc[warp_argmax_abs(wc, n)] < 0.0 ? -1.0 : 1.0;
+  for (int64_t x = lane; x < n; x += 32) VEC[S.u_off + c * n + x] = sign * wc[x];
+}
+
+}  // namespace
+
+// CTAs per sector for a largest k of the launch: one while every column fits an
+// SM's shared memory and a round is a single wave of rotations (k <= 64),
+// then clusters that keep blocks at about 16 columns.  A round costs its latency
+// whatever the width, and a sweep takes k rounds plus an exchange per block pair,
+// so wider clusters only add exchanges.
+int jacobi_cluster(int64_t k) {
+  const int wide = svd_wide_cluster_size() > 0 ? 16 : 8;
+  return k <= 64 ? 1 : k <= 128 ? 4 : k <= 256 ? 8 : wide;
+}
+
+cudaError_t launch_jacobi(const SvdJob* jobs, int32_t njobs, int64_t max_k, double* work, const int64_t* work_off,
+                          int32_t* status, bool acc_j, cudaStream_t st) {
+  if (njobs == 0) return cudaSuccess;
+  const int cl = jacobi_cluster(max_k);
+  const int a = acc_j ? 1 : 0;
+  auto go = [&](auto fn) { return fn(jobs, njobs, max_k, work, work_off, status, cl, a, st); };
+  if (max_k <= 32) return go(launch_class<8, 4, 32, 4, true>);
+  if (max_k <= 64) return go(launch_class<8, 8, 64, 8, true>);
+  if (max_k <= 128) return go(launch_class<16, 8, 32, 8, true>);
+  if (max_k <= 256) return go(launch_class<32, 8, 32, 16, true>);
+  if (max_k <= 512) return go(launch_class<32, 16, 32, 16, true>);
+  if (max_k <= 608) return go(launch_class<32, 19, 64, 19, false>);
+  if (max_k <= 1024) return go(launch_class<32, 32, 32, 12, false>);
+  return go(launch_class<32, 48, 32, 8, false>);
+}
+
+cudaError_t launch_svd_finish(const SvdJob* jobs, int32_t njobs, int64_t max_k, double* u, double* s, double* vh,
+                              double* work, const int64_t* work_off, cudaStream_t st) {
+  if (njobs == 0 || max_k == 0) return cudaSuccess;
+  const dim3 grid((unsigned)njobs, (unsigned)((max_k + kFinishWarps - 1) / kFinishWarps));
+  svd_finish_kernel<<<grid, kFinishWarps * 32, 0, st>>>(jobs, u, s, vh, work, work_off);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_eigh_prepare(const SvdJob* jobs, int32_t njobs, int64_t max_n, const double* a, double* work,
+                                const int64_t* work_off, int32_t* status, cudaStream_t st) {
+  if (njobs == 0 || max_n == 0) return cudaSuccess;
+  eigh_scan_kernel<<<njobs, 1024, 0, st>>>(jobs, a, work, work_off, status);
+  eigh_bound_kernel<<<dim3((unsigned)njobs, (unsigned)((max_n + 15) / 16)), kBoundWarps * 32, 0, st>>>(jobs, a, work,
+                                                                                                     work_off);
+  const unsigned gy = (unsigned)std::min<int64_t>(64, (max_n * max_n + 1023) / 1024);
+  eigh_form_kernel<<<dim3((unsigned)njobs, gy), 256, 0, st>>>(jobs, a, work, work_off);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_eigh_finish(const SvdJob* jobs, int32_t njobs, int64_t max_n, const double* a, double* vecs,
+                               double* vals, double* mags, double* work, const int64_t* work_off, cudaStream_t st) {
+  if (njobs == 0 || max_n == 0) return cudaSuccess;
+  const unsigned nt = (unsigned)((max_n + 31) / 32);
+  const dim3 tiles((unsigned)njobs, nt, nt);
+  eigh_refine_kernel<<<tiles, kRefineWarps * 32, 0, st>>>(jobs, a, vecs, work, work_off, 0);
+  eigh_values_kernel<<<njobs, 1024, 0, st>>>(jobs, vals, mags, work, work_off);
+  eigh_refine_kernel<<<tiles, kRefineWarps * 32, 0, st>>>(jobs, a, vecs, work, work_off, 1);
+  eigh_refine_kernel<<<tiles, kRefineWarps * 32, 0, st>>>(jobs, a, vecs, work, work_off, 2);
+  const dim3 grid((unsigned)njobs, (unsigned)((max_n + kFinishWarps - 1) / kFinishWarps));
+  eigh_finish_kernel<<<grid, kFinishWarps * 32, 0, st>>>(jobs, vecs, work, work_off);
+  return cudaGetLastError();
+}
+
+}  // namespace tnt

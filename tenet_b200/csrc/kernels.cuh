@@ -98,16 +98,38 @@ cudaError_t launch_split_pack_operand(const void* job_table, const GemmJob* host
 cudaError_t launch_svd(const SvdJob* jobs, int32_t njobs, const double* a, double* u, double* s, double* vh,
                        double* work, const int64_t* work_off, int32_t* status, cudaStream_t stream);
 
-// Batched per-sector Householder QR (positive-diagonal gauge) and Jacobi eigh
-// (descending |lambda|, largest-entry-positive vectors), factor.cu.
+// One-sided Jacobi of k x k matrices already in the sectors' scratch (jacobi.cu);
+// max_k (at most kJacobiMaxK) is the largest k of the jobs.
+constexpr int64_t kJacobiMaxK = 1536;
+int jacobi_cluster(int64_t k);
+cudaError_t launch_jacobi(const SvdJob* jobs, int32_t njobs, int64_t max_k, double* work, const int64_t* work_off,
+                          int32_t* status, bool acc_j, cudaStream_t stream);
+cudaError_t launch_svd_finish(const SvdJob* jobs, int32_t njobs, int64_t max_k, double* u, double* s, double* vh,
+                              double* work, const int64_t* work_off, cudaStream_t stream);
+cudaError_t launch_eigh_prepare(const SvdJob* jobs, int32_t njobs, int64_t max_n, const double* a, double* work,
+                                const int64_t* work_off, int32_t* status, cudaStream_t stream);
+cudaError_t launch_eigh_finish(const SvdJob* jobs, int32_t njobs, int64_t max_n, const double* a, double* vecs,
+                               double* vals, double* mags, double* work, const int64_t* work_off, cudaStream_t stream);
+
+// Cluster Householder QR of sectors with at most kQrMaxRows rows (qr.cu), and
+// products with its Q; max_rows / max_cols / max_k over the jobs.
+constexpr int64_t kQrMaxRows = 1408;
+enum : int {
+  kQrFactor = 0,    // tnt_qr: X = A, R to vh, Q (launch_qr_apply) to u
+  kQrSvdFirst = 1,  // rectangular sectors: the long side reduced, reflectors in its output region
+  kQrSvdSecond = 2  // the square rest, transposed; reflectors in the short side's region, R^T to the scratch
+};
+cudaError_t launch_qr_factor(const SvdJob* jobs, int32_t njobs, int64_t max_rows, int64_t max_cols, int mode,
+                             const double* a, double* u, double* vh, double* work, const int64_t* work_off,
+                             cudaStream_t stream);
+cudaError_t launch_qr_apply(const SvdJob* jobs, int32_t njobs, int64_t max_rows, int64_t max_k, int mode, double* u,
+                            double* vh, double* work, const int64_t* work_off, cudaStream_t stream);
+
+// Batched per-sector Householder QR (positive-diagonal gauge) of any size, factor.cu.
 cudaError_t launch_qr(const SvdJob* jobs, int32_t njobs, const double* a, double* q, double* r, double* work,
                       const int64_t* work_off, cudaStream_t stream);
-cudaError_t launch_eigh(const SvdJob* jobs, int32_t njobs, const double* a, double* vecs, double* vals, double* mags,
-                        double* work, const int64_t* work_off, int32_t* status, cudaStream_t stream);
-// True when eigh_kernel keeps an n x n sector (matrix and vectors) in shared memory.
-bool eigh_on_chip(int64_t n);
 // Eigendecomposition through the batched SVD of B = A + ||A||_F I, for plans
-// with sectors beyond eigh_on_chip: b (a's layout), u, s, vh (the SVD
+// with sectors beyond the Jacobi engine: b (a's layout), u, s, vh (the SVD
 // layouts of the plan) and shift (one double per job) are scratch; *bad is
 // set to 1 for a non-Hermitian or non-finite sector (not cleared here).
 cudaError_t launch_eigh_by_svd(const SvdJob* jobs, int32_t n_cluster, int32_t njobs, int64_t max_n, const double* a,

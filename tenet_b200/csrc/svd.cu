@@ -1,4 +1,7 @@
-// Batched per-sector SVD and cross-sector truncation on the device.
+// General batched per-sector SVD and cross-sector truncation on the device.
+// Sectors of at most 1408 rows run on the QR-preconditioned cluster engine
+// (qr.cu, jacobi.cu); these kernels take longer ones, and every sector of the
+// allocation-free entry point (svd_static.cu), whose scratch they fit.
 //
 // Replaces the serial sector loop of svd_compact_factors_dyn_with_direction
 // (tenet-matrixalgebra/src/factorize.rs:1631-1760), which calls a dense SVD

@@ -76,7 +76,10 @@ class FusionRule:
         return isinstance(other, FusionRule) and self.factors == other.factors and self.codec == other.codec
 
     def __hash__(self):
-        return hash((self.factors, self.codec))
+        h = getattr(self, "_hash", None)  # rules and spaces are immutable: hashed once
+        if h is None:
+            h = self._hash = hash((self.factors, self.codec))
+        return h
 
     def __repr__(self):
         return "FusionRule(" + " x ".join(self.factors) + ")"
@@ -238,10 +241,13 @@ class GradedSpace:
         return (self.rule, self._sectors, self._degs, self.is_dual)
 
     def __eq__(self, other):
-        return isinstance(other, GradedSpace) and self._key() == other._key()
+        return self is other or (isinstance(other, GradedSpace) and self._key() == other._key())
 
     def __hash__(self):
-        return hash(self._key())
+        h = getattr(self, "_hash", None)
+        if h is None:
+            h = self._hash = hash(self._key())
+        return h
 
     def __repr__(self):
         inner = ", ".join(f"{self.rule.unlabel(s)}=>{d}" for s, d in zip(self._sectors, self._degs))
@@ -305,10 +311,16 @@ class HomSpace:
         return (self.rule, self.codomain, self.domain)
 
     def same_as(self, other):
-        return self.key() == other.key()
+        return self is other or self.key() == other.key()
 
     def sectors(self):
         """``[(coupled label, rows, cols, offset)]`` in storage order."""
+        got = getattr(self, "_sectors", None)
+        if got is None:
+            got = self._sectors = self._read_sectors()
+        return list(got)
+
+    def _read_sectors(self):
         nf = self.rule.nfactors
         labels = (i32 * max(1, self.nsectors * nf))()
         rows, cols, offs = (i64 * max(1, self.nsectors))(), (i64 * max(1, self.nsectors))(), (i64 * max(1, self.nsectors))()
@@ -577,9 +589,35 @@ class FactorPlan:
         we = i64()
         call("tnt_fplan_work", h, C.byref(we))
         self.work_elems = we.value
+        self._sector_list = space.sectors()
+        self._bonds: Dict = {}
+        self._ranks: Dict = {}
 
     def __del__(self):
         _release("tnt_fplan_destroy", getattr(self, "_h", None))
+
+    def _kept(self, table: Dict, key, make):
+        """A device table of this plan, made once per value of ``key`` (at most 64 kept).
+
+        Its upload is complete before it is first used (a blocking copy), and
+        every use records the stream, so any stream may use it and it may be
+        dropped while work that reads it is queued."""
+        got = table.get(key)
+        if got is None:
+            while len(table) >= 64:
+                table.pop(next(iter(table)), None)
+            got = table[key] = make()
+        got[0].record_stream(torch().cuda.current_stream(got[0].device))
+        return got
+
+    def space_ranks(self, ranks: Sequence[int], device):
+        """Per-sector ranks of a space truncation, on the device."""
+        t = torch()
+        return self._kept(self._ranks, (tuple(ranks), device), lambda: (t.tensor(ranks, dtype=t.int64).to(device),))[0]
+
+    def bond(self, rt: "Runtime", ranks: Sequence[int], device) -> "_Bond":
+        """The bond with ``ranks[i]`` states in coupled sector i: the factors' spaces and copy tables."""
+        return self._kept(self._bonds, (tuple(ranks), device), lambda: _make_bond(rt, self, ranks, device))
 
 
 # ---------------------------------------------------------------------------
@@ -868,20 +906,26 @@ class TensorMap:
         plan = rt.fplan(self.space)
         dev = self.data.device
         u = t.empty(max(1, plan.u_size), dtype=t.float64, device=dev)
-        s = t.empty(max(1, plan.s_size), dtype=t.float64, device=dev)
         vh = t.empty(max(1, plan.v_size), dtype=t.float64, device=dev)
+        # values, error and kept ranks side by side: one copy brings them to the host
+        small = t.empty(plan.s_size + 1 + plan.nsectors, dtype=t.float64, device=dev)
         call("tnt_svd", rt._h, plan._h, C.c_void_p(self.data.data_ptr()), C.c_void_p(u.data_ptr()),
-             C.c_void_p(s.data_ptr()), C.c_void_p(vh.data_ptr()), rt.stream())
-        kept_d = t.empty(max(1, plan.nsectors), dtype=t.int64, device=dev)
-        err_d = t.empty(1, dtype=t.float64, device=dev)
-        ranks = None
-        sectors = self.space.sectors()
-        if truncation.policy == _lib.TRUNC_SPACE:
-            ranks = arr(i64, [truncation.ranks.get(lab, 0) for lab, _, _, _ in sectors])
-        call("tnt_truncate", rt._h, plan._h, C.c_void_p(s.data_ptr()), truncation.policy, truncation.p0,
-             truncation.p1, ranks, C.c_void_p(kept_d.data_ptr()), C.c_void_p(err_d.data_ptr()), rt.stream())
-        return SvdResult(self, plan, u, s, vh, kept_d, err_d)
+             C.c_void_p(small.data_ptr()), C.c_void_p(vh.data_ptr()), rt.stream())
+        host = self._truncate(plan, small, small.data_ptr(), plan.s_size, truncation)
+        return SvdResult(self, plan, u, vh, host)
 
+    def _truncate(self, plan, small, values, at, truncation):
+        """Select on the spectra at ``values``; error and kept ranks go to ``small[at:]``; all of it to the host."""
+        rt = self.runtime
+        err = small.data_ptr() + 8 * at
+        ranks = None
+        if truncation.policy == _lib.TRUNC_SPACE:
+            ranks = plan.space_ranks([truncation.ranks.get(lab, 0) for lab, _, _, _ in plan._sector_list], small.device)
+            ranks = C.c_void_p(ranks.data_ptr())
+        call("tnt_truncate_async", rt._h, plan._h, C.c_void_p(values), truncation.policy, truncation.p0, truncation.p1,
+             ranks, C.c_void_p(err + 8), C.c_void_p(err), rt.stream())
+        host = small.cpu().numpy()
+        return host[:at], float(host[at]), host[at + 1:].view(np.int64).tolist()
 
     def qr_compact(self):
         """``TensorMap::qr_compact`` (typed.rs:1393): ``self = Q o R`` per coupled sector on the device.
@@ -933,40 +977,64 @@ class TensorMap:
         plan = rt.fplan(self.space)
         dev = self.data.device
         vecs = t.empty(max(1, plan.u_size), dtype=t.float64, device=dev)
-        vals = t.empty(max(1, plan.s_size), dtype=t.float64, device=dev)
-        mags = t.empty(max(1, plan.s_size), dtype=t.float64, device=dev)
+        n = plan.s_size
+        small = t.empty(2 * n + 1 + plan.nsectors, dtype=t.float64, device=dev)  # values, magnitudes, error, kept
         call("tnt_eigh", rt._h, plan._h, C.c_void_p(self.data.data_ptr()), C.c_void_p(vecs.data_ptr()),
-             C.c_void_p(vals.data_ptr()), C.c_void_p(mags.data_ptr()), rt.stream())
-        kept_d = t.empty(max(1, plan.nsectors), dtype=t.int64, device=dev)
-        err_d = t.empty(1, dtype=t.float64, device=dev)
-        ranks = None
-        if truncation.policy == _lib.TRUNC_SPACE:
-            ranks = arr(i64, [truncation.ranks.get(lab, 0) for lab, _, _, _ in self.space.sectors()])
-        call("tnt_truncate", rt._h, plan._h, C.c_void_p(mags.data_ptr()), truncation.policy, truncation.p0,
-             truncation.p1, ranks, C.c_void_p(kept_d.data_ptr()), C.c_void_p(err_d.data_ptr()), rt.stream())
-        return EighResult(self, plan, vecs, vals, kept_d, err_d)
+             C.c_void_p(small.data_ptr()), C.c_void_p(small.data_ptr() + 8 * n), rt.stream())
+        host = self._truncate(plan, small, small.data_ptr() + 8 * n, 2 * n, truncation)
+        return EighResult(self, plan, vecs, small, host)
+
+
+class _Bond(tuple):
+    """(table, left, right, n_left, n_right, n_diag, diag space): device copy
+    table (rows of the left factor, the right factor, the diagonal), the spaces
+    codomain <- W, W <- domain and W <- W (None unless an endomorphism)."""
+
+
+def _make_bond(rt, plan: "FactorPlan", ranks, device) -> _Bond:
+    space = plan.space
+    W = GradedSpace(space.rule, [(lab, k) for (lab, _, _, _), k in zip(plan._sector_list, ranks) if k > 0])
+    left, right = rt.space(space.rule, space.codomain, [W]), rt.space(space.rule, [W], space.domain)
+    endo = list(space.codomain) == list(space.domain)
+    diag = rt.space(space.rule, [W], [W]) if endo else None
+    off = lambda sp: {lab: (r, o) for lab, r, _, o in sp.sectors()} if sp is not None else {}
+    lsec, rsec, dsec = off(left), off(right), off(diag)
+    rows_l, rows_r, rows_d = [], [], []
+    for (lab, m, n, _), rec, k in zip(plan._sector_list, plan.records.tolist(), ranks):
+        if k == 0:
+            continue
+        kk = rec[2]
+        rows_l.append([rec[4], lsec[lab][1], m, k, m, m, -1])
+        rows_r.append([rec[6], rsec[lab][1], k, n, kk, k, -1])
+        if endo:
+            r, o = dsec[lab]
+            rows_d.append([rec[5], o, 1, k, 1, r + 1, -1])
+    t = torch()
+    table = t.tensor(rows_l + rows_r + rows_d + [[0] * 7], dtype=t.int64).to(device)
+    return _Bond((table, left, right, len(rows_l), len(rows_r), len(rows_d), diag))
+
+
+def _copy_rows(rt, table, first, count, src, dst):
+    """``count`` strided block copies of a bond's table, from row ``first`` on, in one launch."""
+    if count:
+        call("tnt_copy_segments_async", rt._h, count, C.c_void_p(table.data_ptr() + 56 * first),
+             C.c_void_p(src.data_ptr()), C.c_void_p(dst.data_ptr()), None, rt.stream())
 
 
 def _bond_factors(src: "TensorMap", plan: "FactorPlan", ranks, left, right):
     """Left factor (codomain <- W) and right factor (W <- domain) over the bond W
     with ``ranks[i]`` states in coupled sector i, cut from the plan's U / Vh
-    layouts (column-major m x k and k x n per sector, leading columns / rows kept)."""
+    layouts (column-major m x k and k x n per sector, leading columns / rows
+    kept): one copy launch each (every sector of the factors is one of src's).
+    ``right`` None: the left factor alone."""
     rt = src.runtime
-    rule = src.rule
-    sectors = src.space.sectors()
-    bond = GradedSpace(rule, [(lab, k) for (lab, _, _, _), k in zip(sectors, ranks) if k > 0])
-    # every sector of L and R is one of src's and is written below
-    L = TensorMap.uninitialized(rt, rt.space(rule, src.space.codomain, [bond]))
-    R = TensorMap.uninitialized(rt, rt.space(rule, [bond], src.space.domain))
-    lsec = {lab: off for lab, _, _, off in L.space.sectors()}
-    rsec = {lab: off for lab, _, _, off in R.space.sectors()}
-    for (lab, m, n, _), rec, k in zip(sectors, plan.records, ranks):
-        if k == 0:
-            continue
-        kk = int(rec[2])
-        L.data[lsec[lab]: lsec[lab] + m * k] = left[rec[4]: rec[4] + m * k]
-        full = right[rec[6]: rec[6] + kk * n].view(n, kk)  # column-major kk x n
-        R.data[rsec[lab]: rsec[lab] + k * n] = full[:, :k].contiguous().view(-1)
+    table, lsp, rsp, nl, nr, _, _ = plan.bond(rt, ranks, left.device)
+    L = TensorMap.uninitialized(rt, lsp)
+    _copy_rows(rt, table, 0, nl, left, L.data)
+    if right is None:
+        return L
+    R = TensorMap.uninitialized(rt, rsp)
+    _copy_rows(rt, table, nl, nr, right, R.data)
     return L, R
 
 
@@ -979,16 +1047,15 @@ class SpectrumEntry:
 class SvdResult:
     """Truncated SVD factors: ``u`` (codomain <- bond), ``s`` per sector, ``vh`` (bond <- domain)."""
 
-    def __init__(self, src: TensorMap, plan: FactorPlan, u, s, vh, kept_d, err_d):
+    def __init__(self, src: TensorMap, plan: FactorPlan, u, vh, host):
         self._src, self._plan = src, plan
-        self._u, self._s, self._vh = u, s, vh
-        self.kept = [int(x) for x in kept_d.cpu().numpy()[: plan.nsectors]]
-        self.error = float(err_d.cpu().numpy()[0])
-        s_host = s.cpu().numpy()
-        self.singular_values = []
+        self._u, self._vh = u, vh
+        values, self.error, self.kept = host
         rule = src.rule
-        for (lab, r, c, off), rec, k in zip(src.space.sectors(), plan.records, self.kept):
-            self.singular_values.append(SpectrumEntry(rule.unlabel(lab), s_host[rec[5]: rec[5] + k].copy()))
+        self.singular_values = [
+            SpectrumEntry(rule.unlabel(lab), values[rec[5]: rec[5] + k].copy())
+            for (lab, _, _, _), rec, k in zip(plan._sector_list, plan.records.tolist(), self.kept)
+        ]
 
     def bond_space(self) -> GradedSpace:
         rule = self._src.rule
@@ -1004,32 +1071,23 @@ class EighResult:
     """Truncated eigendecomposition: kept eigenvalues per sector (signed, descending |lambda|),
     the eigenvector isometry ``v`` (codomain <- W) and the diagonal ``d`` (W <- W)."""
 
-    def __init__(self, src: TensorMap, plan: FactorPlan, vecs, vals, kept_d, err_d):
+    def __init__(self, src: TensorMap, plan: FactorPlan, vecs, vals, host):
         self._src, self._plan = src, plan
         self._vecs, self._vals = vecs, vals
-        self.kept = [int(x) for x in kept_d.cpu().numpy()[: plan.nsectors]]
-        self.error = float(err_d.cpu().numpy()[0])
-        v_host = vals.cpu().numpy()
+        values, self.error, self.kept = host
         rule = src.rule
-        self.eigenvalues = []
-        for (lab, _, _, _), rec, k in zip(src.space.sectors(), plan.records, self.kept):
-            if k > 0:
-                self.eigenvalues.append(SpectrumEntry(rule.unlabel(lab), v_host[rec[5]: rec[5] + k].copy()))
+        self.eigenvalues = [
+            SpectrumEntry(rule.unlabel(lab), values[rec[5]: rec[5] + k].copy())
+            for (lab, _, _, _), rec, k in zip(plan._sector_list, plan.records.tolist(), self.kept) if k > 0
+        ]
 
     def factors(self):
         """``(d, v)``: the diagonal of kept eigenvalues and the kept eigenvectors."""
-        t = torch()
         src, plan = self._src, self._plan
-        V, _ = _bond_factors(src, plan, self.kept, self._vecs, t.zeros(max(1, plan.v_size), dtype=t.float64,
-                                                                         device=self._vecs.device))
-        bond = V.space.domain
-        D = TensorMap.zeros(src.runtime, bond, bond)
-        dsec = {lab: (r, off) for lab, r, _, off in D.space.sectors()}
-        for (lab, _, _, _), rec, k in zip(src.space.sectors(), plan.records, self.kept):
-            if k == 0:
-                continue
-            r, off = dsec[lab]
-            D.data[off: off + r * r].view(r, r).diagonal().copy_(self._vals[rec[5]: rec[5] + k])
+        V = _bond_factors(src, plan, self.kept, self._vecs, None)
+        table, _, _, nl, nr, nd, dsp = plan.bond(src.runtime, self.kept, self._vecs.device)
+        D = TensorMap(src.runtime, dsp)
+        _copy_rows(src.runtime, table, nl + nr, nd, self._vals, D.data)
         return D, V
 
 

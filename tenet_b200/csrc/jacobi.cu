@@ -16,16 +16,23 @@
 //    read and written there instead of two read twice and written once;
 //  * short columns take few lanes each (G = 8 up to k = 64, 16 up to 128), so the
 //    reduction and the angle are shared by several pairs of a warp;
-//  * squared norms are formed when a block is loaded and updated per rotation,
-//    so a pair needs one dot product;
+//  * columns carry a scale (fast rotations: p - a q and q + b p, two FMAs per
+//    element instead of two products and two FMAs), taken out once per block pair;
+//  * squared norms are formed once and updated per rotation, so a pair needs one
+//    dot product;
 //  * tests and the tangent run in single precision (its error only leaves 1e-6 of
-//    the pair's cosine behind), the cosine and sine come from one third-order
-//    step in FP64, so c^2 + s^2 = 1 to FP64 rounding;
-//  * rotations accumulate in 2w x 2w matrices kept below the staged columns, and
-//    J's columns are multiplied by them once per block pair on the FP64 tensor
-//    cores (m8n8k4);
+//    the pair's cosine behind); the scale factor (1 + t^2)^{-1/2} comes from one
+//    third-order step in FP64, so a rotation is orthogonal to FP64 rounding;
 //  * the sweep that only confirms convergence is left out when the sweep
 //    before it cannot have left a cosine above the tolerance (below).
+//
+// Two kernels.  While all columns, with J's rows stacked below W's, fit the
+// cluster's shared memory twice (k <= 320, or 448 without J), they never leave it:
+// blocks move to the CTA of their next pair through distributed shared memory.
+// Beyond, blocks are staged through L2, the rotations of a block pair accumulate
+// in a 2w x 2w matrix below the staged columns, and J's columns are multiplied by
+// it on the FP64 tensor cores.  (Handing columns from warp to warp on a count of
+// their rounds instead of a CTA-wide barrier measured the same there.)
 // Measured on a B200 against the general kernels of svd.cu and a two-sided
 // Jacobi in shared memory: truncated SVD of the D = 2048 chain (six sectors of
 // 586, two of 293) 94.9 -> 22.4 ms, a whole two-site update at D = 224 (104 x 104)
@@ -43,17 +50,14 @@ using namespace panel;
 constexpr int kMaxSweeps = 40;
 constexpr size_t kJacobiSmem = 216 * 1024;
 
-// Stride of a staged column: k rounded up to 32, the zr rows of its accumulator,
-// and a pad that keeps the accesses conflict-free (8-lane columns side by side:
-// 8 mod 16; MMA fragments of the accumulator: 4 mod 16).
-__host__ __device__ __forceinline__ int col_stride(int k, int zr, int g) {
-  return (k + 31) / 32 * 32 + zr + (g == 8 ? 8 : 4);
-}
+// Stride of a staged column: its rows, the zr rows of its accumulator, and a pad
+// that keeps the MMA fragments of the accumulator conflict-free (4 mod 16).
+__host__ __device__ constexpr int col_stride(int rows, int zr) { return rows + zr + 4; }
 
-// Block width and (even) block count for k columns on cl CTAs of `owners` column
-// owners each.
-__host__ __device__ __forceinline__ void block_split(int k, int cl, int owners, int zr, int g, int& w, int& nb) {
-  int cap = (int)(kJacobiSmem / 8 / (2 * col_stride(k, zr, g)));
+// Block width and (even) block count for k columns of `rows` rows on cl CTAs of
+// `owners` column owners each.
+__host__ __device__ __forceinline__ void block_split(int k, int rows, int cl, int owners, int zr, int& w, int& nb) {
+  int cap = (int)(kJacobiSmem / 8 / (2 * col_stride(rows, zr)));
   if (cap > owners) cap = owners;
   if (cap > zr / 2) cap = zr / 2;
   int per = 1;  // block pairs per CTA and round
@@ -67,8 +71,9 @@ struct Thresholds {
   float tol, noise2, floor;
 };
 
+// Tangent t, (1 + t^2)^{-1/2} and its inverse, t * gamma (the norms' change).
 struct Rotation {
-  double c, s, tg;  // cosine, sine, tangent * gamma (the norms' change)
+  double t, c, ic, tg;
 };
 
 __device__ __forceinline__ float rcp_approx(float x) {
@@ -101,8 +106,9 @@ __device__ __forceinline__ bool rotation(double al, double be, double ga, const 
   t = z < 0.0f ? -t : t;
   const double td = (double)t, y = (double)rsqrt_approx(fmaf(t, t, 1.0f)), x = fma(td, td, 1.0);
   const double e = fma(-x * y, y, 1.0);  // y (1 + e/2 + 3 e^2 / 8) = x^{-1/2} up to e^3
+  R.t = td;
   R.c = fma(y * e, fma(0.375, e, 0.5), y);
-  R.s = R.c * td;
+  R.ic = x * R.c;
   R.tg = td * ga;
   // Cosine of the pair, and the most this rotation can put back between one of
   // its columns and a third per unit of the other's cosine with it.
@@ -119,33 +125,403 @@ __device__ __forceinline__ double group_sum(double v) {
   return v;
 }
 
-// Both columns in shared memory (pairs inside a block); every lane of the warp calls it.
-template <int G, int ZR>
-__device__ __forceinline__ void rotate_smem(bool live, double* p, double* q, double* np, double* nq, int pw, bool acc_j,
+// Squared norm, scale and inverse scale of the columns of a block pair (block bi's
+// at 0 .. w - 1, block bj's from w on): true column = scale * stored column.
+struct Columns {
+  double *nrm, *d, *id;
+};
+
+// Both columns in shared memory (pairs inside a block); every lane of the warp
+// calls it.  PW elements per lane enter the dot product, NZ further ones (G apart
+// from row G PW on) only rotate, when acc.  KEEP: all of them are loaded before
+// the first store (the compiler cannot move a load over one).
+template <int G, int PW, int NZ, bool KEEP>
+__device__ __forceinline__ void rotate_smem(bool live, double* base, int ls, int ip, int iq, const Columns& col, bool acc,
                                             const Thresholds& th, float& cosmax, float& fillmax) {
   const int gl = threadIdx.x % G;
-  double ga = 0.0, al = 0.0, be = 0.0;
-  if (live) {
-    al = *np;
-    be = *nq;
-    for (int j = 0; j < pw; ++j) ga = fma(p[gl + G * j], q[gl + G * j], ga);
+  double ga = 0.0, gb = 0.0, al = 0.0, be = 0.0, dp = 1.0, dq = 1.0;
+  double u[KEEP ? PW : 1], v[KEEP ? PW : 1], uz[NZ], vz[NZ];
+  double* p = base + (live ? ip : 0) * ls + gl;
+  double* q = base + (live ? iq : 0) * ls + gl;
+#pragma unroll
+  for (int j = 0; j < PW; ++j) {
+    const double x = p[G * j], y = q[G * j];
+    if constexpr (KEEP) {
+      u[j] = x;
+      v[j] = y;
+    }
+    if (j & 1) gb = fma(x, y, gb);
+    else ga = fma(x, y, ga);
   }
-  ga = group_sum<G>(ga);
+  if (live) {
+    al = col.nrm[ip];
+    be = col.nrm[iq];
+    dp = col.d[ip];
+    dq = col.d[iq];
+  }
+  ga = group_sum<G>(ga + gb) * (dp * dq);
   Rotation R;
   if (live && rotation(al, be, ga, th, R, cosmax, fillmax)) {
-    const int n = acc_j ? pw + ZR / G : pw;
-    for (int j = 0; j < n; ++j) {
-      const double u = p[gl + G * j], v = q[gl + G * j];
-      p[gl + G * j] = R.c * u - R.s * v;
-      q[gl + G * j] = R.s * u + R.c * v;
+    const double ip_ = col.id[ip], iq_ = col.id[iq];
+    const double a = -R.t * (dq * ip_), b = R.t * (dp * iq_);
+    if constexpr (!KEEP) asm volatile("" ::: "memory");
+    if (acc) {
+#pragma unroll
+      for (int j = 0; j < NZ; ++j) {
+        uz[j] = p[G * (PW + j)];
+        vz[j] = q[G * (PW + j)];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < PW; ++j) {
+      const double x = KEEP ? u[KEEP ? j : 0] : p[G * j], y = KEEP ? v[KEEP ? j : 0] : q[G * j];
+      p[G * j] = fma(a, y, x);
+      q[G * j] = fma(b, x, y);
+    }
+    if (acc) {
+#pragma unroll
+      for (int j = 0; j < NZ; ++j) {
+        p[G * (PW + j)] = fma(a, vz[j], uz[j]);
+        q[G * (PW + j)] = fma(b, uz[j], vz[j]);
+      }
     }
     if (gl == 0) {
-      *np = al - R.tg;
-      *nq = be + R.tg;
+      col.nrm[ip] = al - R.tg;
+      col.nrm[iq] = be + R.tg;
+      col.d[ip] = dp * R.c;
+      col.d[iq] = dq * R.c;
+      col.id[ip] = ip_ * R.ic;
+      col.id[iq] = iq_ * R.ic;
     }
   }
   __syncwarp();
 }
+
+// The pairs inside the two blocks: a round robin in each, all warps.
+template <int G, int PW, int NZ, int NW, bool KEEP>
+__device__ __forceinline__ void rotate_within(double* base, int ls, int w, int np, int nq, const Columns& col, bool acc,
+                                              const Thresholds& th, float& cosmax, float& fillmax) {
+  constexpr int PP = 32 / G;
+  const int warp = threadIdx.x >> 5, sub = (threadIdx.x & 31) / G;
+  const int n2 = (w + 1) & ~1, half = n2 / 2;
+  for (int r = 0; r < n2 - 1; ++r) {
+    for (int e0 = warp * PP; e0 < n2; e0 += NW * PP) {
+      const int e = e0 + sub, b = e >= half;
+      int p = 0, q = 0;
+      bool live = e < n2;
+      if (live) {
+        tournament_pair(r, b ? e - half : e, n2, p, q);
+        live = q < (b ? nq : np);
+        p += b ? w : 0;
+        q += b ? w : 0;
+      }
+      rotate_smem<G, PW, NZ, KEEP>(live, base, ls, p, q, col, acc, th, cosmax, fillmax);
+    }
+    __syncthreads();
+  }
+}
+
+// Thresholds from ||W||_F^2 (the same sum in the same order in every CTA): a pair
+// is rotated only while its cosine exceeds the rounding level of a length-k dot
+// product and both columns stand above the rounding noise k eps ||A||_F (columns of
+// the null space shrink to that level, and every rotation refills them with
+// noise whose cosine is O(1)).  Every warp leaves its columns' squared norms in
+// sv first; part: 32 doubles of shared memory.
+__device__ __forceinline__ double make_thresholds(const FacWork& f, int64_t ldw, int k, int rank, int cl, double* part,
+                                                  Thresholds& th) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  for (int c = rank * nwarps + warp; c < k; c += cl * nwarps) {
+    double s = 0.0;
+    for (int x = lane; x < k; x += 32) {
+      const double v = __ldcg(f.W + (int64_t)c * ldw + x);
+      s = fma(v, v, s);
+    }
+    s = warp_sum(s);
+    if (lane == 0) f.sv[c] = s;
+  }
+  cluster_barrier(cl);
+  double fs = 0.0;
+  for (int c = tid; c < k; c += blockDim.x) fs += __ldcg(f.sv + c);
+  fs = warp_sum(fs);
+  if (lane == 0) part[warp] = fs;
+  __syncthreads();
+  double frob2 = 0.0;
+  for (int i = 0; i < nwarps; ++i) frob2 += part[i];
+  const double tol = 4.0 * sqrt((double)k) * DBL_EPSILON;
+  th.tol = (float)tol;
+  th.noise2 = (float)(((double)k * DBL_EPSILON) * ((double)k * DBL_EPSILON) * frob2);
+  th.floor = (float)(1e-33 * frob2);  // below every gamma above the tolerance of two columns above the noise
+  return tol;
+}
+
+// After a sweep with these largest values: no pair above the tolerance means
+// done.  Otherwise, a cosine zeroed in the sweep can only come back through later
+// rotations of its two columns (at most 2 k of them), each adding at most
+// fill * cosine, and the single-precision tangent leaves at most 2e-6 of a cosine
+// behind: when both stay below the tolerance, a further sweep would rotate nothing.
+__device__ __forceinline__ bool converged(int k, double tol, float cosmax, float fillmax) {
+  return cosmax == 0.0f || (2.0 * k * (double)fillmax * (double)cosmax <= tol && 2e-6 * (double)cosmax <= tol);
+}
+
+// ---------------------------------------------------------------------------
+// Columns resident in the cluster's shared memory
+// ---------------------------------------------------------------------------
+
+// CTA and slot half (0: block bi's, 1: block bj's) of block x in round r.
+__device__ __forceinline__ void block_place(int x, int r, int nb, int& cta, int& side) {
+  const int m = nb - 1;
+  int other;
+  if (x == m) {
+    cta = 0;
+    other = r;
+  } else {
+    int d = x - r;
+    if (d < 0) d += m;
+    cta = d <= m / 2 ? d : m - d;  // nb even: m / 2 = nb / 2 - 1 pairs beside the fixed player's
+    if (d == 0) {
+      other = m;
+    } else {
+      other = 2 * r - x;
+      if (other < 0) other += m;
+      if (other >= m) other -= m;
+    }
+  }
+  side = x < other ? 0 : 1;
+}
+
+__device__ __forceinline__ uint32_t remote_smem(const void* p, int rank) {
+  uint32_t a = (uint32_t)__cvta_generic_to_shared(p), o;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(o) : "r"(a), "r"(rank));
+  return o;
+}
+__device__ __forceinline__ void st_remote(uint32_t a, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void st_remote(uint32_t a, int v) {
+  asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
+// Columns per block and stride of a stored column.
+__host__ __device__ __forceinline__ int ring_width(int k, int cl) { return (k + 2 * cl - 1) / (2 * cl); }
+__host__ __device__ constexpr int ring_stride(int rows, bool acc, int g) {
+  return rows * (acc ? 2 : 1) + (g == 8 ? 8 : 4);
+}
+
+// G lanes per column, PW elements of W (and of J, ACC) each (columns padded with
+// zeros to G PW rows, so that every loop has a constant length); NW warps own
+// 32 / G columns each.
+template <int G, int PW, int NW, bool ACC>
+__global__ void __launch_bounds__(NW * 32, 1)
+    jacobi_ring_kernel(const SvdJob* __restrict__ jobs, double* __restrict__ work, const int64_t* __restrict__ work_off,
+                       int32_t* __restrict__ status, int cl) {
+  constexpr int PP = 32 / G, PJ = ACC ? PW : 1, kSlots = 2 * NW * PP, kp = G * PW, ls = ring_stride(kp, ACC, G);
+  constexpr int kCopy = ((ACC ? 2 : 1) * kp + 31) / 32;  // elements of a whole column per lane
+  const int rank = (int)(blockIdx.x % cl);
+  const SvdJob S = jobs[blockIdx.x / cl];
+  const int k = (int)S.k;
+  const int64_t ldw = S.m > S.n ? S.m : S.n;
+  if (k == 0) return;
+  const FacWork f = fac_work(work + work_off[blockIdx.x / cl], ldw, k);
+  extern __shared__ __align__(16) double sm[];
+  __shared__ double s_nrm[2][kSlots], s_d[kSlots], s_id[kSlots], part[32];
+  __shared__ int s_max[2][16][2], s_cos, s_fill;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int gl = lane % G, owner = warp * PP + lane / G;
+  const int w = ring_width(k, cl), set_len = 2 * w * ls;
+  int nb = (k + w - 1) / w;
+  nb = nb < 2 ? 2 : (nb + 1) & ~1;
+  const bool active = rank < nb / 2;
+  auto bsize = [&](int b) {
+    const int n = k - b * w;
+    return n < 0 ? 0 : n < w ? n : w;
+  };
+  Thresholds th;
+  const double tol = make_thresholds(f, ldw, k, rank, cl, part, th);
+
+  // The first round's pair of blocks from the scratch, J = I.
+  int bi = 0, bj = 0;
+  if (active) {
+    tournament_pair(0, rank, nb, bi, bj);
+    for (int c = warp; c < 2 * w; c += NW) {
+      const int g = c < w ? bi * w + c : bj * w + c - w;
+      if (c < w ? c >= bsize(bi) : c - w >= bsize(bj)) continue;
+      double* d = sm + (int64_t)c * ls;
+      for (int x = lane; x < kp; x += 32) {
+        d[x] = x < k ? __ldcg(f.W + (int64_t)g * ldw + x) : 0.0;
+        if (ACC) d[kp + x] = x == g ? 1.0 : 0.0;
+      }
+    }
+  }
+  if (cl > 1) cluster_barrier(cl);  // every CTA has started (its shared memory can be written) before the first exchange
+  __syncthreads();
+
+  int set = 0, sweep = 0;
+  for (; sweep < kMaxSweeps && k > 1; ++sweep) {
+    float cosmax = 0.0f, fillmax = 0.0f;
+    if (tid == 0) {
+      s_cos = 0;
+      s_fill = 0;
+    }
+    for (int t = 0; t < nb - 1; ++t) {
+      if (active) {
+        tournament_pair(t, rank, nb, bi, bj);
+        const int np = bsize(bi), nq = bsize(bj);
+        double* C = sm + set * set_len;
+        double* Q = C + w * ls;
+        const Columns col{s_nrm[set], s_d, s_id};
+        if (t == 0)
+          for (int c = warp; c < 2 * w; c += NW) {
+            if (c < w ? c >= np : c - w >= nq) continue;
+            double s = 0.0;
+            for (int x = lane; x < kp; x += 32) s = fma(C[c * ls + x], C[c * ls + x], s);
+            s = warp_sum(s);
+            if (lane == 0) col.nrm[c] = s;
+          }
+        for (int c = tid; c < 2 * w; c += NW * 32) s_d[c] = s_id[c] = 1.0;
+        __syncthreads();
+        if (t == 0) rotate_within<G, PW, PJ, NW, true>(C, ls, w, np, nq, col, ACC, th, cosmax, fillmax);
+        // Cross pairs: G lanes keep column `owner` of block bi in registers.
+        double p[PW], pj[PJ];
+        const bool own = owner < np;
+        const double* po = C + (own ? owner : 0) * ls + gl;  // others load a column they never use
+#pragma unroll
+        for (int j = 0; j < PW; ++j) {
+          p[j] = po[G * j];
+          if constexpr (ACC) pj[j] = po[kp + G * j];
+        }
+        double al = own ? col.nrm[owner] : 0.0, dp = own ? s_d[owner] : 1.0, idp = own ? s_id[owner] : 1.0;
+        __syncthreads();
+        for (int r = 0; r < w; ++r) {
+          int jq = owner + r;
+          if (jq >= w) jq -= w;
+          const bool live = own && jq < nq;
+          double* q = Q + (live ? jq : 0) * ls + gl;
+          double ga = 0.0, gb = 0.0, qv[PW], qj[PJ];
+#pragma unroll
+          for (int j = 0; j < PW; ++j) {
+            qv[j] = q[G * j];
+            if (j & 1) gb = fma(p[j], qv[j], gb);
+            else ga = fma(p[j], qv[j], ga);
+          }
+          const double be = live ? col.nrm[w + jq] : 0.0, dq = live ? s_d[w + jq] : 1.0, idq = live ? s_id[w + jq] : 1.0;
+          if constexpr (ACC)
+#pragma unroll
+            for (int j = 0; j < PW; ++j) qj[j] = q[kp + G * j];
+          const double dd = dp * dq;
+          ga = group_sum<G>(ga + gb) * dd;
+          Rotation R;
+          if (live && rotation(al, be, ga, th, R, cosmax, fillmax)) {
+            const double a = -R.t * (dq * idp), b = R.t * (dp * idq);
+#pragma unroll
+            for (int j = 0; j < PW; ++j) {
+              const double u = p[j];
+              p[j] = fma(a, qv[j], u);
+              q[G * j] = fma(b, u, qv[j]);
+            }
+            if constexpr (ACC)
+#pragma unroll
+              for (int j = 0; j < PW; ++j) {
+                const double u = pj[j];
+                pj[j] = fma(a, qj[j], u);
+                q[kp + G * j] = fma(b, u, qj[j]);
+              }
+            al -= R.tg;
+            dp *= R.c;
+            idp *= R.ic;
+            if (gl == 0) {
+              col.nrm[w + jq] = be + R.tg;
+              s_d[w + jq] = dq * R.c;
+              s_id[w + jq] = idq * R.ic;
+            }
+          }
+          __syncthreads();
+        }
+        // On to the next round's places, scales taken out.
+        int ci = 0, si = 0, cj = 0, sj = 1;
+        if (cl > 1) {
+          const int tn = t + 1 < nb - 1 ? t + 1 : 0;
+          block_place(bi, tn, nb, ci, si);
+          block_place(bj, tn, nb, cj, sj);
+        }
+        double* N = sm + (cl > 1 ? (set ^ 1) * set_len : 0);
+        double* nn = s_nrm[cl > 1 ? set ^ 1 : 0];
+        if (own) {
+          const int slot = si * w + owner;
+          const uint32_t a = remote_smem(N + slot * ls + gl, ci);
+#pragma unroll
+          for (int j = 0; j < PW; ++j) {
+            st_remote(a + 8 * G * j, dp * p[j]);
+            if constexpr (ACC) st_remote(a + 8 * (kp + G * j), dp * pj[j]);
+          }
+          if (gl == 0) st_remote(remote_smem(nn + slot, ci), al);
+        }
+        for (int c = warp; c < nq; c += NW) {
+          const double d = s_d[w + c];
+          const int slot = sj * w + c;
+          const uint32_t a = remote_smem(N + slot * ls, cj);
+          double v[kCopy];
+#pragma unroll
+          for (int i = 0; i < kCopy; ++i)
+            if (lane + 32 * i < (ACC ? 2 : 1) * kp) v[i] = d * Q[c * ls + lane + 32 * i];
+#pragma unroll
+          for (int i = 0; i < kCopy; ++i)
+            if (lane + 32 * i < (ACC ? 2 : 1) * kp) st_remote(a + 8 * (lane + 32 * i), v[i]);
+          if (lane == 0 && cl > 1) st_remote(remote_smem(nn + slot, cj), col.nrm[w + c]);
+        }
+      }
+      if (t == nb - 2) {  // the sweep's largest values, to every CTA
+        const int wc = __reduce_max_sync(0xffffffffu, __float_as_int(cosmax));  // non-negative: ordered like their bits
+        const int wf = __reduce_max_sync(0xffffffffu, __float_as_int(fillmax));
+        if (lane == 0) {
+          atomicMax(&s_cos, wc);
+          atomicMax(&s_fill, wf);
+        }
+        __syncthreads();
+        if (tid < cl) {
+          st_remote(remote_smem(&s_max[sweep & 1][rank][0], tid), s_cos);
+          st_remote(remote_smem(&s_max[sweep & 1][rank][1], tid), s_fill);
+        }
+      }
+      cluster_barrier(cl);
+      if (cl > 1) set ^= 1;
+    }
+    int mc = 0, mf = 0;
+    for (int i = 0; i < cl; ++i) {
+      mc = max(mc, s_max[sweep & 1][i][0]);
+      mf = max(mf, s_max[sweep & 1][i][1]);
+    }
+    __syncthreads();  // s_cos and s_fill are cleared next
+    if (converged(k, tol, __int_as_float(mc), __int_as_float(mf))) {
+      ++sweep;
+      break;
+    }
+  }
+  if (rank == 0 && tid == 0) {
+    if (sweep == kMaxSweeps) atomicOr(status, 1);
+    atomicMax(status + 1, sweep);
+  }
+  // Columns, norms and J (eigh: the normalised columns) back to the scratch.
+  if (active) {
+    tournament_pair(0, rank, nb, bi, bj);
+    for (int c = warp; c < 2 * w; c += NW) {
+      const int g = c < w ? bi * w + c : bj * w + c - w;
+      if (c < w ? c >= bsize(bi) : c - w >= bsize(bj)) continue;
+      const double* d = sm + set * set_len + (int64_t)c * ls;
+      double s = 0.0;
+      for (int x = lane; x < k; x += 32) s = fma(d[x], d[x], s);
+      s = sqrt(warp_sum(s));
+      if (lane == 0) f.sv[g] = s;
+      for (int x = lane; x < k; x += 32) {
+        if (ACC) f.W[(int64_t)g * ldw + x] = d[x];
+        f.J[(int64_t)g * k + x] = ACC ? d[kp + x] : d[x] / s;
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Columns staged through L2
+// ---------------------------------------------------------------------------
 
 // Columns of blocks bi and bj of J times the accumulated rotations: J[:, cols] <-
 // J[:, cols] Z, rows split over the warps in strips of 8 (a strip is read whole
@@ -183,14 +559,16 @@ __device__ __forceinline__ void apply_z(double* J, int k, int w, int p0, int np,
   }
 }
 
-// G lanes per column, at most PW elements of W and ZR / G of the accumulator each;
-// NW warps own 32 / G columns each; HOLD: the passing column stays in registers
-// between its dot product and its update.
-template <int G, int PW, int ZR, int NW, bool HOLD>
+// One warp per column, at most PW elements of W (pw of them used) and ZR / 32 of the
+// accumulator per lane; HOLD: the passing column stays in registers between its
+// dot product and its update.  (Two columns of block bi per warp, which reads and
+// writes a passing column once for two rotations, measured slower: 2570 cycles a
+// round at k = 400 against 2 x 1190, and it spills from k = 576 on.)
+template <int PW, int ZR, int NW, bool HOLD>
 __global__ void __launch_bounds__(NW * 32, 1)
     jacobi_kernel(const SvdJob* __restrict__ jobs, double* __restrict__ work, const int64_t* __restrict__ work_off,
                   int32_t* __restrict__ status, int cl, int acc) {
-  constexpr int PP = 32 / G, PZ = ZR / G;
+  constexpr int PZ = ZR / 32, kp = 32 * PW, ls = col_stride(kp, ZR);
   const int rank = (int)(blockIdx.x % cl);
   const SvdJob S = jobs[blockIdx.x / cl];
   const int k = (int)S.k;
@@ -202,50 +580,24 @@ __global__ void __launch_bounds__(NW * 32, 1)
   double* J = f.J;
   int* words = reinterpret_cast<int*>(f.meta + 4);  // per sweep parity: cosine, fill (float bits)
   extern __shared__ __align__(16) double sm[];
-  __shared__ double nrm[ZR];
+  __shared__ double nrm[ZR], s_d[ZR], s_id[ZR];
   __shared__ double part[32];
   __shared__ int s_cos, s_fill;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int gl = lane % G, owner = warp * PP + lane / G;
   int w, nb;
-  block_split(k, cl, NW * PP, ZR, G, w, nb);
-  const int kp = (k + 31) / 32 * 32, pw = kp / G, ls = col_stride(k, ZR, G);
-  const bool resident = cl == 1 && nb == 2;  // every column stays in shared memory for all sweeps
+  block_split(k, kp, cl, NW, ZR, w, nb);
+  const int pw = (k + 31) / 32;
+  const Columns col{nrm, s_d, s_id};
   auto bsize = [&](int b) {
     const int n = k - b * w;
     return n < 0 ? 0 : n < w ? n : w;
   };
-
-  // ||W||_F^2 (the same sum in the same order in every CTA) for the thresholds,
-  // J = I, cleared reduction words.
-  for (int c = rank * NW + warp; c < k; c += cl * NW) {
-    double s = 0.0;
-    for (int x = lane; x < k; x += 32) {
-      const double v = __ldcg(W + (int64_t)c * ldw + x);
-      s = fma(v, v, s);
-      if (acc_j && !resident) J[(int64_t)c * k + x] = x == c ? 1.0 : 0.0;
-    }
-    s = warp_sum(s);
-    if (lane == 0) f.sv[c] = s;
-  }
+  if (acc_j)
+    for (int c = rank * NW + warp; c < k; c += cl * NW)
+      for (int x = lane; x < k; x += 32) J[(int64_t)c * k + x] = x == c ? 1.0 : 0.0;
   if (rank == 0 && tid < 4) words[tid] = 0;
-  cluster_barrier(cl);
-  double fs = 0.0;
-  for (int c = tid; c < k; c += NW * 32) fs += __ldcg(f.sv + c);
-  fs = warp_sum(fs);
-  if (lane == 0) part[warp] = fs;
-  __syncthreads();
-  double frob2 = 0.0;
-  for (int i = 0; i < NW; ++i) frob2 += part[i];
-  // A pair is rotated only while its cosine exceeds the rounding level of a
-  // length-k dot product and both columns stand above the rounding noise
-  // k eps ||A||_F (columns of the null space shrink to that level, and every
-  // rotation refills them with noise whose cosine is O(1)).
-  const double tol = 4.0 * sqrt((double)k) * DBL_EPSILON;
   Thresholds th;
-  th.tol = (float)tol;
-  th.noise2 = (float)(((double)k * DBL_EPSILON) * ((double)k * DBL_EPSILON) * frob2);
-  th.floor = (float)(1e-33 * frob2);  // below every gamma above the tolerance of two columns above the noise
+  const double tol = make_thresholds(f, ldw, k, rank, cl, part, th);
 
   int sweep = 0;
   for (; sweep < kMaxSweeps && k > 1; ++sweep) {
@@ -260,135 +612,127 @@ __global__ void __launch_bounds__(NW * 32, 1)
         tournament_pair(t, i, nb, bi, bj);
         const int np = bsize(bi), nq = bsize(bj), p0 = bi * w, q0 = bj * w;
         const bool within = t == 0;
-        double* Q = sm + (int64_t)w * ls;  // block bj's columns; block bi's at sm while within its own pairs
-        // Stage: block bj (and bi in the first round) in shared memory, one warp per column.
-        if (!resident || sweep == 0) {
-          for (int c = within ? warp : w + warp; c < 2 * w; c += NW) {
-            if (c < w ? c >= np : c - w >= nq) continue;
-            const double* src = W + (int64_t)(c < w ? p0 + c : q0 + c - w) * ldw;
-            double* d = sm + (int64_t)c * ls;
-            for (int x = lane; x < kp; x += 32) d[x] = x < k ? __ldcg(src + x) : 0.0;
-            if (acc_j)
-              for (int z = lane; z < ZR; z += 32) d[kp + z] = z == c ? 1.0 : 0.0;
-          }
-          __syncwarp();
-        } else {
-          __syncthreads();  // the last sweep's columns, written by other warps
-        }
+        double* Q = sm + w * ls;  // block bj's columns; block bi's at sm while within its own pairs
+        // Stage: block bj (and bi in the first round) in shared memory, one warp per
+        // column; norms on the way.
         for (int c = within ? warp : w + warp; c < 2 * w; c += NW) {
+          if (lane == 0) s_d[c] = s_id[c] = 1.0;
           if (c < w ? c >= np : c - w >= nq) continue;
-          const double* d = sm + (int64_t)c * ls;
+          const double* src = W + (int64_t)(c < w ? p0 + c : q0 + c - w) * ldw;
+          double* d = sm + c * ls;
           double s = 0.0;
-          for (int x = lane; x < kp; x += 32) s = fma(d[x], d[x], s);
+          for (int x = lane; x < kp; x += 32) {
+            const double v = x < k ? __ldcg(src + x) : 0.0;
+            d[x] = v;
+            s = fma(v, v, s);
+          }
+          if (acc_j)
+            for (int z = lane; z < ZR; z += 32) d[kp + z] = z == c ? 1.0 : 0.0;
           s = warp_sum(s);
           if (lane == 0) nrm[c] = s;
         }
         if (within) {
           __syncthreads();
-          const int n2 = (w + 1) & ~1, half = n2 / 2;
-          for (int r = 0; r < n2 - 1; ++r) {
-            for (int base = warp * PP; base < n2; base += NW * PP) {
-              const int e = base + lane / G, b = e >= half;
-              int p = 0, q = 0;
-              bool live = e < n2;
-              if (live) {
-                tournament_pair(r, b ? e - half : e, n2, p, q);
-                live = q < (b ? nq : np);
-                p += b ? w : 0;
-                q += b ? w : 0;
-              }
-              rotate_smem<G, ZR>(live, sm + (int64_t)p * ls, sm + (int64_t)q * ls, nrm + p, nrm + q, pw, acc_j, th,
-                                 cosmax, fillmax);
-            }
-            __syncthreads();
-          }
+          rotate_within<32, PW, PZ, NW, false>(sm, ls, w, np, nq, col, acc_j, th, cosmax, fillmax);
         }
-        // Cross pairs: G lanes keep column `owner` of block bi in registers.
+        // Cross pairs: warp i keeps column i of block bi in registers.
         double p[PW], pz[PZ];
-        double al = 0.0;
-        const bool own = owner < np;
+        double al = 0.0, dp = 1.0, idp = 1.0;
+        const bool own = warp < np;
         if (within) {
-          const double* d = sm + (int64_t)(own ? owner : 0) * ls + gl;
+          const double* d = sm + (own ? warp : 0) * ls + lane;
 #pragma unroll
-          for (int j = 0; j < PW; ++j) p[j] = (own && j < pw) ? d[G * j] : 0.0;
+          for (int j = 0; j < PW; ++j) p[j] = (own && j < pw) ? d[32 * j] : 0.0;
 #pragma unroll
-          for (int h = 0; h < PZ; ++h) pz[h] = (own && acc_j) ? d[kp + G * h] : 0.0;
-          al = own ? nrm[owner] : 0.0;
+          for (int h = 0; h < PZ; ++h) pz[h] = (own && acc_j) ? d[kp + 32 * h] : 0.0;
+          if (own) {
+            al = nrm[warp];
+            dp = s_d[warp];
+            idp = s_id[warp];
+          }
         } else {
-          const double* d = W + (int64_t)(p0 + (own ? owner : 0)) * ldw;
+          const double* d = W + (int64_t)(p0 + (own ? warp : 0)) * ldw;
 #pragma unroll
           for (int j = 0; j < PW; ++j) {
-            p[j] = (own && gl + G * j < k) ? __ldcg(d + gl + G * j) : 0.0;
+            p[j] = (own && lane + 32 * j < k) ? __ldcg(d + lane + 32 * j) : 0.0;
             al = fma(p[j], p[j], al);
           }
-          al = group_sum<G>(al);
+          al = warp_sum(al);
 #pragma unroll
-          for (int h = 0; h < PZ; ++h) pz[h] = gl + G * h == owner ? 1.0 : 0.0;  // accumulator row of a block-bi column
+          for (int h = 0; h < PZ; ++h) pz[h] = lane + 32 * h == warp ? 1.0 : 0.0;  // accumulator row of a block-bi column
         }
         __syncthreads();
         for (int r = 0; r < w; ++r) {
-          int jq = owner + r;
+          int jq = warp + r;
           if (jq >= w) jq -= w;
-          const bool live = own && jq < nq;
-          double* q = Q + (int64_t)(live ? jq : 0) * ls + gl;
-          double ga = 0.0, gb = 0.0;
-          double qv[HOLD ? PW : 1];
+          if (own && jq < nq) {
+            double* q = Q + jq * ls + lane;
+            double ga = 0.0, gb = 0.0;
+            double qv[HOLD ? PW : 1];
 #pragma unroll
-          for (int j = 0; j < PW; ++j) {
-            const double v = (j < pw && live) ? q[G * j] : 0.0;
-            if constexpr (HOLD) qv[j] = v;
-            if (j & 1) gb = fma(p[j], v, gb);
-            else ga = fma(p[j], v, ga);
-          }
-          const double be = live ? nrm[w + jq] : 0.0;
-          ga = group_sum<G>(ga + gb);
-          Rotation R;
-          if (live && rotation(al, be, ga, th, R, cosmax, fillmax)) {
-            if constexpr (!HOLD) asm volatile("" ::: "memory");  // read q again: holding it would spill
+            for (int j = 0; j < PW; ++j) {
+              const double v = j < pw ? q[32 * j] : 0.0;
+              if constexpr (HOLD) qv[j] = v;
+              if (j & 1) gb = fma(p[j], v, gb);
+              else ga = fma(p[j], v, ga);
+            }
+            const double be = nrm[w + jq], dq = s_d[w + jq], idq = s_id[w + jq];
+            ga = warp_sum(ga + gb) * (dp * dq);
+            Rotation R;
+            if (rotation(al, be, ga, th, R, cosmax, fillmax)) {
+              const double a = -R.t * (dq * idp), b = R.t * (dp * idq);
+              if constexpr (!HOLD) asm volatile("" ::: "memory");  // read q again: holding it would spill
 #pragma unroll
-            for (int j = 0; j < PW; ++j)
-              if (j < pw) {
-                const double u = p[j], v = HOLD ? qv[HOLD ? j : 0] : q[G * j];
-                p[j] = R.c * u - R.s * v;
-                q[G * j] = R.s * u + R.c * v;
+              for (int j = 0; j < PW; ++j)
+                if (j < pw) {
+                  const double u = p[j], v = HOLD ? qv[HOLD ? j : 0] : q[32 * j];
+                  p[j] = fma(a, v, u);
+                  q[32 * j] = fma(b, u, v);
+                }
+              if (acc_j) {
+#pragma unroll
+                for (int h = 0; h < PZ; ++h) {
+                  const double u = pz[h], v = q[kp + 32 * h];
+                  pz[h] = fma(a, v, u);
+                  q[kp + 32 * h] = fma(b, u, v);
+                }
               }
-            if (acc_j) {
-#pragma unroll
-              for (int h = 0; h < PZ; ++h) {
-                const double u = pz[h], v = q[kp + G * h];
-                pz[h] = R.c * u - R.s * v;
-                q[kp + G * h] = R.s * u + R.c * v;
+              al -= R.tg;
+              dp *= R.c;
+              idp *= R.ic;
+              if (lane == 0) {
+                nrm[w + jq] = be + R.tg;
+                s_d[w + jq] = dq * R.c;
+                s_id[w + jq] = idq * R.ic;
               }
             }
-            al -= R.tg;
-            if (gl == 0) nrm[w + jq] = be + R.tg;
           }
           __syncthreads();
         }
-        // Back: block bi from registers, block bj from shared memory.
+        // Back, scales taken out: block bi from registers, block bj from shared memory.
         if (own) {
-          double* z = sm + (int64_t)owner * ls + gl;
-          double* d = resident ? z : W + (int64_t)(p0 + owner) * ldw + gl;
+          double* d = W + (int64_t)(p0 + warp) * ldw;
 #pragma unroll
           for (int j = 0; j < PW; ++j)
-            if (gl + G * j < (resident ? kp : k)) d[G * j] = p[j];
+            if (lane + 32 * j < k) d[lane + 32 * j] = dp * p[j];
           if (acc_j)
 #pragma unroll
-            for (int h = 0; h < PZ; ++h) z[kp + G * h] = pz[h];
+            for (int h = 0; h < PZ; ++h) sm[warp * ls + kp + 32 * h + lane] = dp * pz[h];
         }
-        if (!resident) {
-          for (int c = warp; c < nq; c += NW) {
-            const double* d = Q + (int64_t)c * ls;
-            for (int x = lane; x < k; x += 32) W[(int64_t)(q0 + c) * ldw + x] = d[x];
-          }
-          if (acc_j) {
-            __syncthreads();
-            apply_z<ZR>(J, k, w, p0, np, q0, nq, sm + kp, ls);
-          }
-          __syncthreads();  // the staging area is reused by the next pair
+        for (int c = warp; c < nq; c += NW) {
+          double* d = Q + c * ls;
+          const double dq = s_d[w + c];
+          for (int x = lane; x < k; x += 32) W[(int64_t)(q0 + c) * ldw + x] = dq * d[x];
+          if (acc_j)
+            for (int z = lane; z < ZR; z += 32) d[kp + z] *= dq;
         }
+        if (acc_j) {
+          __syncthreads();
+          apply_z<ZR>(J, k, w, p0, np, q0, nq, sm + kp, ls);
+        }
+        __syncthreads();  // the staging area is reused by the next pair
       }
-      if (cl > 1) cluster_barrier(cl);
+      cluster_barrier(cl);
     }
     // The sweep's largest cosine before rotation and largest fill factor, over the cluster.
     const int wc = __reduce_max_sync(0xffffffffu, __float_as_int(cosmax));  // non-negative: ordered like their bits
@@ -399,30 +743,19 @@ __global__ void __launch_bounds__(NW * 32, 1)
     }
     __syncthreads();
     int* wd = words + 2 * (sweep & 1);
-    if (cl > 1) {
-      if (tid == 0) {
-        atomicMax(wd, s_cos);
-        atomicMax(wd + 1, s_fill);
-        if (rank == 0) {  // the other parity's words: last read before the previous barrier
-          words[2 * ((sweep & 1) ^ 1)] = 0;
-          words[2 * ((sweep & 1) ^ 1) + 1] = 0;
-        }
+    if (tid == 0) {
+      atomicMax(wd, s_cos);
+      atomicMax(wd + 1, s_fill);
+      if (rank == 0) {  // the other parity's words: last read before the previous barrier
+        words[2 * ((sweep & 1) ^ 1)] = 0;
+        words[2 * ((sweep & 1) ^ 1) + 1] = 0;
       }
-      cluster_barrier(cl);
-      cosmax = __int_as_float(__ldcg(wd));
-      fillmax = __int_as_float(__ldcg(wd + 1));
-      cluster_barrier(cl);  // read by all before the next sweep clears or adds
-    } else {
-      cosmax = __int_as_float(s_cos);
-      fillmax = __int_as_float(s_fill);
-      __syncthreads();
     }
-    // No pair above the tolerance: done.  Otherwise, a cosine zeroed in this
-    // sweep can only come back through later rotations of its two columns (at most
-    // 2 k of them), each adding at most fill * cosine, and the single-precision
-    // tangent leaves at most 2e-6 of a cosine behind: when both stay below the
-    // tolerance, a further sweep would rotate nothing.
-    if (cosmax == 0.0f || (2.0 * k * (double)fillmax * (double)cosmax <= tol && 2e-6 * (double)cosmax <= tol)) {
+    cluster_barrier(cl);
+    cosmax = __int_as_float(__ldcg(wd));
+    fillmax = __int_as_float(__ldcg(wd + 1));
+    cluster_barrier(cl);  // read by all before the next sweep clears or adds
+    if (converged(k, tol, cosmax, fillmax)) {
       ++sweep;
       break;
     }
@@ -430,16 +763,6 @@ __global__ void __launch_bounds__(NW * 32, 1)
   if (rank == 0 && tid == 0) {
     if (sweep == kMaxSweeps) atomicOr(status, 1);
     atomicMax(status + 1, sweep);
-  }
-  if (resident) {
-    for (int c = warp; c < k; c += NW) {
-      const double* d = sm + (int64_t)c * ls;  // column c sits in slot c: bi = 0 fills slots 0 .. w - 1
-      if (k > 1)
-        for (int x = lane; x < k; x += 32) W[(int64_t)c * ldw + x] = d[x];
-      if (acc_j)
-        for (int z = lane; z < k; z += 32) J[(int64_t)c * k + z] = k > 1 ? d[kp + z] : 1.0;
-    }
-    __syncthreads();
   }
   for (int c = rank * NW + warp; c < k; c += cl * NW) {
     double s = 0.0;
@@ -454,19 +777,9 @@ __global__ void __launch_bounds__(NW * 32, 1)
   }
 }
 
-template <int G, int PW, int ZR, int NW, bool HOLD>
-cudaError_t launch_class(const SvdJob* jobs, int32_t njobs, int64_t max_k, double* work, const int64_t* work_off,
-                         int32_t* status, int cl, int acc, cudaStream_t st) {
-  // Single-CTA sectors take what they need (w and the stride grow with k), so
-  // several fit an SM; clusters take the whole staging area.
-  size_t smem = kJacobiSmem;
-  if (cl == 1) {
-    int w, nb;
-    block_split((int)max_k, cl, NW * (32 / G), ZR, G, w, nb);
-    smem = (size_t)2 * w * col_stride((int)max_k, ZR, G) * sizeof(double);
-  }
-  auto fn = jacobi_kernel<G, PW, ZR, NW, HOLD>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kJacobiSmem);
+template <class F, class... A>
+cudaError_t launch_cluster(F fn, int njobs, int cl, int threads, size_t smem, cudaStream_t st, A... args) {
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   if (cl > 8) {
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -474,7 +787,7 @@ cudaError_t launch_class(const SvdJob* jobs, int32_t njobs, int64_t max_k, doubl
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(njobs * cl));
-  cfg.blockDim = dim3(NW * 32);
+  cfg.blockDim = dim3((unsigned)threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
@@ -484,7 +797,7 @@ cudaError_t launch_class(const SvdJob* jobs, int32_t njobs, int64_t max_k, doubl
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, fn, jobs, work, work_off, status, cl, acc);
+  return cudaLaunchKernelEx(&cfg, fn, args...);
 }
 
 // ---------------------------------------------------------------------------
@@ -820,30 +1133,51 @@ __global__ void __launch_bounds__(kFinishWarps * 32)
 
 }  // namespace
 
-// CTAs per sector for a largest k of the launch: one while every column fits an
-// SM's shared memory and a round is a single wave of rotations (k <= 64),
-// then clusters that keep blocks at about 16 columns.  A round costs its latency
-// whatever the width, and a sweep takes k rounds plus an exchange per block pair,
-// so wider clusters only add exchanges.
+// CTAs per sector for a largest k of the launch: one while a round is a single
+// wave of rotations on one SM (k <= 64), four while it is a few, then as many as
+// the device can co-schedule.  A round costs its latency whatever the width, and
+// a sweep takes k rounds plus an exchange per block pair, so wider clusters
+// add exchanges where they no longer shorten the rounds.
 int jacobi_cluster(int64_t k) {
   const int wide = svd_wide_cluster_size() > 0 ? 16 : 8;
-  return k <= 64 ? 1 : k <= 128 ? 4 : k <= 256 ? 8 : wide;
+  return k <= 64 ? 1 : k <= 128 ? 4 : wide;
 }
 
 cudaError_t launch_jacobi(const SvdJob* jobs, int32_t njobs, int64_t max_k, double* work, const int64_t* work_off,
                           int32_t* status, bool acc_j, cudaStream_t st) {
   if (njobs == 0) return cudaSuccess;
   const int cl = jacobi_cluster(max_k);
-  const int a = acc_j ? 1 : 0;
-  auto go = [&](auto fn) { return fn(jobs, njobs, max_k, work, work_off, status, cl, a, st); };
-  if (max_k <= 32) return go(launch_class<8, 4, 32, 4, true>);
-  if (max_k <= 64) return go(launch_class<8, 8, 64, 8, true>);
-  if (max_k <= 128) return go(launch_class<16, 8, 32, 8, true>);
-  if (max_k <= 256) return go(launch_class<32, 8, 32, 16, true>);
-  if (max_k <= 512) return go(launch_class<32, 16, 32, 16, true>);
-  if (max_k <= 608) return go(launch_class<32, 19, 64, 19, false>);
-  if (max_k <= 1024) return go(launch_class<32, 32, 32, 12, false>);
-  return go(launch_class<32, 48, 32, 8, false>);
+  const int k = (int)max_k;
+#define TNT_RING(g, pw, nw)                                                                                          \
+  if (k <= g * pw) {                                                                                                 \
+    const size_t smem = (size_t)(cl > 1 ? 4 : 2) * ring_width(k, cl) * ring_stride(g * pw, acc_j, g) * sizeof(double); \
+    return acc_j ? launch_cluster(jacobi_ring_kernel<g, pw, nw, true>, njobs, cl, nw * 32, smem, st, jobs, work,      \
+                                  work_off, status, cl)                                                              \
+                 : launch_cluster(jacobi_ring_kernel<g, pw, nw, false>, njobs, cl, nw * 32, smem, st, jobs, work,     \
+                                  work_off, status, cl);                                                             \
+  }
+#define TNT_RING_EIGH(g, pw, nw)                                                                                     \
+  if (k <= g * pw && !acc_j)                                                                                         \
+    return launch_cluster(jacobi_ring_kernel<g, pw, nw, false>, njobs, cl, nw * 32,                                  \
+                          (size_t)4 * ring_width(k, cl) * ring_stride(g * pw, false, g) * sizeof(double), st, jobs,  \
+                          work, work_off, status, cl);
+#define TNT_STAGED(pw, zr, nw, hold)                                                                                  \
+  if (k <= 32 * pw)                                                                                                  \
+    return launch_cluster(jacobi_kernel<pw, zr, nw, hold>, njobs, cl, nw * 32, kJacobiSmem, st, jobs, work, work_off,  \
+                          status, cl, acc_j ? 1 : 0);
+  // Ring widths grow with k, so the largest sector's need covers the launch.
+  TNT_RING(8, 2, 2) TNT_RING(8, 4, 4) TNT_RING(8, 6, 6) TNT_RING(8, 8, 8)
+  TNT_RING(16, 6, 6) TNT_RING(16, 7, 7) TNT_RING(16, 8, 8)
+  if (cl == 16) {
+    TNT_RING(32, 5, 5) TNT_RING(32, 6, 6) TNT_RING(32, 7, 7) TNT_RING(32, 8, 8) TNT_RING(32, 9, 9) TNT_RING(32, 10, 10)
+    TNT_RING_EIGH(32, 12, 12) TNT_RING_EIGH(32, 14, 14)
+  }
+  TNT_STAGED(12, 32, 16, true) TNT_STAGED(14, 32, 16, true) TNT_STAGED(16, 32, 16, true)
+  TNT_STAGED(19, 64, 19, false) TNT_STAGED(24, 32, 15, false) TNT_STAGED(32, 32, 12, false) TNT_STAGED(48, 32, 8, false)
+  return cudaErrorInvalidValue;
+#undef TNT_RING
+#undef TNT_RING_EIGH
+#undef TNT_STAGED
 }
 
 cudaError_t launch_svd_finish(const SvdJob* jobs, int32_t njobs, int64_t max_k, double* u, double* s, double* vh,

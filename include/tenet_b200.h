@@ -274,16 +274,18 @@ tnt_status tnt_compose_packed(tnt_ctx* ctx, const tnt_cplan* plan, double* dst, 
                               const void* lhs_packed, const double* rhs, const void* rhs_packed, double alpha,
                               double beta, int32_t precision, int32_t slices, void* stream);
 
-/* Tile-shape autotuning of tnt_compose.  FP64: every coupled-sector job gets
- * one output-tile shape (0: 64x64, 1: 64x32, 2: 32x64, 3: 32x32) minimising
- * ntiles * (ceil(k/16) + 1) * cost[shape]; split precision: tile width 64 or
+/* Tile-shape autotuning of tnt_compose.  FP64: sectors are cut into equal tiles
+ * of at most 32, 48, 64 or 80 a side, chosen per plan and batch count from a cost
+ * per tile and k-tile, g + b * (16 x 16 blocks); split precision: tile width 64 or
  * 128 from the per-MAC throughput ratio eff64.  The per-device costs are
  * measured on the first compose with beta == 0, at least 2e8 flops and no
  * stream capture in progress (it times each candidate on the caller's own
  * operands, so make that call before any capture); TNT_AUTOTUNE=0 keeps the
  * model defaults.  No counterpart in the reference (per-sector GEMM calls).
- * tnt_cplan_tile_shapes: the per-job shapes for the given four costs;
- * tnt_tuning_info: the device's current costs and calibration state. */
+ * tnt_tuning_info: the device's calibration state, with g and b as the costs of
+ * the uniform shapes 64x64, 64x32, 32x64, 32x32; tnt_cplan_tile_shapes: the
+ * per-job shape (0 .. 3) minimising ntiles * (ceil(k/16) + 1) * cost[shape] for
+ * four given costs. */
 tnt_status tnt_cplan_tile_shapes(const tnt_cplan* plan, const double* costs, int32_t* shapes);
 tnt_status tnt_tuning_info(int32_t device, double* f64_costs, int32_t* f64_calibrated, double* split_eff64,
                            int32_t* split_calibrated);

@@ -1188,37 +1188,49 @@ std::pair<GemmTile*, int32_t> f64_tiles(tnt_cplan_s* plan, const ComposeArgs& x,
     jobs_dev = c.jobs;
   }
   const std::vector<GemmJob>& jobs = plan->p->tables.jobs;
-  double cost[4];
+  double g, b;
   bool calibrated;
   {
-    std::lock_guard<std::mutex> g(tuning_mutex());
+    std::lock_guard<std::mutex> lock(tuning_mutex());
     DeviceTuning& T = device_tuning(d);
-    std::copy(T.f64_cost, T.f64_cost + 4, cost);
+    g = T.f64_g;
+    b = T.f64_b;
     calibrated = T.f64_calibrated;
   }
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d);
   if (!calibrated && can_calibrate(plan, x.nbatch, x.beta, st)) {
-    double measured[4];
-    for (int s = 0; s < 4; ++s) {
-      std::vector<int32_t> uniform(jobs.size(), s);
-      std::vector<GemmTile> tv = build_f64_tiles(jobs, x.nbatch, uniform, cost);
+    double ms[2], kt[2], bkt[2];
+    for (int s = 0; s < 2; ++s) {
+      std::vector<GemmTile> tv = build_f64_tiles(jobs, x.nbatch, s == 0 ? 4 : 2, g, b);
       GemmTile* td = upload(tv);
-      const double ms = time_ms(st, 3, [&] {
+      ms[s] = time_ms(st, 3, [&] {
         cuda_check(launch_gemm_f64(jobs_dev, td, (int32_t)tv.size(), x.dst, x.sd, x.lhs, x.sl, x.rhs, x.sr, x.alpha,
                                    x.beta, st),
                    "fp64 grouped gemm launch");
       });
       cudaFree(td);
-      measured[s] = ms / std::max(1.0, f64_tile_units(jobs, tv));
+      f64_tile_units(jobs, tv, kt[s], bkt[s]);
     }
-    std::lock_guard<std::mutex> g(tuning_mutex());
+    // ms = (g ktiles + b block_ktiles) / sms at both caps; a fit outside the
+    // plausible range (a compose too small to fill the GPU) keeps the defaults' ratio.
+    const double det = kt[0] * bkt[1] - kt[1] * bkt[0];
+    double mg = det != 0.0 ? sms * (ms[0] * bkt[1] - ms[1] * bkt[0]) / det : 0.0;
+    double mb = det != 0.0 ? sms * (kt[0] * ms[1] - kt[1] * ms[0]) / det : 0.0;
+    if (!(mb > 0.0 && mg >= 0.5 * mb && mg <= 10.0 * mb)) {
+      mb = sms * ms[0] / std::max(1.0, (g / b) * kt[0] + bkt[0]);
+      mg = mb * (g / b);
+    }
+    std::lock_guard<std::mutex> lock(tuning_mutex());
     DeviceTuning& T = device_tuning(d);
-    std::copy(measured, measured + 4, T.f64_cost);
+    T.f64_g = g = mg;
+    T.f64_b = b = mb;
+    for (int s = 0; s < 4; ++s) T.f64_cost[s] = (g + b * (kShapeM[s] / 16) * (kShapeN[s] / 16)) / sms;
     T.f64_calibrated = true;
-    std::copy(measured, measured + 4, cost);
   }
-  std::vector<GemmTile> tv = build_f64_tiles(jobs, x.nbatch, choose_f64_shapes(jobs, cost), cost);
+  std::vector<GemmTile> tv = build_f64_tiles(jobs, x.nbatch, choose_f64_cap(jobs, x.nbatch, g, b, sms), g, b);
   std::pair<GemmTile*, int32_t> r(upload(tv), (int32_t)tv.size());
-  std::lock_guard<std::mutex> g(plan->mu);
+  std::lock_guard<std::mutex> lock(plan->mu);
   CplanDevice& c = plan->on_device(d);
   auto ins = c.f64_tiles.emplace(x.nbatch, r);
   if (!ins.second) cudaFree(r.first);  // another thread built it first

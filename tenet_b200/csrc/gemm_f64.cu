@@ -4,15 +4,24 @@
 // (tenet-operations/src/fusion_replay.rs:556) and its device twin
 // execute_direct_on_storage (fusion_replay.rs:1168-1290, one cuBLAS call per
 // sector).  Every (sector job, batch entry, output tile) is one work item of a
-// persistent kernel.  Each tile carries its shape: interior tiles take the
-// shape the autotuner picked for the sector (64x64, 64x32, 32x64 or 32x32,
-// from the block-size histogram), and the last row and column blocks of a
-// sector are trimmed to the remainder rounded up to 16, so ragged sectors
-// waste little padding.  Tiles are pre-sorted longest first so the uneven
-// sector sizes balance across the 148 SMs.  Math runs on the FP64 tensor
-// cores (mma.sync m8n8k4 f64, which reaches the same 37 TFLOP/s on B200 as
+// launch.  A sector's rows and columns are cut into equal tiles (multiples of 16, at
+// most 80 by 80); the autotuner picks the largest tile from a cost model per
+// tile and k-tile, g + b * (16 x 16 blocks), whose constants it measures: with
+// g about 3 b (barrier, copies, latency) fewer and larger tiles win wherever there
+// are enough of them to fill the GPU, smaller ones where the longest tile's
+// serial k loop would be the whole time.  Tiles are pre-sorted longest first so
+// the uneven sector sizes balance across the 148 SMs.  Math runs on the FP64
+// tensor cores (mma.sync m8n8k4 f64, which reaches the same 37 TFLOP/s on B200 as
 // the m16n8k* shapes); operands are staged through shared memory by a
-// three-deep cp.async ring.
+// three-deep cp.async ring, A with its rows and B with its k contiguous, as they
+// lie in memory (conflict-free copies and fragments both).
+//
+// Measured: the 64-compose fZ2xU1xSU2 batch 22.8 -> 24.9 TFLOP/s (64 x 64 tiles
+// with trimmed edges before), a scale-1 SU(2) effective Hamiltonian's composes 29.5
+// TFLOP/s of the 35.5 of an 8192^3 cuBLAS DGEMM. Bound by the FP64 MMA pipe (70% busy
+// on the ragged batch, 10% of it on padding) and the start and end of each tile.
+// m16n8k4 instead of m8n8k4 measured the same; leaving out the k-slices beyond K
+// in the last k-tile measured 2% slower (the branch keeps the loads from being hoisted).
 #include "kernels.cuh"
 
 namespace tnt {
@@ -20,13 +29,13 @@ namespace tnt {
 namespace {
 
 constexpr int BK = 16;
-constexpr int SP = 68;  // padded row stride in doubles: conflict-free fragment loads
+constexpr int kMaxTile = 16 * kF64MaxBlocks;
+constexpr int SA = kMaxTile + 4;  // row stride of A's k-slices in doubles: 4 mod 16, conflict-free fragments
+constexpr int SB = BK + 4;        // stride of B's columns: 4 mod 16
+constexpr int kABuf = BK * SA, kBBuf = kMaxTile * SB;
 constexpr int kThreads = 128;
 constexpr int kStages = 3;  // cp.async ring: two k-tiles in flight while one is multiplied
-// Three CTAs per SM: the 64 x 64 tile body needs 168 registers, and capping it
-// at 128 (four CTAs) spills and measured 7% slower on the 64-compose
-// fZ2xU1xSU2 batch (21.2 against 22.8 TFLOP/s).
-constexpr int kMinBlocks = 3;
+constexpr int kMinBlocks = 3;  // 168 registers: the 80 x 80 tile's 50 accumulators and its fragments
 
 __device__ __forceinline__ void cp_async8(double* smem, const double* gmem, bool pred) {
   unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -43,7 +52,7 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
                : "d"(a), "d"(b));
 }
 
-// One BM x BN output tile (BM, BN in {16, 32, 48, 64}) whose first row and
+// One BM x BN output tile (multiples of 16 up to kMaxTile) whose first row and
 // column are m0 and n0; 4 warps in a 2 x 2 layout, each computing
 // (BM/2) x (BN/2) with m8n8k4 FP64 MMAs.  K runs in BK-deep k-tiles through a
 // kStages-deep cp.async ring, one barrier per k-tile.
@@ -51,7 +60,7 @@ template <int BM, int BN>
 __device__ __forceinline__ void tile_body(const GemmJob& J, int64_t m0, int64_t n0, int32_t batch,
                                           double* __restrict__ C, int64_t sc, const double* __restrict__ A,
                                           int64_t sa, const double* __restrict__ B, int64_t sb, double alpha,
-                                          double beta, double (*As)[BK][SP], double (*Bs)[BK][SP]) {
+                                          double beta, double* As, double* Bs) {
   constexpr int WI = BM / 16, WJ = BN / 16;  // 8x8 MMA tiles per warp along M and N
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = warp >> 1, wn = warp & 1;
@@ -65,51 +74,67 @@ __device__ __forceinline__ void tile_body(const GemmJob& J, int64_t m0, int64_t 
 #pragma unroll
     for (int j = 0; j < WJ; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
+  // Copies: A's k-slices warp + 4 q (q < 4), lanes along the rows; B's k row
+  // tid % 16 of columns tid / 16 + 8 r.  One pointer each, stepped per k-tile.
   const int64_t nk = (J.k + BK - 1) / BK;
-  auto load = [&](int64_t kt, int buf) {
-    const int64_t k0 = kt * BK;
+  const int mrem = (int)(J.m - m0 < BM ? J.m - m0 : BM), nrem = (int)(J.n - n0 < BN ? J.n - n0 : BN);
+  const double* pa = a + m0 + lane + (int64_t)warp * J.lda;
+  const int bk = tid & 15, bj = tid >> 4;
+  const double* pb = b + bk + (n0 + bj) * J.ldb;
+  const int64_t sa4 = 4 * J.lda, sb8 = 8 * J.ldb;
+  int64_t kleft = J.k;  // from the k-tile loaded next on
+  auto load = [&](int buf) {
+    double* da = As + buf * kABuf + warp * SA + lane;
+    const double* q = pa;
 #pragma unroll
-    for (int r = 0; r < (BM * BK) / kThreads; ++r) {
-      int idx = tid + r * kThreads;
-      int i = idx % BM, kk = idx / BM;
-      int64_t gm = m0 + i, gk = k0 + kk;
-      bool ok = gm < J.m && gk < J.k;
-      cp_async8(&As[buf][kk][i], ok ? a + gm + gk * J.lda : a, ok);
-    }
+    for (int i = 0; i < BK / 4; ++i, q += sa4)
 #pragma unroll
-    for (int r = 0; r < (BN * BK) / kThreads; ++r) {
-      int idx = tid + r * kThreads;
-      int kk = idx % BK, j = idx / BK;
-      int64_t gn = n0 + j, gk = k0 + kk;
-      bool ok = gn < J.n && gk < J.k;
-      cp_async8(&Bs[buf][kk][j], ok ? b + gk + gn * J.ldb : b, ok);
+      for (int h = 0; h < (BM + 31) / 32; ++h) {
+        if (BM % 32 == 0 || h < BM / 32 || lane < 16) {
+          const bool ok = lane + 32 * h < mrem && warp + 4 * i < kleft;
+          cp_async8(da + 4 * i * SA + 32 * h, ok ? q + 32 * h : a, ok);
+        }
+      }
+    double* db = Bs + buf * kBBuf + bj * SB + bk;
+    const double* r = pb;
+#pragma unroll
+    for (int j = 0; j < BN / 8; ++j, r += sb8) {
+      const bool ok = bj + 8 * j < nrem && bk < kleft;
+      cp_async8(db + 8 * j * SB, ok ? r : b, ok);
     }
+    pa += BK * J.lda;
+    pb += BK;
+    kleft -= BK;
   };
 
   // Prologue: k-tiles 0 .. kStages-2 in flight (empty groups keep the count).
 #pragma unroll
   for (int s = 0; s < kStages - 1; ++s) {
-    if (s < nk) load(s, s);
+    if (s < nk) load(s);
     cp_async_commit();
   }
+  int buf = 0, nxt = kStages - 1;
   for (int64_t kt = 0; kt < nk; ++kt) {
-    const int buf = (int)(kt % kStages);
     cp_async_wait<kStages - 2>();  // k-tile kt has landed
     __syncthreads();               // ... for every thread, and k-tile kt-1's buffer is free
-    if (kt + kStages - 1 < nk) load(kt + kStages - 1, (int)((kt + kStages - 1) % kStages));
+    if (kt + kStages - 1 < nk) load(nxt);
     cp_async_commit();
+    const double* as = As + buf * kABuf + t4 * SA + wm * (BM / 2) + g;
+    const double* bs = Bs + buf * kBBuf + (wn * (BN / 2) + g) * SB + t4;
 #pragma unroll
     for (int kk = 0; kk < BK; kk += 4) {
       double af[WI], bf[WJ];
 #pragma unroll
-      for (int i = 0; i < WI; ++i) af[i] = As[buf][kk + t4][wm * (BM / 2) + i * 8 + g];
+      for (int i = 0; i < WI; ++i) af[i] = as[kk * SA + i * 8];
 #pragma unroll
-      for (int j = 0; j < WJ; ++j) bf[j] = Bs[buf][kk + t4][wn * (BN / 2) + j * 8 + g];
+      for (int j = 0; j < WJ; ++j) bf[j] = bs[j * 8 * SB + kk];
 #pragma unroll
       for (int i = 0; i < WI; ++i)
 #pragma unroll
         for (int j = 0; j < WJ; ++j) dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
     }
+    buf = buf + 1 == kStages ? 0 : buf + 1;
+    nxt = nxt + 1 == kStages ? 0 : nxt + 1;
   }
   cp_async_wait<0>();
   __syncthreads();  // the ring is reused by the CTA's next tile
@@ -135,39 +160,38 @@ __device__ __forceinline__ void tile_body(const GemmJob& J, int64_t m0, int64_t 
 template <int BM>
 __device__ __forceinline__ void tile_rows(int bn16, const GemmJob& J, int64_t m0, int64_t n0, int32_t batch,
                                           double* C, int64_t sc, const double* A, int64_t sa, const double* B,
-                                          int64_t sb, double alpha, double beta, double (*As)[BK][SP],
-                                          double (*Bs)[BK][SP]) {
+                                          int64_t sb, double alpha, double beta, double* As, double* Bs) {
   switch (bn16) {
     case 1: tile_body<BM, 16>(J, m0, n0, batch, C, sc, A, sa, B, sb, alpha, beta, As, Bs); break;
     case 2: tile_body<BM, 32>(J, m0, n0, batch, C, sc, A, sa, B, sb, alpha, beta, As, Bs); break;
     case 3: tile_body<BM, 48>(J, m0, n0, batch, C, sc, A, sa, B, sb, alpha, beta, As, Bs); break;
-    default: tile_body<BM, 64>(J, m0, n0, batch, C, sc, A, sa, B, sb, alpha, beta, As, Bs); break;
+    case 4: tile_body<BM, 64>(J, m0, n0, batch, C, sc, A, sa, B, sb, alpha, beta, As, Bs); break;
+    default: tile_body<BM, 80>(J, m0, n0, batch, C, sc, A, sa, B, sb, alpha, beta, As, Bs); break;
   }
 }
 
-// One CTA per tile.  A tile's `shape` is its geometry code
-// f64_tile_code(BM, BN) and (tm, tn) its first row and column in units of
-// 16: interior tiles have the job's chosen shape, the last row and column
-// blocks are trimmed to the remainder rounded up to 16.
+// One CTA per tile.  A tile's `shape` is its geometry code f64_tile_code(BM, BN)
+// and (tm, tn) its first row and column in units of 16.
 __global__ void __launch_bounds__(kThreads, kMinBlocks) gemm_f64_kernel(const GemmJob* __restrict__ jobs,
                                                             const GemmTile* __restrict__ tiles, int32_t ntiles,
                                                             double* __restrict__ C, int64_t sc,
                                                             const double* __restrict__ A, int64_t sa,
                                                             const double* __restrict__ B, int64_t sb, double alpha,
                                                             double beta) {
-  extern __shared__ __align__(16) double ring[];  // kStages x (A, B) k-tiles: 52 KB, above the static limit
-  auto As = reinterpret_cast<double(*)[BK][SP]>(ring);
-  auto Bs = reinterpret_cast<double(*)[BK][SP]>(ring + kStages * BK * SP);
+  extern __shared__ __align__(16) double ring[];  // kStages x (A, B) k-tiles: 70 KB
+  double* As = ring;
+  double* Bs = ring + kStages * kABuf;
   for (int32_t it = blockIdx.x; it < ntiles; it += gridDim.x) {
     const GemmTile tile = tiles[it];
     const GemmJob J = jobs[tile.job];
     const int64_t m0 = (int64_t)tile.tm * 16, n0 = (int64_t)tile.tn * 16;
-    const int bm16 = (tile.shape >> 2) + 1, bn16 = (tile.shape & 3) + 1;
+    const int bm16 = (tile.shape >> 3) + 1, bn16 = (tile.shape & 7) + 1;
     switch (bm16) {
       case 1: tile_rows<16>(bn16, J, m0, n0, tile.batch, C, sc, A, sa, B, sb, alpha, beta, As, Bs); break;
       case 2: tile_rows<32>(bn16, J, m0, n0, tile.batch, C, sc, A, sa, B, sb, alpha, beta, As, Bs); break;
       case 3: tile_rows<48>(bn16, J, m0, n0, tile.batch, C, sc, A, sa, B, sb, alpha, beta, As, Bs); break;
-      default: tile_rows<64>(bn16, J, m0, n0, tile.batch, C, sc, A, sa, B, sb, alpha, beta, As, Bs); break;
+      case 4: tile_rows<64>(bn16, J, m0, n0, tile.batch, C, sc, A, sa, B, sb, alpha, beta, As, Bs); break;
+      default: tile_rows<80>(bn16, J, m0, n0, tile.batch, C, sc, A, sa, B, sb, alpha, beta, As, Bs); break;
     }
   }
 }
@@ -186,7 +210,7 @@ cudaError_t launch_gemm_f64(const GemmJob* jobs, const GemmTile* tiles, int32_t 
   // over a fixed number of CTAs per SM measured 6-11% slower on the
   // 64-compose fZ2xU1xSU2 batch).
   int grid = ntiles;
-  constexpr size_t smem = 2 * kStages * BK * SP * sizeof(double);
+  constexpr size_t smem = kStages * (kABuf + kBBuf) * sizeof(double);
   cudaError_t e = cudaFuncSetAttribute(gemm_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   gemm_f64_kernel<<<grid, kThreads, smem, stream>>>(jobs, tiles, ntiles, c, sc, a, sa, b, sb, alpha, beta);

@@ -102,7 +102,8 @@ def lanczos(H: EffectiveHamiltonian, x0: "typed.TensorMap", iterations: int = 30
         raise ValueError("at most 48 Lanczos steps (device eigensolver limit)")
     fplan = rt.fplan(space)
     dev = x0.data.device
-    V = torch.empty((m, n), dtype=torch.float64, device=dev)
+    ld = -(-n // 32) * 32  # every vector starts on a 256-byte boundary, as an allocation would
+    V = torch.empty((m, ld), dtype=torch.float64, device=dev)
     h = torch.empty(m, dtype=torch.float64, device=dev)
     h2 = torch.empty(m, dtype=torch.float64, device=dev)
     nrm = torch.empty(1, dtype=torch.float64, device=dev)
@@ -110,26 +111,26 @@ def lanczos(H: EffectiveHamiltonian, x0: "typed.TensorMap", iterations: int = 30
     P = lambda t: C.c_void_p(t.data_ptr())
 
     def wdot(k, vecs, y, out):
-        call("tnt_wdot", rt._h, fplan._h, k, P(vecs), n, P(y), P(out), st)
+        call("tnt_wdot", rt._h, fplan._h, k, P(vecs), ld, P(y), P(out), st)
 
-    v = x0.data.clone()
-    wdot(1, v, v, nrm)
-    v /= torch.sqrt(nrm[0])
-    alphas, betas = [], []
+    # Nothing on the host waits for the device before the tridiagonal matrix is
+    # complete: coefficients stay in device arrays, vectors in their rows of V.
+    alpha_d = torch.empty(m, dtype=torch.float64, device=dev)
+    beta_d = torch.empty(m, dtype=torch.float64, device=dev)
+    wdot(1, x0.data, x0.data, nrm)
+    torch.div(x0.data.detach(), torch.sqrt(nrm), out=V[0, :n])
     for j in range(m):
-        V[j].copy_(v)
-        w = H.apply(typed.TensorMap(rt, space, V[j].clone()), precision, slices).data
+        w = H.apply(typed.TensorMap(rt, space, V[j, :n]), precision, slices).data
         for hv in (h, h2):  # classical Gram-Schmidt, twice
             wdot(j + 1, V, w, hv)
             neg = -hv[: j + 1]
-            call("tnt_axpy_many", rt._h, n, j + 1, P(V), n, P(neg), 1.0, None, P(w), st)
-        alpha = float(h[j] + h2[j])
+            call("tnt_axpy_many", rt._h, n, j + 1, P(V), ld, P(neg), 1.0, None, P(w), st)
+        torch.add(h[j], h2[j], out=alpha_d[j])
         wdot(1, w, w, nrm)
-        beta = float(torch.sqrt(nrm[0]))
-        alphas.append(alpha)
-        betas.append(beta)
+        torch.sqrt(nrm[0], out=beta_d[j])
         if j + 1 < m:
-            v = w / beta
+            torch.div(w, beta_d[j], out=V[j + 1, :n])
+    alphas, betas = alpha_d.cpu().tolist(), beta_d.cpu().tolist()
     T = np.diag(alphas) + np.diag(betas[:-1], 1) + np.diag(betas[:-1], -1)
     Td = torch.as_tensor(np.asfortranarray(T).ravel(order="F"), device=dev)
     evals = torch.empty(m, dtype=torch.float64, device=dev)
@@ -137,7 +138,7 @@ def lanczos(H: EffectiveHamiltonian, x0: "typed.TensorMap", iterations: int = 30
     call("tnt_symeig", rt._h, m, P(Td), P(evals), P(evecs), st)
     c0 = evecs[:m].contiguous()
     ritz = torch.zeros(n, dtype=torch.float64, device=dev)
-    call("tnt_axpy_many", rt._h, n, m, P(V), n, P(c0), 0.0, None, P(ritz), st)
+    call("tnt_axpy_many", rt._h, n, m, P(V), ld, P(c0), 0.0, None, P(ritz), st)
     return float(evals[0]), typed.TensorMap(rt, space, ritz), alphas, betas
 
 

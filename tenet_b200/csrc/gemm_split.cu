@@ -40,9 +40,18 @@
 // bulk copy (cp.async.bulk, no tensor map, no multicast) and the UMMA
 // shared-memory descriptors use the SWIZZLE_64B K-major canonical layout.
 // Warp roles per CTA (one 128 x TN output tile at a time): warp 0 issues the
-// copies, warp 1 owns TMEM and issues tcgen05.mma from one thread, warps 2-9
-// drain the accumulators (two warps per TMEM lane quarter, one per half of
-// the columns) and write C.
+// copies, warp 1 owns TMEM and issues tcgen05.mma from one thread, warps 2-17
+// drain the accumulators (four warps per TMEM lane quarter, one per quarter of
+// the columns) and write C, warp 18 lays out what they need of the next tile.
+//
+// What bounds it (int8, S = 5): shared memory.  A 64-deep K block is 60 KB
+// written by the copies and 108 KB read by the MMAs, 1310 cycles at 128 bytes a
+// cycle against 960 of tensor work; 1170 - 1390 are measured, plus some 1700 per
+// tile to hand the accumulators over.  64 Hubbard composes (237 tiles of four K
+// blocks per SM): 1435 -> 1094 us; the effective-Hamiltonian products: 1395 ->
+// 1210 us, before and after 16 epilogue warps, their records laid out ahead, the
+// copies issued by 2 S lanes, and rows, columns and half K blocks of padding
+// left out.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -60,8 +69,9 @@ constexpr int TM = kSplitTileM;   // 128 rows per tile (TMEM lanes)
 constexpr int KB = 32;            // K elements per block: one 64-byte swizzle row
 constexpr int KCHUNK = 512;       // exact-accumulation chunk
 constexpr int KB_PER_CHUNK = KCHUNK / KB;
-constexpr int kEpiWarps = 8;  // two epilogue warps per TMEM lane quarter, one per half of the tile's columns
-constexpr int kSplitThreads = 32 * (2 + kEpiWarps);
+constexpr int kEpiWarps = 16;  // four epilogue warps per TMEM lane quarter, one per quarter of the tile's columns
+constexpr int kTableWarp = 2 + kEpiWarps;  // feeds the epilogue (see EpiTile)
+constexpr int kSplitThreads = 32 * (3 + kEpiWarps);
 constexpr int A_TILE_BYTES = TM * KB * 2;  // 8 KiB
 template <int TN>
 __host__ __device__ constexpr int b_tile_bytes() { return TN * KB * 2; }  // 4 KiB (N = 64) or 8 KiB (N = 128)
@@ -174,13 +184,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// 32 lanes x 16 columns of 32-bit words, no wait (pair with tmem_ld_wait).
-__device__ __forceinline__ void tmem_ld16_raw(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
+// 32 lanes x 8 columns of 32-bit words, no wait (pair with tmem_ld_wait).
+__device__ __forceinline__ void tmem_ld8_raw(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
 
@@ -542,6 +550,22 @@ __global__ void __launch_bounds__(256, 4) pack_b_kernel(const SplitJob* __restri
   }
 }
 
+// What the epilogue needs of one tile, put into shared memory ahead of time by
+// a warp of its own: the chain tile -> job -> scales is three dependent loads
+// (2000 cycles), which the epilogue of a short tile would otherwise wait for.
+template <int TN>
+struct EpiTile {
+  int64_t c_off, ldc;           // element offset of the tile in C, column stride
+  int32_t rows, cols, nchunks;  // live rows and columns, exact-accumulation chunks
+  int32_t pad;
+  int64_t b_at;                 // offset of the tile's column scales
+  double sr[TM];                  // row scales times alpha and the digits' power of two
+  double tau[TN == 64 ? TN : 1];  // column scales (width 128: read by the epilogue itself)
+};
+// Width 128 leaves room for one record beside two stages of seven slices.
+template <int TN>
+__host__ __device__ constexpr int epi_slots() { return TN == 64 ? 2 : 1; }
+
 __host__ __device__ constexpr uint32_t tmem_cols_pow2(uint32_t c) {
   return c <= 32 ? 32 : c <= 64 ? 64 : c <= 128 ? 128 : c <= 256 ? 256 : 512;
 }
@@ -588,12 +612,15 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
   uint64_t* empty = full + nstage;
   uint64_t* acc_full = empty + nstage;   // [2]
   uint64_t* acc_empty = acc_full + 2;    // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  constexpr int NEPI = epi_slots<TN>();
+  uint64_t* epi_full = acc_empty + 2;    // [NEPI]
+  uint64_t* epi_empty = epi_full + NEPI; // [NEPI]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(epi_empty + NEPI);
   volatile int* bail = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  EpiTile<TN>* epi = reinterpret_cast<EpiTile<TN>*>(tmem_slot + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int32_t step = (int32_t)gridDim.x;
-  auto nkb_of = [](const GemmTile& tl) { return (int64_t)((tl.k + 63) / 64) * (64 / KBX); };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < nstage; ++s) {
@@ -602,7 +629,11 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&acc_full[s], 1);
-      mbar_init(&acc_empty[s], 32 * kEpiWarps);
+      mbar_init(&acc_empty[s], kEpiWarps);
+    }
+    for (int s = 0; s < NEPI; ++s) {
+      mbar_init(&epi_full[s], 32);
+      mbar_init(&epi_empty[s], kEpiWarps);
     }
     *bail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -620,73 +651,85 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
 
   if (warp == 0) {
     // ---- bulk-copy producer ------------------------------------------------
-    if (lane == 0) {
-      int64_t it = 0;
-      int32_t t = blockIdx.x;
-      // Two tiles and one job ahead, so no load of the tile table waits at a tile boundary.
-      GemmTile t1 = t < ntiles ? tiles[t] : GemmTile{};
-      GemmTile t2 = t + step < ntiles ? tiles[t + step] : GemmTile{};
-      SplitJob j1 = jobs[t < ntiles ? t1.job : 0];
-      for (; t < ntiles && !*bail; t += step) {
-        const GemmTile tile = t1;
-        const SplitJob J = j1;
-        t1 = t2;
-        if (t + step < ntiles) j1 = jobs[t1.job];
-        if (t + 2 * step < ntiles) t2 = tiles[t + 2 * step];
-        const int64_t nkb = J.k_pad / KBX;
-        const int64_t abase = tile.batch * dims.a_stride + J.a_pack + (int64_t)tile.tm * TM * KBX;
-        const int64_t bbase = tile.batch * dims.b_stride + J.b_pack + (int64_t)tile.tn * TN * KBX;
-        for (int64_t kb = 0; kb < nkb; ++kb, ++it) {
-          const int st = (int)(it % nstage);
-          if (!mbar_wait(&empty[st], (uint32_t)(((it / nstage) & 1) ^ 1))) {
-            atomicExch(err, 1);
-            *bail = 1;
-            break;
-          }
-          uint8_t* sbase = smem + st * stage_bytes;
-          mbar_expect_tx(&full[st], (uint32_t)stage_bytes);
-#pragma unroll
-          for (int s = 0; s < S; ++s) {
-            const int64_t ea = abase + (int64_t)s * J.m_pad * J.k_pad + kb * J.m_pad * KBX;
-            bulk_load(sbase + s * A_TILE_BYTES, apack + ea * kElem, A_TILE_BYTES, &full[st]);
-            const int64_t eb = bbase + (int64_t)s * J.n_pad * J.k_pad + kb * J.n_pad * KBX;
-            bulk_load(sbase + S * A_TILE_BYTES + s * B_TILE_BYTES, bpack + eb * kElem, B_TILE_BYTES, &full[st]);
-          }
+    // Lane s < S copies slice s of A, lane S + s slice s of B: one thread that
+    // issued all 2 S copies of a k-block, with two 64-bit divisions for the stage,
+    // took 1200 - 1650 cycles for it, as long as the k-block's MMAs.
+    const bool is_a = lane < S, copies = lane < 2 * S;
+    const int slice = is_a ? lane : lane - S;
+    int st = 0;
+    uint32_t phase = 1;  // parity of the wait on empty[st]: the first pass finds it free
+    int32_t t = blockIdx.x;
+    // Two tiles and one job ahead, so no load of the tile table waits at a tile boundary.
+    GemmTile t1 = t < ntiles ? tiles[t] : GemmTile{};
+    GemmTile t2 = t + step < ntiles ? tiles[t + step] : GemmTile{};
+    SplitJob j1 = jobs[t < ntiles ? t1.job : 0];
+    for (; t < ntiles; t += step) {
+      if (__any_sync(0xffffffffu, *bail)) break;
+      const GemmTile tile = t1;
+      const SplitJob J = j1;
+      t1 = t2;
+      if (t + step < ntiles) j1 = jobs[t1.job];
+      if (t + 2 * step < ntiles) t2 = tiles[t + 2 * step];
+      const int32_t nkb = (int32_t)(J.k_pad / KBX);
+      // Rows and columns beyond m and n (in whole 8-row swizzle groups) are not
+      // copied: what they multiply reaches only accumulators that are not written.
+      const int64_t mrows = J.m - (int64_t)tile.tm * TM, ncols = J.n - (int64_t)tile.tn * TN;
+      const uint32_t abytes = mrows < TM ? (uint32_t)((mrows + 7) / 8) * 512u : (uint32_t)A_TILE_BYTES;
+      const uint32_t bbytes = ncols < TN ? (uint32_t)((ncols + 7) / 8) * 512u : (uint32_t)B_TILE_BYTES;
+      // This lane's slice, from k-block 0 on: one k-block is all the job's rows of 64 bytes.
+      const int64_t rows_pad = is_a ? J.m_pad : J.n_pad;
+      const int64_t first = is_a ? tile.batch * dims.a_stride + J.a_pack : tile.batch * dims.b_stride + J.b_pack;
+      const uint8_t* src = (is_a ? apack : bpack) + (first + slice * rows_pad * J.k_pad) * kElem +
+                           (is_a ? (int64_t)tile.tm * TM : (int64_t)tile.tn * TN) * 64;
+      const uint32_t bytes = is_a ? abytes : bbytes;
+      const uint32_t at = is_a ? slice * A_TILE_BYTES : S * A_TILE_BYTES + slice * B_TILE_BYTES;
+      for (int32_t kb = 0; kb < nkb; ++kb, src += rows_pad * 64) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&empty[st], phase))) {
+          atomicExch(err, 1);
+          *bail = 1;
+          break;
+        }
+        if (lane == 0) mbar_expect_tx(&full[st], S * (abytes + bbytes));
+        __syncwarp();
+        if (copies) bulk_load(smem + st * stage_bytes + at, src, bytes, &full[st]);
+        if (++st == nstage) {
+          st = 0;
+          phase ^= 1;
         }
       }
     }
   } else if (warp == 1) {
     // ---- MMA issuer (one thread) -------------------------------------------
     if (lane == 0) {
-      int64_t it = 0, round = 0;
+      int st = 0;
+      uint32_t phase = 0, round = 0;
       int32_t t = blockIdx.x;
       GemmTile nxt = t < ntiles ? tiles[t] : GemmTile{};
       for (; t < ntiles && !*bail; t += step) {
         const GemmTile tile = nxt;
         if (t + step < ntiles) nxt = tiles[t + step];
-        const int64_t nkb = nkb_of(tile);
+        const int32_t nkb = (tile.k + 63) / 64 * (64 / KBX);
         uint32_t tacc = 0;
         bool fresh[NACC];
 #pragma unroll
         for (int a = 0; a < NACC; ++a) fresh[a] = true;
-        for (int64_t kb = 0; kb < nkb; ++kb, ++it) {
-          const int64_t kin = kb % KCH;
+        for (int32_t kb = 0; kb < nkb; ++kb) {
+          const int32_t kin = kb % KCH;
           if (kin == 0) {
-            const int set = (int)(round % NSETS);
+            const uint32_t set = round % NSETS;
             if (round >= NSETS) {
-              if (!mbar_wait(&acc_empty[set], (uint32_t)((round / NSETS - 1) & 1))) {
+              if (!mbar_wait(&acc_empty[set], (round / NSETS - 1) & 1)) {
                 atomicExch(err, 2);
                 *bail = 1;
                 break;
               }
             }
             tc_fence_after();
-            tacc = tmem + (uint32_t)set * SET_COLS;
+            tacc = tmem + set * SET_COLS;
 #pragma unroll
             for (int a = 0; a < NACC; ++a) fresh[a] = true;
           }
-          const int st = (int)(it % nstage);
-          if (!mbar_wait(&full[st], (uint32_t)((it / nstage) & 1))) {
+          if (!mbar_wait(&full[st], phase)) {
             atomicExch(err, 3);
             *bail = 1;
             break;
@@ -697,6 +740,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
           if constexpr (I8) {
 #pragma unroll
             for (int kk = 0; kk < 2; ++kk) {  // two 32-byte K steps per 64-byte row
+              if (kk == 1 && kb * KB8 + KB8 / 2 >= tile.k) break;  // the last k-block's second half is padding
               // The first MMA of a chunk (i = 0 spans every accumulator) overwrites.
               const uint32_t first = (kin == 0 && kk == 0) ? 0u : 1u;
 #pragma unroll
@@ -733,97 +777,166 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
             umma_commit(&acc_full[round % NSETS]);
             ++round;
           }
+          if (++st == nstage) {
+            st = 0;
+            phase ^= 1;
+          }
         }
       }
     }
-  } else {
-    // ---- epilogue: warps 2..9; TMEM lane quarter = warp % 4, column half = (warp - 2) / 4
-    // Each chunk's accumulators are summed in FP64 and added into C directly
-    // (the first chunk applies alpha/beta), so no FP64 tile lives in registers.
-    const int q = warp & 3;
-    const int half = (warp - 2) >> 2;
-    constexpr int HC = TN / 2;  // columns per epilogue warp
-    int64_t round = 0;
+  } else if (warp == kTableWarp) {
+    // ---- the epilogue's records ---------------------------------------------
+    // kTileScale: 2^-12 2^{-8(H-1)} (digits, H = min(S, 3) high diagonals) or 2^-14 (slices)
+    constexpr double kTileScale = I8 ? (S == 1 ? 1.0 / 4096.0 : S == 2 ? 1.0 / 1048576.0 : 1.0 / 268435456.0)
+                                     : 1.0 / 16384.0;
+    uint32_t n = 0;
     int32_t t = blockIdx.x;
     GemmTile nxt = t < ntiles ? tiles[t] : GemmTile{};
-    for (; t < ntiles; t += step) {
-      if (*bail) break;
+    for (; t < ntiles && !*bail; t += step, ++n) {
       const GemmTile tile = nxt;
       if (t + step < ntiles) nxt = tiles[t + step];
       const SplitJob J = jobs[tile.job];
-      const int64_t nkb = J.k_pad / KBX;
-      const int64_t nchunks = (nkb + KCH - 1) / KCH;
-      const int64_t row = (int64_t)tile.tm * TM + q * 32 + lane;
-      const bool live = row < J.m;
-      // 2^-12 2^{-8(H-1)} (digits, H = min(S, 3) high diagonals) or 2^-14 (slices)
-      constexpr double kTileScale = I8 ? (S == 1 ? 1.0 / 4096.0 : S == 2 ? 1.0 / 1048576.0 : 1.0 / 268435456.0)
-                                       : 1.0 / 16384.0;
-      const double sr = live ? a_scales[tile.batch * dims.as_stride + J.a_scale + row] * kTileScale * alpha : 0.0;
-      const double* tcs = b_scales + tile.batch * dims.bs_stride + J.b_scale + (int64_t)tile.tn * TN;
-      // The column scales of this warp's columns, one per lane (read before
-      // the accumulators are ready; the writes fetch them by shuffle).
-      constexpr int NTS = (HC + 31) / 32;
-      double tsc[NTS];
+      const int64_t row0 = (int64_t)tile.tm * TM, col0 = (int64_t)tile.tn * TN;
+      const double* as = a_scales + tile.batch * dims.as_stride + J.a_scale + row0;
+      const double* bs = b_scales + tile.batch * dims.bs_stride + J.b_scale + col0;
+      double sr[TM / 32], tau[2] = {0.0, 0.0};
 #pragma unroll
-      for (int u = 0; u < NTS; ++u) tsc[u] = (32 * u + lane < HC) ? __ldg(tcs + half * HC + 32 * u + lane) : 0.0;
-      double* crow = C + tile.batch * sc + J.c_off + row;
+      for (int u = 0; u < TM / 32; ++u)
+        sr[u] = row0 + 32 * u + lane < J.m ? as[32 * u + lane] * kTileScale * alpha : 0.0;
+      if constexpr (TN == 64) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) tau[u] = col0 + 32 * u + lane < J.n ? bs[32 * u + lane] : 0.0;
+      }
+      EpiTile<TN>& e = epi[n % NEPI];
+      if (!mbar_wait(&epi_empty[n % NEPI], ((n / NEPI) & 1) ^ 1)) {
+        atomicExch(err, 5);
+        *bail = 1;
+        break;
+      }
+#pragma unroll
+      for (int u = 0; u < TM / 32; ++u) e.sr[32 * u + lane] = sr[u];
+      if constexpr (TN == 64) {
+        e.tau[lane] = tau[0];
+        e.tau[32 + lane] = tau[1];
+      }
+      if (lane == 0) {
+        e.c_off = tile.batch * sc + J.c_off + row0 + col0 * J.ldc;
+        e.ldc = J.ldc;
+        e.rows = (int32_t)(J.m - row0 < TM ? J.m - row0 : TM);
+        e.cols = (int32_t)(J.n - col0 < TN ? J.n - col0 : TN);
+        e.nchunks = (int32_t)((J.k_pad / KBX + KCH - 1) / KCH);
+        e.b_at = tile.batch * dims.bs_stride + J.b_scale + col0;
+      }
+      mbar_arrive(&epi_full[n % NEPI]);
+    }
+  } else {
+    // ---- epilogue: warps 2..17; TMEM lane quarter = warp % 4, column quarter = (warp - 2) / 4
+    // Each chunk's accumulators are summed in FP64 and added into C directly
+    // (the first chunk applies alpha/beta), so no FP64 tile lives in registers.
+    const int q = warp & 3;
+    const int part = (warp - 2) >> 2;
+    constexpr int HC = TN / (kEpiWarps / 4);  // columns per epilogue warp
+    uint32_t round = 0, n = 0;
+    for (int32_t t = blockIdx.x; t < ntiles; t += step, ++n) {
+      // Votes keep the warp together: a wait that ran out on one lane ends all of them.
+      if (__any_sync(0xffffffffu, *bail)) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(&epi_full[n % NEPI], (n / NEPI) & 1))) {
+        atomicExch(err, 6);
+        *bail = 1;
+        break;
+      }
+      const EpiTile<TN>& e = epi[n % NEPI];
+      const int32_t nchunks = e.nchunks;
       if (nchunks == 0) {  // k == 0: C = beta C on this warp's columns
-        if (live)
-          for (int cc = half * HC; cc < (half + 1) * HC; ++cc) {
-            const int64_t col = (int64_t)tile.tn * TN + cc;
-            if (col < J.n) {
-              double* p = crow + col * J.ldc;
-              *p = beta == 0.0 ? 0.0 : beta * *p;
-            }
-          }
-        continue;
+        double* crow = C + e.c_off + q * 32 + lane;
+        if (q * 32 + lane < e.rows)
+          for (int i = part * HC; i < e.cols && i < (part + 1) * HC; ++i)
+            crow[i * e.ldc] = beta == 0.0 ? 0.0 : beta * crow[i * e.ldc];
       }
       bool ok = true;
-      for (int64_t chunk = 0; chunk < nchunks; ++chunk, ++round) {
-        const int set = (int)(round % NSETS);
-        if (!mbar_wait(&acc_full[set], (uint32_t)((round / NSETS) & 1))) {
+      for (int32_t chunk = 0; chunk < nchunks; ++chunk, ++round) {
+        const uint32_t set = round % NSETS;
+        if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[set], (round / NSETS) & 1))) {
           atomicExch(err, 4);
           *bail = 1;
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)set * SET_COLS;
-        // Sum of the accumulators of columns [c0, c0 + 16) in FP64.
-        auto drain16 = [&](int c0, double (&sum)[16]) {
-          if constexpr (I8) {
-            // The exact integer sum in two parts: hi = sum_{a<H} acc_a
-            // 256^{H-1-a} (|hi| < 2^43) and lo = sum_{a<L} acc_{H+a}
-            // 256^{L-1-a} (|lo| < 2^47), both exact as doubles; the value
-            // hi + lo 2^{-8L} is rounded once (the FMA), and the remaining
-            // 2^{-8(H-1)} sits in kTileScale.  The loads of up to three
-            // accumulators are in flight before each wait.
-            constexpr int H = NACC < 3 ? NACC : 3, L = NACC - H;
-            uint32_t r[3][16];
+        const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + set * SET_COLS + part * HC;
+        // This warp's share of the accumulators may be overwritten from here on.
+        auto release = [&] {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&acc_empty[set]);
+        };
+        // Writes columns [c0, c0 + 16) of this warp's share; value(i) is column c0 + i.
+        auto write16 = [&](int c0, auto&& value) {
+          const double bb = chunk > 0 ? 1.0 : beta;  // later chunks add to what the first one wrote
+          const double sr = e.sr[q * 32 + lane];
+          const int ncol = q * 32 + lane < e.rows ? e.cols - part * HC - c0 : 0;
+          const int64_t ldc = e.ldc;
+          double* p = C + e.c_off + q * 32 + lane + (part * HC + c0) * ldc;
+          double tsc = 0.0;
+          if constexpr (TN != 64)
+            if (lane < 16 && part * HC + c0 + lane < e.cols) tsc = __ldg(b_scales + e.b_at + part * HC + c0 + lane);
 #pragma unroll
-            for (int a = 0; a < H; ++a) tmem_ld16_raw(tbase + (uint32_t)(a * TN + c0), r[a]);
+          for (int i = 0; i < 16; ++i, p += ldc) {
+            const double tau = TN == 64 ? e.tau[part * HC + c0 + i] : __shfl_sync(0xffffffffu, tsc, i);
+            const double v = sr * tau * value(i);
+            if (i < ncol) *p = bb == 0.0 ? v : fma(bb, *p, v);
+          }
+        };
+        if constexpr (I8) {
+          // The exact integer sum over the first H diagonals, hi = sum_a acc_a
+          // 256^{H-1-a} (|hi| < 2^43), and the other L, lo = sum_a acc_{H+a}
+          // 256^{L-1-a} (|lo| < 2^47): with up to two of those, one integer hi
+          // 256^L + lo below 2^60; with three, hi plus the carry of lo, and the 24
+          // bits below it.  The accumulators are released as soon as the integers
+          // are formed (eight columns at a time: the 96 registers that 19 warps
+          // leave hold no more), so the next tile's MMAs run while these are
+          // converted, exactly in two parts and rounded once by the FMA, and
+          // written.  The remaining 2^{-8(H-1)} sits in the row scales.
+          static_assert(HC == 16, "int8 digits run at width 64");
+          constexpr int H = NACC < 3 ? NACC : 3, L = NACC - H;
+          constexpr int kLoBits = 8 * L, kOne = L <= 2 ? kLoBits : 0;
+          long long v[16];
+          uint32_t low[16];
+#pragma unroll
+          for (int b = 0; b < 16; b += 8) {
+            uint32_t r[NACC][8];
+#pragma unroll
+            for (int a = 0; a < NACC; ++a) tmem_ld8_raw(tbase + (uint32_t)(a * TN + b), r[a]);
             tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              long long h = 0;
+            for (int i = 0; i < 8; ++i) {
+              long long hi = 0, lo = 0;
 #pragma unroll
-              for (int a = 0; a < H; ++a) h = h * 256 + (long long)(int32_t)r[a][i];
-              sum[i] = i51_to_f64(h);
-            }
-            if constexpr (L > 0) {
+              for (int a = 0; a < H; ++a) hi = hi * 256 + (long long)(int32_t)r[a][i];
 #pragma unroll
-              for (int a = 0; a < L; ++a) tmem_ld16_raw(tbase + (uint32_t)((H + a) * TN + c0), r[a]);
-              tmem_ld_wait();
-              constexpr double kLo = L == 1 ? 1.0 / 256.0 : L == 2 ? 1.0 / 65536.0 : 1.0 / 16777216.0;
-#pragma unroll
-              for (int i = 0; i < 16; ++i) {
-                long long l = 0;
-#pragma unroll
-                for (int a = 0; a < L; ++a) l = l * 256 + (long long)(int32_t)r[a][i];
-                sum[i] = fma(i51_to_f64(l), kLo, sum[i]);
+              for (int a = H; a < NACC; ++a) lo = lo * 256 + (long long)(int32_t)r[a][i];
+              low[b + i] = 0;
+              if constexpr (L <= 2) {
+                v[b + i] = hi * (1LL << kOne) + lo;
+              } else {
+                v[b + i] = hi + (lo >> kLoBits);
+                low[b + i] = (uint32_t)lo & ((1u << kLoBits) - 1);
               }
             }
-          } else {
+          }
+          release();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) asm volatile("" : "+l"(v[i]), "+r"(low[i]));  // converted after the release
+          write16(0, [&](int i) {
+            if constexpr (L == 0) return i51_to_f64(v[i]);
+            constexpr double kLo = 1.0 / (double)(1 << kLoBits);
+            const uint32_t l = L <= 2 ? (uint32_t)v[i] & ((1u << kLoBits) - 1) : low[i];
+            return fma(i51_to_f64((long long)l), kLo, i51_to_f64(v[i] >> kOne));
+          });
+        } else {
+#pragma unroll 1
+          for (int c0 = 0; c0 < HC; c0 += 16) {
+            double sum[16];
 #pragma unroll
             for (int i = 0; i < 16; ++i) sum[i] = 0.0;
 #pragma unroll
@@ -833,44 +946,13 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
 #pragma unroll
               for (int i = 0; i < 16; ++i) sum[i] += (double)v[i];
             }
+            if (c0 + 16 == HC) release();
+            write16(c0, [&](int i) { return sum[i]; });
           }
-        };
-        auto write16 = [&](int c0, const double (&sum)[16]) {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const int cw = c0 - half * HC + i;  // column within this warp's share (uniform)
-            const double tau = __shfl_sync(0xffffffffu, tsc[cw >> 5], cw & 31);
-            const int64_t col = (int64_t)tile.tn * TN + c0 + i;
-            if (live && col < J.n) {
-              double* p = crow + col * J.ldc;
-              const double v = sr * tau * sum[i];
-              if (chunk > 0) *p += v;
-              else *p = beta == 0.0 ? v : fma(beta, *p, v);
-            }
-          }
-        };
-        if constexpr (HC == 32) {
-          // Release the accumulators as soon as the second 16 columns are in
-          // registers, so the next tile's MMAs run while they are written
-          // (holding all 32 columns would spill at this block size).
-          double sum[16];
-          drain16(half * HC, sum);
-          write16(half * HC, sum);
-          drain16(half * HC + 16, sum);
-          tc_fence_before();
-          mbar_arrive(&acc_empty[set]);
-          write16(half * HC + 16, sum);
-        } else {
-#pragma unroll 1
-          for (int c0 = half * HC; c0 < (half + 1) * HC; c0 += 16) {
-            double sum[16];
-            drain16(c0, sum);
-            write16(c0, sum);
-          }
-          tc_fence_before();
-          mbar_arrive(&acc_empty[set]);
         }
       }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&epi_empty[n % NEPI]);
       if (!ok) break;
     }
   }
@@ -1226,9 +1308,12 @@ cudaError_t launch_gemm_split(const void* job_table, const GemmJob* host_jobs, i
   const uint8_t* mb = static_cast<const uint8_t*>(bpack);
   const int stage_bytes = slices * (A_TILE_BYTES + tile_n * 64);
   const int max_smem = 227 * 1024;
-  int nstage = std::min(4, (max_smem - 2048) / stage_bytes);
+  // alignment slack, barriers and the epilogue's records beside the stages
+  const int extra = 1024 + 128 + (tile_n == 64 ? epi_slots<64>() * (int)sizeof(EpiTile<64>)
+                                               : epi_slots<128>() * (int)sizeof(EpiTile<128>));
+  int nstage = std::min(4, (max_smem - extra) / stage_bytes);
   if (nstage < 1) return cudaErrorInvalidValue;
-  const size_t smem = 1024 + (size_t)nstage * stage_bytes + 256;
+  const size_t smem = (size_t)nstage * stage_bytes + extra;
   return launch_mma(slices, tile_n, i8, ntiles, smem, stream, ma, mb, djobs, tiles, L.dims, ascale, bscale, c, sc,
                     alpha, beta, nstage, err);
 }

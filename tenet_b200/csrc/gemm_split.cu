@@ -206,6 +206,24 @@ __device__ __forceinline__ double pow2_scale(double amax) {
   return ldexp(1.0, e);
 }
 
+// The scale is a power of two, so the exponent of a row's maximum, in its high
+// word, decides it: two integer instructions per value instead of an FP64
+// maximum's five, and the digits' power of two joins it in one multiplier.  Rows
+// whose largest magnitude is zero, subnormal or tiny (below 2^-959), at least
+// 2^1022, infinite or NaN take the general rule.
+// The high words between which a maximum's exponent alone gives the scale.
+constexpr uint32_t kScaleLo = 64u << 20, kScaleHi = 2045u << 20;
+
+__device__ __forceinline__ uint32_t hi_abs(double x) { return (uint32_t)__double2hiint(x) & 0x7fffffffu; }
+
+// sigma of a row with largest high word h in [kScaleLo, kScaleHi), and `unit`
+// (the digits' power of two) over sigma.
+__device__ __forceinline__ void fast_scale(uint32_t h, double unit, double& sigma, double& mul) {
+  const uint32_t e = h >> 20;  // amax in [2^(e-1023), 2^(e-1022))
+  sigma = __hiloint2double((int)((e + 1) << 20), 0);
+  mul = unit * __hiloint2double((int)((2045 - e) << 20), 0);
+}
+
 // Cut 8 consecutive values (|x| < 1) into S slices of 7 bits each, 16 bytes
 // (8 bf16) per slice: x ~ sum_s q_s 2^{-7(s+1)} with q_s the balanced
 // base-128 digits of X = rint(x 2^{7S}) (one power-of-two scaling and one
@@ -214,14 +232,15 @@ __device__ __forceinline__ double pow2_scale(double amax) {
 // in [-64, 63], sum_s q_s 128^{S-1-s} = X.  Slice s is stored pre-scaled by
 // 2^{-7s}: an integer of magnitude <= 128 times a power of two, exact in BF16.
 template <int S>
-__device__ __forceinline__ void cut8_store(const double (&x)[8], __nv_bfloat16* dst, int64_t slice_stride) {
-  constexpr int kShift = 7 * S;
+__host__ __device__ constexpr double cut_scale() { return (double)(1ull << (7 * S)); }
+template <int S>
+__device__ __forceinline__ void cut8_store(const double (&x)[8], __nv_bfloat16* dst, int64_t slice_stride,
+                                           double scale = cut_scale<S>()) {
   constexpr long long kOffset = [] {
     long long c = 0;
     for (int j = 0; j < S; ++j) c = c * 128 + 64;
     return c;
   }();
-  const double scale = (double)(1ull << kShift);
   long long y[8];
 #pragma unroll
   for (int t = 0; t < 8; ++t) y[t] = __double2ll_rn(x[t] * scale) + kOffset;
@@ -285,27 +304,24 @@ __device__ __forceinline__ uint32_t gather_byte(uint32_t w0, uint32_t w1, uint32
 // the top digit d_0 itself (Y = d_0 256^{S-1} + sum u_s 256^{S-1-s}).  The
 // digits are then a byte transpose of the eight values' low words.
 template <int S>
-__device__ __forceinline__ void cut8_store_s8(const double (&x)[8], int8_t* dst, int64_t slice_stride) {
+__host__ __device__ constexpr double cut_scale_s8() { return (double)(1ull << (8 * S - 2)); }
+template <int S>
+__device__ __forceinline__ void cut8_store_s8(const double (&x)[8], int8_t* dst, int64_t slice_stride,
+                                              double scale = cut_scale_s8<S>()) {
   static_assert(S >= 1 && S <= kMaxI8Slices, "8-bit digits: 1..6 per value");
   constexpr unsigned long long kOffset = [] {
     unsigned long long c = 0;
     for (int j = 0; j < S - 1; ++j) c = c * 256 + 128;
     return c;
   }();
-  constexpr unsigned long long kFlip = [] {
-    unsigned long long m = 0;
-    for (int j = 0; j < S - 1; ++j) m |= 0x80ull << (8 * j);
-    return m;
-  }();
   constexpr double kMagic = 6755399441055744.0 + (double)kOffset;  // 1.5 * 2^52 + C, an exact integer
-  const double scale = (double)(1ull << (8 * S - 2));
   uint32_t w[2][S];  // digit s of values 0-3 (w[0]) and 4-7 (w[1])
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     uint32_t lo[4], hi[4];
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
-      const unsigned long long v = (unsigned long long)__double_as_longlong(fma(x[4 * h + t], scale, kMagic)) ^ kFlip;
+      const unsigned long long v = (unsigned long long)__double_as_longlong(fma(x[4 * h + t], scale, kMagic));
       lo[t] = (uint32_t)v;
       hi[t] = (uint32_t)(v >> 32);
     }
@@ -313,6 +329,7 @@ __device__ __forceinline__ void cut8_store_s8(const double (&x)[8], int8_t* dst,
     for (int s = 0; s < S; ++s) {
       const int b = S - 1 - s;  // byte of digit s
       w[h][s] = b < 4 ? gather_byte(lo[0], lo[1], lo[2], lo[3], b) : gather_byte(hi[0], hi[1], hi[2], hi[3], b - 4);
+      if (s > 0) w[h][s] ^= 0x80808080u;  // u_s back to the int8 bits of d_s
     }
   }
 #pragma unroll
@@ -352,13 +369,16 @@ __global__ void __launch_bounds__(256, 4) pack_a_kernel(const SplitJob* __restri
                                                      const double* __restrict__ A, int64_t sa,
                                                      double* __restrict__ scales, void* __restrict__ pack) {
   __shared__ double red[8][32];
-  __shared__ __align__(16) uint8_t tile[(I8 ? 1 : 2) * S * 2048];  // one iteration's slices
+  __shared__ uint32_t redh[8][32];
+  // One iteration's slices; a second tile saves a barrier per iteration where four CTAs still fit.
+  constexpr int kBufs = I8 ? 2 : 1, kTile = (I8 ? 1 : 2) * S * 2048;
+  __shared__ __align__(16) uint8_t tiles[kBufs][kTile];
   const int64_t group = blockIdx.x, batch = blockIdx.y;
   const SplitJob J = jobs[group_job[group]];
   // A group made only of padding rows (m_pad rounds m up to the 128-row
   // tile) is skipped: an output row depends only on its own row of A, and the
   // multiply never writes rows beyond m, so those digits and scales are never
-  // used.  Padding rows inside a live group still get zero digits.
+  // used.
   if (group * 32 - J.a_scale >= J.m) return;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t row = group * 32 - J.a_scale + lane;  // row within the job (padded rows beyond m read zero)
@@ -385,12 +405,37 @@ __global__ void __launch_bounds__(256, 4) pack_a_kernel(const SplitJob* __restri
     }
   };
   double* srow = scales + batch * dims.as_stride + J.a_scale + row;
-  double m = 0.0;
-  if constexpr (MODE != kPackCut) {
-    double amax = 0.0;
+  constexpr double kUnit = I8 ? cut_scale_s8<S>() : cut_scale<S>();
+  uint32_t h = 0;
+  if constexpr (MODE == kPackFused) {
     if (live) {
       int64_t it = it0;
       for (; it + 1 < nit; it += 2) {  // two iterations of loads in flight
+        double u[8], v[8];
+        load(u, it);
+        load(v, it + 1);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) h = max(h, max(hi_abs(u[i]), hi_abs(v[i])));
+      }
+      if (it < nit) {
+        double u[8];
+        load(u, it);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) h = max(h, hi_abs(u[i]));
+      }
+    }
+    redh[w][lane] = h;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) h = max(h, redh[i][lane]);
+  }
+  double m = 0.0;
+  const bool general = MODE != kPackFused || __syncthreads_or(live && !(h >= kScaleLo && h < kScaleHi));
+  if (MODE != kPackCut && general) {
+    double amax = 0.0;
+    if (live) {
+      int64_t it = it0;
+      for (; it + 1 < nit; it += 2) {
         double u[8], v[8];
         load(u, it);
         load(v, it + 1);
@@ -414,10 +459,20 @@ __global__ void __launch_bounds__(256, 4) pack_a_kernel(const SplitJob* __restri
         atomicMax(reinterpret_cast<unsigned long long*>(srow), (unsigned long long)__double_as_longlong(m));
       return;
     }
-  } else {
-    m = *srow;  // the full row maximum left by the kPackAmax launch
   }
-  const double sigma = pow2_scale(m), inv = 1.0 / sigma;
+  if constexpr (MODE == kPackCut) {
+    m = *srow;  // the full row maximum left by the kPackAmax launch
+    h = hi_abs(m);
+  }
+  const bool slow = !(h >= kScaleLo && h < kScaleHi);
+  double sigma, mul, inv = 1.0;  // digits of x: x * inv * mul, inv = 1 but for the general rule
+  fast_scale(h, kUnit, sigma, mul);
+  if (slow) {
+    sigma = pow2_scale(m);
+    inv = 1.0 / sigma;
+    mul = kUnit;
+  }
+  const bool any_slow = __any_sync(0xffffffffu, slow && live);
   if (MODE == kPackFused && w == 0) *srow = sigma;
   // Pass 2.  Each iteration cuts 32 rows x 64 k into shared memory (lane =
   // row, coalesced reads) and writes every slice's 32 x 64-byte piece -- one
@@ -430,33 +485,39 @@ __global__ void __launch_bounds__(256, 4) pack_a_kernel(const SplitJob* __restri
   uint8_t* base = static_cast<uint8_t*>(pack) + (batch * dims.a_stride + J.a_pack) * elem +
                   (group * 32 - J.a_scale) * 64;  // row 0 of this group, k-block 0, slice 0
   const int swz = (lane >> 1) & 3;
+  const int64_t left = J.m - (group * 32 - J.a_scale);  // live rows from the group's first on
   double x[8];
   if (nit > it0) load(x, it0);
   for (int64_t it = it0; it < nit; ++it) {
     double nx[8];
     if (it + 1 < nit) load(nx, it + 1);
+    if (any_slow)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) x[i] *= inv;
+      for (int i = 0; i < 8; ++i) x[i] *= inv;
+    uint8_t* tile = tiles[it % kBufs];
     if constexpr (I8) {
       // tile[s][row][64 bytes]; warp w holds bytes 8w .. 8w + 7 of the row
       cut8_store_s8<S>(x, reinterpret_cast<int8_t*>(tile) + lane * 64 + ((((w >> 1) ^ swz) << 4) | ((w & 1) << 3)),
-                       32 * 64);
+                       32 * 64, mul);
     } else {
       // tile[s][kb 0..1][row][32 bf16]; warp w holds chunk w & 3 of k-block w >> 2
       cut8_store<S>(x, reinterpret_cast<__nv_bfloat16*>(tile) + (w >> 2) * 32 * 32 + lane * 32 + (((w & 3) ^ swz) << 3),
-                    2 * 32 * 32);
+                    2 * 32 * 32, mul);
     }
     __syncthreads();
     constexpr int kPieces = I8 ? S : 2 * S;  // 2 KB pieces per iteration
-    const int c = threadIdx.x & 127;
-    for (int p = threadIdx.x >> 7; p < kPieces; p += 2) {
+    // Left out: 8-row groups beyond m, and of int8 digits the 32 k of a last block
+    // that lie beyond K (neither is multiplied).
+    const int c = threadIdx.x & 127, cr = c >> 2;
+    const bool skip = (cr & ~7) >= left || (I8 && it * 64 + 32 >= J.k && (((c & 3) ^ (cr >> 1)) & 2));
+    for (int p = skip ? kPieces : threadIdx.x >> 7; p < kPieces; p += 2) {
       const int s = I8 ? p : p >> 1;
       const int64_t kb = I8 ? it : 2 * it + (p & 1);
       const uint4* src = reinterpret_cast<const uint4*>(tile + p * 2048);
       uint4* dst = reinterpret_cast<uint4*>(base + s * slice_bytes + kb * J.m_pad * 64);
       dst[c] = src[c];  // the tile is already in the 64-byte swizzle
     }
-    __syncthreads();
+    if constexpr (kBufs == 1) __syncthreads();
     if (it + 1 < nit) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) x[i] = nx[i];
@@ -546,6 +607,119 @@ __global__ void __launch_bounds__(256, 4) pack_b_kernel(const SplitJob* __restri
     if (it + 1 < nit) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) x[i] = nx[i];
+    }
+  }
+}
+
+// log2 of the passes over a 32-column group of this K.
+template <int ITS>
+__device__ __forceinline__ int keep_parts(int64_t k_pad) {
+  return k_pad <= 64 * ITS ? 0 : k_pad <= 128 * ITS ? 1 : 2;
+}
+
+// B up to K = 1024: one read, values kept in registers.  The kernel above reads B
+// twice (maxima, then digits, the second time from L2) and waits for memory in
+// every 64-deep iteration.  Here a thread holds all its values from the first
+// read: kKeepIts iterations of 8, with 8 lanes per column, or 16 (two columns of a
+// warp at a time), or the whole warp where K is longer.  Two iterations leave room
+// for three CTAs per SM and reach K = 512, four reach 1024.  64 Hubbard composes,
+// int8, S = 5 (1.41 GB read, 0.9 GB written): 566 -> 464 us with two, 479 with
+// four; 8 in BF16: 1151 -> 902.  The same for A (three barriers and a pass through
+// shared memory per iteration, which want more CTAs) was slower: 496 -> 555 us.
+// Before the cut each warp transposes its 256 values of an iteration through
+// shared memory, so that every lane holds 8 consecutive k.  Value e of the 256 sits
+// at e ^ ((e >> 3) & 15): conflict-free both ways.
+template <int S, bool I8, int kKeepIts>
+__global__ void __launch_bounds__(256, kKeepIts == 2 ? 3 : 2) pack_b_keep_kernel(const SplitJob* __restrict__ jobs,
+                                                          const int32_t* __restrict__ group_job, SplitDims dims,
+                                                          const double* __restrict__ B, int64_t sb,
+                                                          double* __restrict__ scales, void* __restrict__ pack) {
+  constexpr double kUnit = I8 ? cut_scale_s8<S>() : cut_scale<S>();
+  __shared__ double tr[8][256];
+  const int64_t group = blockIdx.x, batch = blockIdx.y;
+  const SplitJob J = jobs[group_job[group]];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int P = keep_parts<kKeepIts>(J.k_pad), LPC = 8 << P;
+  const int seg = lane & (LPC - 1), cl = lane >> (3 + P);
+  const int64_t slice_stride = J.n_pad * J.k_pad;
+  double* t = tr[warp];
+  for (int part = 0; part < 1 << P; ++part) {
+    const int64_t col0 = group * 32 - J.b_scale + warp * 4 + part * (4 >> P), col = col0 + cl;
+    if (col0 >= J.n) break;  // padding columns: never reach a written output column
+    const bool live = col < J.n;
+    const double* b = B + batch * sb + J.b_off + col * J.ldb;
+    double x[kKeepIts][8];
+#pragma unroll
+    for (int it = 0; it < kKeepIts; ++it) {
+      const int64_t kf = (int64_t)it * (64 << P), k0 = kf + seg;
+      if (live && kf + (64 << P) <= J.k) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[it][i] = __ldg(b + k0 + LPC * i);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[it][i] = (live && k0 + LPC * i < J.k) ? __ldg(b + k0 + LPC * i) : 0.0;
+      }
+    }
+    uint32_t h = 0;
+#pragma unroll
+    for (int it = 0; it < kKeepIts; ++it)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) h = max(h, hi_abs(x[it][i]));
+#pragma unroll
+    for (int o = 1; o <= 4; o <<= 1) h = max(h, __shfl_xor_sync(0xffffffffu, h, o));
+    if (P > 0) h = max(h, __shfl_xor_sync(0xffffffffu, h, 8));
+    if (P > 1) h = max(h, __shfl_xor_sync(0xffffffffu, h, 16));
+    const bool slow = live && !(h >= kScaleLo && h < kScaleHi);
+    double sigma = 1.0, mul = 0.0;
+    fast_scale(h, kUnit, sigma, mul);
+    if (__any_sync(0xffffffffu, slow)) {
+      double amax = 0.0;
+#pragma unroll
+      for (int it = 0; it < kKeepIts; ++it)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) amax = fmax(amax, fabs(x[it][i]));
+      for (int o = 1; o < LPC; o <<= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+      if (slow) {
+        sigma = pow2_scale(amax);
+        mul = kUnit;
+        const double inv = 1.0 / sigma;
+#pragma unroll
+        for (int it = 0; it < kKeepIts; ++it)
+#pragma unroll
+          for (int i = 0; i < 8; ++i) x[it][i] *= inv;
+      }
+    }
+    if (!live) mul = 0.0;
+    if (seg == 0 && live) scales[batch * dims.bs_stride + J.b_scale + col] = sigma;
+#pragma unroll
+    for (int it = 0; it < kKeepIts; ++it) {
+      if (it * (64 << P) < J.k_pad) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int e = (cl << (6 + P)) + seg + (i << (3 + P));
+          t[e ^ ((e >> 3) & 15)] = x[it][i];
+        }
+        __syncwarp();
+        double y[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) y[j] = t[(8 * lane + j) ^ (lane & 15)];  // k = 8 seg + j of column cl
+        __syncwarp();
+        const int s8 = seg & 7;
+        const int64_t kb64 = ((int64_t)it << P) + (seg >> 3);
+        // 32 k beyond K are not multiplied (int8) and not written
+        if (live && kb64 * 64 + (I8 ? s8 & 4 : 0) * 8 < (I8 ? J.k : J.k_pad)) {
+          if constexpr (I8) {
+            int8_t* dst = static_cast<int8_t*>(pack) + batch * dims.b_stride + J.b_pack + kb64 * J.n_pad * KB8 +
+                          col * KB8 + ((((s8 >> 1) ^ (int)((col >> 1) & 3)) << 4) | ((s8 & 1) << 3));
+            cut8_store_s8<S>(y, dst, slice_stride, mul);
+          } else {
+            const int64_t kb = kb64 * 2 + (s8 >> 2);
+            __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(pack) + batch * dims.b_stride + J.b_pack +
+                                 kb * J.n_pad * KB + col * KB + (((s8 & 3) ^ (int)((col >> 1) & 3)) << 3);
+            cut8_store<S>(y, dst, slice_stride, mul);
+          }
+        }
+      }
     }
   }
 }
@@ -1063,23 +1237,34 @@ void pack_a_launch(cudaStream_t st, const SplitJob* jobs, const int32_t* agj, Sp
   pack_scale_kernel<<<(unsigned)(blocks < 4096 ? blocks : 4096), 256, 0, st>>>(ascale, nscale);
 }
 
+template <int S, bool I8>
+void pack_b_launch(cudaStream_t st, const SplitJob* jobs, const int32_t* bgj, SplitDims dims, const double* b, int64_t sb,
+                   void* bpack, double* bscale, int64_t nbatch, int keep) {
+  const dim3 gb((unsigned)(dims.bs_stride / 32), (unsigned)nbatch);
+  if (keep == 2)
+    pack_b_keep_kernel<S, I8, 2><<<gb, 256, 0, st>>>(jobs, bgj, dims, b, sb, bscale, bpack);
+  else if (keep == 4)
+    pack_b_keep_kernel<S, I8, 4><<<gb, 256, 0, st>>>(jobs, bgj, dims, b, sb, bscale, bpack);
+  else
+    pack_b_kernel<S, I8><<<gb, 256, 0, st>>>(jobs, bgj, dims, b, sb, bscale, bpack);
+}
+
 template <int S>
 cudaError_t split_passes_t(cudaStream_t st, const SplitJob* jobs, const int32_t* agj, const int32_t* bgj, SplitDims dims,
                            const double* a,
                            int64_t sa, void* apack, double* ascale, const double* b, int64_t sb, void* bpack,
-                           double* bscale, int64_t nbatch, bool i8, int kchunks) {
+                           double* bscale, int64_t nbatch, bool i8, int kchunks, int keep) {
   // A null source skips that side (its packs were made beforehand).
-  const dim3 gb((unsigned)(dims.bs_stride / 32), (unsigned)nbatch);
   if (i8) {
     if constexpr (S <= kMaxI8Slices) {
       if (a) pack_a_launch<S, true>(st, jobs, agj, dims, a, sa, apack, ascale, nbatch, kchunks);
-      if (b) pack_b_kernel<S, true><<<gb, 256, 0, st>>>(jobs, bgj, dims, b, sb, bscale, bpack);
+      if (b) pack_b_launch<S, true>(st, jobs, bgj, dims, b, sb, bpack, bscale, nbatch, keep);
     } else {
       return cudaErrorInvalidValue;
     }
   } else {
     if (a) pack_a_launch<S, false>(st, jobs, agj, dims, a, sa, apack, ascale, nbatch, kchunks);
-    if (b) pack_b_kernel<S, false><<<gb, 256, 0, st>>>(jobs, bgj, dims, b, sb, bscale, bpack);
+    if (b) pack_b_launch<S, false>(st, jobs, bgj, dims, b, sb, bpack, bscale, nbatch, keep);
   }
   return cudaGetLastError();
 }
@@ -1087,11 +1272,12 @@ cudaError_t split_passes_t(cudaStream_t st, const SplitJob* jobs, const int32_t*
 cudaError_t launch_split_passes(int S, cudaStream_t st, const SplitJob* jobs, const int32_t* agj, const int32_t* bgj,
                                 SplitDims dims,
                                 const double* a, int64_t sa, void* apack, double* ascale, const double* b, int64_t sb,
-                                void* bpack, double* bscale, int64_t nbatch, bool i8, int kchunks) {
+                                void* bpack, double* bscale, int64_t nbatch, bool i8, int kchunks, int keep) {
   switch (S) {
 #define TNT_SPLIT_CASE(n) \
   case n:                 \
-    return split_passes_t<n>(st, jobs, agj, bgj, dims, a, sa, apack, ascale, b, sb, bpack, bscale, nbatch, i8, kchunks);
+    return split_passes_t<n>(st, jobs, agj, bgj, dims, a, sa, apack, ascale, b, sb, bpack, bscale, nbatch, i8,   \
+                             kchunks, keep);
     TNT_SPLIT_CASE(1) TNT_SPLIT_CASE(2) TNT_SPLIT_CASE(3) TNT_SPLIT_CASE(4)
     TNT_SPLIT_CASE(5) TNT_SPLIT_CASE(6) TNT_SPLIT_CASE(7) TNT_SPLIT_CASE(8)
 #undef TNT_SPLIT_CASE
@@ -1215,6 +1401,13 @@ int pack_a_chunks(const Layout& L, int64_t nbatch) {
   return 1;
 }
 
+// Iterations that B's pass keeps in registers (see pack_b_keep_kernel): 0 where a job's K is beyond it.
+int pack_keeps(const Layout& L) {
+  int64_t k = 0;
+  for (const SplitJob& j : L.jobs) k = std::max(k, j.k_pad);
+  return k <= 512 ? 2 : k <= 1024 ? 4 : 0;
+}
+
 // Byte offsets of one side's slices and scales inside a pre-packed operand
 // (one batch entry): [slices][scales], each 1024-byte aligned.
 struct OperandLayout {
@@ -1253,9 +1446,9 @@ cudaError_t launch_split_pack_operand(const void* job_table, const GemmJob* host
   double* scale = reinterpret_cast<double*>(base + o.scale);
   if (side == 0)
     return launch_split_passes(slices, stream, djobs, agj, bgj, L.dims, src, 0, base + o.pack, scale, nullptr, 0,
-                               nullptr, nullptr, 1, i8, pack_a_chunks(L, 1));
+                               nullptr, nullptr, 1, i8, pack_a_chunks(L, 1), pack_keeps(L));
   return launch_split_passes(slices, stream, djobs, agj, bgj, L.dims, nullptr, 0, nullptr, nullptr, src, 0,
-                             base + o.pack, scale, 1, i8, 1);
+                             base + o.pack, scale, 1, i8, 1, pack_keeps(L));
 }
 
 cudaError_t launch_gemm_split(const void* job_table, const GemmJob* host_jobs, int32_t njobs, const GemmTile* tiles,
@@ -1301,7 +1494,7 @@ cudaError_t launch_gemm_split(const void* job_table, const GemmJob* host_jobs, i
   if (!pre_a || !pre_b) {
     cudaError_t e = launch_split_passes(slices, stream, djobs, agj, bgj, L.dims, pre_a ? nullptr : a, sa, apack,
                                         ascale, pre_b ? nullptr : b, sb, bpack, bscale, nbatch, i8,
-                                        pre_a ? 1 : pack_a_chunks(L, nbatch));
+                                        pre_a ? 1 : pack_a_chunks(L, nbatch), pack_keeps(L));
     if (e != cudaSuccess) return e;
   }
   const uint8_t* ma = static_cast<const uint8_t*>(apack);

@@ -73,3 +73,42 @@ def test_split_edges_match_numpy(shapes, precision, slices, alpha, beta, nbatch)
             for j in range(n):
                 gaps[c0 + j * ldc: c0 + j * ldc + m] = False
         assert np.array_equal(got[q][gaps], c[q][gaps], equal_nan=True)
+
+
+# K per pass over B: two or four iterations in registers, one to three splits of a warp, and the two-pass kernel
+@pytest.mark.parametrize("k", [40, 200, 300, 700, 1500])
+@pytest.mark.parametrize("precision,slices", [("i8", 5), ("bf16", 5)])
+def test_split_scales_over_the_exponent_range(k, precision, slices):
+    """Rows and columns whose scales are at both ends of the exponent range, and zero ones:
+    powers of two commute with the digits, so the bound is the unscaled product's."""
+    import torch
+
+    import tenet_b200 as tb
+    from tenet_b200 import _lib
+    from tenet_b200._lib import arr, call, i64
+
+    rt = tb.Runtime(0)
+    e = np.array([0, -1015, -961, -959, -957, 1020, 1021, 1022, 3, 500] * 4)
+    m = n = len(e)
+    rng = np.random.default_rng(k)
+    A, B = rng.uniform(-1, 1, (m, k)), rng.uniform(-1, 1, (k, n))
+    A[8::10], B[:, 8::10] = 0.0, 0.0
+    As, Bs = np.ldexp(A, e[:, None]), np.ldexp(B, e[None, :])
+    h = C.c_void_p()
+    call("tnt_cplan_from_jobs", 1, arr(i64, [m, n, k, 0, 0, 0, m, k, m]), m * k, k * n, m * n, C.byref(h))
+    da, db = (torch.as_tensor(np.ascontiguousarray(x.T).ravel(), device="cuda") for x in (As, Bs))
+    dc = torch.empty(m * n, dtype=torch.float64, device="cuda")
+    ptr = lambda t: C.c_void_p(t.data_ptr())
+    call("tnt_compose", rt._h, h, 1, ptr(dc), m * n, ptr(da), m * k, ptr(db), k * n, 1.0, 0.0,
+         _lib.PREC_INT8X if precision == "i8" else _lib.PREC_BF16X, slices, rt.stream())
+    got = dc.cpu().numpy().reshape(n, m).T
+    _lib.lib().tnt_cplan_destroy(h)
+    if precision == "i8":
+        unit = 1.01 * (slices + 1) * 2.0 ** (2 - 8 * slices) + 2.0 ** -50
+    else:
+        unit = 1.01 * (slices + 1) * 2.0 ** (-7 * slices) + 2.0 ** -31
+    s = e[:, None] + e[None, :]
+    ok = abs(s) <= 900  # products that FP64 holds
+    assert ok.sum() > m
+    back = np.ldexp(np.where(ok, got, 0.0), np.where(ok, -s, 0))
+    assert np.all(abs(back - np.where(ok, A @ B, 0.0)) <= k * unit)

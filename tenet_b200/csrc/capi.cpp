@@ -142,9 +142,9 @@ struct tnt_xplan_s {
     if (it != dev.end()) return it->second;
     const XformTables& t = p->tables;
     DevXform x;
-    x.groups = upload(t.groups);
-    x.src = upload(t.src_entries);
-    x.dst = upload(t.dst_entries);
+    x.groups = upload(t.fgroups);
+    x.src = upload(t.fsrc);
+    x.dst = upload(t.fdst);
     x.coef = upload(t.coef);
     // One launch per kernel path: tiles grouped by kind (stable within a kind).
     std::vector<XTile> tiles(t.tiles);
@@ -153,6 +153,9 @@ struct tnt_xplan_s {
     for (int k = 1; k < kXKinds; ++k) x.kind_begin[k] = x.kind_begin[k - 1] + x.kind_count[k - 1];
     x.tiles = upload(tiles);
     x.ntiles = (int32_t)tiles.size();
+    x.tr_tiles = upload(t.tr_tiles);
+    x.ntr = (int32_t)t.tr_tiles.size();
+    for (const XTrTile& tl : t.tr_tiles) x.tr_cap = std::max(x.tr_cap, tl.np * tl.r * (tl.jn | 1));
     x.max_nsrc = t.max_nsrc;
     x.max_ndst = t.max_ndst;
     return dev.emplace(d, x).first->second;
@@ -1912,9 +1915,31 @@ tnt_status tnt_xplan_concat(int32_t n, const tnt_xplan* const* plans, const int6
         T.dst_entries.push_back(e);
       }
       T.coef.insert(T.coef.end(), t.coef.begin(), t.coef.end());
+      const int32_t fsbase = (int32_t)T.fsrc.size(), fdbase = (int32_t)T.fdst.size();
+      for (XGroup g : t.fgroups) {
+        g.src_first += fsbase;
+        g.dst_first += fdbase;
+        g.coef_off += cbase;
+        T.fgroups.push_back(g);
+      }
+      for (XEntry e : t.fsrc) {
+        e.offset += src_offs[i];
+        T.fsrc.push_back(e);
+      }
+      for (XEntry e : t.fdst) {
+        e.offset += dst_offs[i];
+        T.fdst.push_back(e);
+      }
       for (XTile tile : t.tiles) {
         tile.group += gbase;
         T.tiles.push_back(tile);
+      }
+      for (XTrTile tile : t.tr_tiles) {
+        tile.group += gbase;
+        tile.src += src_offs[i];
+        tile.dst += dst_offs[i];
+        tile.coef += cbase;
+        T.tr_tiles.push_back(tile);
       }
       T.src_size = std::max(T.src_size, src_offs[i] + t.src_size);
       T.dst_size = std::max(T.dst_size, dst_offs[i] + t.dst_size);

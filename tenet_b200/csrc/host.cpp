@@ -801,42 +801,156 @@ Terms braid_pair_terms(const Rule& r, const TreePair& p, const std::vector<int>&
 //
 // A single-block group whose source is strided along destination axis 0 but
 // contiguous along another axis k* (extent above 1) is a transposing copy
-// (kernel path 4): its tiles are ranges of planes (axis 0 x axis k*) over the
-// remaining axes instead of ranges of columns.
-static int xform_transposing_axis(const XformTables& t, const XGroup& g) {
+// (kernel path 4), cut into tiles of its own: planes (axis 0 x axis k*) over the
+// remaining axes, in pieces that fit the kernel's staging buffer.
+static int xform_transposing_axis(const XGroup& g, const XEntry& e) {
   if (g.nsrc != 1 || g.ndst != 1 || g.rank < 2 || g.dims[0] < 4) return 0;
-  const XEntry& e = t.src_entries[g.src_first];
   if (e.strides[0] == 1) return 0;
   for (int k = 1; k < g.rank; ++k)
     if (e.strides[k] == 1 && g.dims[k] > 1) return g.dims[k] >= 4 ? k : 0;
   return 0;
 }
 
-static void split_tiles(XformTables& t) {
-  t.tiles.clear();
-  const int64_t slots = 148 * 3;
-  auto kind_of = [&](const XGroup& g) { return xform_transposing_axis(t, g) > 0 ? 4 : xform_kind(g); };
-  int64_t total[kXKinds] = {}, ngroups[kXKinds] = {}, target[kXKinds] = {};
+// The group with neighbouring axes merged where every entry, source and
+// destination, steps over the one as over the continuation of the other, and
+// axes of extent 1 left out.  The elements and their order are the same; rows get
+// longer and the rank smaller (a U(1) tensor's (a, b | c, d) -> (c, d | a, b) is a
+// plain matrix transpose of every block).  Axis 0 grows to at most `cap0`, since
+// tiles are made of whole columns.  The kernels write along axis 0 with stride 1,
+// so a leading axis of extent 1 is left out only if the next one has that stride.
+static XGroup fold_group(const XformTables& t, const XGroup& g, int64_t cap0, std::vector<XEntry>& src,
+                         std::vector<XEntry>& dst) {
+  src.assign(t.src_entries.begin() + g.src_first, t.src_entries.begin() + g.src_first + g.nsrc);
+  dst.assign(t.dst_entries.begin() + g.dst_first, t.dst_entries.begin() + g.dst_first + g.ndst);
+  auto every = [&](auto&& f) { return std::all_of(src.begin(), src.end(), f) && std::all_of(dst.begin(), dst.end(), f); };
+  XGroup f = g;
+  int n = 0;  // axes kept, in place: axis n is written at or before the axis k that is read
+  for (int k = 0; k < g.rank; ++k) {
+    const int64_t d = g.dims[k];
+    if (d == 1 && n > 0) continue;
+    if (n == 1 && f.dims[0] == 1 &&
+        std::all_of(dst.begin(), dst.end(), [&](const XEntry& e) { return e.strides[k] == 1; }))
+      n = 0;
+    const int64_t merged = n > 0 ? f.dims[n - 1] * d : 0;
+    if (n > 0 && f.dims[n - 1] > 1 && merged <= (n == 1 ? std::min<int64_t>(cap0, 65535) : 65535) &&
+        every([&](const XEntry& e) { return e.strides[k] == e.strides[n - 1] * f.dims[n - 1]; })) {
+      f.dims[n - 1] = (int32_t)merged;
+      continue;
+    }
+    f.dims[n] = (int32_t)d;
+    for (XEntry& e : src) e.strides[n] = e.strides[k];
+    for (XEntry& e : dst) e.strides[n] = e.strides[k];
+    ++n;
+  }
+  f.rank = n;
+  for (int k = n; k < kMaxRank; ++k) {
+    f.dims[k] = 1;
+    for (XEntry& e : src) e.strides[k] = 0;
+    for (XEntry& e : dst) e.strides[k] = 0;
+  }
+  return f;
+}
+
+static void fold_axes(XformTables& t) {
+  t.fgroups.clear();
+  t.fsrc.clear();
+  t.fdst.clear();
+  int64_t total = 0;
+  for (auto& g : t.groups) total += g.nelem;
+  // Axis 0 of a copy that is not transposing: rows no longer than a slot's share of the plan.
+  const int64_t cap0 = std::min<int64_t>(1024, total / (148 * 3));
+  std::vector<XEntry> src, dst;
   for (auto& g : t.groups) {
-    total[kind_of(g)] += g.nelem;
-    ngroups[kind_of(g)] += 1;
+    int lead = 0;  // a source with stride 1 along the leading axis is not transposed
+    while (lead < g.rank && g.dims[lead] == 1) ++lead;
+    const bool strided = g.nsrc == 1 && g.ndst == 1 && lead < g.rank && t.src_entries[g.src_first].strides[lead] != 1;
+    XGroup f = fold_group(t, g, strided ? 65535 : cap0, src, dst);
+    if (strided && xform_transposing_axis(f, src[0]) == 0) f = fold_group(t, g, cap0, src, dst);
+    f.src_first = (int32_t)t.fsrc.size();
+    f.dst_first = (int32_t)t.fdst.size();
+    t.fsrc.insert(t.fsrc.end(), src.begin(), src.end());
+    t.fdst.insert(t.fdst.end(), dst.begin(), dst.end());
+    t.fgroups.push_back(f);
+  }
+}
+
+// Tiles of one transposing group: pieces of up to `cap` staged doubles (rows
+// padded to an odd length), columns and rows cut evenly, small planes batched.
+static void transposing_tiles(XformTables& t, int32_t gi, int ks, int64_t cap) {
+  const XGroup& g = t.fgroups[gi];
+  const XEntry &s = t.fsrc[g.src_first], &d = t.fdst[g.dst_first];
+  const int64_t d0 = g.dims[0], dj = g.dims[ks], planes = g.nelem / (d0 * dj);
+  auto even = [](int64_t n, int64_t most) { return (n + (n + most - 1) / most - 1) / ((n + most - 1) / most); };
+  const int64_t J = even(dj, cap >= kTrCap / 2 ? 64 : 32), Jp = J | 1, R = even(d0, std::max<int64_t>(1, cap / Jp));
+  XTrTile tile{};
+  tile.s0 = s.strides[0];
+  tile.dks = d.strides[ks];
+  tile.group = gi;
+  tile.ks = ks;
+  tile.coef = g.coef_off;
+  const int64_t per = R == d0 && J == dj ? std::min<int64_t>(kTrPlanes, std::max<int64_t>(1, cap / (R * Jp))) : 1;
+  for (int64_t o = 0; o < planes; o += per) {
+    tile.first = o;
+    tile.np = (int32_t)std::min(per, planes - o);
+    if (tile.np > 1) {
+      tile.src = s.offset;
+      tile.dst = d.offset;
+      tile.r = (int32_t)R;
+      tile.jn = (int32_t)J;
+      t.tr_tiles.push_back(tile);
+      continue;
+    }
+    int64_t sb = s.offset, db = d.offset, rem = o;
+    for (int k = 1; k < g.rank; ++k)
+      if (k != ks) {
+        sb += rem % g.dims[k] * s.strides[k];
+        db += rem % g.dims[k] * d.strides[k];
+        rem /= g.dims[k];
+      }
+    for (int64_t i = 0; i < d0; i += R)
+      for (int64_t j = 0; j < dj; j += J) {
+        tile.src = sb + i * tile.s0 + j;
+        tile.dst = db + i + j * tile.dks;
+        tile.r = (int32_t)std::min(R, d0 - i);
+        tile.jn = (int32_t)std::min(J, dj - j);
+        t.tr_tiles.push_back(tile);
+      }
+  }
+}
+
+static void split_tiles(XformTables& t) {
+  for (auto& g : t.groups)
+    for (int k = 0; k < g.rank; ++k)
+      if (g.dims[k] > 65535) throw std::invalid_argument("a block extent above 65535 is not supported");
+  fold_axes(t);
+  t.tiles.clear();
+  t.tr_tiles.clear();
+  const int64_t slots = 148 * 3;
+  auto axis_of = [&](const XGroup& g) { return g.nsrc == 1 ? xform_transposing_axis(g, t.fsrc[g.src_first]) : 0; };
+  int64_t total[kXKinds + 1] = {}, ngroups[kXKinds + 1] = {}, target[kXKinds] = {};
+  for (auto& g : t.fgroups) {
+    const int kind = axis_of(g) > 0 ? kXTransposing : xform_kind(g);
+    total[kind] += g.nelem;
+    ngroups[kind] += 1;
   }
   for (int k = 0; k < kXKinds; ++k) {
     const int64_t waves = std::max<int64_t>(1, ((total[k] + 32767) / 32768 + ngroups[k] + slots - 1) / slots);
     target[k] = std::min<int64_t>(
         32768, std::max<int64_t>(512, total[k] / std::max<int64_t>(1, waves * slots - ngroups[k])));
   }
-  for (size_t gi = 0; gi < t.groups.size(); ++gi) {
-    const XGroup& g = t.groups[gi];
-    for (int k = 0; k < g.rank; ++k)
-      if (g.dims[k] > 65535) throw std::invalid_argument("a block extent above 65535 is not supported");
-    const int kind = kind_of(g);
-    const int ks = kind == 4 ? xform_transposing_axis(t, g) : 0;
-    // work units: columns (all axes but 0), or planes (all axes but 0 and k*)
-    const int64_t unit = (g.rank > 0 ? g.dims[0] : 1) * (kind == 4 ? g.dims[ks] : 1);
+  // Transposing tiles fill the staging buffer once a plan has two waves of such
+  // tiles; smaller plans spread over the slots.
+  const int64_t tr_cap = std::min<int64_t>(kTrCap, std::max<int64_t>(512, total[kXTransposing] / (2 * slots)));
+  for (size_t gi = 0; gi < t.fgroups.size(); ++gi) {
+    const XGroup& g = t.fgroups[gi];
+    if (const int ks = axis_of(g)) {
+      transposing_tiles(t, (int32_t)gi, ks, tr_cap);
+      continue;
+    }
+    const int kind = xform_kind(g);
+    const int64_t unit = g.rank > 0 ? g.dims[0] : 1;  // work units: columns (all axes but 0)
     const int64_t cols = g.nelem / unit;
-    const int64_t per =
-        std::max<int64_t>(1, kind == 4 ? target[kind] / unit : std::min<int64_t>(256, target[kind] / unit));
+    const int64_t per = std::max<int64_t>(1, std::min<int64_t>(256, target[kind] / unit));
     for (int64_t s = 0; s < cols; s += per) {
       XTile tile;
       tile.group = (int32_t)gi;
@@ -847,9 +961,8 @@ static void split_tiles(XformTables& t) {
     }
   }
   auto elems = [&](const XTile& x) {
-    const XGroup& g = t.groups[x.group];
-    const int64_t unit = (g.rank > 0 ? (int64_t)g.dims[0] : 1) * (x.kind == 4 ? g.dims[xform_transposing_axis(t, g)] : 1);
-    return x.count * unit;
+    const XGroup& g = t.fgroups[x.group];
+    return x.count * (g.rank > 0 ? (int64_t)g.dims[0] : 1);
   };
   std::stable_sort(t.tiles.begin(), t.tiles.end(), [&](const XTile& a, const XTile& b) {
     if (a.kind != b.kind) return a.kind < b.kind;

@@ -30,9 +30,13 @@ struct XGroup {
 // else, 3 = abelian copy with long rows (one source, one destination, d0 >=
 // 64: each column walked down axis 0 with four 16-byte loads in flight),
 // 4 = transposing abelian copy (assigned by the host tiler, which sees the
-// entries: see xform_transposing_axis).  Shared by the host tiler and the
-// device kernels.
-constexpr int kXKinds = 5;
+// entries: see xform_transposing_axis; a kernel and tiles of its own).  Shared by
+// the host tiler and the device kernels.
+constexpr int kXKinds = 4;
+constexpr int kXTransposing = 4;
+// Staging of a transposing tile: doubles per buffer, planes.
+constexpr int kTrCap = 4096;
+constexpr int kTrPlanes = 64;
 inline int xform_kind(const XGroup& g) {
   const int d0 = g.rank > 0 ? g.dims[0] : 1;
   if (g.nsrc == 1 && g.ndst == 1) return d0 < 64 ? 0 : 3;
@@ -57,11 +61,30 @@ struct XTile {
   int64_t count;
 };
 
+// One tile of a transposing copy (kind 4): `np` planes of r x jn elements, rows
+// along destination axis 0, columns along the axis on which the source is
+// contiguous.  np = 1: src and dst are the offsets of the tile's first element.
+// np > 1: planes first .. first + np - 1 of a block whose whole planes are r x jn;
+// src and dst are the block's offsets.
+struct XTrTile {
+  int64_t src, dst;
+  int64_t s0, dks;  // source stride between rows, destination stride between columns
+  int64_t first;
+  int32_t r, jn, np;
+  int32_t group, ks;  // folded group and its contiguous axis
+  int32_t coef;
+};
+
 struct XformTables {
   std::vector<XGroup> groups;
   std::vector<XEntry> src_entries, dst_entries;
   std::vector<double> coef;
+  // What the device runs: the groups with their axes folded (see fold_axes; one
+  // per group, entries of their own), and the tiles over those.
+  std::vector<XGroup> fgroups;
+  std::vector<XEntry> fsrc, fdst;
   std::vector<XTile> tiles;
+  std::vector<XTrTile> tr_tiles;
   int64_t src_size = 0, dst_size = 0;
   int32_t max_nsrc = 0, max_ndst = 0;
 };

@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(kXThreads, 3) xform_kernel(const XTile* __rest
       }
     }
     const bool abelian = KIND == 0 || KIND == 3;
-    for (int c = tid; c < (KIND == 4 ? 0 : ncols); c += kXThreads) {
+    for (int c = tid; c < ncols; c += kXThreads) {
       int64_t col = tile.start + c;
       int64_t sb = 0, db = 0;
       const XEntry* es = abelian ? &src_e[g.src_first] : nullptr;
@@ -114,95 +114,6 @@ __global__ void __launch_bounds__(kXThreads, 3) xform_kernel(const XTile* __rest
     while (W < d0 && W < 32) W <<= 1;
     const int H = kXThreads / W;
     const int tx = tid % W, ty = tid / W;
-
-    if constexpr (KIND == 4) {
-      // Transposing copies (one source and one destination block, source
-      // stride 1 along a destination axis k* > 0, not along axis 0): the
-      // block is a stack of planes (axis 0 x axis k*) over the remaining
-      // axes; a tile is a range of planes.  Planes, cut into sub-planes of at
-      // most 64 columns of k* and as many rows of axis 0 as shared memory
-      // holds, are staged in batches: loaded with consecutive threads along
-      // k* (contiguous in the source), written with consecutive threads along
-      // axis 0 (contiguous in the destination), every lane active.
-      constexpr int kTrCap = 4096;  // doubles of staging
-      constexpr int kTrPlanes = 64;
-      __shared__ double tbuf[kTrCap];
-      __shared__ int64_t pbase[kTrPlanes][2];
-      const double u = alpha * Ug[0];
-      // k*: the first axis after 0 with source stride 1 and extent above 1
-      // (the host assigns this path only when there is one).
-      int ks = 1;
-      while (ks < rank - 1 && !(ent[0].strides[ks] == 1 && g.dims[ks] > 1)) ++ks;
-      const int64_t s0 = ent[0].strides[0], sks = ent[0].strides[ks], dks = ent[1].strides[ks];
-      const int dj = g.dims[ks];
-      const int J = dj < 64 ? dj : 64, Jp = J + 1;
-      const int R = d0 < kTrCap / Jp ? d0 : kTrCap / Jp;
-      const int64_t o_end = tile.start + tile.count;
-      for (int i0 = 0; i0 < d0; i0 += R) {
-        const int r = d0 - i0 < R ? d0 - i0 : R;
-        for (int j0 = 0; j0 < dj; j0 += J) {
-          const int jn = dj - j0 < J ? dj - j0 : J;
-          const int ps = r * Jp;  // staging doubles per plane
-          const int npmax = kTrCap / ps < kTrPlanes ? kTrCap / ps : kTrPlanes;  // >= 1: ps <= kTrCap
-          for (int64_t o0 = tile.start; o0 < o_end; o0 += npmax) {
-            const int np = o_end - o0 < npmax ? (int)(o_end - o0) : npmax;
-            if (tid < np) {
-              int64_t rem = o0 + tid, sb = ent[0].offset, db = ent[1].offset;
-#pragma unroll
-              for (int k = 1; k < kMaxRank; ++k) {
-                if (k < rank && k != ks) {
-                  const int32_t dk = g.dims[k];
-                  const int64_t q = rem / dk;
-                  const int64_t v = rem - q * dk;
-                  rem = q;
-                  sb += v * ent[0].strides[k];
-                  db += v * ent[1].strides[k];
-                }
-              }
-              pbase[tid][0] = sb + (int64_t)i0 * s0 + (int64_t)j0 * sks;
-              pbase[tid][1] = db + i0 + (int64_t)j0 * dks;
-            }
-            __syncthreads();
-            // Load: flat over (plane, row, k* column), k* fastest (contiguous in
-            // the source); eight loads in flight per thread.  Quotients by
-            // float reciprocal: exact here, since e < 4096 keeps the product's
-            // error below 2^-11, under half of 1 / divisor for divisors below 1024.
-            const int n_el = np * r * jn;
-            const float inv_jn = 1.0f / (float)jn, inv_r = 1.0f / (float)r;
-            for (int e0 = tid; e0 < n_el; e0 += 8 * kXThreads) {
-              double v[8];
-              int at[8];
-#pragma unroll
-              for (int q = 0; q < 8; ++q) {
-                const int e = e0 + q * kXThreads;
-                at[q] = -1;
-                if (e < n_el) {
-                  const int row = __float2int_rz(((float)e + 0.5f) * inv_jn), j = e - row * jn;
-                  const int p = __float2int_rz(((float)row + 0.5f) * inv_r), i = row - p * r;
-                  v[q] = __ldg(src + pbase[p][0] + (int64_t)i * s0 + (int64_t)j * sks);
-                  at[q] = p * ps + i * Jp + j;
-                }
-              }
-#pragma unroll
-              for (int q = 0; q < 8; ++q)
-                if (at[q] >= 0) tbuf[at[q]] = v[q];
-            }
-            __syncthreads();
-            // Store: flat over (plane, k* column, row), rows fastest (contiguous
-            // in the destination).
-            for (int e = tid; e < n_el; e += kXThreads) {
-              const int col = __float2int_rz(((float)e + 0.5f) * inv_r), i = e - col * r;
-              const int p = __float2int_rz(((float)col + 0.5f) * inv_jn), j = col - p * jn;
-              const double x = u * tbuf[p * ps + i * Jp + j];
-              double* dp = dst + pbase[p][1] + (int64_t)j * dks + i;
-              *dp = beta == 0.0 ? x : fma(beta, *dp, x);
-            }
-            __syncthreads();
-          }
-        }
-      }
-      continue;
-    }
 
     if constexpr (KIND == 0) {
       // Abelian groups: a scaled permuted copy.  Each thread issues kUnroll
@@ -462,11 +373,145 @@ __global__ void __launch_bounds__(kXThreads, 3) xform_kernel(const XTile* __rest
   }
 }
 
+__device__ __forceinline__ void cp_async8(double* smem, const double* gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem)
+               : "memory");
+}
+
+// Transposing copies (one source and one destination block, source stride 1 along
+// a destination axis k* > 0, not along axis 0).  A tile's planes of r rows (axis 0)
+// x jn columns (axis k*) are loaded along k* and written along axis 0, both
+// contiguous, through shared memory with rows of odd length.
+//
+// Bound by memory: what it takes is enough bytes in flight and few instructions
+// per element.  Loads are cp.async into the second of two buffers while the first
+// is written, positions step by additions (two divisions per tile and thread, not
+// two per element), and folded axes make the planes large.  0.6 GB U(1) tensor,
+// (a, b | c, d) -> (c, d | a, b): 186 -> 129 us, of 93 at the copy rate.
+__global__ void __launch_bounds__(kXThreads, 3) xform_transpose_kernel(
+    const XTrTile* __restrict__ tiles, int32_t ntiles, const XGroup* __restrict__ groups,
+    const XEntry* __restrict__ src_e, const XEntry* __restrict__ dst_e, const double* __restrict__ coef,
+    const double* __restrict__ src, double* __restrict__ dst, double alpha, double beta, int cap) {
+  extern __shared__ double tbuf[];              // [2][cap]
+  __shared__ int64_t pbase[3][kTrPlanes][2];    // first element of each plane, source and destination
+  const int tid = threadIdx.x;
+
+  auto place = [&](const XTrTile& T, int slot) {
+    if (tid >= T.np) return;
+    int64_t sb = T.src, db = T.dst;
+    if (T.np > 1) {
+      const XGroup& g = groups[T.group];
+      const XEntry &es = src_e[g.src_first], &ed = dst_e[g.dst_first];
+      int64_t rem = T.first + tid;
+      for (int k = 1; k < g.rank; ++k) {
+        if (k == T.ks) continue;
+        const int32_t dk = g.dims[k];
+        const int64_t q = rem / dk, v = rem - q * dk;
+        rem = q;
+        sb += v * es.strides[k];
+        db += v * ed.strides[k];
+      }
+    }
+    pbase[slot][tid][0] = sb;
+    pbase[slot][tid][1] = db;
+  };
+  // Visits the elements e = tid, tid + 256, .. of np planes of b x a, position x
+  // along a (fastest), y along b, plane p.  np * a * b <= 4096, so the quotients by
+  // float reciprocal are exact: the error is below 2^-11, under half of 1 / a.
+  auto walk = [&](int a, int b, int np, auto&& f) {
+    const int n = np * a * b;
+    const float inv_a = 1.0f / (float)a, inv_b = 1.0f / (float)b;
+    int y = __float2int_rz(((float)tid + 0.5f) * inv_a), x = tid - y * a;
+    const int dy = __float2int_rz(((float)kXThreads + 0.5f) * inv_a), dx = kXThreads - dy * a;
+    if (np == 1) {
+#pragma unroll 4
+      for (int e = tid; e < n; e += kXThreads) {
+        f(x, y, 0);
+        x += dx;
+        y += dy;
+        if (x >= a) {
+          x -= a;
+          ++y;
+        }
+      }
+      return;
+    }
+    int p = __float2int_rz(((float)y + 0.5f) * inv_b);
+    y -= p * b;
+    const int dp = __float2int_rz(((float)dy + 0.5f) * inv_b), dyb = dy - dp * b;
+#pragma unroll 4
+    for (int e = tid; e < n; e += kXThreads) {
+      f(x, y, p);
+      x += dx;
+      y += dyb;
+      p += dp;
+      if (x >= a) {
+        x -= a;
+        ++y;
+      }
+      if (y >= b) {
+        y -= b;
+        ++p;
+      }
+    }
+  };
+  auto load = [&](const XTrTile& T, double* buf, int slot) {
+    const int jp = T.jn | 1, ps = T.r * jp;
+    if (T.np == 1) {
+      const double* q = src + T.src;
+      walk(T.jn, T.r, 1, [&](int j, int i, int) { cp_async8(buf + i * jp + j, q + i * T.s0 + j); });
+    } else {
+      walk(T.jn, T.r, T.np, [&](int j, int i, int p) {
+        cp_async8(buf + p * ps + i * jp + j, src + pbase[slot][p][0] + i * T.s0 + j);
+      });
+    }
+  };
+  auto store = [&](const XTrTile& T, const double* buf, int slot) {
+    const int jp = T.jn | 1, ps = T.r * jp;
+    const double u = alpha * coef[T.coef];
+    auto put = [&](double* o, double v) { *o = beta == 0.0 ? u * v : fma(beta, *o, u * v); };
+    if (T.np == 1) {
+      double* q = dst + T.dst;
+      walk(T.r, T.jn, 1, [&](int i, int j, int) { put(q + j * T.dks + i, buf[i * jp + j]); });
+    } else {
+      walk(T.r, T.jn, T.np, [&](int i, int j, int p) {
+        put(dst + pbase[slot][p][1] + j * T.dks + i, buf[p * ps + i * jp + j]);
+      });
+    }
+  };
+
+  int32_t t = blockIdx.x;
+  if (t >= ntiles) return;
+  XTrTile cur = tiles[t], nxt = cur;
+  if (t + (int32_t)gridDim.x < ntiles) nxt = tiles[t + gridDim.x];
+  place(cur, 0);
+  __syncthreads();
+  load(cur, tbuf, 0);
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+  for (int it = 0;; ++it) {
+    const bool more = t + (int32_t)gridDim.x < ntiles;
+    // Three sets of plane positions: a thread that is ahead writes the next one
+    // while another still stores with this one's.
+    if (more) place(nxt, (it + 1) % 3);
+    __syncthreads();  // positions are in place, and the other buffer has been written out
+    if (more) load(nxt, tbuf + ((it + 1) & 1) * cap, (it + 1) % 3);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    __syncthreads();  // every thread's part of this tile has arrived
+    const XTrTile done = cur;
+    cur = nxt;
+    t += gridDim.x;
+    if (t + (int32_t)gridDim.x < ntiles) nxt = tiles[t + gridDim.x];
+    store(done, tbuf + (it & 1) * cap, it % 3);
+    if (!more) break;
+  }
+}
+
 }  // namespace
 
 cudaError_t launch_xform(const DevXform& x, double* dst, const double* src, double alpha, double beta,
                          cudaStream_t stream) {
-  if (x.ntiles == 0) return cudaSuccess;
+  if (x.ntiles == 0 && x.ntr == 0) return cudaSuccess;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -481,10 +526,19 @@ cudaError_t launch_xform(const DevXform& x, double* dst, const double* src, doub
       xform_kernel<1><<<grid, kXThreads, 0, stream>>>(t, n, x.groups, x.src, x.dst, x.coef, src, dst, alpha, beta);
     else if (k == 3)
       xform_kernel<3><<<grid, kXThreads, 0, stream>>>(t, n, x.groups, x.src, x.dst, x.coef, src, dst, alpha, beta);
-    else if (k == 4)
-      xform_kernel<4><<<grid, kXThreads, 0, stream>>>(t, n, x.groups, x.src, x.dst, x.coef, src, dst, alpha, beta);
     else
       xform_kernel<2><<<grid, kXThreads, 0, stream>>>(t, n, x.groups, x.src, x.dst, x.coef, src, dst, alpha, beta);
+  }
+  if (x.ntr > 0) {
+    const int smem = 2 * x.tr_cap * (int)sizeof(double);
+    if (smem > 40 * 1024) {  // beyond what a launch may ask for without it, next to the plane positions
+      const cudaError_t e =
+          cudaFuncSetAttribute(xform_transpose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      if (e != cudaSuccess) return e;
+    }
+    const int grid = x.ntr < sms * 3 ? x.ntr : sms * 3;
+    xform_transpose_kernel<<<grid, kXThreads, smem, stream>>>(x.tr_tiles, x.ntr, x.groups, x.src, x.dst, x.coef, src,
+                                                             dst, alpha, beta, x.tr_cap);
   }
   return cudaGetLastError();
 }

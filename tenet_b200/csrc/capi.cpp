@@ -146,7 +146,7 @@ struct tnt_xplan_s {
     x.src = upload(t.fsrc);
     x.dst = upload(t.fdst);
     x.coef = upload(t.coef);
-    // One launch per kernel path: tiles grouped by kind (stable within a kind).
+    // Each kernel path walks its own tiles: grouped by kind (stable within a kind).
     std::vector<XTile> tiles(t.tiles);
     std::stable_sort(tiles.begin(), tiles.end(), [](const XTile& a, const XTile& b) { return a.kind < b.kind; });
     for (const XTile& tl : tiles) x.kind_count[tl.kind] += 1;

@@ -789,7 +789,7 @@ Terms braid_pair_terms(const Rule& r, const TreePair& p, const std::vector<int>&
 // ---------------------------------------------------------------------------
 
 // Work tiles of whole columns (all axes but destination axis 0).  Each
-// kernel path is its own launch, and its tiles are sized to fill whole waves
+// kernel path has CTAs of its own, and its tiles are sized to fill whole waves
 // of the transform kernel's resident CTAs (three per SM on the 148 SMs of a
 // B200): a path is counted in waves of tiles of at most 32768 elements plus
 // one partial tile per group, and the per-tile target divides the path's

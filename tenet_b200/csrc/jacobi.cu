@@ -35,8 +35,8 @@
 // their rounds instead of a CTA-wide barrier measured the same there.)
 // Measured on a B200 against the general kernels of svd.cu and a two-sided
 // Jacobi in shared memory: truncated SVD of the D = 2048 chain (six sectors of
-// 586, two of 293) 94.9 -> 22.4 ms, a whole two-site update at D = 224 (104 x 104)
-// 5.4 -> 1.65 ms, eigh at D = 224 6.4 -> 1.3 ms with eigenvalues to 4e-16 (1.4e-14).
+// 586, two of 293) 94.9 -> 21.8 ms, a whole two-site update at D = 224 (104 x 104)
+// 5.2 -> 1.15 ms, eigh at D = 224 6.4 -> 0.87 ms with eigenvalues to 4e-16 (1.4e-14).
 #include <algorithm>
 
 #include "panel.cuh"

@@ -5,7 +5,7 @@
 // (tenet-operations/src/fusion_replay.rs:556, 1168-1290) with an emulated-FP64
 // product whose error is set by the slice count.
 //
-// Splitting (pack_a_kernel / pack_b_kernel, one fused pass per operand):
+// Splitting (pack_a_kernel / pack_b_keep_kernel, one fused pass per operand):
 // every row of A and every column of B is scaled by a power of two sigma so
 // its largest magnitude is below 1, then cut into S fixed-point slices of 7
 // bits, the balanced base-128 digits of one rounded integer:
@@ -344,9 +344,7 @@ __device__ __forceinline__ void cut8_store_s8(const double (&x)[8], int8_t* dst,
 // takes k = 64 it + 8 w .. + 7.  Pass 1 reduces the row maxima over the whole
 // K (across the 8 warps in shared memory) into the power-of-two scale; pass 2
 // re-reads the same rows (now cached) and writes every slice.  B: one CTA per
-// 32-column group; 8 threads per column, each taking 8 consecutive k (64
-// contiguous doubles of a column per iteration), maxima reduced by shuffles
-// within the 8-lane group.  BF16 slices fill two 32-wide k-blocks per
+// 32-column group, 8 to 32 lanes per column (below).  BF16 slices fill two 32-wide k-blocks per
 // iteration; int8 digits one 64-wide k-block.
 
 // K-chunked packing of A (operands with few rows and a long K, whose fused
@@ -525,102 +523,15 @@ __global__ void __launch_bounds__(256, 4) pack_a_kernel(const SplitJob* __restri
   }
 }
 
-// B: one CTA per 32-column group, one warp per 4 columns, 8 lanes per
-// column.  Loads are coalesced along K (lane j of a column reads
-// k = 64 it + j + 8 i: 64 contiguous bytes per column per load); before the
-// cut, each warp transposes its 4 x 64 values through shared memory so every
-// lane holds 8 consecutive k (the 8-byte digit words).  The shared-memory
-// index k ^ ((k >> 3) & 7) in the low three bits keeps both the strided
-// writes and the consecutive reads at the 2-wavefront minimum.
-template <int S, bool I8>
-__global__ void __launch_bounds__(256, 4) pack_b_kernel(const SplitJob* __restrict__ jobs,
-                                                     const int32_t* __restrict__ group_job, SplitDims dims,
-                                                     const double* __restrict__ B, int64_t sb,
-                                                     double* __restrict__ scales, void* __restrict__ pack) {
-  __shared__ double tr[8][4][64];
-  const int64_t group = blockIdx.x, batch = blockIdx.y;
-  const SplitJob J = jobs[group_job[group]];
-  if (group * 32 - J.b_scale >= J.n) return;  // only padding columns: never reach a written output column
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c = lane >> 3, seg = lane & 7;
-  const int64_t col = group * 32 - J.b_scale + (threadIdx.x >> 3);
-  const bool live = col < J.n;
-  const double* b = B + batch * sb + J.b_off + col * J.ldb;
-  const int64_t nit = J.k_pad / 64;
-  // Loads of one 64-k iteration of this thread: k = 64 it + seg + 8 i.
-  auto load = [&](double (&v)[8], int64_t it) {
-    const int64_t k0 = it * 64 + seg;
-    const double* p = b + k0;
-    if (live && it * 64 + 64 <= J.k) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = __ldg(p + 8 * i);
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = (live && k0 + 8 * i < J.k) ? __ldg(p + 8 * i) : 0.0;
-    }
-  };
-  double amax = 0.0;
-  if (live) {
-    int64_t it = 0;
-    for (; it + 1 < nit; it += 2) {  // two iterations of loads in flight
-      double u[8], v[8];
-      load(u, it);
-      load(v, it + 1);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) amax = fmax(amax, fmax(fabs(u[i]), fabs(v[i])));
-    }
-    if (it < nit) {
-      double u[8];
-      load(u, it);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) amax = fmax(amax, fabs(u[i]));
-    }
-  }
-#pragma unroll
-  for (int o = 4; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  const double sigma = pow2_scale(amax), inv = 1.0 / sigma;
-  if (seg == 0) scales[batch * dims.bs_stride + J.b_scale + col] = sigma;
-  const int64_t slice_stride = J.n_pad * J.k_pad;
-  double* t = &tr[warp][c][0];
-  double x[8];
-  if (nit > 0) load(x, 0);
-  for (int64_t it = 0; it < nit; ++it) {
-    double nx[8];  // the next iteration's loads, in flight while this one is cut
-    if (it + 1 < nit) load(nx, it + 1);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) t[8 * i + (seg ^ i)] = x[i] * inv;  // k = seg + 8 i
-    __syncwarp();
-    double y[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) y[j] = t[8 * seg + (j ^ seg)];  // k = 8 seg + j
-    __syncwarp();
-    if constexpr (I8) {
-      int8_t* dst = static_cast<int8_t*>(pack) + batch * dims.b_stride + J.b_pack + it * J.n_pad * KB8 + col * KB8 +
-                    ((((seg >> 1) ^ (int)((col >> 1) & 3)) << 4) | ((seg & 1) << 3));
-      cut8_store_s8<S>(y, dst, slice_stride);
-    } else {
-      const int64_t kb = it * 2 + (seg >> 2);
-      __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(pack) + batch * dims.b_stride + J.b_pack +
-                           kb * J.n_pad * KB + col * KB + (((seg & 3) ^ (int)((col >> 1) & 3)) << 3);
-      cut8_store<S>(y, dst, slice_stride);
-    }
-    if (it + 1 < nit) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = nx[i];
-    }
-  }
-}
-
 // log2 of the passes over a 32-column group of this K.
 template <int ITS>
 __device__ __forceinline__ int keep_parts(int64_t k_pad) {
   return k_pad <= 64 * ITS ? 0 : k_pad <= 128 * ITS ? 1 : 2;
 }
 
-// B up to K = 1024: one read, values kept in registers.  The kernel above reads B
-// twice (maxima, then digits, the second time from L2) and waits for memory in
-// every 64-deep iteration.  Here a thread holds all its values from the first
-// read: kKeepIts iterations of 8, with 8 lanes per column, or 16 (two columns of a
+// B up to K = 1024: one read, values kept in registers.  Two reads (maxima, then
+// digits, the second time from L2) wait for memory in every 64-deep iteration.
+// Here a thread holds all its values from the first read: kKeepIts iterations of 8, with 8 lanes per column, or 16 (two columns of a
 // warp at a time), or the whole warp where K is longer.  Two iterations leave room
 // for three CTAs per SM and reach K = 512, four reach 1024.  64 Hubbard composes,
 // int8, S = 5 (1.41 GB read, 0.9 GB written): 566 -> 464 us with two, 479 with
@@ -718,6 +629,103 @@ __global__ void __launch_bounds__(256, kKeepIts == 2 ? 3 : 2) pack_b_keep_kernel
                                  kb * J.n_pad * KB + col * KB + (((s8 & 3) ^ (int)((col >> 1) & 3)) << 3);
             cut8_store<S>(y, dst, slice_stride, mul);
           }
+        }
+      }
+    }
+  }
+}
+
+// B beyond K = 1024: a warp per column, which goes through its registers twice in
+// chunks of 1024 (maxima, then digits), all loads of a chunk in flight at once.
+// Each 32-column group is dealt to four CTAs, since such operands have few columns:
+// with one CTA per group and one 64-deep iteration in flight the effective-Hamiltonian
+// network's longest B took 141 us, now 106.
+template <int S, bool I8>
+__global__ void __launch_bounds__(256, 2) pack_b_long_kernel(const SplitJob* __restrict__ jobs,
+                                                          const int32_t* __restrict__ group_job, SplitDims dims,
+                                                          const double* __restrict__ B, int64_t sb,
+                                                          double* __restrict__ scales, void* __restrict__ pack) {
+  constexpr double kUnit = I8 ? cut_scale_s8<S>() : cut_scale<S>();
+  constexpr int kIts = I8 ? 4 : 2;  // four iterations of BF16 slices spill
+  __shared__ double tr[8][256];
+  const int64_t group = blockIdx.x, batch = blockIdx.y;
+  const SplitJob J = jobs[group_job[group]];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, s8 = lane & 7;
+  const int64_t col = group * 32 - J.b_scale + blockIdx.z * 8 + warp;
+  if (col >= J.n) return;  // padding columns: never reach a written output column
+  const int64_t slice_stride = J.n_pad * J.k_pad, nchunk = (J.k_pad + 256 * kIts - 1) / (256 * kIts);
+  const double* b = B + batch * sb + J.b_off + col * J.ldb;
+  double* t = tr[warp];
+  double x[kIts][8];
+  auto load = [&](int64_t chunk) {
+#pragma unroll
+    for (int it = 0; it < kIts; ++it) {
+      const int64_t kf = (chunk * kIts + it) * 256, k0 = kf + lane;
+      if (kf + 256 <= J.k) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[it][i] = __ldg(b + k0 + 32 * i);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[it][i] = k0 + 32 * i < J.k ? __ldg(b + k0 + 32 * i) : 0.0;
+      }
+    }
+  };
+  uint32_t h = 0;
+  for (int64_t chunk = 0; chunk < nchunk; ++chunk) {
+    load(chunk);
+#pragma unroll
+    for (int it = 0; it < kIts; ++it)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) h = max(h, hi_abs(x[it][i]));
+  }
+  h = __reduce_max_sync(0xffffffffu, h);
+  const bool slow = !(h >= kScaleLo && h < kScaleHi);
+  double sigma, mul, inv = 1.0;
+  fast_scale(h, kUnit, sigma, mul);
+  if (slow) {  // the whole warp: one column
+    double amax = 0.0;
+    for (int64_t chunk = 0; chunk < nchunk; ++chunk) {
+      load(chunk);
+#pragma unroll
+      for (int it = 0; it < kIts; ++it)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) amax = fmax(amax, fabs(x[it][i]));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    sigma = pow2_scale(amax);
+    inv = 1.0 / sigma;
+    mul = kUnit;
+  }
+  if (lane == 0) scales[batch * dims.bs_stride + J.b_scale + col] = sigma;
+  for (int64_t chunk = 0; chunk < nchunk; ++chunk) {
+    if (nchunk > 1 || slow) load(chunk);
+#pragma unroll
+    for (int it = 0; it < kIts; ++it) {
+      const int64_t kf = (chunk * kIts + it) * 256;
+      if (kf >= J.k_pad) break;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int e = lane + 32 * i;
+        t[e ^ ((e >> 3) & 15)] = slow ? x[it][i] * inv : x[it][i];
+      }
+      __syncwarp();
+      double y[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) y[j] = t[(8 * lane + j) ^ (lane & 15)];  // k = kf + 8 lane + j
+      __syncwarp();
+      const int64_t kb64 = kf / 64 + (lane >> 3);
+      // 32 k beyond K are not multiplied (int8) and not written
+      if (kb64 * 64 + (I8 ? s8 & 4 : 0) * 8 < (I8 ? J.k : J.k_pad)) {
+        if constexpr (I8) {
+          int8_t* dst = static_cast<int8_t*>(pack) + batch * dims.b_stride + J.b_pack + kb64 * J.n_pad * KB8 +
+                        col * KB8 + ((((s8 >> 1) ^ (int)((col >> 1) & 3)) << 4) | ((s8 & 1) << 3));
+          cut8_store_s8<S>(y, dst, slice_stride, mul);
+        } else {
+          const int64_t kb = kb64 * 2 + (s8 >> 2);
+          __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(pack) + batch * dims.b_stride + J.b_pack +
+                               kb * J.n_pad * KB + col * KB + (((s8 & 3) ^ (int)((col >> 1) & 3)) << 3);
+          cut8_store<S>(y, dst, slice_stride, mul);
         }
       }
     }
@@ -1246,7 +1254,7 @@ void pack_b_launch(cudaStream_t st, const SplitJob* jobs, const int32_t* bgj, Sp
   else if (keep == 4)
     pack_b_keep_kernel<S, I8, 4><<<gb, 256, 0, st>>>(jobs, bgj, dims, b, sb, bscale, bpack);
   else
-    pack_b_kernel<S, I8><<<gb, 256, 0, st>>>(jobs, bgj, dims, b, sb, bscale, bpack);
+    pack_b_long_kernel<S, I8><<<dim3(gb.x, gb.y, 4), 256, 0, st>>>(jobs, bgj, dims, b, sb, bscale, bpack);
 }
 
 template <int S>

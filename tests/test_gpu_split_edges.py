@@ -20,6 +20,7 @@ SHAPES = [
     [(1, 1, 1), (7, 9, 31), (8, 8, 32), (9, 7, 33), (63, 65, 63), (64, 64, 64)],
     [(65, 63, 65), (127, 129, 95), (128, 128, 96), (129, 127, 97), (136, 200, 161), (5, 6, 0)],
     [(130, 256, 40), (255, 257, 600)],
+    [(40, 33, 1100), (20, 40, 1025), (9, 65, 70), (5, 8, 2049), (3, 4, 0)],
     [(20 + i, 150 - i, 30 + i) for i in range(100)],
 ]
 

@@ -804,12 +804,13 @@ cudaError_t launch_cluster(F fn, int njobs, int cl, int threads, size_t smem, cu
 // Outputs
 // ---------------------------------------------------------------------------
 
-__device__ __forceinline__ int64_t warp_argmax_abs(const double* x, int64_t len) {
+template <class X>
+__device__ __forceinline__ int64_t warp_argmax_abs(int64_t len, X&& x) {
   const int lane = threadIdx.x & 31;
   double best = -1.0;
   int64_t at = 0;
   for (int64_t i = lane; i < len; i += 32) {
-    const double v = fabs(x[i]);
+    const double v = fabs(x(i));
     if (v > best) {
       best = v;
       at = i;
@@ -830,7 +831,7 @@ __device__ __forceinline__ int64_t warp_argmax_abs(const double* x, int64_t len)
 constexpr int kFinishWarps = 8;
 
 // Singular triplets in descending order, one warp per column: W's column over its
-// norm and J's column, the left vector's largest-|.| entry positive
+// norm and J's column (rows back from the places of the QR pass), the left vector's largest-|.| entry positive
 // (factorize.rs:3836-3852, 3945-3962; the first maximum wins).
 __global__ void __launch_bounds__(kFinishWarps * 32)
     svd_finish_kernel(const SvdJob* __restrict__ jobs, double* __restrict__ U, double* __restrict__ SV,
@@ -856,10 +857,11 @@ __global__ void __launch_bounds__(kFinishWarps * 32)
   const double* jc = f.J + c * k;
   double* u = U + S.u_off + pos * m;
   double* vh = VH + S.v_off + pos;
-  const double* lv = wide ? jc : wc;
-  const double sign = lv[warp_argmax_abs(lv, wide ? k : m)] < 0.0 ? -1.0 : 1.0;
-  for (int64_t x = lane; x < m; x += 32) u[x] = wide ? sign * jc[x] : sign * wc[x] * inv;
-  for (int64_t x = lane; x < n; x += 32) vh[x * k] = wide ? sign * wc[x] * inv : sign * jc[x];
+  auto j = [&](int64_t x) { return jc[(int)f.rk[x]]; };
+  auto left = [&](int64_t x) { return wide ? j(x) : wc[x]; };
+  const double sign = left(warp_argmax_abs(m, left)) < 0.0 ? -1.0 : 1.0;
+  for (int64_t x = lane; x < m; x += 32) u[x] = wide ? sign * j(x) : sign * wc[x] * inv;
+  for (int64_t x = lane; x < n; x += 32) vh[x * k] = wide ? sign * wc[x] * inv : sign * j(x);
   if (lane == 0) SV[S.s_off + pos] = sc / f.meta[0];
 }
 
@@ -1127,7 +1129,7 @@ __global__ void __launch_bounds__(kFinishWarps * 32)
   if (c >= n) return;
   const FacWork f = fac_work(work + work_off[blockIdx.x], n, n);
   const double* wc = f.W + c * n;
-  const double sign = wc[warp_argmax_abs(wc, n)] < 0.0 ? -1.0 : 1.0;
+  const double sign = wc[warp_argmax_abs(n, [&](int64_t x) { return wc[x]; })] < 0.0 ? -1.0 : 1.0;
   for (int64_t x = lane; x < n; x += 32) VEC[S.u_off + c * n + x] = sign * wc[x];
 }
 

@@ -15,8 +15,8 @@
 // of kernels against one CTA per sector.
 //
 // The SVD factors X^T = Q R once (twice for a rectangular sector, whose first pass
-// makes it square) and gives R^T to the Jacobi engine: its columns are graded and
-// nearly orthogonal, which takes 9 to 10 sweeps where the sector's own columns
+// makes it square; in the last pass the rows of X^T in falling order) and gives R^T to
+// the Jacobi engine: its columns are graded and nearly orthogonal, which takes 9 to 10 sweeps where the sector's own columns
 // take 11 (N(0, 1)) to 18 (a spectrum over three decades) at 104 x 104.
 #include <algorithm>
 
@@ -269,11 +269,40 @@ __global__ void __launch_bounds__(PWD * 32, 1)
   const double* a = A + S.a_off;
   const int64_t gt = (int64_t)rank * blockDim.x + tid, gn = (int64_t)cl * blockDim.x;
 
-  // The SVD scales the sector by a power of two to a largest magnitude in
-  // [1/2, 1), so no product of its Jacobi sweeps leaves the range of a float.
-  double scale = 1.0;
-  if (mode == kQrSvdFirst || (mode == kQrSvdSecond && square)) {
-    double mx = 0.0;
+  // The SVD's last pass takes the rows of X by falling largest entry: Householder QR
+  // is accurate row by row only in that order, and X's rows (a sector's columns, which
+  // can stand decades apart) carry the relative accuracy of the small singular values.
+  // Without it ten decades in random order left 1e-8 of a value, with it 1e-14.
+  // Largest entries to sv, and every CTA counts every row's place (k^2 comparisons in
+  // shared memory); places to rk, for svd_finish_kernel.
+  double mx = 0.0;
+  const int* place = reinterpret_cast<const int*>(s.V + v.nref);
+  if (mode == kQrSvdSecond) {
+    const QrView f1 = qr_view(kQrSvdFirst, S, f, U, VH);
+    const double* rows = square ? a : f1.Y;  // row x of X: contiguous from x * ld
+    const int64_t ld = square ? S.m : f1.ldy;
+    for (int x = rank * PWD + warp; x < v.rows; x += cl * PWD) {
+      double top = 0.0;
+      for (int c = lane; c < (square ? v.ncols : x + 1); c += 32) top = fmax(top, fabs(__ldcg(rows + c + x * ld)));
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+      if (lane == 0) f.sv[x] = top;
+    }
+    cluster_barrier(cl);
+    static_assert(PWD * QrSmem<PWD, PLR>::ldv >= 2 * 32 * PLR, "keys and places fit V");
+    for (int x = tid; x < v.rows; x += PWD * 32) s.V[x] = __ldcg(f.sv + x);
+    __syncthreads();
+    for (int x = tid; x < v.rows; x += PWD * 32) {
+      const double top = s.V[x];
+      int at = 0;
+      for (int o = 0; o < v.rows; ++o) at += (s.V[o] > top || (s.V[o] == top && o < x)) ? 1 : 0;
+      reinterpret_cast<int*>(s.V + v.nref)[x] = at;
+      if (rank == 0) f.rk[x] = (double)at;
+      if (at == 0) red[0] = top;
+    }
+    __syncthreads();
+    mx = red[0];
+  } else if (mode == kQrSvdFirst) {
     for (int64_t i = gt; i < S.m * S.n; i += gn) mx = fmax(mx, fabs(a[i]));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -287,6 +316,11 @@ __global__ void __launch_bounds__(PWD * 32, 1)
     }
     cluster_barrier(cl);
     mx = __longlong_as_double((long long)__ldcg(slot));
+  }
+  // The SVD scales the sector by a power of two to a largest magnitude in
+  // [1/2, 1), so no product of its Jacobi sweeps leaves the range of a float.
+  double scale = 1.0;
+  if (mode == kQrSvdFirst || (mode == kQrSvdSecond && square)) {
     if (mx > 0.0 && mx <= DBL_MAX) {
       int e;
       frexp(mx, &e);
@@ -303,13 +337,13 @@ __global__ void __launch_bounds__(PWD * 32, 1)
   } else if (mode == kQrSvdFirst || square) {  // A^T: X(x, c) = A[c + x ncols]
     for (int64_t i = gt; i < total; i += gn) {
       const int64_t x = i / v.ncols, c = i - x * v.ncols;
-      v.Y[x + c * v.ldy] = a[i] * scale;
+      v.Y[(mode == kQrSvdSecond ? place[x] : x) + c * v.ldy] = a[i] * scale;
     }
   } else {  // R1^T of the first pass, lower triangular
     const QrView f1 = qr_view(kQrSvdFirst, S, f, U, VH);
     for (int64_t i = gt; i < total; i += gn) {
       const int64_t x = i / v.ncols, c = i - x * v.ncols;
-      v.Y[x + c * v.ldy] = c <= x ? __ldcg(f1.Y + c + x * f1.ldy) : 0.0;
+      v.Y[place[x] + c * v.ldy] = c <= x ? __ldcg(f1.Y + c + x * f1.ldy) : 0.0;
     }
   }
   cluster_barrier(cl);

@@ -6,6 +6,12 @@
 // W J = columns orthogonal to 4 sqrt(k) eps, J (SVD only) in the scratch, column
 // norms in sv.
 //
+// The rounding of some 10 k rotations moves the length of J's columns by a random walk
+// and a small bias, and W J's with them (k = 300: -13 eps on average, -34 eps at most; a
+// value's error 25 eps of the largest).  So at the end both are divided by the length
+// of J's column, which leaves the values 4 eps and the product of the factors 23
+// (38 before, 24 by the general kernels).
+//
 // Columns are split into nb blocks (nb even, w columns each); a sweep is a
 // round-robin tournament of the blocks, one pair per CTA and round, with the
 // pairs inside each block rotated in the first round.  What bounds a round is
@@ -117,6 +123,11 @@ __device__ __forceinline__ bool rotation(double al, double be, double ga, const 
   return true;
 }
 
+// 1 / d from an estimate good to a few roundings: the product of the rotations' inverse
+// factors walks away from the inverse of the product, and a rotation whose two
+// coefficients disagree is not orthogonal.
+__device__ __forceinline__ double reciprocal_step(double d, double id) { return fma(id, fma(-d, id, 1.0), id); }
+
 // Sum over the G lanes of a column.
 template <int G>
 __device__ __forceinline__ double group_sum(double v) {
@@ -188,10 +199,11 @@ __device__ __forceinline__ void rotate_smem(bool live, double* base, int ls, int
     if (gl == 0) {
       col.nrm[ip] = al - R.tg;
       col.nrm[iq] = be + R.tg;
-      col.d[ip] = dp * R.c;
-      col.d[iq] = dq * R.c;
-      col.id[ip] = ip_ * R.ic;
-      col.id[iq] = iq_ * R.ic;
+      const double d0 = dp * R.c, d1 = dq * R.c;
+      col.d[ip] = d0;
+      col.d[iq] = d1;
+      col.id[ip] = reciprocal_step(d0, ip_ * R.ic);
+      col.id[iq] = reciprocal_step(d1, iq_ * R.ic);
     }
   }
   __syncwarp();
@@ -427,11 +439,12 @@ __global__ void __launch_bounds__(NW * 32, 1)
               }
             al -= R.tg;
             dp *= R.c;
-            idp *= R.ic;
+            idp = reciprocal_step(dp, idp * R.ic);
             if (gl == 0) {
               col.nrm[w + jq] = be + R.tg;
-              s_d[w + jq] = dq * R.c;
-              s_id[w + jq] = idq * R.ic;
+              const double d = dq * R.c;
+              s_d[w + jq] = d;
+              s_id[w + jq] = reciprocal_step(d, idq * R.ic);
             }
           }
           __syncthreads();
@@ -507,13 +520,17 @@ __global__ void __launch_bounds__(NW * 32, 1)
       const int g = c < w ? bi * w + c : bj * w + c - w;
       if (c < w ? c >= bsize(bi) : c - w >= bsize(bj)) continue;
       const double* d = sm + set * set_len + (int64_t)c * ls;
-      double s = 0.0;
-      for (int x = lane; x < k; x += 32) s = fma(d[x], d[x], s);
-      s = sqrt(warp_sum(s));
-      if (lane == 0) f.sv[g] = s;
+      double s = 0.0, jj = 0.0;
       for (int x = lane; x < k; x += 32) {
-        if (ACC) f.W[(int64_t)g * ldw + x] = d[x];
-        f.J[(int64_t)g * k + x] = ACC ? d[kp + x] : d[x] / s;
+        s = fma(d[x], d[x], s);
+        if (ACC) jj = fma(d[kp + x], d[kp + x], jj);
+      }
+      s = sqrt(warp_sum(s));
+      const double in = ACC ? 1.0 / sqrt(warp_sum(jj)) : 0.0;
+      if (lane == 0) f.sv[g] = ACC ? s * in : s;
+      for (int x = lane; x < k; x += 32) {
+        if (ACC) f.W[(int64_t)g * ldw + x] = d[x] * in;
+        f.J[(int64_t)g * k + x] = ACC ? d[kp + x] * in : d[x] / s;
       }
     }
   }
@@ -699,11 +716,12 @@ __global__ void __launch_bounds__(NW * 32, 1)
               }
               al -= R.tg;
               dp *= R.c;
-              idp *= R.ic;
+              idp = reciprocal_step(dp, idp * R.ic);
               if (lane == 0) {
                 nrm[w + jq] = be + R.tg;
-                s_d[w + jq] = dq * R.c;
-                s_id[w + jq] = idq * R.ic;
+                const double d = dq * R.c;
+                s_d[w + jq] = d;
+                s_id[w + jq] = reciprocal_step(d, idq * R.ic);
               }
             }
           }
@@ -765,15 +783,25 @@ __global__ void __launch_bounds__(NW * 32, 1)
     atomicMax(status + 1, sweep);
   }
   for (int c = rank * NW + warp; c < k; c += cl * NW) {
-    double s = 0.0;
+    double* wc = W + (int64_t)c * ldw;
+    double* jc = J + (int64_t)c * k;
+    double s = 0.0, jj = 0.0;
     for (int x = lane; x < k; x += 32) {
-      const double v = __ldcg(W + (int64_t)c * ldw + x);
+      const double v = __ldcg(wc + x), j = acc_j ? __ldcg(jc + x) : 0.0;
       s = fma(v, v, s);
+      jj = fma(j, j, jj);
     }
     s = sqrt(warp_sum(s));
-    if (lane == 0) f.sv[c] = s;
-    if (!acc_j)  // eigh: the normalised columns
-      for (int x = lane; x < k; x += 32) J[(int64_t)c * k + x] = __ldcg(W + (int64_t)c * ldw + x) / s;
+    const double in = acc_j ? 1.0 / sqrt(warp_sum(jj)) : 0.0;
+    if (lane == 0) f.sv[c] = acc_j ? s * in : s;
+    for (int x = lane; x < k; x += 32) {
+      if (acc_j) {
+        wc[x] = __ldcg(wc + x) * in;
+        jc[x] = __ldcg(jc + x) * in;
+      } else {
+        jc[x] = __ldcg(wc + x) / s;  // eigh: the normalised columns
+      }
+    }
   }
 }
 

@@ -352,6 +352,12 @@ tnt_status tnt_ctx_sync(tnt_ctx* ctx, void* stream);
 /* Jacobi sweeps the slowest sector of the last tnt_svd / tnt_svd_ws on this
  * context needed (diagnostic). */
 tnt_status tnt_ctx_svd_sweeps(const tnt_ctx* ctx, int32_t* sweeps);
+/* How the factorisations take a plan's sectors on a device whose widest cluster is
+ * `wide` CTAs (16, or 0 where only portable clusters of 8 fit).  counts (4): sectors on
+ * the general kernels, of these the ones on clusters and on 16-CTA clusters, and the
+ * number of runs of the others; runs (nullable, 2 per run, at most one run per sector):
+ * sectors and CTAs per sector.  Host only; each device's tables keep their own. */
+tnt_status tnt_fplan_schedule(const tnt_fplan* plan, int32_t wide, int32_t* counts, int32_t* runs);
 /* Doubles of SVD workspace a plan needs (tnt_svd_ws). */
 tnt_status tnt_fplan_work(const tnt_fplan* plan, int64_t* work_elems);
 /* tnt_svd with a caller-provided device workspace of tnt_fplan_work doubles

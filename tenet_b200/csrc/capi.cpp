@@ -233,15 +233,93 @@ struct FacRun {
   bool rectangular = false;  // some sector is not square
 };
 
+// How the factorisations take a plan's sectors on a device whose widest cluster is
+// `wide` CTAs (16, or 0 where only portable clusters of 8 fit): a value of the jobs
+// and that width alone, kept with each device's tables.
+struct FacSchedule {
+  std::vector<size_t> order;  // the largest-first table, as indices of the plan's jobs
+  int32_t n_old = 0;          // its leading jobs, beyond the cluster QR and Jacobi kernels,
+  int32_t n_cluster = 0;      // ... of which the first n_cluster run their SVD on clusters,
+  int32_t n_wide = 0;         // ... and the first n_wide of these on 16-CTA clusters
+  std::vector<FacRun> runs;   // the other jobs, by falling k
+};
+
+static FacSchedule factor_schedule(const std::vector<SvdJob>& jobs, int wide) {
+  FacSchedule S;
+  S.order.resize(jobs.size());
+  for (size_t i = 0; i < S.order.size(); ++i) S.order[i] = i;
+  auto cost = [&](size_t i) {
+    const double r = (double)std::max(jobs[i].m, jobs[i].n), k = (double)jobs[i].k;
+    return r * k * k;
+  };
+  // Sectors too long for the cluster QR and Jacobi kernels (old = true) go
+  // first; of these, the ones whose blocked Jacobi has at least one column block
+  // per cluster CTA run on a thread-block cluster (svd_cluster_kernel), those
+  // with a block for each of 16 CTAs (where the device allows such clusters)
+  // ahead of the 8-CTA ones.  The rest follow by falling k.
+  auto old = [&](size_t i) { return std::max(jobs[i].m, jobs[i].n) > kQrMaxRows; };
+  auto clustered = [&](size_t i) {
+    const int64_t rows = std::max(jobs[i].m, jobs[i].n), k = jobs[i].k;
+    if (!old(i) || svd_on_chip(rows, k)) return 0;
+    const int bw = svd_block_width(rows, k);
+    if (bw <= 0) return 0;
+    const int64_t nb = (k + bw - 1) / bw;
+    return wide > 0 && nb >= wide ? 2 : nb >= svd_cluster_size() ? 1 : 0;
+  };
+  std::stable_sort(S.order.begin(), S.order.end(), [&](size_t a, size_t b) {
+    if (old(a) != old(b)) return old(a);
+    if (!old(a)) return jobs[a].k > jobs[b].k;
+    const int ca = clustered(a), cb = clustered(b);
+    if (ca != cb) return ca > cb;
+    return cost(a) > cost(b);
+  });
+  for (size_t i : S.order) {
+    S.n_old += old(i) ? 1 : 0;
+    S.n_cluster += clustered(i) > 0 ? 1 : 0;
+    S.n_wide += clustered(i) == 2 ? 1 : 0;
+  }
+  // One run per cluster width of the Jacobi kernel, each its own launch; a
+  // narrower run joins the one before it while all clusters of the joint
+  // launch fit the GPU's SMs at once (apart they would run one after the other).
+  std::vector<FacRun>& runs = S.runs;
+  for (size_t i = (size_t)S.n_old; i < S.order.size(); ++i) {
+    const SvdJob& J = jobs[S.order[i]];
+    if (runs.empty() || jacobi_cluster(runs.back().max_k, wide) != jacobi_cluster(J.k, wide)) {
+      FacRun r;
+      r.first = (int32_t)i;
+      r.max_k = J.k;
+      runs.push_back(r);
+    }
+    FacRun& r = runs.back();
+    r.count += 1;
+    r.max_rows = std::max({r.max_rows, J.m, J.n});
+    r.max_cols = std::max(r.max_cols, J.n);
+    r.rectangular |= J.m != J.n;
+  }
+  for (size_t i = runs.size(); i-- > 1;) {
+    FacRun &x = runs[i - 1], &y = runs[i];
+    if ((int64_t)(x.count + y.count) * jacobi_cluster(x.max_k, wide) > 128) continue;
+    x.count += y.count;
+    x.max_rows = std::max(x.max_rows, y.max_rows);
+    x.max_cols = std::max(x.max_cols, y.max_cols);
+    x.rectangular |= y.rectangular;
+    runs.erase(runs.begin() + (long)i);
+  }
+  return S;
+}
+
+// A device's largest-first tables and the schedule they were laid out for.
+struct FacDevice {
+  SvdJob* jobs = nullptr;
+  int64_t* off = nullptr;
+  FacSchedule sched;
+};
+
 struct tnt_fplan_s {
   std::shared_ptr<FactorPlan> p;
   std::mutex mu;
   std::map<int, std::pair<SvdJob*, int64_t*>> dev;  // jobs, work offsets (sector order)
-  std::map<int, std::pair<SvdJob*, int64_t*>> lpt;  // the same, cluster jobs then largest first
-  int32_t n_old = 0;      // leading jobs of the lpt tables beyond the cluster QR and Jacobi kernels
-  int32_t n_cluster = 0;  // ... of which the first n_cluster run their SVD on clusters,
-  int32_t n_wide = 0;     // ... and the first n_wide of these on 16-CTA clusters
-  std::vector<FacRun> runs;  // the other jobs, by falling k
+  std::map<int, FacDevice> lpt;                     // the same, in the order of the schedule
   std::map<int, FplanChunks> chunks;                // weighted-dot chunk tables
   int64_t work_elems = 0;
   std::vector<int64_t> work_off;
@@ -254,8 +332,8 @@ struct tnt_fplan_s {
       cudaFree(kv.second.second);
       auto lt = lpt.find(kv.first);
       if (lt != lpt.end()) {
-        cudaFree(lt->second.first);
-        cudaFree(lt->second.second);
+        cudaFree(lt->second.jobs);
+        cudaFree(lt->second.off);
       }
       auto it = chunks.find(kv.first);
       if (it != chunks.end()) {
@@ -287,90 +365,29 @@ struct tnt_fplan_s {
     dev.emplace(d, r);
     return r;
   }
-  // Job and work-offset tables ordered longest-first (rows * k^2 descending)
-  // for the one-CTA-per-sector factorisation kernels: each job carries its
-  // own output offsets, so the order only changes which CTA starts first,
-  // and the largest sectors no longer start in the last wave.
-  std::pair<SvdJob*, int64_t*> lpt_on_device() {
+  // Job and work-offset tables of the current device in the order of its schedule:
+  // each job carries its own output offsets, so the order only changes which CTA
+  // starts first, and the largest sectors no longer start in the last wave.  An entry
+  // is complete before it is published and never changes, so callers read it without
+  // the lock while other threads add other devices (map nodes do not move).
+  const FacDevice& lpt_on_device() {
     on_device();  // sector-order tables first (needed by truncation and dots)
     int d = current_device();
     std::lock_guard<std::mutex> g(mu);
     auto it = lpt.find(d);
     if (it != lpt.end()) return it->second;
     const auto& jobs = p->tables.jobs;
-    std::vector<size_t> order(jobs.size());
-    for (size_t i = 0; i < order.size(); ++i) order[i] = i;
-    auto cost = [&](size_t i) {
-      const double r = (double)std::max(jobs[i].m, jobs[i].n), k = (double)jobs[i].k;
-      return r * k * k;
-    };
-    // Sectors too long for the cluster QR and Jacobi kernels (old = true) go
-    // first; of these, the ones whose blocked Jacobi has at least one column block
-    // per cluster CTA run on a thread-block cluster (svd_cluster_kernel), those
-    // with a block for each of 16 CTAs (where the device allows such clusters)
-    // ahead of the 8-CTA ones.  The rest follow by falling k.
-    const int wide = svd_wide_cluster_size();
-    auto old = [&](size_t i) { return std::max(jobs[i].m, jobs[i].n) > kQrMaxRows; };
-    auto clustered = [&](size_t i) {
-      const int64_t rows = std::max(jobs[i].m, jobs[i].n), k = jobs[i].k;
-      if (!old(i) || svd_on_chip(rows, k)) return 0;
-      const int bw = svd_block_width(rows, k);
-      if (bw <= 0) return 0;
-      const int64_t nb = (k + bw - 1) / bw;
-      return wide > 0 && nb >= wide ? 2 : nb >= svd_cluster_size() ? 1 : 0;
-    };
-    std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) {
-      if (old(a) != old(b)) return old(a);
-      if (!old(a)) return jobs[a].k > jobs[b].k;
-      const int ca = clustered(a), cb = clustered(b);
-      if (ca != cb) return ca > cb;
-      return cost(a) > cost(b);
-    });
-    n_old = 0;
-    n_cluster = 0;
-    n_wide = 0;
-    for (size_t i = 0; i < order.size(); ++i) {
-      n_old += old(order[i]) ? 1 : 0;
-      n_cluster += clustered(order[i]) > 0 ? 1 : 0;
-      n_wide += clustered(order[i]) == 2 ? 1 : 0;
-    }
-    // One run per cluster width of the Jacobi kernel, each its own launch; a
-    // narrower run joins the one before it while all clusters of the joint
-    // launch fit the GPU's SMs at once (apart they would run one after the other).
-    runs.clear();
-    for (size_t i = (size_t)n_old; i < order.size(); ++i) {
-      const SvdJob& J = jobs[order[i]];
-      const int cl = jacobi_cluster(J.k);
-      if (runs.empty() || jacobi_cluster(runs.back().max_k) != cl) {
-        FacRun r;
-        r.first = (int32_t)i;
-        r.max_k = J.k;
-        runs.push_back(r);
-      }
-      FacRun& r = runs.back();
-      r.count += 1;
-      r.max_rows = std::max({r.max_rows, J.m, J.n});
-      r.max_cols = std::max(r.max_cols, J.n);
-      r.rectangular |= J.m != J.n;
-    }
-    for (size_t i = runs.size(); i-- > 1;) {
-      FacRun &x = runs[i - 1], &y = runs[i];
-      if ((int64_t)(x.count + y.count) * jacobi_cluster(x.max_k) > 128) continue;
-      x.count += y.count;
-      x.max_rows = std::max(x.max_rows, y.max_rows);
-      x.max_cols = std::max(x.max_cols, y.max_cols);
-      x.rectangular |= y.rectangular;
-      runs.erase(runs.begin() + (long)i);
-    }
+    FacDevice x;
+    x.sched = factor_schedule(jobs, svd_wide_cluster_size());
     std::vector<SvdJob> sj(jobs.size());
     std::vector<int64_t> sw(jobs.size());
-    for (size_t i = 0; i < order.size(); ++i) {
-      sj[i] = jobs[order[i]];
-      sw[i] = work_off[order[i]];
+    for (size_t i = 0; i < jobs.size(); ++i) {
+      sj[i] = jobs[x.sched.order[i]];
+      sw[i] = work_off[x.sched.order[i]];
     }
-    auto r = std::make_pair(upload(sj), upload(sw));
-    lpt.emplace(d, r);
-    return r;
+    x.jobs = upload(sj);
+    x.off = upload(sw);
+    return lpt.emplace(d, std::move(x)).first->second;
   }
 };
 
@@ -1615,15 +1632,15 @@ namespace {
 // The batched SVD of a plan: sectors beyond kQrMaxRows on the general Jacobi
 // kernels; the others reduced to R^T (rectangular ones made square first), swept by
 // the cluster Jacobi engine, their factors taken back through the reflectors.
-cudaError_t svd_launches(tnt_fplan_s* plan, std::pair<SvdJob*, int64_t*> dev, const double* a, double* u, double* s,
-                         double* vh, double* work, int32_t* status, cudaStream_t st) {
+cudaError_t svd_launches(const FacDevice& dev, const double* a, double* u, double* s, double* vh, double* work,
+                         int32_t* status, cudaStream_t st) {
+  const FacSchedule& q = dev.sched;
   cudaError_t e = cudaSuccess;
-  if (plan->n_old > 0)
-    e = launch_svd_split(dev.first, plan->n_cluster, plan->n_old, a, u, s, vh, work, dev.second, status, st,
-                         plan->n_wide);
-  for (const FacRun& r : plan->runs) {
-    const SvdJob* j = dev.first + r.first;
-    const int64_t* off = dev.second + r.first;
+  if (q.n_old > 0)
+    e = launch_svd_split(dev.jobs, q.n_cluster, q.n_old, a, u, s, vh, work, dev.off, status, st, q.n_wide);
+  for (const FacRun& r : q.runs) {
+    const SvdJob* j = dev.jobs + r.first;
+    const int64_t* off = dev.off + r.first;
     auto then = [&](cudaError_t x) { e = e == cudaSuccess ? x : e; };
     if (e == cudaSuccess && r.rectangular)
       then(launch_qr_factor(j, r.count, r.max_rows, r.max_k, kQrSvdFirst, a, u, vh, work, off, st));
@@ -1650,7 +1667,7 @@ tnt_status tnt_svd(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, double
     const SvdTables& t = plan->p->tables;
     if (t.jobs.empty()) return;
     need(a && u && s && vh, "null operand");
-    auto dev = plan->lpt_on_device();
+    const FacDevice& dev = plan->lpt_on_device();
     std::lock_guard<std::recursive_mutex> g(ctx->mu);
     if (ctx->svd_work_elems < (size_t)plan->work_elems) {
       cudaFree(ctx->svd_work);
@@ -1661,7 +1678,7 @@ tnt_status tnt_svd(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, double
     }
     cudaStream_t st = (cudaStream_t)stream;
     cuda_check(cudaMemsetAsync(ctx->status, 0, 2 * sizeof(int32_t), st), "memset status");
-    cuda_check(svd_launches(plan, dev, a, u, s, vh, ctx->svd_work, ctx->status, st),
+    cuda_check(svd_launches(dev, a, u, s, vh, ctx->svd_work, ctx->status, st),
                "svd kernel launch");
     int32_t hs[2] = {0, 0};
     cuda_check(cudaMemcpyAsync(hs, ctx->status, sizeof(hs), cudaMemcpyDeviceToHost, st), "read svd status");
@@ -1680,11 +1697,27 @@ tnt_status tnt_svd_ws_async(tnt_ctx* ctx, const tnt_fplan* fplan, const double* 
     const SvdTables& t = plan->p->tables;
     if (t.jobs.empty()) return;
     need(a && u && s && vh && work && status, "null operand");
-    auto dev = plan->lpt_on_device();
+    const FacDevice& dev = plan->lpt_on_device();
     cudaStream_t st = (cudaStream_t)stream;
     cuda_check(cudaMemsetAsync(status, 0, 2 * sizeof(int32_t), st), "memset status");
-    cuda_check(svd_launches(plan, dev, a, u, s, vh, work, status, st),
+    cuda_check(svd_launches(dev, a, u, s, vh, work, status, st),
                "svd kernel launch");
+  });
+}
+
+tnt_status tnt_fplan_schedule(const tnt_fplan* plan, int32_t wide, int32_t* counts, int32_t* runs) {
+  return guarded([&] {
+    need(plan && counts, "null argument");
+    need(wide == 0 || wide == 16, "the widest cluster is 16 CTAs, or 0 where only portable ones fit");
+    const FacSchedule s = factor_schedule(plan->p->tables.jobs, wide);
+    counts[0] = s.n_old;
+    counts[1] = s.n_cluster;
+    counts[2] = s.n_wide;
+    counts[3] = (int32_t)s.runs.size();
+    for (size_t i = 0; runs && i < s.runs.size(); ++i) {
+      runs[2 * i] = s.runs[i].count;
+      runs[2 * i + 1] = jacobi_cluster(s.runs[i].max_k, wide);
+    }
   });
 }
 
@@ -1704,11 +1737,11 @@ tnt_status tnt_svd_ws(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, dou
     const SvdTables& t = plan->p->tables;
     if (t.jobs.empty()) return;
     need(a && u && s && vh && work, "null operand");
-    auto dev = plan->lpt_on_device();
+    const FacDevice& dev = plan->lpt_on_device();
     cudaStream_t st = (cudaStream_t)stream;
     std::lock_guard<std::recursive_mutex> g(ctx->mu);  // the status words are the context's
     cuda_check(cudaMemsetAsync(ctx->status, 0, 2 * sizeof(int32_t), st), "memset status");
-    cuda_check(svd_launches(plan, dev, a, u, s, vh, work, ctx->status, st),
+    cuda_check(svd_launches(dev, a, u, s, vh, work, ctx->status, st),
                "svd kernel launch");
     int32_t hs[2] = {0, 0};
     cuda_check(cudaMemcpyAsync(hs, ctx->status, sizeof(hs), cudaMemcpyDeviceToHost, st), "read svd status");
@@ -1741,14 +1774,14 @@ tnt_status tnt_qr(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, double*
     const SvdTables& t = plan->p->tables;
     if (t.jobs.empty()) return;
     need(a && q && r, "null operand");
-    auto dev = plan->lpt_on_device();
+    const FacDevice& dev = plan->lpt_on_device();
     std::lock_guard<std::recursive_mutex> g(ctx->mu);
     double* work = factor_work(ctx, plan);
     cudaStream_t st = (cudaStream_t)stream;
-    cuda_check(launch_qr(dev.first, plan->n_old, a, q, r, work, dev.second, st), "qr kernel launch");
-    for (const FacRun& x : plan->runs) {
-      const SvdJob* j = dev.first + x.first;
-      const int64_t* off = dev.second + x.first;
+    cuda_check(launch_qr(dev.jobs, dev.sched.n_old, a, q, r, work, dev.off, st), "qr kernel launch");
+    for (const FacRun& x : dev.sched.runs) {
+      const SvdJob* j = dev.jobs + x.first;
+      const int64_t* off = dev.off + x.first;
       cuda_check(launch_qr_factor(j, x.count, x.max_rows, x.max_cols, kQrFactor, a, q, r, work, off, st),
                  "cluster qr launch");
       cuda_check(launch_qr_apply(j, x.count, x.max_rows, x.max_k, kQrFactor, q, r, work, off, st),
@@ -1769,7 +1802,7 @@ tnt_status tnt_eigh(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, doubl
     need(a && vecs && vals, "null operand");
     for (const SvdJob& j : t.jobs)
       need(j.m == j.n, "eigh requires an endomorphism (square coupled-sector blocks)");
-    auto dev = plan->lpt_on_device();
+    const FacDevice& dev = plan->lpt_on_device();
     std::lock_guard<std::recursive_mutex> g(ctx->mu);
     double* work = factor_work(ctx, plan);
     cudaStream_t st = (cudaStream_t)stream;
@@ -1777,7 +1810,7 @@ tnt_status tnt_eigh(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, doubl
     for (const SvdJob& j : t.jobs) max_n = std::max<int64_t>(max_n, j.m);
     cuda_check(cudaMemsetAsync(ctx->status, 0, 2 * sizeof(int32_t), st), "memset status");
     int32_t hs[2] = {0, 0};
-    if (plan->n_old > 0) {
+    if (dev.sched.n_old > 0) {
       // Sectors beyond the cluster engine go through the general SVD of the
       // shifted, positive semidefinite A + ||A||_F I.
       const size_t njobs = t.jobs.size();
@@ -1796,14 +1829,14 @@ tnt_status tnt_eigh(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, doubl
       double* shift = vh + t.v_size;
       int32_t* bad = reinterpret_cast<int32_t*>(shift + njobs);
       cuda_check(cudaMemsetAsync(bad, 0, sizeof(int32_t), st), "memset eigh flag");
-      cuda_check(launch_eigh_by_svd(dev.first, plan->n_cluster, plan->n_old, max_n, a, b, u, sv, vh, shift, bad, vecs,
-                                    vals, mags, work, dev.second, ctx->status, st, plan->n_wide),
+      cuda_check(launch_eigh_by_svd(dev.jobs, dev.sched.n_cluster, dev.sched.n_old, max_n, a, b, u, sv, vh, shift, bad,
+                                    vecs, vals, mags, work, dev.off, ctx->status, st, dev.sched.n_wide),
                  "eigh (shifted SVD) launch");
       cuda_check(cudaMemcpyAsync(&hs[1], bad, sizeof(int32_t), cudaMemcpyDeviceToHost, st), "read eigh flag");
     }
-    for (const FacRun& r : plan->runs) {
-      const SvdJob* j = dev.first + r.first;
-      const int64_t* off = dev.second + r.first;
+    for (const FacRun& r : dev.sched.runs) {
+      const SvdJob* j = dev.jobs + r.first;
+      const int64_t* off = dev.off + r.first;
       cuda_check(launch_eigh_prepare(j, r.count, r.max_k, a, work, off, ctx->status, st), "eigh preparation launch");
       cuda_check(launch_jacobi(j, r.count, r.max_k, work, off, ctx->status, false, st), "eigh sweeps launch");
       cuda_check(launch_eigh_finish(j, r.count, r.max_k, a, vecs, vals, mags, work, off, st), "eigh output launch");

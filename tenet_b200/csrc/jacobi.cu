@@ -1168,15 +1168,12 @@ __global__ void __launch_bounds__(kFinishWarps * 32)
 // the device can co-schedule.  A round costs its latency whatever the width, and
 // a sweep takes k rounds plus an exchange per block pair, so wider clusters
 // add exchanges where they no longer shorten the rounds.
-int jacobi_cluster(int64_t k) {
-  const int wide = svd_wide_cluster_size() > 0 ? 16 : 8;
-  return k <= 64 ? 1 : k <= 128 ? 4 : wide;
-}
+int jacobi_cluster(int64_t k, int wide) { return k <= 64 ? 1 : k <= 128 ? 4 : wide > 0 ? 16 : 8; }
 
 cudaError_t launch_jacobi(const SvdJob* jobs, int32_t njobs, int64_t max_k, double* work, const int64_t* work_off,
                           int32_t* status, bool acc_j, cudaStream_t st) {
   if (njobs == 0) return cudaSuccess;
-  const int cl = jacobi_cluster(max_k);
+  const int cl = jacobi_cluster(max_k, svd_wide_cluster_size());
   const int k = (int)max_k;
 #define TNT_RING(g, pw, nw)                                                                                          \
   if (k <= g * pw) {                                                                                                 \

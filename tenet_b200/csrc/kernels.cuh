@@ -105,7 +105,7 @@ cudaError_t launch_svd(const SvdJob* jobs, int32_t njobs, const double* a, doubl
 // One-sided Jacobi of k x k matrices already in the sectors' scratch (jacobi.cu);
 // max_k (at most kJacobiMaxK) is the largest k of the jobs.
 constexpr int64_t kJacobiMaxK = 1536;
-int jacobi_cluster(int64_t k);
+int jacobi_cluster(int64_t k, int wide);  // wide: svd_wide_cluster_size() of the device
 cudaError_t launch_jacobi(const SvdJob* jobs, int32_t njobs, int64_t max_k, double* work, const int64_t* work_off,
                           int32_t* status, bool acc_j, cudaStream_t stream);
 cudaError_t launch_svd_finish(const SvdJob* jobs, int32_t njobs, int64_t max_k, double* u, double* s, double* vh,

@@ -805,9 +805,13 @@ __global__ void __launch_bounds__(NW * 32, 1)
   }
 }
 
+// The kernel's limit on dynamic shared memory belongs to the device, not to the call:
+// always the engine's bound, never this launch's own need, which another thread's
+// larger launch would find between its own set and its launch.
 template <class F, class... A>
 cudaError_t launch_cluster(F fn, int njobs, int cl, int threads, size_t smem, cudaStream_t st, A... args) {
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (smem > kJacobiSmem) return cudaErrorInvalidValue;
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kJacobiSmem);
   if (e != cudaSuccess) return e;
   if (cl > 8) {
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);

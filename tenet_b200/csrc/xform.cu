@@ -562,8 +562,10 @@ cudaError_t launch_xform(const DevXform& x, double* dst, const double* src, doub
   if (x.ntr > 0) {
     const int smem = 2 * x.tr_cap * (int)sizeof(double);
     if (smem > 40 * 1024) {  // beyond what a launch may ask for without it, next to the plane positions
-      const cudaError_t e =
-          cudaFuncSetAttribute(xform_transpose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      // Always the largest tile's need: the limit is the device's, and another thread's plan
+      // may be launched between this call and the launch.
+      const cudaError_t e = cudaFuncSetAttribute(xform_transpose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 2 * kTrCap * (int)sizeof(double));
       if (e != cudaSuccess) return e;
     }
     const int grid = x.ntr < sms * 3 ? x.ntr : sms * 3;

@@ -132,6 +132,7 @@ struct tnt_xplan_s {
       cudaFree(kv.second.dst);
       cudaFree(kv.second.coef);
       cudaFree(kv.second.tiles);
+      cudaFree(kv.second.tr_tiles);
       if (prev >= 0) cudaSetDevice(prev);
     }
   }

@@ -748,6 +748,19 @@ struct EpiTile {
 template <int TN>
 __host__ __device__ constexpr int epi_slots() { return TN == 64 ? 2 : 1; }
 
+// What follows the stages in shared memory (from a 1024-byte boundary, 1023 bytes in
+// at most: kMmaSlack).
+constexpr int kMaxStages = 4, kMmaSlack = 1024;
+template <int TN>
+struct MmaTail {
+  uint64_t full[kMaxStages], empty[kMaxStages];
+  uint64_t acc_full[2], acc_empty[2];
+  uint64_t epi_full[epi_slots<TN>()], epi_empty[epi_slots<TN>()];
+  uint32_t tmem_slot;
+  int bail;
+  EpiTile<TN> epi[epi_slots<TN>()];
+};
+
 __host__ __device__ constexpr uint32_t tmem_cols_pow2(uint32_t c) {
   return c <= 32 ? 32 : c <= 64 ? 64 : c <= 128 ? 128 : c <= 256 ? 256 : 512;
 }
@@ -790,16 +803,13 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   constexpr int stage_bytes = S * (A_TILE_BYTES + b_tile_bytes<TN>());
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + nstage * stage_bytes);
-  uint64_t* empty = full + nstage;
-  uint64_t* acc_full = empty + nstage;   // [2]
-  uint64_t* acc_empty = acc_full + 2;    // [2]
   constexpr int NEPI = epi_slots<TN>();
-  uint64_t* epi_full = acc_empty + 2;    // [NEPI]
-  uint64_t* epi_empty = epi_full + NEPI; // [NEPI]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(epi_empty + NEPI);
-  volatile int* bail = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  EpiTile<TN>* epi = reinterpret_cast<EpiTile<TN>*>(tmem_slot + 2);
+  MmaTail<TN>& tail = *reinterpret_cast<MmaTail<TN>*>(smem + nstage * stage_bytes);
+  uint64_t *full = tail.full, *empty = tail.empty, *acc_full = tail.acc_full, *acc_empty = tail.acc_empty;
+  uint64_t *epi_full = tail.epi_full, *epi_empty = tail.epi_empty;
+  uint32_t* tmem_slot = &tail.tmem_slot;
+  volatile int* bail = &tail.bail;
+  EpiTile<TN>* epi = tail.epi;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int32_t step = (int32_t)gridDim.x;
@@ -1509,10 +1519,8 @@ cudaError_t launch_gemm_split(const void* job_table, const GemmJob* host_jobs, i
   const uint8_t* mb = static_cast<const uint8_t*>(bpack);
   const int stage_bytes = slices * (A_TILE_BYTES + tile_n * 64);
   const int max_smem = 227 * 1024;
-  // alignment slack, barriers and the epilogue's records beside the stages
-  const int extra = 1024 + 128 + (tile_n == 64 ? epi_slots<64>() * (int)sizeof(EpiTile<64>)
-                                               : epi_slots<128>() * (int)sizeof(EpiTile<128>));
-  int nstage = std::min(4, (max_smem - extra) / stage_bytes);
+  const int extra = kMmaSlack + (int)(tile_n == 64 ? sizeof(MmaTail<64>) : sizeof(MmaTail<128>));
+  int nstage = std::min(kMaxStages, (max_smem - extra) / stage_bytes);
   if (nstage < 1) return cudaErrorInvalidValue;
   const size_t smem = (size_t)nstage * stage_bytes + extra;
   return launch_mma(slices, tile_n, i8, ntiles, smem, stream, ma, mb, djobs, tiles, L.dims, ascale, bscale, c, sc,

@@ -1811,6 +1811,15 @@ tnt_status tnt_eigh(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, doubl
     for (const SvdJob& j : t.jobs) max_n = std::max<int64_t>(max_n, j.m);
     cuda_check(cudaMemsetAsync(ctx->status, 0, 2 * sizeof(int32_t), st), "memset status");
     int32_t hs[2] = {0, 0};
+    int32_t* bad = nullptr;
+    // All sectors are checked and swept before any of them writes its outputs: a call
+    // that fails leaves them as they were.
+    for (const FacRun& r : dev.sched.runs) {
+      const SvdJob* j = dev.jobs + r.first;
+      const int64_t* off = dev.off + r.first;
+      cuda_check(launch_eigh_prepare(j, r.count, r.max_k, a, work, off, ctx->status, st), "eigh preparation launch");
+      cuda_check(launch_jacobi(j, r.count, r.max_k, work, off, ctx->status, false, st), "eigh sweeps launch");
+    }
     if (dev.sched.n_old > 0) {
       // Sectors beyond the cluster engine go through the general SVD of the
       // shifted, positive semidefinite A + ||A||_F I.
@@ -1828,20 +1837,17 @@ tnt_status tnt_eigh(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, doubl
       double* sv = u + t.u_size;
       double* vh = sv + t.s_size;
       double* shift = vh + t.v_size;
-      int32_t* bad = reinterpret_cast<int32_t*>(shift + njobs);
+      bad = reinterpret_cast<int32_t*>(shift + njobs);
       cuda_check(cudaMemsetAsync(bad, 0, sizeof(int32_t), st), "memset eigh flag");
       cuda_check(launch_eigh_by_svd(dev.jobs, dev.sched.n_cluster, dev.sched.n_old, max_n, a, b, u, sv, vh, shift, bad,
                                     vecs, vals, mags, work, dev.off, ctx->status, st, dev.sched.n_wide),
                  "eigh (shifted SVD) launch");
       cuda_check(cudaMemcpyAsync(&hs[1], bad, sizeof(int32_t), cudaMemcpyDeviceToHost, st), "read eigh flag");
     }
-    for (const FacRun& r : dev.sched.runs) {
-      const SvdJob* j = dev.jobs + r.first;
-      const int64_t* off = dev.off + r.first;
-      cuda_check(launch_eigh_prepare(j, r.count, r.max_k, a, work, off, ctx->status, st), "eigh preparation launch");
-      cuda_check(launch_jacobi(j, r.count, r.max_k, work, off, ctx->status, false, st), "eigh sweeps launch");
-      cuda_check(launch_eigh_finish(j, r.count, r.max_k, a, vecs, vals, mags, work, off, st), "eigh output launch");
-    }
+    for (const FacRun& r : dev.sched.runs)
+      cuda_check(launch_eigh_finish(dev.jobs + r.first, r.count, r.max_k, a, vecs, vals, mags, work, dev.off + r.first,
+                                    ctx->status, bad, st),
+                 "eigh output launch");
     cuda_check(cudaMemcpyAsync(&hs[0], ctx->status, sizeof(int32_t), cudaMemcpyDeviceToHost, st), "read eigh status");
     cuda_check(cudaStreamSynchronize(st), "stream synchronize");
     if (hs[1] != 0 || (hs[0] & 2)) throw std::invalid_argument("eigh requires Hermitian coupled-sector blocks");

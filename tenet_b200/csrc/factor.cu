@@ -21,7 +21,7 @@
 // eigh_from_svd_kernel below).
 #include <cfloat>
 
-#include "kernels.cuh"
+#include "panel.cuh"
 
 namespace tnt {
 
@@ -328,7 +328,10 @@ __global__ void __launch_bounds__(kFacThreads) eigh_from_svd_kernel(const SvdJob
                                                                     const double* __restrict__ VH,
                                                                     const double* __restrict__ shift,
                                                                     double* __restrict__ VEC, double* __restrict__ VAL,
-                                                                    double* __restrict__ MAG) {
+                                                                    double* __restrict__ MAG,
+                                                                    const int32_t* __restrict__ status,
+                                                                    const int32_t* __restrict__ bad) {
+  if (panel::factor_failed(status, bad)) return;
   const SvdJob J = jobs[blockIdx.x];
   const int64_t n = J.m, k = J.k;
   if (n == 0) return;
@@ -406,7 +409,7 @@ cudaError_t launch_eigh_by_svd(const SvdJob* jobs, int32_t n_cluster, int32_t nj
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(eigh_from_svd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFacSmemBytes);
   if (e != cudaSuccess) return e;
-  eigh_from_svd_kernel<<<njobs, kFacThreads, post_smem, stream>>>(jobs, s, vh, shift, vecs, vals, mags);
+  eigh_from_svd_kernel<<<njobs, kFacThreads, post_smem, stream>>>(jobs, s, vh, shift, vecs, vals, mags, status, bad);
   return cudaGetLastError();
 }
 

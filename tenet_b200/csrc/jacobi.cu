@@ -1055,9 +1055,13 @@ __device__ __forceinline__ double frag(const double* a, int64_t ld, int r, int x
 constexpr int kRefineWarps = 4;  // a CTA takes a 32 x 32 tile, a warp 16 x 16 of it
 
 // step 0: W = scale A V.  step 1: X (into VEC).  step 2: W[:, rank] = V + V X.
+// From step 1 on the outputs are written, so every kernel leaves a call that has
+// failed alone (a sector that is not Hermitian, or sweeps that did not converge).
 __global__ void __launch_bounds__(kRefineWarps * 32)
     eigh_refine_kernel(const SvdJob* __restrict__ jobs, const double* __restrict__ A, double* __restrict__ VEC,
-                       double* __restrict__ work, const int64_t* __restrict__ work_off, int step) {
+                       double* __restrict__ work, const int64_t* __restrict__ work_off,
+                       const int32_t* __restrict__ status, const int32_t* __restrict__ bad, int step) {
+  if (factor_failed(status, bad)) return;
   const SvdJob S = jobs[blockIdx.x];
   const int n = (int)S.m;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
@@ -1117,7 +1121,10 @@ __global__ void __launch_bounds__(kRefineWarps * 32)
 // ascending value, then index) into rk; the sorted values out.
 __global__ void __launch_bounds__(1024) eigh_values_kernel(const SvdJob* __restrict__ jobs, double* __restrict__ VAL,
                                                            double* __restrict__ MAG, double* __restrict__ work,
-                                                           const int64_t* __restrict__ work_off) {
+                                                           const int64_t* __restrict__ work_off,
+                                                           const int32_t* __restrict__ status,
+                                                           const int32_t* __restrict__ bad) {
+  if (factor_failed(status, bad)) return;
   const SvdJob S = jobs[blockIdx.x];
   const int n = (int)S.m, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   if (n == 0) return;
@@ -1153,7 +1160,9 @@ __global__ void __launch_bounds__(1024) eigh_values_kernel(const SvdJob* __restr
 // Each vector's largest-|.| entry positive (factorize.rs:3902-3913).
 __global__ void __launch_bounds__(kFinishWarps * 32)
     eigh_finish_kernel(const SvdJob* __restrict__ jobs, double* __restrict__ VEC, double* __restrict__ work,
-                       const int64_t* __restrict__ work_off) {
+                       const int64_t* __restrict__ work_off, const int32_t* __restrict__ status,
+                       const int32_t* __restrict__ bad) {
+  if (factor_failed(status, bad)) return;
   const SvdJob S = jobs[blockIdx.x];
   const int64_t n = S.m;
   const int lane = threadIdx.x & 31;
@@ -1231,16 +1240,17 @@ cudaError_t launch_eigh_prepare(const SvdJob* jobs, int32_t njobs, int64_t max_n
 }
 
 cudaError_t launch_eigh_finish(const SvdJob* jobs, int32_t njobs, int64_t max_n, const double* a, double* vecs,
-                               double* vals, double* mags, double* work, const int64_t* work_off, cudaStream_t st) {
+                               double* vals, double* mags, double* work, const int64_t* work_off,
+                               const int32_t* status, const int32_t* bad, cudaStream_t st) {
   if (njobs == 0 || max_n == 0) return cudaSuccess;
   const unsigned nt = (unsigned)((max_n + 31) / 32);
   const dim3 tiles((unsigned)njobs, nt, nt);
-  eigh_refine_kernel<<<tiles, kRefineWarps * 32, 0, st>>>(jobs, a, vecs, work, work_off, 0);
-  eigh_values_kernel<<<njobs, 1024, 0, st>>>(jobs, vals, mags, work, work_off);
-  eigh_refine_kernel<<<tiles, kRefineWarps * 32, 0, st>>>(jobs, a, vecs, work, work_off, 1);
-  eigh_refine_kernel<<<tiles, kRefineWarps * 32, 0, st>>>(jobs, a, vecs, work, work_off, 2);
+  eigh_refine_kernel<<<tiles, kRefineWarps * 32, 0, st>>>(jobs, a, vecs, work, work_off, status, bad, 0);
+  eigh_values_kernel<<<njobs, 1024, 0, st>>>(jobs, vals, mags, work, work_off, status, bad);
+  eigh_refine_kernel<<<tiles, kRefineWarps * 32, 0, st>>>(jobs, a, vecs, work, work_off, status, bad, 1);
+  eigh_refine_kernel<<<tiles, kRefineWarps * 32, 0, st>>>(jobs, a, vecs, work, work_off, status, bad, 2);
   const dim3 grid((unsigned)njobs, (unsigned)((max_n + kFinishWarps - 1) / kFinishWarps));
-  eigh_finish_kernel<<<grid, kFinishWarps * 32, 0, st>>>(jobs, vecs, work, work_off);
+  eigh_finish_kernel<<<grid, kFinishWarps * 32, 0, st>>>(jobs, vecs, work, work_off, status, bad);
   return cudaGetLastError();
 }
 

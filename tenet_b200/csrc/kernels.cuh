@@ -113,7 +113,8 @@ cudaError_t launch_svd_finish(const SvdJob* jobs, int32_t njobs, int64_t max_k, 
 cudaError_t launch_eigh_prepare(const SvdJob* jobs, int32_t njobs, int64_t max_n, const double* a, double* work,
                                 const int64_t* work_off, int32_t* status, cudaStream_t stream);
 cudaError_t launch_eigh_finish(const SvdJob* jobs, int32_t njobs, int64_t max_n, const double* a, double* vecs,
-                               double* vals, double* mags, double* work, const int64_t* work_off, cudaStream_t stream);
+                               double* vals, double* mags, double* work, const int64_t* work_off,
+                               const int32_t* status, const int32_t* bad, cudaStream_t stream);
 
 // Cluster Householder QR of sectors with at most kQrMaxRows rows (qr.cu), and
 // products with its Q; max_rows / max_cols / max_k over the jobs.
@@ -135,7 +136,8 @@ cudaError_t launch_qr(const SvdJob* jobs, int32_t njobs, const double* a, double
 // Eigendecomposition through the batched SVD of B = A + ||A||_F I, for plans
 // with sectors beyond the Jacobi engine: b (a's layout), u, s, vh (the SVD
 // layouts of the plan) and shift (one double per job) are scratch; *bad is
-// set to 1 for a non-Hermitian or non-finite sector (not cleared here).
+// set to 1 for a non-Hermitian or non-finite sector (not cleared here).  Nothing is
+// written to the outputs once *bad or *status says that the call has failed.
 cudaError_t launch_eigh_by_svd(const SvdJob* jobs, int32_t n_cluster, int32_t njobs, int64_t max_n, const double* a,
                                double* b, double* u, double* s, double* vh, double* shift, int32_t* bad,
                                double* vecs, double* vals, double* mags, double* work, const int64_t* work_off,

@@ -60,6 +60,12 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
                : "d"(a), "d"(b));
 }
 
+// Whether a sector of this call was refused (status, bit 1; bad, of the general eigh
+// kernels, may be null) or has not converged (status, bit 0).
+__device__ __forceinline__ bool factor_failed(const int32_t* status, const int32_t* bad) {
+  return *status != 0 || (bad != nullptr && *bad != 0);
+}
+
 // Round-robin pairing of k2 (even) players: round r, pair i.
 __device__ __forceinline__ void tournament_pair(int r, int i, int k2, int& p, int& q) {
   int a, b;

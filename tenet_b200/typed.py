@@ -16,6 +16,7 @@ from __future__ import annotations
 
 import ctypes as C
 import itertools
+import threading
 from dataclasses import dataclass
 from typing import Dict, Optional, Sequence, Tuple
 
@@ -592,6 +593,7 @@ class FactorPlan:
         self._sector_list = space.sectors()
         self._bonds: Dict = {}
         self._ranks: Dict = {}
+        self._kept_lock = threading.Lock()
 
     def __del__(self):
         _release("tnt_fplan_destroy", getattr(self, "_h", None))
@@ -602,11 +604,12 @@ class FactorPlan:
         Its upload is complete before it is first used (a blocking copy), and
         every use records the stream, so any stream may use it and it may be
         dropped while work that reads it is queued."""
-        got = table.get(key)
-        if got is None:
-            while len(table) >= 64:
-                table.pop(next(iter(table)), None)
-            got = table[key] = make()
+        with self._kept_lock:  # several threads may use one plan
+            got = table.get(key)
+            if got is None:
+                while len(table) >= 64:
+                    table.pop(next(iter(table)))
+                got = table[key] = make()
         got[0].record_stream(torch().cuda.current_stream(got[0].device))
         return got
 

@@ -549,6 +549,7 @@ __global__ void __launch_bounds__(256, kKeepIts == 2 ? 3 : 2) pack_b_keep_kernel
   __shared__ double tr[8][256];
   const int64_t group = blockIdx.x, batch = blockIdx.y;
   const SplitJob J = jobs[group_job[group]];
+  if (J.k_pad > 256 * kKeepIts) return;  // pack_b_long_kernel's
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int P = keep_parts<kKeepIts>(J.k_pad), LPC = 8 << P;
   const int seg = lane & (LPC - 1), cl = lane >> (3 + P);
@@ -636,20 +637,24 @@ __global__ void __launch_bounds__(256, kKeepIts == 2 ? 3 : 2) pack_b_keep_kernel
 }
 
 // B beyond K = 1024: a warp per column, which goes through its registers twice in
-// chunks of 1024 (maxima, then digits), all loads of a chunk in flight at once.
-// Each 32-column group is dealt to four CTAs, since such operands have few columns:
+// chunks of 1024 (int8 digits; 512 for BF16 slices), maxima and then digits, all loads
+// of a chunk in flight at once.  Each 32-column group is dealt to four CTAs, since such operands have few columns:
 // with one CTA per group and one 64-deep iteration in flight the effective-Hamiltonian
-// network's longest B took 141 us, now 106.
+// network's longest B took 141 us, now 106.  Sectors up to `kept` are left to
+// pack_b_keep_kernel: a column of K = 64 would use a quarter of its warp's loads (twenty
+// 256 x 2048 x 64 sectors beside one of K = 1100, int8 x5: 55 us all here, now 28).
 template <int S, bool I8>
 __global__ void __launch_bounds__(256, 2) pack_b_long_kernel(const SplitJob* __restrict__ jobs,
                                                           const int32_t* __restrict__ group_job, SplitDims dims,
                                                           const double* __restrict__ B, int64_t sb,
-                                                          double* __restrict__ scales, void* __restrict__ pack) {
+                                                          double* __restrict__ scales, void* __restrict__ pack,
+                                                          int kept) {
   constexpr double kUnit = I8 ? cut_scale_s8<S>() : cut_scale<S>();
   constexpr int kIts = I8 ? 4 : 2;  // four iterations of BF16 slices spill
   __shared__ double tr[8][256];
   const int64_t group = blockIdx.x, batch = blockIdx.y;
   const SplitJob J = jobs[group_job[group]];
+  if (J.k_pad <= kept) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, s8 = lane & 7;
   const int64_t col = group * 32 - J.b_scale + blockIdx.z * 8 + warp;
   if (col >= J.n) return;  // padding columns: never reach a written output column
@@ -1255,23 +1260,30 @@ void pack_a_launch(cudaStream_t st, const SplitJob* jobs, const int32_t* agj, Sp
   pack_scale_kernel<<<(unsigned)(blocks < 4096 ? blocks : 4096), 256, 0, st>>>(ascale, nscale);
 }
 
+// The passes over B that a plan needs: iterations kept in registers (pack_b_keep_kernel;
+// 0: none of its sectors), and whether some K is beyond them (pack_b_long_kernel).
+struct PackKeeps {
+  int its = 0;
+  bool beyond = false;
+};
+
 template <int S, bool I8>
 void pack_b_launch(cudaStream_t st, const SplitJob* jobs, const int32_t* bgj, SplitDims dims, const double* b, int64_t sb,
-                   void* bpack, double* bscale, int64_t nbatch, int keep) {
+                   void* bpack, double* bscale, int64_t nbatch, PackKeeps keep) {
   const dim3 gb((unsigned)(dims.bs_stride / 32), (unsigned)nbatch);
-  if (keep == 2)
+  if (keep.its == 2)
     pack_b_keep_kernel<S, I8, 2><<<gb, 256, 0, st>>>(jobs, bgj, dims, b, sb, bscale, bpack);
-  else if (keep == 4)
+  else if (keep.its == 4)
     pack_b_keep_kernel<S, I8, 4><<<gb, 256, 0, st>>>(jobs, bgj, dims, b, sb, bscale, bpack);
-  else
-    pack_b_long_kernel<S, I8><<<dim3(gb.x, gb.y, 4), 256, 0, st>>>(jobs, bgj, dims, b, sb, bscale, bpack);
+  if (keep.beyond)
+    pack_b_long_kernel<S, I8><<<dim3(gb.x, gb.y, 4), 256, 0, st>>>(jobs, bgj, dims, b, sb, bscale, bpack, 256 * keep.its);
 }
 
 template <int S>
 cudaError_t split_passes_t(cudaStream_t st, const SplitJob* jobs, const int32_t* agj, const int32_t* bgj, SplitDims dims,
                            const double* a,
                            int64_t sa, void* apack, double* ascale, const double* b, int64_t sb, void* bpack,
-                           double* bscale, int64_t nbatch, bool i8, int kchunks, int keep) {
+                           double* bscale, int64_t nbatch, bool i8, int kchunks, PackKeeps keep) {
   // A null source skips that side (its packs were made beforehand).
   if (i8) {
     if constexpr (S <= kMaxI8Slices) {
@@ -1290,7 +1302,7 @@ cudaError_t split_passes_t(cudaStream_t st, const SplitJob* jobs, const int32_t*
 cudaError_t launch_split_passes(int S, cudaStream_t st, const SplitJob* jobs, const int32_t* agj, const int32_t* bgj,
                                 SplitDims dims,
                                 const double* a, int64_t sa, void* apack, double* ascale, const double* b, int64_t sb,
-                                void* bpack, double* bscale, int64_t nbatch, bool i8, int kchunks, int keep) {
+                                void* bpack, double* bscale, int64_t nbatch, bool i8, int kchunks, PackKeeps keep) {
   switch (S) {
 #define TNT_SPLIT_CASE(n) \
   case n:                 \
@@ -1419,11 +1431,19 @@ int pack_a_chunks(const Layout& L, int64_t nbatch) {
   return 1;
 }
 
-// Iterations that B's pass keeps in registers (see pack_b_keep_kernel): 0 where a job's K is beyond it.
-int pack_keeps(const Layout& L) {
-  int64_t k = 0;
-  for (const SplitJob& j : L.jobs) k = std::max(k, j.k_pad);
-  return k <= 512 ? 2 : k <= 1024 ? 4 : 0;
+// Where some K is beyond 1024, pack_b_long_kernel takes K above 512 as well (a warp's loads
+// are at least half used: sixteen 600-deep sectors beside one of 1100 are 28 us so, 34 in two
+// passes), and the rest too unless its columns are worth a pass of their own: about 1 us per
+// 1000 columns in the long kernel against 4 us for a further launch.
+PackKeeps pack_keeps(const Layout& L, int64_t nbatch) {
+  constexpr int64_t kOwnPass = 4096;  // columns
+  int64_t longest = 0, columns = 0;
+  for (const SplitJob& j : L.jobs) {
+    longest = std::max(longest, j.k_pad);
+    if (j.k_pad <= 512) columns += j.n;
+  }
+  if (longest <= 1024) return PackKeeps{longest <= 512 ? 2 : 4, false};
+  return PackKeeps{columns * nbatch >= kOwnPass ? 2 : 0, true};
 }
 
 // Byte offsets of one side's slices and scales inside a pre-packed operand
@@ -1464,9 +1484,9 @@ cudaError_t launch_split_pack_operand(const void* job_table, const GemmJob* host
   double* scale = reinterpret_cast<double*>(base + o.scale);
   if (side == 0)
     return launch_split_passes(slices, stream, djobs, agj, bgj, L.dims, src, 0, base + o.pack, scale, nullptr, 0,
-                               nullptr, nullptr, 1, i8, pack_a_chunks(L, 1), pack_keeps(L));
+                               nullptr, nullptr, 1, i8, pack_a_chunks(L, 1), pack_keeps(L, 1));
   return launch_split_passes(slices, stream, djobs, agj, bgj, L.dims, nullptr, 0, nullptr, nullptr, src, 0,
-                             base + o.pack, scale, 1, i8, 1, pack_keeps(L));
+                             base + o.pack, scale, 1, i8, 1, pack_keeps(L, 1));
 }
 
 cudaError_t launch_gemm_split(const void* job_table, const GemmJob* host_jobs, int32_t njobs, const GemmTile* tiles,
@@ -1512,7 +1532,7 @@ cudaError_t launch_gemm_split(const void* job_table, const GemmJob* host_jobs, i
   if (!pre_a || !pre_b) {
     cudaError_t e = launch_split_passes(slices, stream, djobs, agj, bgj, L.dims, pre_a ? nullptr : a, sa, apack,
                                         ascale, pre_b ? nullptr : b, sb, bpack, bscale, nbatch, i8,
-                                        pre_a ? 1 : pack_a_chunks(L, nbatch), pack_keeps(L));
+                                        pre_a ? 1 : pack_a_chunks(L, nbatch), pack_keeps(L, nbatch));
     if (e != cudaSuccess) return e;
   }
   const uint8_t* ma = static_cast<const uint8_t*>(apack);

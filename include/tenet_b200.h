@@ -282,10 +282,16 @@ tnt_status tnt_compose_packed(tnt_ctx* ctx, const tnt_cplan* plan, double* dst, 
  * stream capture in progress (it times each candidate on the caller's own
  * operands, so make that call before any capture); TNT_AUTOTUNE=0 keeps the
  * model defaults.  No counterpart in the reference (per-sector GEMM calls).
+ * tnt_cplan_f64_tiles: the largest tile side in 16-row blocks that a plan takes for
+ * given costs and SMs, and the tiles that then run (nullable, 6 per tile, longest first:
+ * job, batch entry, first row and column, rows and columns, the last ones of a sector
+ * rounded up to 16).
  * tnt_tuning_info: the device's calibration state, with g and b as the costs of
- * the uniform shapes 64x64, 64x32, 32x64, 32x32; tnt_cplan_tile_shapes: the
- * per-job shape (0 .. 3) minimising ntiles * (ceil(k/16) + 1) * cost[shape] for
- * four given costs. */
+ * the uniform shapes 64x64, 64x32, 32x64, 32x32.  tnt_cplan_tile_shapes (kept for
+ * callers of the four-shape rule; no kernel uses it): the per-job shape (0 .. 3)
+ * minimising ntiles * (ceil(k/16) + 1) * cost[shape] for four given costs. */
+tnt_status tnt_cplan_f64_tiles(const tnt_cplan* plan, int64_t nbatch, double g, double b, int32_t sms, int32_t* cap,
+                               int64_t* ntiles, int64_t max_tiles, int32_t* tiles);
 tnt_status tnt_cplan_tile_shapes(const tnt_cplan* plan, const double* costs, int32_t* shapes);
 tnt_status tnt_tuning_info(int32_t device, double* f64_costs, int32_t* f64_calibrated, double* split_eff64,
                            int32_t* split_calibrated);

@@ -111,6 +111,7 @@ _SIGS = {
     "tnt_split_operand_bytes": [vp, i32, i32, i32, P(C.c_size_t)],
     "tnt_split_pack_operand": [vp, vp, i32, vp, i32, i32, vp, C.c_size_t, vp],
     "tnt_compose_packed": [vp, vp, vp, vp, vp, vp, vp, f64, f64, i32, i32, vp],
+    "tnt_cplan_f64_tiles": [vp, i64, f64, f64, i32, P(i32), P(i64), i64, P(i32)],
     "tnt_cplan_tile_shapes": [vp, P(f64), P(i32)],
     "tnt_tuning_info": [i32, P(f64), P(i32), P(f64), P(i32)],
     "tnt_eigh": [vp, vp, vp, vp, vp, vp, vp],

@@ -6,7 +6,7 @@
 #include <cstring>
 #include <functional>
 #include <map>
-#include <queue>
+#include <tuple>
 
 namespace tnt {
 
@@ -69,27 +69,42 @@ int tile_blocks(const GemmTile& t) { return ((t.shape >> 3) + 1) * ((t.shape & 7
 }  // namespace
 
 std::vector<GemmTile> build_f64_tiles(const std::vector<GemmJob>& jobs, int64_t nbatch, int cap, double g, double b) {
-  std::vector<std::pair<double, GemmTile>> v;
-  for (int64_t q = 0; q < nbatch; ++q)
-    for (size_t j = 0; j < jobs.size(); ++j) {
-      const GemmJob& J = jobs[j];
-      const int mb = blocks16(J.m), nb = blocks16(J.n);
-      const int mt = (mb + cap - 1) / cap, nt = (nb + cap - 1) / cap;
-      if (mt == 0 || nt == 0) continue;
-      // one cost per job (its largest tile's), so a job's tiles stay adjacent
-      const double c = (double)ksteps(J) * (g + b * ceil_div(mb, mt) * ceil_div(nb, nt));
-      for (int x = 0; x < mt; ++x)
-        for (int y = 0; y < nt; ++y) {
-          int m0, h, n0, w;
-          piece(mb, cap, x, m0, h);
-          piece(nb, cap, y, n0, w);
-          v.push_back({c, GemmTile{(int32_t)j, (int32_t)q, m0, n0, f64_tile_code(16 * h, 16 * w), 0}});
-        }
-    }
-  std::stable_sort(v.begin(), v.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
+  // Jobs by falling cost (a job's largest tile's), so that only they are sorted and
+  // the tiles are written in place; a job's tiles stay adjacent, and of jobs of one
+  // cost each batch entry's come together.
+  struct Cut {
+    double cost;
+    int32_t job;
+    int mb, nb, mt, nt;
+  };
+  std::vector<Cut> cuts;
+  cuts.reserve(jobs.size());
+  size_t total = 0;
+  for (size_t j = 0; j < jobs.size(); ++j) {
+    const GemmJob& J = jobs[j];
+    Cut c{0.0, (int32_t)j, blocks16(J.m), blocks16(J.n), 0, 0};
+    c.mt = (c.mb + cap - 1) / cap;
+    c.nt = (c.nb + cap - 1) / cap;
+    if (c.mt == 0 || c.nt == 0) continue;
+    c.cost = (double)ksteps(J) * (g + b * ceil_div(c.mb, c.mt) * ceil_div(c.nb, c.nt));
+    total += (size_t)c.mt * c.nt;
+    cuts.push_back(c);
+  }
+  std::stable_sort(cuts.begin(), cuts.end(), [](const Cut& x, const Cut& y) { return x.cost > y.cost; });
   std::vector<GemmTile> out;
-  out.reserve(v.size());
-  for (auto& x : v) out.push_back(x.second);
+  out.reserve(total * (size_t)nbatch);
+  for (size_t i = 0, e; i < cuts.size(); i = e) {
+    for (e = i + 1; e < cuts.size() && cuts[e].cost == cuts[i].cost;) ++e;
+    for (int64_t q = 0; q < nbatch; ++q)
+      for (size_t c = i; c < e; ++c)
+        for (int x = 0; x < cuts[c].mt; ++x)
+          for (int y = 0; y < cuts[c].nt; ++y) {
+            int m0, h, n0, w;
+            piece(cuts[c].mb, cap, x, m0, h);
+            piece(cuts[c].nb, cap, y, n0, w);
+            out.push_back(GemmTile{cuts[c].job, (int32_t)q, m0, n0, f64_tile_code(16 * h, 16 * w), 0});
+          }
+  }
   return out;
 }
 
@@ -104,30 +119,101 @@ void f64_tile_units(const std::vector<GemmJob>& jobs, const std::vector<GemmTile
 
 int choose_f64_cap(const std::vector<GemmJob>& jobs, int64_t nbatch, double g, double b, int sms) {
   // More tiles than this keep every SM busy at any cap: the sums decide.
-  constexpr size_t kDeal = 20000;
-  int best = kF64MaxBlocks;
+  constexpr double kDeal = 20000;
+  // Jobs of one size count as one: this runs on the first compose of every plan.
+  struct Size {
+    int64_t ks, count;
+    int mb, nb;
+  };
+  std::vector<Size> sizes;
+  sizes.reserve(jobs.size());
+  for (const GemmJob& J : jobs)
+    if (J.m > 0 && J.n > 0) sizes.push_back({ksteps(J), nbatch, blocks16(J.m), blocks16(J.n)});
+  auto key = [](const Size& x) { return std::make_tuple(x.ks, x.mb, x.nb); };
+  std::sort(sizes.begin(), sizes.end(), [&](const Size& x, const Size& y) { return key(x) > key(y); });
+  size_t kinds = 0;
+  for (size_t i = 0; i < sizes.size(); ++i)
+    if (kinds > 0 && key(sizes[kinds - 1]) == key(sizes[i]))
+      sizes[kinds - 1].count += nbatch;
+    else
+      sizes[kinds++] = sizes[i];
+  sizes.resize(kinds);
+
+  // Per cap: tiles by cost, and bounds on the time of a longest-first deal of them to
+  // the SMs: at least the SMs' mean load and the longest tile's chain (alone on its SM
+  // a tile still takes its latency, about six block times, per k-tile), at most the mean
+  // and one tile more.
+  struct Class {
+    double largest, cost;  // of the job's tiles (their place in the list), and of these
+    int64_t count;
+  };
+  struct Option {
+    std::vector<Class> classes;
+    double tiles = 0.0, mean = 0.0, chain = 0.0, least = 0.0, most = 0.0;
+  };
+  Option opt[kF64MaxBlocks + 1];
+  double bound = 0.0;
+  for (int cap = kF64MaxBlocks; cap >= 2; --cap) {
+    Option& o = opt[cap];
+    double top = 0.0;
+    for (const Size& z : sizes) {
+      const int mt = (z.mb + cap - 1) / cap, nt = (z.nb + cap - 1) / cap;
+      const double largest = (double)z.ks * (g + b * ceil_div(z.mb, mt) * ceil_div(z.nb, nt));
+      for (int h = 1; h >= 0; --h)      // pieces one block taller than the others, then these
+        for (int w = 1; w >= 0; --w) {  // and wider
+          const int64_t n = z.count * (h ? z.mb % mt : mt - z.mb % mt) * (w ? z.nb % nt : nt - z.nb % nt);
+          if (n == 0) continue;
+          const double blocks = (double)(z.mb / mt + h) * (z.nb / nt + w), c = (double)z.ks * (g + b * blocks);
+          o.classes.push_back({largest, c, n});
+          o.tiles += (double)n;
+          o.mean += c * (double)n / sms;
+          top = std::max(top, c);
+          o.chain = std::max(o.chain, (double)z.ks * b * (6.0 + blocks));
+        }
+    }
+    const bool deal = o.tiles <= kDeal;
+    o.least = deal ? std::max({o.mean, o.chain, top}) : o.mean;
+    o.most = deal ? std::max(o.mean + top, o.chain) : o.mean;
+    bound = cap == kF64MaxBlocks ? o.most : std::min(bound, o.most);
+  }
+  // Only caps that can still be the best are dealt out.
+  int best = 0, open = 0;
+  for (int cap = kF64MaxBlocks; cap >= 2; --cap)
+    if (opt[cap].least <= bound) {
+      best = open == 0 ? cap : best;
+      ++open;
+    }
+  if (open == 1) return best;
   double best_t = 0.0;
   for (int cap = kF64MaxBlocks; cap >= 2; --cap) {
-    const std::vector<GemmTile> tiles = build_f64_tiles(jobs, nbatch, cap, g, b);
-    double kt, bkt;
-    f64_tile_units(jobs, tiles, kt, bkt);
-    double t = (g * kt + b * bkt) / sms;
-    if (tiles.size() <= kDeal) {
-      // Longest-first deal to the SMs, and the longest chain: alone on its SM a tile
-      // still takes its latency (about six block times) per k-tile.
-      std::priority_queue<double, std::vector<double>, std::greater<double>> load;
-      for (int i = 0; i < sms; ++i) load.push(0.0);
+    Option& o = opt[cap];
+    if (o.least > bound) continue;
+    double t = o.mean;
+    if (o.tiles <= kDeal) {
+      std::sort(o.classes.begin(), o.classes.end(), [](const Class& x, const Class& y) {
+        return std::make_tuple(x.largest, x.cost) > std::make_tuple(y.largest, y.cost);
+      });
+      std::vector<double> load(sms, 0.0);  // a heap, least loaded SM first
       double top = 0.0;
-      for (const GemmTile& x : tiles) {
-        const double ks = (double)ksteps(jobs[x.job]), c = ks * (g + b * tile_blocks(x));
-        const double l = load.top() + c;
-        load.pop();
-        load.push(l);
-        top = std::max({top, l, ks * b * (6.0 + tile_blocks(x))});
+      for (const Class& c : o.classes) {
+        int64_t n = c.count;
+        // Loads within one tile of each other: every SM takes one in each full round.
+        const double low = load.front();
+        if (n >= sms && top - low <= c.cost) {
+          const double add = (double)(n / sms) * c.cost;
+          for (double& l : load) l += add;
+          top += add;
+          n %= sms;
+        }
+        for (; n > 0; --n) {
+          std::pop_heap(load.begin(), load.end(), std::greater<double>());
+          top = std::max(top, load.back() += c.cost);
+          std::push_heap(load.begin(), load.end(), std::greater<double>());
+        }
       }
-      t = top;
+      t = std::max(top, o.chain);
     }
-    if (cap == kF64MaxBlocks || t < best_t) {
+    if (cap == best || t < best_t) {
       best = cap;
       best_t = t;
     }

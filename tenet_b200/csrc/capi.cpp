@@ -1541,6 +1541,24 @@ tnt_status tnt_cplan_tile_shapes(const tnt_cplan* plan, const double* costs, int
   });
 }
 
+tnt_status tnt_cplan_f64_tiles(const tnt_cplan* plan, int64_t nbatch, double g, double b, int32_t sms, int32_t* cap,
+                               int64_t* ntiles, int64_t max_tiles, int32_t* tiles) {
+  return guarded([&] {
+    need(plan && cap && ntiles, "null argument");
+    need(nbatch >= 0 && sms > 0 && g > 0.0 && b > 0.0, "batch count, SMs and costs must be positive");
+    const auto& jobs = plan->p->tables.jobs;
+    *cap = choose_f64_cap(jobs, nbatch, g, b, sms);
+    const std::vector<GemmTile> v = build_f64_tiles(jobs, nbatch, *cap, g, b);
+    *ntiles = (int64_t)v.size();
+    if (!tiles) return;
+    need(max_tiles >= *ntiles, "tile buffer too small");
+    for (const GemmTile& t : v) {
+      const int32_t r[6] = {t.job, t.batch, 16 * t.tm, 16 * t.tn, 16 * ((t.shape >> 3) + 1), 16 * ((t.shape & 7) + 1)};
+      tiles = std::copy(r, r + 6, tiles);
+    }
+  });
+}
+
 tnt_status tnt_tuning_info(int32_t device, double* f64_costs, int32_t* f64_calibrated, double* split_eff64,
                            int32_t* split_calibrated) {
   return guarded([&] {

@@ -55,13 +55,16 @@ cudaError_t launch_gemm_f64(const GemmJob* jobs, const GemmTile* tiles, int32_t 
                             cudaStream_t stream);
 
 // FP64 grouped GEMM of plans whose every K is at most kThinMaxK (gemm_thin.cu):
-// one streaming pass over tiles of kThinRows x kThinCols outputs, or ranges of
-// columns where a job has fewer than kThinWide rows.
-constexpr int kThinMaxK = 8, kThinRows = 512, kThinCols = 32, kThinWide = 32, kThinWideElems = 2048;
+// one streaming pass over tiles of rows x columns, or ranges of columns where a job has
+// fewer than kThinWide rows.
+constexpr int kThinMaxK = 8, kThinPitch = kThinMaxK + 1;  // pitch of a staged column: odd, conflict-free
+constexpr int kThinThreads = 256, kThinRows = 512, kThinCols = 256;
+constexpr int kThinWide = 9, kThinTall = 1024, kThinWideElems = 2048;
 struct ThinTile {
   int32_t job, batch;
   int64_t row, col;
   int32_t nrow, ncol;
+  int32_t lanes;  // threads along the rows (kThinThreads: each takes several)
 };
 bool thin_plan(const std::vector<GemmJob>& jobs);
 std::vector<ThinTile> build_thin_tiles(const std::vector<GemmJob>& jobs, int64_t nbatch);

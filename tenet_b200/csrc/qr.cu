@@ -529,11 +529,18 @@ cudaError_t apply_class(const SvdJob* jobs, int32_t njobs, int64_t max_k, double
   return cudaGetLastError();
 }
 
-// CTAs of a sector's cluster: one while the trailing update is a few column
-// groups, up to 16 where it is the larger part.
-int qr_cluster(int64_t max_cols) {
+// CTAs of a sector's cluster: one while the trailing update is a few column groups, up
+// to 16 where it is the larger part; but no wider than lets every cluster of the launch
+// run at once (a CTA fills its SM, and eight clusters of 16, 16 of 8, 36 of 4 or 74 of 2 fit
+// 148 SMs in their GPCs).  A second wave costs as much as the first, a narrower cluster
+// at most a third more: 300 x 300 sectors, 1 / 10 / 37 / 80 of them, in ms:
+//   16 CTAs 0.79 / 1.48 / 4.40 / 8.80, 8 0.82 / 0.82 / 2.42 / 4.83, 4 0.88 / 0.89 / 1.83 / 2.86,
+//   2 1.01 / 1.02 / 1.18 / 2.34, 1 1.27 / 1.27 / 1.44 / 1.75.
+int qr_cluster(int64_t max_cols, int32_t njobs) {
   const int wide = svd_wide_cluster_size() > 0 ? 16 : 8;
-  return max_cols <= 48 ? 1 : max_cols <= 128 ? 4 : max_cols <= 256 ? 8 : wide;
+  const int most = max_cols <= 48 ? 1 : max_cols <= 128 ? 4 : max_cols <= 256 ? 8 : wide;
+  const int fits = njobs <= 8 ? 16 : njobs <= 16 ? 8 : njobs <= 36 ? 4 : njobs <= 74 ? 2 : 1;
+  return std::min(most, fits);
 }
 
 }  // namespace
@@ -542,7 +549,7 @@ cudaError_t launch_qr_factor(const SvdJob* jobs, int32_t njobs, int64_t max_rows
                              const double* a, double* u, double* vh, double* work, const int64_t* work_off,
                              cudaStream_t st) {
   if (njobs == 0) return cudaSuccess;
-  const int cl = qr_cluster(max_cols);
+  const int cl = qr_cluster(max_cols, njobs);
   if (max_rows <= 64) return factor_class<32, 2>(jobs, njobs, a, u, vh, work, work_off, cl, mode, st);
   if (max_rows <= 256) return factor_class<32, 8>(jobs, njobs, a, u, vh, work, work_off, cl, mode, st);
   if (max_rows <= 640) return factor_class<32, 20>(jobs, njobs, a, u, vh, work, work_off, cl, mode, st);

@@ -359,9 +359,10 @@ tnt_status tnt_ctx_sync(tnt_ctx* ctx, void* stream);
  * context needed (diagnostic). */
 tnt_status tnt_ctx_svd_sweeps(const tnt_ctx* ctx, int32_t* sweeps);
 /* How the factorisations take a plan's sectors on a device whose widest cluster is
- * `wide` CTAs (16, or 0 where only portable clusters of 8 fit).  counts (4): sectors on
- * the general kernels, of these the ones on clusters and on 16-CTA clusters, and the
- * number of runs of the others; runs (nullable, 2 per run, at most one run per sector):
+ * `wide` CTAs (16, or 0 where only portable clusters of 8 fit).  counts (6): sectors on
+ * the general kernels, of these the ones on clusters and on 16-CTA clusters, the
+ * number of runs of the others, and whether (0 or 1) the SVD and the QR take all sectors
+ * in one launch of the one-CTA kernels because they have few columns; runs (nullable, 2 per run, at most one run per sector):
  * sectors and CTAs per sector.  Host only; each device's tables keep their own. */
 tnt_status tnt_fplan_schedule(const tnt_fplan* plan, int32_t wide, int32_t* counts, int32_t* runs);
 /* Doubles of SVD workspace a plan needs (tnt_svd_ws). */

@@ -243,6 +243,7 @@ struct FacSchedule {
   int32_t n_cluster = 0;      // ... of which the first n_cluster run their SVD on clusters,
   int32_t n_wide = 0;         // ... and the first n_wide of these on 16-CTA clusters
   std::vector<FacRun> runs;   // the other jobs, by falling k
+  bool few_svd = false, few_qr = false;  // all jobs have few columns: the one-CTA kernels in one launch
 };
 
 static FacSchedule factor_schedule(const std::vector<SvdJob>& jobs, int wide) {
@@ -274,6 +275,22 @@ static FacSchedule factor_schedule(const std::vector<SvdJob>& jobs, int wide) {
     if (ca != cb) return ca > cb;
     return cost(a) > cost(b);
   });
+  // The engine's four to six launches cost more than they gain where every sector has
+  // few columns: one sector or a hundred of 4 x 4, SVD 65 us against 44 in one launch, QR 30
+  // against 22.  The SVD's one-CTA kernel has a CTA's shared memory to itself and rotates
+  // on full columns, so from 5 columns on it takes one wave of sectors of up to 640 rows
+  // (300 of 5 x 5: 119 against 111 us; 1400 x 5: 131 against 120).  The QR's walks a column
+  // per reflector in every warp: tall sectors up to 3000 elements (600 x 5 40 against 48 us,
+  // 1400 x 3 52 against 42), wide ones by their trailing updates (200 columns: 4 rows 35
+  // against 38 us, 5 rows 42 against 38), for which many sectors have narrower clusters
+  // (600 columns and 4 rows, one 64 against 45, 60 of them 65 against 78, 148 66 against 115).
+  const int64_t wide_most = jobs.size() <= 36 ? 4096 : jobs.size() <= 74 ? 10000 : 20000;
+  S.few_svd = S.few_qr = !jobs.empty();
+  for (const SvdJob& J : jobs) {
+    const int64_t rows = std::max(J.m, J.n);
+    S.few_svd &= rows <= kQrMaxRows && (J.k <= 4 || (J.k <= 8 && jobs.size() <= 148 && rows <= 640));
+    S.few_qr &= J.k <= 8 && (J.m >= J.n ? J.m * J.n <= 3000 : J.n * J.m * J.m <= wide_most);
+  }
   for (size_t i : S.order) {
     S.n_old += old(i) ? 1 : 0;
     S.n_cluster += clustered(i) > 0 ? 1 : 0;
@@ -1654,6 +1671,7 @@ namespace {
 cudaError_t svd_launches(const FacDevice& dev, const double* a, double* u, double* s, double* vh, double* work,
                          int32_t* status, cudaStream_t st) {
   const FacSchedule& q = dev.sched;
+  if (q.few_svd) return launch_svd(dev.jobs, (int32_t)q.order.size(), a, u, s, vh, work, dev.off, status, st, true);
   cudaError_t e = cudaSuccess;
   if (q.n_old > 0)
     e = launch_svd_split(dev.jobs, q.n_cluster, q.n_old, a, u, s, vh, work, dev.off, status, st, q.n_wide);
@@ -1733,6 +1751,8 @@ tnt_status tnt_fplan_schedule(const tnt_fplan* plan, int32_t wide, int32_t* coun
     counts[1] = s.n_cluster;
     counts[2] = s.n_wide;
     counts[3] = (int32_t)s.runs.size();
+    counts[4] = s.few_svd ? 1 : 0;
+    counts[5] = s.few_qr ? 1 : 0;
     for (size_t i = 0; runs && i < s.runs.size(); ++i) {
       runs[2 * i] = s.runs[i].count;
       runs[2 * i + 1] = jacobi_cluster(s.runs[i].max_k, wide);
@@ -1797,8 +1817,11 @@ tnt_status tnt_qr(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, double*
     std::lock_guard<std::recursive_mutex> g(ctx->mu);
     double* work = factor_work(ctx, plan);
     cudaStream_t st = (cudaStream_t)stream;
-    cuda_check(launch_qr(dev.jobs, dev.sched.n_old, a, q, r, work, dev.off, st), "qr kernel launch");
-    for (const FacRun& x : dev.sched.runs) {
+    const FacSchedule& sched = dev.sched;
+    const int32_t one_cta = sched.few_qr ? (int32_t)sched.order.size() : sched.n_old;
+    cuda_check(launch_qr(dev.jobs, one_cta, a, q, r, work, dev.off, st), "qr kernel launch");
+    for (const FacRun& x : sched.runs) {
+      if (sched.few_qr) break;
       const SvdJob* j = dev.jobs + x.first;
       const int64_t* off = dev.off + x.first;
       cuda_check(launch_qr_factor(j, x.count, x.max_rows, x.max_cols, kQrFactor, a, q, r, work, off, st),

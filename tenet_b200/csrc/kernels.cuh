@@ -101,9 +101,10 @@ cudaError_t launch_split_pack_operand(const void* job_table, const GemmJob* host
                                       const double* src, int slices, int tile_n, bool i8, void* packed,
                                       cudaStream_t stream);
 
-// Batched one-sided Jacobi SVD, one CTA per coupled sector.
+// Batched one-sided Jacobi SVD, one CTA per coupled sector; few: sectors of few columns
+// (FacSchedule::few_svd), scaled as by the cluster engine.
 cudaError_t launch_svd(const SvdJob* jobs, int32_t njobs, const double* a, double* u, double* s, double* vh,
-                       double* work, const int64_t* work_off, int32_t* status, cudaStream_t stream);
+                       double* work, const int64_t* work_off, int32_t* status, cudaStream_t stream, bool few = false);
 
 // One-sided Jacobi of k x k matrices already in the sectors' scratch (jacobi.cu);
 // max_k (at most kJacobiMaxK) is the largest k of the jobs.

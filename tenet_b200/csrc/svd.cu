@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(kSvdThreads) svd_jacobi_kernel(const SvdJob* _
                                                                  double* __restrict__ S, double* __restrict__ VH,
                                                                  double* __restrict__ work,
                                                                  const int64_t* __restrict__ work_off,
-                                                                 int32_t* __restrict__ status) {
+                                                                 int32_t* __restrict__ status, bool few) {
   const SvdJob J = jobs[blockIdx.x];
   const int64_t m = J.m, n = J.n, k = J.k;
   if (k == 0) return;
@@ -243,12 +243,33 @@ __global__ void __launch_bounds__(kSvdThreads) svd_jacobi_kernel(const SvdJob* _
   const double* a = A + J.a_off;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
 
+  double mx = 0.0;
   for (int64_t idx = tid; idx < rows * k; idx += blockDim.x) {
     int64_t r = idx % rows, c = idx / rows;
-    W[idx] = wide ? a[c + r * m] : a[r + c * m];
+    const double x = wide ? a[c + r * m] : a[r + c * m];
+    W[idx] = x;
+    mx = fmax(mx, fabs(x));
   }
   for (int64_t idx = tid; idx < k * k; idx += blockDim.x) V[idx] = (idx % k == idx / k) ? 1.0 : 0.0;
   __shared__ double red[32];
+  // Sectors of few columns, which the cluster engine would take as well, keep its range:
+  // where a fourth power of their entries could leave FP64's, they are scaled by a power of
+  // two to a largest magnitude in [1/2, 1).
+  double scale = 1.0;
+  if (few) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (lane == 0) red[warp] = mx;
+    __syncthreads();
+    for (int w = 0; w < nwarps; ++w) mx = fmax(mx, red[w]);
+    if (mx > 0.0 && mx <= DBL_MAX && (mx < 1e-60 || mx > 1e60)) {
+      int e;
+      frexp(mx, &e);
+      scale = ldexp(1.0, e < -1022 ? 1022 : -e);
+      for (int64_t idx = tid; idx < rows * k; idx += blockDim.x) W[idx] *= scale;
+    }
+    __syncthreads();  // red is used again
+  }
   double f2 = 0.0;
   for (int64_t idx = tid; idx < rows * k; idx += blockDim.x) f2 = fma(W[idx], W[idx], f2);
   f2 = warp_sum(f2);
@@ -267,7 +288,9 @@ __global__ void __launch_bounds__(kSvdThreads) svd_jacobi_kernel(const SvdJob* _
   // SVD, so nothing is lost.
   const double abs_floor = 1e-28 * frob2;
   const double tol = 4.0 * sqrt((double)rows) * DBL_EPSILON;
-  const double noise2 = ((double)rows * DBL_EPSILON) * ((double)rows * DBL_EPSILON) * frob2;
+  // (of few columns a null one is at rounding level after its first rotation, however long)
+  const double level = (few && rows > 64 ? 64.0 : (double)rows) * DBL_EPSILON;
+  const double noise2 = level * level * frob2;
 
   __shared__ int rotated;
   const int k2 = (int)((k + 1) & ~1LL);
@@ -462,7 +485,7 @@ __global__ void __launch_bounds__(kSvdThreads) svd_jacobi_kernel(const SvdJob* _
       for (int64_t x = lane; x < m; x += 32) u[x + pos * m] = sign * vc[x];
       for (int64_t x = lane; x < n; x += 32) vh[pos + x * k] = sign * wc[x] * inv;
     }
-    if (lane == 0) s[pos] = sc;
+    if (lane == 0) s[pos] = sc / scale;
   }
 }
 
@@ -770,12 +793,12 @@ __global__ void __launch_bounds__(1024) truncate_kernel(const SvdJob* __restrict
 }  // namespace
 
 cudaError_t launch_svd(const SvdJob* jobs, int32_t njobs, const double* a, double* u, double* s, double* vh,
-                       double* work, const int64_t* work_off, int32_t* status, cudaStream_t stream) {
+                       double* work, const int64_t* work_off, int32_t* status, cudaStream_t stream, bool few) {
   if (njobs == 0) return cudaSuccess;
   cudaError_t e = cudaFuncSetAttribute(svd_jacobi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kSvdSmemBytes);
   if (e != cudaSuccess) return e;
-  svd_jacobi_kernel<<<njobs, kSvdThreads, kSvdSmemBytes, stream>>>(jobs, a, u, s, vh, work, work_off, status);
+  svd_jacobi_kernel<<<njobs, kSvdThreads, kSvdSmemBytes, stream>>>(jobs, a, u, s, vh, work, work_off, status, few);
   return cudaGetLastError();
 }
 

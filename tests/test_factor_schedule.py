@@ -24,9 +24,9 @@ def plan_of(sectors):
 
 
 def schedule(plan, wide):
-    counts, runs = (C.c_int32 * 4)(), (C.c_int32 * (2 * plan.nsectors))()
+    counts, runs = (C.c_int32 * 6)(), (C.c_int32 * (2 * plan.nsectors))()
     _lib.call("tnt_fplan_schedule", plan._h, wide, counts, runs)
-    return list(counts), [tuple(runs[2 * i: 2 * i + 2]) for i in range(counts[3])]
+    return list(counts[:4]), [tuple(runs[2 * i: 2 * i + 2]) for i in range(counts[3])]
 
 
 def test_grouping_follows_the_cluster_width():

@@ -908,17 +908,9 @@ __global__ void __launch_bounds__(kFinishWarps * 32)
 // meta[1].  Sectors that fail the reference's Hermiticity check
 // (normwise_hermitian, factorize.rs:5999-6021: ||A - A^T||_F <= 2 * 64 eps ||A||_F,
 // every entry finite) set bit 1 of *status.
-__global__ void __launch_bounds__(1024) eigh_scan_kernel(const SvdJob* __restrict__ jobs, const double* __restrict__ A,
-                                                         double* __restrict__ work,
-                                                         const int64_t* __restrict__ work_off,
-                                                         int32_t* __restrict__ status) {
-  const SvdJob S = jobs[blockIdx.x];
-  const int64_t n = S.m;
-  if (n == 0) return;
-  const FacWork f = fac_work(work + work_off[blockIdx.x], n, n);
-  const double* a = A + S.a_off;
+__device__ void eigh_scan(const double* a, int64_t n, const FacWork& f, int32_t* status) {
   __shared__ double red[2][32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
   double mx = 0.0;
   int finite = 1;
   for (int64_t i = tid; i < n * n; i += blockDim.x) {
@@ -930,7 +922,7 @@ __global__ void __launch_bounds__(1024) eigh_scan_kernel(const SvdJob* __restric
   for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   if (lane == 0) red[0][warp] = mx;
   __syncthreads();
-  for (int i = 0; i < 32; ++i) mx = fmax(mx, red[0][i]);
+  for (int i = 0; i < nwarps; ++i) mx = fmax(mx, red[0][i]);
   __syncthreads();
   double scale = 1.0;
   if (finite && mx > 0.0) {
@@ -954,7 +946,7 @@ __global__ void __launch_bounds__(1024) eigh_scan_kernel(const SvdJob* __restric
   __syncthreads();
   if (tid == 0) {
     f2 = d2 = 0.0;
-    for (int i = 0; i < 32; ++i) {
+    for (int i = 0; i < nwarps; ++i) {
       f2 += red[0][i];
       d2 += red[1][i];
     }
@@ -966,23 +958,25 @@ __global__ void __launch_bounds__(1024) eigh_scan_kernel(const SvdJob* __restric
   }
 }
 
+__global__ void __launch_bounds__(1024) eigh_scan_kernel(const SvdJob* __restrict__ jobs, const double* __restrict__ A,
+                                                         double* __restrict__ work,
+                                                         const int64_t* __restrict__ work_off,
+                                                         int32_t* __restrict__ status) {
+  const SvdJob S = jobs[blockIdx.x];
+  if (S.m == 0) return;
+  eigh_scan(A + S.a_off, S.m, fac_work(work + work_off[blockIdx.x], S.m, S.m), status);
+}
+
 constexpr int kBoundWarps = 8;
 
-// Row sums of |A^2| for 16 rows per CTA (8 x 8 tiles on the FP64 tensor cores, A's
-// symmetry giving rows as columns); their maximum to meta[2].
-__global__ void __launch_bounds__(kBoundWarps * 32)
-    eigh_bound_kernel(const SvdJob* __restrict__ jobs, const double* __restrict__ A, double* __restrict__ work,
-                      const int64_t* __restrict__ work_off) {
-  const SvdJob S = jobs[blockIdx.x];
-  const int n = (int)S.m, r0 = 16 * (int)blockIdx.y;
-  if (r0 >= n) return;
-  const FacWork f = fac_work(work + work_off[blockIdx.x], n, n);
+// Row sums of |A^2| for the 16 rows from r0 on, by kBoundWarps warps (8 x 8 tiles on the
+// FP64 tensor cores, A's symmetry giving rows as columns); their maximum to meta[2].
+// Every thread of the CTA calls it (rows beyond n: no work).
+__device__ void eigh_bound(const double* a, int n, const FacWork& f, int r0, int warp, double (*rows)[16]) {
   const double scale = f.meta[0];
-  const double* a = A + S.a_off;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
-  __shared__ double rows[kBoundWarps][16];
+  const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   double sum[2] = {0.0, 0.0};
-  for (int c0 = 16 * warp; c0 < n; c0 += 16 * kBoundWarps) {
+  for (int c0 = 16 * warp; c0 < n && r0 < n; c0 += 16 * kBoundWarps) {
     double d[2][2][2] = {};
 #pragma unroll 2
     for (int x0 = 0; x0 < n; x0 += 4) {
@@ -1011,15 +1005,25 @@ __global__ void __launch_bounds__(kBoundWarps * 32)
     if (t4 == 0) rows[warp][8 * h + g] = sum[h];
   }
   __syncthreads();
-  if (threadIdx.x < 16) {
+  if (warp == 0 && lane < 16 && r0 < n) {
     double t = 0.0;
-    for (int i = 0; i < kBoundWarps; ++i) t += rows[i][threadIdx.x];
+    for (int i = 0; i < kBoundWarps; ++i) t += rows[i][lane];
     atomicMax(reinterpret_cast<unsigned long long*>(f.meta) + 2, (unsigned long long)__double_as_longlong(t));
   }
 }
 
-__device__ __forceinline__ double eigh_shift(const double* meta) {
-  const double c = fmin(1.125 * meta[1], 1.0625 * sqrt(meta[2]));
+__global__ void __launch_bounds__(kBoundWarps * 32)
+    eigh_bound_kernel(const SvdJob* __restrict__ jobs, const double* __restrict__ A, double* __restrict__ work,
+                      const int64_t* __restrict__ work_off) {
+  const SvdJob S = jobs[blockIdx.x];
+  if (16 * (int64_t)blockIdx.y >= S.m) return;
+  __shared__ double rows[kBoundWarps][16];
+  eigh_bound(A + S.a_off, (int)S.m, fac_work(work + work_off[blockIdx.x], S.m, S.m), 16 * (int)blockIdx.y,
+             threadIdx.x >> 5, rows);
+}
+
+__device__ __forceinline__ double eigh_shift(const double* meta) {  // meta[2] comes from atomics
+  const double c = fmin(1.125 * meta[1], 1.0625 * sqrt(__ldcg(meta + 2)));
   return c > 0.0 ? c : 1.0;  // a zero sector (or one that failed the scan)
 }
 
@@ -1036,6 +1040,34 @@ __global__ void __launch_bounds__(256) eigh_form_kernel(const SvdJob* __restrict
     f.W[i] = fma(a[i], scale, (i % n) == (i / n) ? c : 0.0);
 }
 
+// Sectors up to kEighSmall: scan, bound and shifted matrix in one launch, and all of the
+// output stage in another, a CTA per sector.  In launches of their own the seven steps
+// were most of the time (n = 4: 70 us, 45 so).
+constexpr int64_t kEighSmall = 64;
+constexpr int kSmallThreads = 512;
+
+__global__ void __launch_bounds__(kSmallThreads) eigh_prepare_small_kernel(const SvdJob* __restrict__ jobs,
+                                                                           const double* __restrict__ A,
+                                                                           double* __restrict__ work,
+                                                                           const int64_t* __restrict__ work_off,
+                                                                           int32_t* __restrict__ status) {
+  const SvdJob S = jobs[blockIdx.x];
+  const int n = (int)S.m;
+  if (n == 0) return;
+  const FacWork f = fac_work(work + work_off[blockIdx.x], n, n);
+  const double* a = A + S.a_off;
+  __shared__ double rows[kSmallThreads / 32][16];
+  eigh_scan(a, n, f, status);
+  __syncthreads();  // meta
+  const int warp = threadIdx.x >> 5, part = warp / kBoundWarps;
+  for (int r0 = 0; r0 < n; r0 += 16 * (kSmallThreads / 32 / kBoundWarps)) {
+    eigh_bound(a, n, f, r0 + 16 * part, warp % kBoundWarps, rows + part * kBoundWarps);
+    __syncthreads();  // rows are used again, and the maxima are in place
+  }
+  const double scale = f.meta[0], c = eigh_shift(f.meta);
+  for (int i = threadIdx.x; i < n * n; i += kSmallThreads) f.W[i] = fma(a[i], scale, (i % n) == (i / n) ? c : 0.0);
+}
+
 // One refinement step of the eigenvectors V (Ogita and Aishima, "Iterative
 // refinement for symmetric eigenvalue decomposition", 2018): the sweeps' rounding
 // errors, a random walk of about 12 n rotations at the scale of c, are replaced by
@@ -1047,30 +1079,26 @@ __global__ void __launch_bounds__(256) eigh_form_kernel(const SvdJob* __restrict
 // the errors) it is left out.
 
 // Fragments of an m x 4 slice: rows g of a matrix walked down its columns (TR) or
-// across them.
+// across them.  OWN: the matrix was written by this launch.
+template <bool OWN>
 __device__ __forceinline__ double frag(const double* a, int64_t ld, int r, int x, int n, bool tr) {
-  return (r < n && x < n) ? __ldg(tr ? a + x + (int64_t)r * ld : a + r + (int64_t)x * ld) : 0.0;
+  if (r >= n || x >= n) return 0.0;
+  const double* p = tr ? a + x + (int64_t)r * ld : a + r + (int64_t)x * ld;
+  return OWN ? *p : __ldg(p);
 }
 
 constexpr int kRefineWarps = 4;  // a CTA takes a 32 x 32 tile, a warp 16 x 16 of it
 
-// step 0: W = scale A V.  step 1: X (into VEC).  step 2: W[:, rank] = V + V X.
-// From step 1 on the outputs are written, so every kernel leaves a call that has
-// failed alone (a sector that is not Hermitian, or sweeps that did not converge).
-__global__ void __launch_bounds__(kRefineWarps * 32)
-    eigh_refine_kernel(const SvdJob* __restrict__ jobs, const double* __restrict__ A, double* __restrict__ VEC,
-                       double* __restrict__ work, const int64_t* __restrict__ work_off,
-                       const int32_t* __restrict__ status, const int32_t* __restrict__ bad, int step) {
-  if (factor_failed(status, bad)) return;
-  const SvdJob S = jobs[blockIdx.x];
-  const int n = (int)S.m;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
-  const int r0 = 32 * (int)blockIdx.y + 16 * (warp & 1), c0 = 32 * (int)blockIdx.z + 16 * (warp >> 1);
+// The 16 x 16 tile at r0, c0, by one warp.  step 0: W = scale A V.  step 1: X (into vec).
+// step 2: W[:, rank] = V + V X.
+template <bool OWN>
+__device__ __forceinline__ void eigh_refine(const double* a, double* vec, const FacWork& f, int n, int r0, int c0,
+                                            int step) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   if (r0 >= n || c0 >= n) return;
-  const FacWork f = fac_work(work + work_off[blockIdx.x], n, n);
-  const double *V = f.J, *a = A + S.a_off, *X = VEC + S.u_off;
+  const double* V = f.J;
   const double* lhs = step == 0 ? a : V;
-  const double* rhs = step == 0 ? V : step == 1 ? f.W : X;
+  const double* rhs = step == 0 ? V : step == 1 ? f.W : vec;
   double d[2][2][2] = {}, e[2][2][2] = {}, t[2][2][2] = {};
 #pragma unroll 2
   for (int x0 = 0; x0 < n; x0 += 4) {
@@ -1078,10 +1106,10 @@ __global__ void __launch_bounds__(kRefineWarps * 32)
     double u[2], v[2], w[2], z[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      u[h] = frag(lhs, n, r0 + 8 * h + g, x, n, step == 1);
-      v[h] = frag(rhs, n, c0 + 8 * h + g, x, n, true);
-      w[h] = step == 1 ? frag(V, n, c0 + 8 * h + g, x, n, true) : 0.0;
-      z[h] = step == 1 ? frag(f.W, n, r0 + 8 * h + g, x, n, true) : 0.0;
+      u[h] = frag<OWN>(lhs, n, r0 + 8 * h + g, x, n, step == 1);
+      v[h] = frag<OWN>(rhs, n, c0 + 8 * h + g, x, n, true);
+      w[h] = step == 1 ? frag<OWN>(V, n, c0 + 8 * h + g, x, n, true) : 0.0;
+      z[h] = step == 1 ? frag<OWN>(f.W, n, r0 + 8 * h + g, x, n, true) : 0.0;
     }
 #pragma unroll
     for (int h = 0; h < 2; ++h)
@@ -1110,25 +1138,31 @@ __global__ void __launch_bounds__(kRefineWarps * 32)
           const double mid = 0.5 * (d[h][i][q] + t[h][i][q] + (lr + lc) * res), gap = lc - lr;
           double x = 0.5 * res;
           if (r != c && fabs(mid) < 1e-8 * fabs(gap)) x += mid / gap;
-          VEC[S.u_off + r + (int64_t)c * n] = x;
+          vec[r + (int64_t)c * n] = x;
         } else {
           f.W[r + (int64_t)f.rk[c] * n] = V[r + (int64_t)c * n] + d[h][i][q];
         }
       }
 }
 
-// lambda_c = (v_c, A v_c) / (v_c, v_c) into sv; ranks by descending |lambda| (ties:
-// ascending value, then index) into rk; the sorted values out.
-__global__ void __launch_bounds__(1024) eigh_values_kernel(const SvdJob* __restrict__ jobs, double* __restrict__ VAL,
-                                                           double* __restrict__ MAG, double* __restrict__ work,
-                                                           const int64_t* __restrict__ work_off,
-                                                           const int32_t* __restrict__ status,
-                                                           const int32_t* __restrict__ bad) {
+// From step 1 on the outputs are written, so every kernel leaves a call that has
+// failed alone (a sector that is not Hermitian, or sweeps that did not converge).
+__global__ void __launch_bounds__(kRefineWarps * 32)
+    eigh_refine_kernel(const SvdJob* __restrict__ jobs, const double* __restrict__ A, double* __restrict__ VEC,
+                       double* __restrict__ work, const int64_t* __restrict__ work_off,
+                       const int32_t* __restrict__ status, const int32_t* __restrict__ bad, int step) {
   if (factor_failed(status, bad)) return;
   const SvdJob S = jobs[blockIdx.x];
-  const int n = (int)S.m, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int n = (int)S.m, warp = threadIdx.x >> 5;
   if (n == 0) return;
-  const FacWork f = fac_work(work + work_off[blockIdx.x], n, n);
+  eigh_refine<false>(A + S.a_off, VEC + S.u_off, fac_work(work + work_off[blockIdx.x], n, n), n,
+                     32 * (int)blockIdx.y + 16 * (warp & 1), 32 * (int)blockIdx.z + 16 * (warp >> 1), step);
+}
+
+// lambda_c = (v_c, A v_c) / (v_c, v_c) into sv; ranks by descending |lambda| (ties:
+// ascending value, then index) into rk; the sorted values out.
+__device__ void eigh_values(const FacWork& f, int n, double* val, double* mag) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   for (int c = warp; c < n; c += nwarps) {
     const double *v = f.J + (int64_t)c * n, *w = f.W + (int64_t)c * n;
     double s = 0.0, q = 0.0;
@@ -1151,27 +1185,61 @@ __global__ void __launch_bounds__(1024) eigh_values_kernel(const SvdJob* __restr
     pos = __reduce_add_sync(0xffffffffu, pos);
     if (lane == 0) {
       f.rk[c] = (double)pos;
-      VAL[S.s_off + pos] = lc / f.meta[0];
-      if (MAG) MAG[S.s_off + pos] = ac / f.meta[0];
+      val[pos] = lc / f.meta[0];
+      if (mag) mag[pos] = ac / f.meta[0];
     }
   }
 }
 
-// Each vector's largest-|.| entry positive (factorize.rs:3902-3913).
+__global__ void __launch_bounds__(1024) eigh_values_kernel(const SvdJob* __restrict__ jobs, double* __restrict__ VAL,
+                                                           double* __restrict__ MAG, double* __restrict__ work,
+                                                           const int64_t* __restrict__ work_off,
+                                                           const int32_t* __restrict__ status,
+                                                           const int32_t* __restrict__ bad) {
+  const SvdJob S = jobs[blockIdx.x];
+  if (S.m == 0 || factor_failed(status, bad)) return;
+  eigh_values(fac_work(work + work_off[blockIdx.x], S.m, S.m), (int)S.m, VAL + S.s_off, MAG ? MAG + S.s_off : nullptr);
+}
+
+// Column c of a sector, its largest-|.| entry positive (factorize.rs:3902-3913), by one warp.
+__device__ __forceinline__ void eigh_column(const FacWork& f, int64_t n, int64_t c, double* vec) {
+  const double* wc = f.W + c * n;
+  const double sign = wc[warp_argmax_abs(n, [&](int64_t x) { return wc[x]; })] < 0.0 ? -1.0 : 1.0;
+  for (int64_t x = threadIdx.x & 31; x < n; x += 32) vec[c * n + x] = sign * wc[x];
+}
+
 __global__ void __launch_bounds__(kFinishWarps * 32)
     eigh_finish_kernel(const SvdJob* __restrict__ jobs, double* __restrict__ VEC, double* __restrict__ work,
                        const int64_t* __restrict__ work_off, const int32_t* __restrict__ status,
                        const int32_t* __restrict__ bad) {
   if (factor_failed(status, bad)) return;
   const SvdJob S = jobs[blockIdx.x];
-  const int64_t n = S.m;
-  const int lane = threadIdx.x & 31;
   const int64_t c = (int64_t)blockIdx.y * kFinishWarps + (threadIdx.x >> 5);
-  if (c >= n) return;
+  if (c >= S.m) return;
+  eigh_column(fac_work(work + work_off[blockIdx.x], S.m, S.m), S.m, c, VEC + S.u_off);
+}
+
+__global__ void __launch_bounds__(kSmallThreads)
+    eigh_finish_small_kernel(const SvdJob* __restrict__ jobs, const double* __restrict__ A, double* __restrict__ VEC,
+                             double* __restrict__ VAL, double* __restrict__ MAG, double* __restrict__ work,
+                             const int64_t* __restrict__ work_off, const int32_t* __restrict__ status,
+                             const int32_t* __restrict__ bad) {
+  const SvdJob S = jobs[blockIdx.x];
+  const int n = (int)S.m;
+  if (n == 0 || factor_failed(status, bad)) return;
   const FacWork f = fac_work(work + work_off[blockIdx.x], n, n);
-  const double* wc = f.W + c * n;
-  const double sign = wc[warp_argmax_abs(n, [&](int64_t x) { return wc[x]; })] < 0.0 ? -1.0 : 1.0;
-  for (int64_t x = lane; x < n; x += 32) VEC[S.u_off + c * n + x] = sign * wc[x];
+  const int warp = threadIdx.x >> 5, nwarps = kSmallThreads / 32, nt = (n + 15) / 16;
+  double* vec = VEC + S.u_off;
+  for (int step = 0; step < 3; ++step) {
+    for (int t = warp; t < nt * nt; t += nwarps)
+      eigh_refine<true>(A + S.a_off, vec, f, n, 16 * (t % nt), 16 * (t / nt), step);
+    __syncthreads();
+    if (step == 0) {
+      eigh_values(f, n, VAL + S.s_off, MAG ? MAG + S.s_off : nullptr);
+      __syncthreads();
+    }
+  }
+  for (int c = warp; c < n; c += nwarps) eigh_column(f, n, c, vec);
 }
 
 }  // namespace
@@ -1231,6 +1299,10 @@ cudaError_t launch_svd_finish(const SvdJob* jobs, int32_t njobs, int64_t max_k, 
 cudaError_t launch_eigh_prepare(const SvdJob* jobs, int32_t njobs, int64_t max_n, const double* a, double* work,
                                 const int64_t* work_off, int32_t* status, cudaStream_t st) {
   if (njobs == 0 || max_n == 0) return cudaSuccess;
+  if (max_n <= kEighSmall) {
+    eigh_prepare_small_kernel<<<njobs, kSmallThreads, 0, st>>>(jobs, a, work, work_off, status);
+    return cudaGetLastError();
+  }
   eigh_scan_kernel<<<njobs, 1024, 0, st>>>(jobs, a, work, work_off, status);
   eigh_bound_kernel<<<dim3((unsigned)njobs, (unsigned)((max_n + 15) / 16)), kBoundWarps * 32, 0, st>>>(jobs, a, work,
                                                                                                      work_off);
@@ -1243,6 +1315,10 @@ cudaError_t launch_eigh_finish(const SvdJob* jobs, int32_t njobs, int64_t max_n,
                                double* vals, double* mags, double* work, const int64_t* work_off,
                                const int32_t* status, const int32_t* bad, cudaStream_t st) {
   if (njobs == 0 || max_n == 0) return cudaSuccess;
+  if (max_n <= kEighSmall) {
+    eigh_finish_small_kernel<<<njobs, kSmallThreads, 0, st>>>(jobs, a, vecs, vals, mags, work, work_off, status, bad);
+    return cudaGetLastError();
+  }
   const unsigned nt = (unsigned)((max_n + 31) / 32);
   const dim3 tiles((unsigned)njobs, nt, nt);
   eigh_refine_kernel<<<tiles, kRefineWarps * 32, 0, st>>>(jobs, a, vecs, work, work_off, status, bad, 0);

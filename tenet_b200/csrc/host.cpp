@@ -856,14 +856,25 @@ static void fold_axes(XformTables& t) {
   t.fsrc.clear();
   t.fdst.clear();
   int64_t total = 0;
-  for (auto& g : t.groups) total += g.nelem;
-  // Axis 0 of a copy that is not transposing: rows no longer than a slot's share of the plan.
-  const int64_t cap0 = std::min<int64_t>(1024, total / (148 * 3));
+  bool copies = true;
+  for (auto& g : t.groups) {
+    total += g.nelem;
+    copies &= g.nsrc == 1 && g.ndst == 1;
+  }
+  // Axis 0 where the copy is not transposing: rows no longer than a slot's share of the
+  // plan.  Recoupling plans, where column setup is the larger part, gain up to rows of
+  // 1024 (SU(2), 25-dimensional legs, 288 MB: 136 us at 128, 72 at 1024).  Plans of plain
+  // copies already keep eight columns' loads in flight, and rows of a few hundred walk a warp each
+  // with fewer: up to 128 (Z2, 24-dimensional legs, 42 MB: 7.6 us, 11.3 at 576; 32 and 134 MB:
+  // 28.2, 31.5 at 1024), and not below four columns a slot.
+  const int64_t group0 = std::min<int64_t>(1024, total / (148 * 3));
+  const int64_t copy0 = std::min<int64_t>(128, total / (148 * 3 * 4));
   std::vector<XEntry> src, dst;
   for (auto& g : t.groups) {
     int lead = 0;  // a source with stride 1 along the leading axis is not transposed
     while (lead < g.rank && g.dims[lead] == 1) ++lead;
     const bool strided = g.nsrc == 1 && g.ndst == 1 && lead < g.rank && t.src_entries[g.src_first].strides[lead] != 1;
+    const int64_t cap0 = copies ? copy0 : group0;
     XGroup f = fold_group(t, g, strided ? 65535 : cap0, src, dst);
     if (strided && xform_transposing_axis(f, src[0]) == 0) f = fold_group(t, g, cap0, src, dst);
     f.src_first = (int32_t)t.fsrc.size();
@@ -938,9 +949,9 @@ static void split_tiles(XformTables& t) {
     target[k] = std::min<int64_t>(
         32768, std::max<int64_t>(512, total[k] / std::max<int64_t>(1, waves * slots - ngroups[k])));
   }
-  // Transposing tiles fill the staging buffer once a plan has two waves of such
-  // tiles; smaller plans spread over the slots.
-  const int64_t tr_cap = std::min<int64_t>(kTrCap, std::max<int64_t>(512, total[kXTransposing] / (2 * slots)));
+  // Transposing tiles fill the staging buffer once a plan has a wave of such tiles;
+  // smaller plans spread over the slots.
+  const int64_t tr_cap = std::min<int64_t>(kTrCap, std::max<int64_t>(512, total[kXTransposing] / slots));
   for (size_t gi = 0; gi < t.fgroups.size(); ++gi) {
     const XGroup& g = t.fgroups[gi];
     if (const int ks = axis_of(g)) {

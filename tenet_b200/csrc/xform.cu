@@ -143,13 +143,17 @@ __device__ __forceinline__ void xform_tiles(XShared& sh, const XTile* __restrict
               od[u] = cbase[cl][1] + i0;
             }
           }
+          if (beta != 0.0) {  // added in place before the first is written
 #pragma unroll
-          for (int u = 0; u < kUnroll; ++u) {
-            if (od[u] >= 0) {
-              const double x = scale * v[u];
-              dst[od[u]] = beta == 0.0 ? x : fma(beta, dst[od[u]], x);
-            }
+            for (int u = 0; u < kUnroll; ++u)
+              if (od[u] >= 0) v[u] = fma(beta, dst[od[u]], scale * v[u]);
+          } else {
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) v[u] *= scale;
           }
+#pragma unroll
+          for (int u = 0; u < kUnroll; ++u)
+            if (od[u] >= 0) dst[od[u]] = v[u];
         }
       }
       continue;
@@ -175,19 +179,20 @@ __device__ __forceinline__ void xform_tiles(XShared& sh, const XTile* __restrict
 #pragma unroll
             for (int q = 0; q < 4; ++q)
               if (p0 + q * W < np) v[q] = __ldg(sp + p0 + q * W);
+            if (beta != 0.0) {  // added in place before the first is written
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const int p = p0 + q * W;
-              if (p < np) {
-                const double2 a = make_double2(u * v[q].x, u * v[q].y);
-                if (beta == 0.0) {
-                  op[p] = a;
-                } else {
-                  const double2 b = op[p];
-                  op[p] = make_double2(fma(beta, b.x, a.x), fma(beta, b.y, a.y));
+              for (int q = 0; q < 4; ++q)
+                if (p0 + q * W < np) {
+                  const double2 b = op[p0 + q * W];
+                  v[q] = make_double2(fma(beta, b.x, u * v[q].x), fma(beta, b.y, u * v[q].y));
                 }
-              }
+            } else {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) v[q] = make_double2(u * v[q].x, u * v[q].y);
             }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              if (p0 + q * W < np) op[p0 + q * W] = v[q];
           }
         } else {
           for (int i0 = tx; i0 < d0; i0 += 4 * W) {
@@ -195,14 +200,18 @@ __device__ __forceinline__ void xform_tiles(XShared& sh, const XTile* __restrict
 #pragma unroll
             for (int q = 0; q < 4; ++q)
               if (i0 + q * W < d0) v[q] = __ldg(src + sbase + (int64_t)(i0 + q * W) * s0);
+            double* op = dst + dbase + i0;
+            if (beta != 0.0) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const int i = i0 + q * W;
-              if (i < d0) {
-                double* o = dst + dbase + i;
-                *o = beta == 0.0 ? u * v[q] : fma(beta, *o, u * v[q]);
-              }
+              for (int q = 0; q < 4; ++q)
+                if (i0 + q * W < d0) v[q] = fma(beta, op[q * W], u * v[q]);
+            } else {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) v[q] *= u;
             }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              if (i0 + q * W < d0) op[q * W] = v[q];
           }
         }
       }
@@ -503,15 +512,44 @@ __global__ void __launch_bounds__(kXThreads, 3) xform_transpose_kernel(
   auto store = [&](const XTrTile& T, const double* buf, int slot) {
     const int jp = T.jn | 1, ps = T.r * jp;
     const double u = alpha * coef[T.coef];
-    auto put = [&](double* o, double v) { *o = beta == 0.0 ? u * v : fma(beta, *o, u * v); };
-    if (T.np == 1) {
-      double* q = dst + T.dst;
-      walk(T.r, T.jn, 1, [&](int i, int j, int) { put(q + j * T.dks + i, buf[i * jp + j]); });
-    } else {
-      walk(T.r, T.jn, T.np, [&](int i, int j, int p) {
-        put(dst + pbase[slot][p][1] + j * T.dks + i, buf[p * ps + i * jp + j]);
-      });
+    auto visit = [&](auto&& put) {
+      if (T.np == 1) {
+        double* q = dst + T.dst;
+        walk(T.r, T.jn, 1, [&](int i, int j, int) { put(q + j * T.dks + i, u * buf[i * jp + j]); });
+      } else {
+        walk(T.r, T.jn, T.np, [&](int i, int j, int p) {
+          put(dst + pbase[slot][p][1] + j * T.dks + i, u * buf[p * ps + i * jp + j]);
+        });
+      }
+    };
+    if (beta == 0.0) {
+      visit([](double* at, double x) { *at = x; });
+      return;
     }
+    // Four elements are read before they are written: otherwise every load waits for
+    // the store before it (24 MB of ragged U(1) blocks 20 us, now 14).
+    double* at[4];
+    double v[4];
+    int have = 0;
+    auto flush = [&] {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (q < have) v[q] = fma(beta, *at[q], v[q]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (q < have) *at[q] = v[q];
+      have = 0;
+    };
+    visit([&](double* o, double x) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (q == have) {
+          at[q] = o;
+          v[q] = x;
+        }
+      if (++have == 4) flush();
+    });
+    flush();
   };
 
   int32_t t = blockIdx.x;

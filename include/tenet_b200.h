@@ -306,7 +306,8 @@ tnt_status tnt_compose_host(tnt_ctx* ctx, const tnt_cplan* plan, int64_t nbatch,
 
 /* Compact SVD of every coupled sector: u (m x k), s (k), vh (k x n) per
  * sector at the offsets of tnt_fplan_info, largest-|U| column gauge
- * (factorize.rs:3836-3852). */
+ * (factorize.rs:3836-3852).  u or vh may be a itself where the offsets agree; such a
+ * call runs every sector on one CTA. */
 tnt_status tnt_svd(tnt_ctx* ctx, const tnt_fplan* plan, const double* a, double* u, double* s, double* vh,
                    void* stream);
 

@@ -1667,14 +1667,23 @@ namespace {
 
 // The batched SVD of a plan: sectors beyond kQrMaxRows on the general Jacobi
 // kernels; the others reduced to R^T (rectangular ones made square first), swept by
-// the cluster Jacobi engine, their factors taken back through the reflectors.
-cudaError_t svd_launches(const FacDevice& dev, const double* a, double* u, double* s, double* vh, double* work,
-                         int32_t* status, cudaStream_t st) {
+// the cluster Jacobi engine, their factors taken back through the reflectors.  The engine
+// keeps reflectors in u and vh while others still read a, so factors written over a
+// (in place) come from the one-CTA kernels, which read a sector whole before they write.
+cudaError_t svd_launches(const SvdTables& t, const FacDevice& dev, const double* a, double* u, double* s, double* vh,
+                         double* work, int32_t* status, cudaStream_t st) {
   const FacSchedule& q = dev.sched;
-  if (q.few_svd) return launch_svd(dev.jobs, (int32_t)q.order.size(), a, u, s, vh, work, dev.off, status, st, true);
+  const int32_t njobs = (int32_t)q.order.size();
+  if (q.few_svd) return launch_svd(dev.jobs, njobs, a, u, s, vh, work, dev.off, status, st, true);
   cudaError_t e = cudaSuccess;
   if (q.n_old > 0)
     e = launch_svd_split(dev.jobs, q.n_cluster, q.n_old, a, u, s, vh, work, dev.off, status, st, q.n_wide);
+  auto over_a = [&](const double* x, int64_t n) {
+    const uintptr_t p = (uintptr_t)x, r = (uintptr_t)a;
+    return p < r + sizeof(double) * (uintptr_t)t.a_size && r < p + sizeof(double) * (uintptr_t)n;
+  };
+  if (e == cudaSuccess && (over_a(u, t.u_size) || over_a(vh, t.v_size)))
+    return launch_svd(dev.jobs + q.n_old, njobs - q.n_old, a, u, s, vh, work, dev.off + q.n_old, status, st, true);
   for (const FacRun& r : q.runs) {
     const SvdJob* j = dev.jobs + r.first;
     const int64_t* off = dev.off + r.first;
@@ -1715,7 +1724,7 @@ tnt_status tnt_svd(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, double
     }
     cudaStream_t st = (cudaStream_t)stream;
     cuda_check(cudaMemsetAsync(ctx->status, 0, 2 * sizeof(int32_t), st), "memset status");
-    cuda_check(svd_launches(dev, a, u, s, vh, ctx->svd_work, ctx->status, st),
+    cuda_check(svd_launches(t, dev, a, u, s, vh, ctx->svd_work, ctx->status, st),
                "svd kernel launch");
     int32_t hs[2] = {0, 0};
     cuda_check(cudaMemcpyAsync(hs, ctx->status, sizeof(hs), cudaMemcpyDeviceToHost, st), "read svd status");
@@ -1737,7 +1746,7 @@ tnt_status tnt_svd_ws_async(tnt_ctx* ctx, const tnt_fplan* fplan, const double* 
     const FacDevice& dev = plan->lpt_on_device();
     cudaStream_t st = (cudaStream_t)stream;
     cuda_check(cudaMemsetAsync(status, 0, 2 * sizeof(int32_t), st), "memset status");
-    cuda_check(svd_launches(dev, a, u, s, vh, work, status, st),
+    cuda_check(svd_launches(t, dev, a, u, s, vh, work, status, st),
                "svd kernel launch");
   });
 }
@@ -1780,7 +1789,7 @@ tnt_status tnt_svd_ws(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, dou
     cudaStream_t st = (cudaStream_t)stream;
     std::lock_guard<std::recursive_mutex> g(ctx->mu);  // the status words are the context's
     cuda_check(cudaMemsetAsync(ctx->status, 0, 2 * sizeof(int32_t), st), "memset status");
-    cuda_check(svd_launches(dev, a, u, s, vh, work, ctx->status, st),
+    cuda_check(svd_launches(t, dev, a, u, s, vh, work, ctx->status, st),
                "svd kernel launch");
     int32_t hs[2] = {0, 0};
     cuda_check(cudaMemcpyAsync(hs, ctx->status, sizeof(hs), cudaMemcpyDeviceToHost, st), "read svd status");

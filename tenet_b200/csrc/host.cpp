@@ -865,8 +865,8 @@ static void fold_axes(XformTables& t) {
   // plan.  Recoupling plans, where column setup is the larger part, gain up to rows of
   // 1024 (SU(2), 25-dimensional legs, 288 MB: 136 us at 128, 72 at 1024).  Plans of plain
   // copies already keep eight columns' loads in flight, and rows of a few hundred walk a warp each
-  // with fewer: up to 128 (Z2, 24-dimensional legs, 42 MB: 7.6 us, 11.3 at 576; 32 and 134 MB:
-  // 28.2, 31.5 at 1024), and not below four columns a slot.
+  // with fewer: up to 128 (Z2, 24-dimensional legs, 42 MB: 7.6 us, 11.3 at 576;
+  // 32-dimensional, 134 MB: 28.2 us, 31.5 at 1024), and not below four columns a slot.
   const int64_t group0 = std::min<int64_t>(1024, total / (148 * 3));
   const int64_t copy0 = std::min<int64_t>(128, total / (148 * 3 * 4));
   std::vector<XEntry> src, dst;

@@ -101,8 +101,8 @@ cudaError_t launch_split_pack_operand(const void* job_table, const GemmJob* host
                                       const double* src, int slices, int tile_n, bool i8, void* packed,
                                       cudaStream_t stream);
 
-// Batched one-sided Jacobi SVD, one CTA per coupled sector; few: sectors of few columns
-// (FacSchedule::few_svd), scaled as by the cluster engine.
+// Batched one-sided Jacobi SVD, one CTA per coupled sector; few: in place of the cluster
+// engine (few columns, or outputs over the input), scaled as by it.
 cudaError_t launch_svd(const SvdJob* jobs, int32_t njobs, const double* a, double* u, double* s, double* vh,
                        double* work, const int64_t* work_off, int32_t* status, cudaStream_t stream, bool few = false);
 

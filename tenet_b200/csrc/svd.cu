@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(kSvdThreads) svd_jacobi_kernel(const SvdJob* _
   }
   for (int64_t idx = tid; idx < k * k; idx += blockDim.x) V[idx] = (idx % k == idx / k) ? 1.0 : 0.0;
   __shared__ double red[32];
-  // Sectors of few columns, which the cluster engine would take as well, keep its range:
+  // Sectors that the cluster engine would take as well keep its range:
   // where a fourth power of their entries could leave FP64's, they are scaled by a power of
   // two to a largest magnitude in [1/2, 1).
   double scale = 1.0;
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(kSvdThreads) svd_jacobi_kernel(const SvdJob* _
   const double abs_floor = 1e-28 * frob2;
   const double tol = 4.0 * sqrt((double)rows) * DBL_EPSILON;
   // (of few columns a null one is at rounding level after its first rotation, however long)
-  const double level = (few && rows > 64 ? 64.0 : (double)rows) * DBL_EPSILON;
+  const double level = (few && k <= 8 && rows > 64 ? 64.0 : (double)rows) * DBL_EPSILON;
   const double noise2 = level * level * frob2;
 
   __shared__ int rotated;

@@ -1,0 +1,45 @@
+"""Factorisations whose output is written over their input."""
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from tests.test_gpu_cluster_factor import EPS
+
+pytestmark = pytest.mark.gpu
+
+# (rows, columns, output over the input): the whole of a is one factor
+CASES = [("svd", 60, 60, "u"), ("svd", 60, 60, "vh"), ("svd", 200, 30, "u"), ("svd", 30, 200, "vh"), ("svd", 150, 150, "vh"),
+         ("svd", 330, 330, "vh"), ("svd", 6, 6, "vh"), ("svd", 9, 1409, "vh"), ("qr", 90, 60, "u"), ("qr", 40, 300, "vh"),
+         ("qr", 5, 5, "vh"), ("eigh", 40, 40, "u"), ("eigh", 150, 150, "u")]
+
+
+@pytest.mark.parametrize("kind,m,n,over", CASES)
+def test_output_over_input(kind, m, n, over):
+    import torch
+
+    import tenet_b200 as tb
+    from tenet_b200 import _lib
+
+    rt = tb.Runtime(0)
+    rule, k = tb.U1FusionRule(), min(m, n)
+    plan = rt.fplan(rt.space(rule, [tb.GradedSpace(rule, [(0, m)])], [tb.GradedSpace(rule, [(0, n)])]))
+    A = np.random.default_rng(m + n).standard_normal((m, n))
+    if kind == "eigh":
+        A = A + A.T
+    a = torch.as_tensor(A.T.ravel().copy(), device="cuda")
+    new = lambda x: torch.full((x,), np.nan, dtype=torch.float64, device="cuda")
+    u = a if over == "u" else new(m * k)
+    v = a if over == "vh" else new(k * n)
+    s = new(k)
+    p = lambda t: C.c_void_p(t.data_ptr())
+    args = {"svd": (u, s, v), "qr": (u, v), "eigh": (u, s, None)}[kind]
+    _lib.call(f"tnt_{kind}", rt._h, plan._h, p(a), *(p(t) if t is not None else None for t in args), rt.stream())
+    h = lambda t, r, c: t.cpu().numpy().reshape(c, r).T
+    U = h(u, m, k)
+    V = U.T if kind == "eigh" else h(v, k, n)
+    S = np.ones(k) if kind == "qr" else s.cpu().numpy()
+    tol = 100 * np.sqrt(k) * EPS
+    assert np.linalg.norm((U * S) @ V - A) <= np.sqrt(k) * tol * np.linalg.norm(A)
+    assert np.abs(U.T @ U - np.eye(k)).max() <= tol

@@ -876,11 +876,14 @@ __global__ void __launch_bounds__(kFinishWarps * 32)
   const bool wide = m < n;
   const int64_t ldw = wide ? n : m;
   const FacWork f = fac_work(work + work_off[blockIdx.x], ldw, k);
-  const double sc = f.sv[c];
+  // A sector with an entry that is not finite has values that are not: they come first,
+  // so that every place is written.
+  auto value = [&](int64_t x) { return isnan(f.sv[x]) ? DBL_MAX * 2.0 : f.sv[x]; };
+  const double sc = f.sv[c], top = value(c);
   int64_t pos = 0;
   for (int64_t o = lane; o < k; o += 32) {
-    const double so = f.sv[o];
-    pos += (so > sc || (so == sc && o < c)) ? 1 : 0;
+    const double so = value(o);
+    pos += (so > top || (so == top && o < c)) ? 1 : 0;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) pos += __shfl_xor_sync(0xffffffffu, pos, o);

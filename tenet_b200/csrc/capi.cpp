@@ -326,6 +326,48 @@ static FacSchedule factor_schedule(const std::vector<SvdJob>& jobs, int wide) {
   return S;
 }
 
+// Where a plan's sectors lie in a, u and vh: element ranges, rising, neighbours joined (a
+// concatenated plan's buffers are usually one arena, which overlaps as a whole).
+struct FacSpans {
+  using Ranges = std::vector<std::pair<int64_t, int64_t>>;
+  Ranges a, u, v;
+  static Ranges joined(Ranges r) {
+    std::sort(r.begin(), r.end());
+    Ranges out;
+    for (const auto& x : r) {
+      if (x.first == x.second) continue;
+      if (!out.empty() && x.first <= out.back().second)
+        out.back().second = std::max(out.back().second, x.second);
+      else
+        out.push_back(x);
+    }
+    return out;
+  }
+  explicit FacSpans(const std::vector<SvdJob>& jobs) {
+    for (const SvdJob& J : jobs) {
+      a.push_back({J.a_off, J.a_off + J.m * J.n});
+      u.push_back({J.u_off, J.u_off + J.m * J.k});
+      v.push_back({J.v_off, J.v_off + J.k * J.n});
+    }
+    a = joined(a);
+    u = joined(u);
+    v = joined(v);
+  }
+  // Whether ranges x from px and y from py have a byte in common.
+  static bool overlap(const double* px, const Ranges& x, const double* py, const Ranges& y) {
+    auto at = [](const double* p, int64_t i) { return (uintptr_t)p + sizeof(double) * (uintptr_t)i; };
+    for (size_t i = 0, j = 0; i < x.size() && j < y.size();) {
+      if (at(px, x[i].second) <= at(py, y[j].first))
+        ++i;
+      else if (at(py, y[j].second) <= at(px, x[i].first))
+        ++j;
+      else
+        return true;
+    }
+    return false;
+  }
+};
+
 // A device's largest-first tables and the schedule they were laid out for.
 struct FacDevice {
   SvdJob* jobs = nullptr;
@@ -339,6 +381,7 @@ struct tnt_fplan_s {
   std::map<int, std::pair<SvdJob*, int64_t*>> dev;  // jobs, work offsets (sector order)
   std::map<int, FacDevice> lpt;                     // the same, in the order of the schedule
   std::map<int, FplanChunks> chunks;                // weighted-dot chunk tables
+  std::unique_ptr<FacSpans> span;                   // made by the first SVD
   int64_t work_elems = 0;
   std::vector<int64_t> work_off;
   ~tnt_fplan_s() {
@@ -382,6 +425,11 @@ struct tnt_fplan_s {
     auto r = std::make_pair(upload(p->tables.jobs), upload(work_off));
     dev.emplace(d, r);
     return r;
+  }
+  const FacSpans& spans() {
+    std::lock_guard<std::mutex> g(mu);
+    if (!span) span = std::make_unique<FacSpans>(p->tables.jobs);
+    return *span;
   }
   // Job and work-offset tables of the current device in the order of its schedule:
   // each job carries its own output offsets, so the order only changes which CTA
@@ -1670,7 +1718,7 @@ namespace {
 // the cluster Jacobi engine, their factors taken back through the reflectors.  The engine
 // keeps reflectors in u and vh while others still read a, so factors written over a
 // (in place) come from the one-CTA kernels, which read a sector whole before they write.
-cudaError_t svd_launches(const SvdTables& t, const FacDevice& dev, const double* a, double* u, double* s, double* vh,
+cudaError_t svd_launches(const FacSpans& spans, const FacDevice& dev, const double* a, double* u, double* s, double* vh,
                          double* work, int32_t* status, cudaStream_t st) {
   const FacSchedule& q = dev.sched;
   const int32_t njobs = (int32_t)q.order.size();
@@ -1678,11 +1726,7 @@ cudaError_t svd_launches(const SvdTables& t, const FacDevice& dev, const double*
   cudaError_t e = cudaSuccess;
   if (q.n_old > 0)
     e = launch_svd_split(dev.jobs, q.n_cluster, q.n_old, a, u, s, vh, work, dev.off, status, st, q.n_wide);
-  auto over_a = [&](const double* x, int64_t n) {
-    const uintptr_t p = (uintptr_t)x, r = (uintptr_t)a;
-    return p < r + sizeof(double) * (uintptr_t)t.a_size && r < p + sizeof(double) * (uintptr_t)n;
-  };
-  if (e == cudaSuccess && (over_a(u, t.u_size) || over_a(vh, t.v_size)))
+  if (e == cudaSuccess && (spans.overlap(a, spans.a, u, spans.u) || spans.overlap(a, spans.a, vh, spans.v)))
     return launch_svd(dev.jobs + q.n_old, njobs - q.n_old, a, u, s, vh, work, dev.off + q.n_old, status, st, true);
   for (const FacRun& r : q.runs) {
     const SvdJob* j = dev.jobs + r.first;
@@ -1724,7 +1768,7 @@ tnt_status tnt_svd(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, double
     }
     cudaStream_t st = (cudaStream_t)stream;
     cuda_check(cudaMemsetAsync(ctx->status, 0, 2 * sizeof(int32_t), st), "memset status");
-    cuda_check(svd_launches(t, dev, a, u, s, vh, ctx->svd_work, ctx->status, st),
+    cuda_check(svd_launches(plan->spans(), dev, a, u, s, vh, ctx->svd_work, ctx->status, st),
                "svd kernel launch");
     int32_t hs[2] = {0, 0};
     cuda_check(cudaMemcpyAsync(hs, ctx->status, sizeof(hs), cudaMemcpyDeviceToHost, st), "read svd status");
@@ -1746,7 +1790,7 @@ tnt_status tnt_svd_ws_async(tnt_ctx* ctx, const tnt_fplan* fplan, const double* 
     const FacDevice& dev = plan->lpt_on_device();
     cudaStream_t st = (cudaStream_t)stream;
     cuda_check(cudaMemsetAsync(status, 0, 2 * sizeof(int32_t), st), "memset status");
-    cuda_check(svd_launches(t, dev, a, u, s, vh, work, status, st),
+    cuda_check(svd_launches(plan->spans(), dev, a, u, s, vh, work, status, st),
                "svd kernel launch");
   });
 }
@@ -1789,7 +1833,7 @@ tnt_status tnt_svd_ws(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, dou
     cudaStream_t st = (cudaStream_t)stream;
     std::lock_guard<std::recursive_mutex> g(ctx->mu);  // the status words are the context's
     cuda_check(cudaMemsetAsync(ctx->status, 0, 2 * sizeof(int32_t), st), "memset status");
-    cuda_check(svd_launches(t, dev, a, u, s, vh, work, ctx->status, st),
+    cuda_check(svd_launches(plan->spans(), dev, a, u, s, vh, work, ctx->status, st),
                "svd kernel launch");
     int32_t hs[2] = {0, 0};
     cuda_check(cudaMemcpyAsync(hs, ctx->status, sizeof(hs), cudaMemcpyDeviceToHost, st), "read svd status");

@@ -43,3 +43,27 @@ def test_output_over_input(kind, m, n, over):
     tol = 100 * np.sqrt(k) * EPS
     assert np.linalg.norm((U * S) @ V - A) <= np.sqrt(k) * tol * np.linalg.norm(A)
     assert np.abs(U.T @ U - np.eye(k)).max() <= tol
+
+
+def test_factors_in_one_arena_are_not_in_place():
+    """All operands in one allocation (a serving arena): ranges that only neighbour are as apart."""
+    import torch
+
+    import tenet_b200 as tb
+    from tenet_b200 import _lib
+
+    rt = tb.Runtime(0)
+    rule = tb.U1FusionRule()
+    leg = [tb.GradedSpace(rule, [(0, 90), (1, 40)])]
+    plan = rt.fplan(rt.space(rule, leg, leg))
+    sizes = [plan.u_size, plan.u_size, plan.s_size, plan.v_size]
+    x = np.random.default_rng(2).standard_normal(sizes[0])
+    arena = torch.zeros(sum(sizes), dtype=torch.float64, device="cuda")
+    apart = [torch.zeros(n, dtype=torch.float64, device="cuda") for n in sizes]
+    at = np.concatenate([[0], np.cumsum(sizes)])
+    together = [arena[at[i]: at[i + 1]] for i in range(4)]
+    for a, u, s, v in (together, apart):
+        a.copy_(torch.as_tensor(x))
+        p = lambda t: C.c_void_p(t.data_ptr())
+        _lib.call("tnt_svd", rt._h, plan._h, p(a), p(u), p(s), p(v), rt.stream())
+    assert all(torch.equal(x, y) for x, y in zip(together, apart))

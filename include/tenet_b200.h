@@ -359,13 +359,15 @@ tnt_status tnt_ctx_sync(tnt_ctx* ctx, void* stream);
 /* Jacobi sweeps the slowest sector of the last tnt_svd / tnt_svd_ws on this
  * context needed (diagnostic). */
 tnt_status tnt_ctx_svd_sweeps(const tnt_ctx* ctx, int32_t* sweeps);
-/* How the factorisations take a plan's sectors on a device whose widest cluster is
- * `wide` CTAs (16, or 0 where only portable clusters of 8 fit).  counts (6): sectors on
- * the general kernels, of these the ones on clusters and on 16-CTA clusters, the
- * number of runs of the others, and whether (0 or 1) the SVD and the QR take all sectors
- * in one launch of the one-CTA kernels because they have few columns; runs (nullable, 2 per run, at most one run per sector):
- * sectors and CTAs per sector.  Host only; each device's tables keep their own. */
-tnt_status tnt_fplan_schedule(const tnt_fplan* plan, int32_t wide, int32_t* counts, int32_t* runs);
+/* How an operation (0 SVD, 1 QR, 2 eigh) takes a plan's sectors on a device whose widest
+ * cluster is `wide` CTAs (16, or 0 where only portable clusters of 8 fit).  counts (4):
+ * sectors on the general kernels, of these the ones on clusters and on 16-CTA clusters,
+ * and the number of runs of the others; runs (nullable, 2 per run, at most one run per
+ * sector): sectors, and the class they share, 0 for few columns (one CTA each), else the
+ * largest size of the class.  A sector's class follows from its own size, so that its
+ * results do not depend on the plan it is in.  Host only; each device's tables keep
+ * their own. */
+tnt_status tnt_fplan_schedule(const tnt_fplan* plan, int32_t op, int32_t wide, int32_t* counts, int32_t* runs);
 /* Doubles of SVD workspace a plan needs (tnt_svd_ws). */
 tnt_status tnt_fplan_work(const tnt_fplan* plan, int64_t* work_elems);
 /* tnt_svd with a caller-provided device workspace of tnt_fplan_work doubles

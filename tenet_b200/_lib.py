@@ -97,7 +97,7 @@ _SIGS = {
     "tnt_xplan_concat": [i32, P(vp), P(i64), P(i64), P(vp)],
     "tnt_cplan_concat": [i32, P(vp), P(i64), P(i64), P(i64), P(vp)],
     "tnt_fplan_concat": [i32, P(vp), P(i64), P(i64), P(i64), P(i64), P(i64), P(vp)],
-    "tnt_fplan_schedule": [vp, i32, P(i32), P(i32)],
+    "tnt_fplan_schedule": [vp, i32, i32, P(i32), P(i32)],
     "tnt_fplan_work": [vp, P(i64)],
     "tnt_svd_ws": [vp, vp, vp, vp, vp, vp, vp, vp],
     "tnt_qr": [vp, vp, vp, vp, vp, vp],

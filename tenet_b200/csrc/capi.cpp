@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -116,6 +117,13 @@ struct tnt_ctx_s {
   cudaEvent_t scratch_done = nullptr;
   cudaStream_t scratch_user = nullptr;
   bool scratch_user_valid = false;
+  // Side streams of a factorisation's runs and the events around them (FacFork).
+  struct Side {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t end = nullptr;
+  };
+  std::vector<Side> side;
+  cudaEvent_t side_begin = nullptr, side_gate = nullptr;
 };
 
 struct tnt_xplan_s {
@@ -227,101 +235,113 @@ struct FplanChunks {
   int64_t n = 0;
 };
 
-// Consecutive jobs of the largest-first table that run in one launch per stage.
+enum FacOp : int { kOpSvd = 0, kOpQr = 1, kOpEigh = 2 };
+
+// Consecutive jobs of an operation's table that run in one launch per stage.
 struct FacRun {
   int32_t first = 0, count = 0;
-  int64_t max_k = 0, max_rows = 0, max_cols = 0;
+  int64_t max_k = 0, max_rows = 0;
+  int first_cl = 1, cl = 1;  // CTAs per sector of the QR passes (first_cl: an SVD's rectangular sectors)
   bool rectangular = false;  // some sector is not square
+  bool one_cta = false;      // few columns: the one-CTA kernels, one launch
 };
 
-// How the factorisations take a plan's sectors on a device whose widest cluster is
-// `wide` CTAs (16, or 0 where only portable clusters of 8 fit): a value of the jobs
-// and that width alone, kept with each device's tables.
+// How an operation takes a plan's sectors on a device whose widest cluster is `wide` CTAs
+// (16, or 0 where only portable clusters of 8 fit): a value of the jobs and that width
+// alone, kept with each device's tables.
 struct FacSchedule {
-  std::vector<size_t> order;  // the largest-first table, as indices of the plan's jobs
+  std::vector<size_t> order;  // the table, as indices of the plan's jobs
   int32_t n_old = 0;          // its leading jobs, beyond the cluster QR and Jacobi kernels,
   int32_t n_cluster = 0;      // ... of which the first n_cluster run their SVD on clusters,
   int32_t n_wide = 0;         // ... and the first n_wide of these on 16-CTA clusters
-  std::vector<FacRun> runs;   // the other jobs, by falling k
-  bool few_svd = false, few_qr = false;  // all jobs have few columns: the one-CTA kernels in one launch
+  std::vector<FacRun> runs;   // the other jobs, longest chains first
 };
 
-static FacSchedule factor_schedule(const std::vector<SvdJob>& jobs, int wide) {
+// Sectors of few columns, for which the engine's four to six launches cost more than they
+// gain: one or a hundred of 4 x 4, SVD 65 us against 44 in one launch, QR 30 against 22.
+// The SVD's one-CTA kernel has a CTA's shared memory to itself and rotates on full columns
+// (1400 x 4 71 us against 109, 1400 x 5 131 against 120; 600 x 8 106 against 133, 9 x 9 no
+// gain).  The QR's walks a column per reflector in every warp: tall sectors up to 3000
+// elements (600 x 5 40 us against 48, 1400 x 3 52 against 42), wide ones by their trailing
+// updates (600 columns, 4 rows: one 64 against 45, 148 of them 66 against 115).
+static bool few_columns(FacOp op, const SvdJob& J) {
+  const int64_t rows = std::max(J.m, J.n);
+  if (op == kOpSvd) return J.k <= 4 || (J.k <= 8 && rows <= 640);
+  if (op == kOpQr) return J.k <= 8 && (J.m >= J.n ? J.m * J.n <= 3000 : J.n * J.m * J.m <= 10000);
+  return false;
+}
+
+// A sector's arithmetic must not depend on what else its plan holds (a request gives the
+// same bits alone and in a batch), so its kernels, lanes per column, panel width and
+// cluster of the sweeps follow from its own size: only sectors of one class share a run.
+static FacSchedule factor_schedule(const std::vector<SvdJob>& jobs, int wide, FacOp op) {
   FacSchedule S;
   S.order.resize(jobs.size());
   for (size_t i = 0; i < S.order.size(); ++i) S.order[i] = i;
-  auto cost = [&](size_t i) {
-    const double r = (double)std::max(jobs[i].m, jobs[i].n), k = (double)jobs[i].k;
-    return r * k * k;
-  };
+  auto rows = [&](size_t i) { return std::max(jobs[i].m, jobs[i].n); };
+  auto cost = [&](size_t i) { return (double)rows(i) * (double)jobs[i].k * (double)jobs[i].k; };
   // Sectors too long for the cluster QR and Jacobi kernels (old = true) go
   // first; of these, the ones whose blocked Jacobi has at least one column block
   // per cluster CTA run on a thread-block cluster (svd_cluster_kernel), those
   // with a block for each of 16 CTAs (where the device allows such clusters)
-  // ahead of the 8-CTA ones.  The rest follow by falling k.
-  auto old = [&](size_t i) { return std::max(jobs[i].m, jobs[i].n) > kQrMaxRows; };
-  auto clustered = [&](size_t i) {
-    const int64_t rows = std::max(jobs[i].m, jobs[i].n), k = jobs[i].k;
-    if (!old(i) || svd_on_chip(rows, k)) return 0;
-    const int bw = svd_block_width(rows, k);
+  // ahead of the 8-CTA ones.  The engine's classes follow, then few columns.
+  auto old = [&](size_t i) { return rows(i) > kQrMaxRows; };
+  auto clustered = [&](size_t i) -> int64_t {
+    const int64_t k = jobs[i].k;
+    if (!old(i) || svd_on_chip(rows(i), k)) return 0;
+    const int bw = svd_block_width(rows(i), k);
     if (bw <= 0) return 0;
     const int64_t nb = (k + bw - 1) / bw;
     return wide > 0 && nb >= wide ? 2 : nb >= svd_cluster_size() ? 1 : 0;
   };
+  using Key = std::array<int64_t, 4>;
+  std::vector<Key> key(jobs.size());
+  for (size_t i = 0; i < jobs.size(); ++i) {
+    const int64_t k = jobs[i].k;
+    if (old(i))
+      key[i] = Key{2, clustered(i), 0, 0};
+    else if (few_columns(op, jobs[i]))
+      key[i] = Key{0, 0, 0, 0};
+    else
+      key[i] = Key{1, op == kOpQr ? 0 : jacobi_class(k, wide, op == kOpSvd), op == kOpSvd ? qr_class(k) : 0,
+                   op == kOpEigh ? 0 : qr_class(rows(i))};
+  }
   std::stable_sort(S.order.begin(), S.order.end(), [&](size_t a, size_t b) {
-    if (old(a) != old(b)) return old(a);
-    if (!old(a)) return jobs[a].k > jobs[b].k;
-    const int ca = clustered(a), cb = clustered(b);
-    if (ca != cb) return ca > cb;
+    if (key[a] != key[b]) return key[a] > key[b];
+    if (key[a][0] == 1) return jobs[a].k > jobs[b].k;
     return cost(a) > cost(b);
   });
-  // The engine's four to six launches cost more than they gain where every sector has
-  // few columns: one sector or a hundred of 4 x 4, SVD 65 us against 44 in one launch, QR 30
-  // against 22.  The SVD's one-CTA kernel has a CTA's shared memory to itself and rotates
-  // on full columns, so from 5 columns on it takes one wave of sectors of up to 640 rows
-  // (300 of 5 x 5: 119 against 111 us; 1400 x 5: 131 against 120).  The QR's walks a column
-  // per reflector in every warp: tall sectors up to 3000 elements (600 x 5 40 against 48 us,
-  // 1400 x 3 52 against 42), wide ones by their trailing updates (200 columns: 4 rows 35
-  // against 38 us, 5 rows 42 against 38), for which many sectors have narrower clusters
-  // (600 columns and 4 rows, one 64 against 45, 60 of them 65 against 78, 148 66 against 115).
-  const int64_t wide_most = jobs.size() <= 36 ? 4096 : jobs.size() <= 74 ? 10000 : 20000;
-  S.few_svd = S.few_qr = !jobs.empty();
-  for (const SvdJob& J : jobs) {
-    const int64_t rows = std::max(J.m, J.n);
-    S.few_svd &= rows <= kQrMaxRows && (J.k <= 4 || (J.k <= 8 && jobs.size() <= 148 && rows <= 640));
-    S.few_qr &= J.k <= 8 && (J.m >= J.n ? J.m * J.n <= 3000 : J.n * J.m * J.m <= wide_most);
-  }
-  for (size_t i : S.order) {
-    S.n_old += old(i) ? 1 : 0;
-    S.n_cluster += clustered(i) > 0 ? 1 : 0;
-    S.n_wide += clustered(i) == 2 ? 1 : 0;
-  }
-  // One run per cluster width of the Jacobi kernel, each its own launch; a
-  // narrower run joins the one before it while all clusters of the joint
-  // launch fit the GPU's SMs at once (apart they would run one after the other).
-  std::vector<FacRun>& runs = S.runs;
-  for (size_t i = (size_t)S.n_old; i < S.order.size(); ++i) {
-    const SvdJob& J = jobs[S.order[i]];
-    if (runs.empty() || jacobi_cluster(runs.back().max_k, wide) != jacobi_cluster(J.k, wide)) {
-      FacRun r;
-      r.first = (int32_t)i;
-      r.max_k = J.k;
-      runs.push_back(r);
+  for (size_t n = 0; n < S.order.size(); ++n) {
+    const size_t i = S.order[n];
+    if (key[i][0] == 2) {
+      S.n_old += 1;
+      S.n_cluster += key[i][1] > 0 ? 1 : 0;
+      S.n_wide += key[i][1] == 2 ? 1 : 0;
+      continue;
     }
-    FacRun& r = runs.back();
+    if (S.runs.empty() || key[S.order[n - 1]] != key[i]) {
+      FacRun r;
+      r.first = (int32_t)n;
+      r.one_cta = key[i][0] == 0;
+      S.runs.push_back(r);
+    }
+    const SvdJob& J = jobs[i];
+    FacRun& r = S.runs.back();
     r.count += 1;
+    r.max_k = std::max(r.max_k, J.k);
     r.max_rows = std::max({r.max_rows, J.m, J.n});
-    r.max_cols = std::max(r.max_cols, J.n);
     r.rectangular |= J.m != J.n;
   }
-  for (size_t i = runs.size(); i-- > 1;) {
-    FacRun &x = runs[i - 1], &y = runs[i];
-    if ((int64_t)(x.count + y.count) * jacobi_cluster(x.max_k, wide) > 128) continue;
-    x.count += y.count;
-    x.max_rows = std::max(x.max_rows, y.max_rows);
-    x.max_cols = std::max(x.max_cols, y.max_cols);
-    x.rectangular |= y.rectangular;
-    runs.erase(runs.begin() + (long)i);
+  for (FacRun& r : S.runs) {
+    if (r.one_cta || op == kOpEigh) continue;
+    std::vector<QrSize> first, last;
+    for (int32_t n = r.first; n < r.first + r.count; ++n) {
+      const SvdJob& J = jobs[S.order[n]];
+      if (op == kOpSvd && J.m != J.n) first.push_back({std::max(J.m, J.n), J.k});
+      last.push_back(op == kOpSvd ? QrSize{J.k, J.k} : QrSize{J.m, J.n});
+    }
+    if (!first.empty()) r.first_cl = qr_cluster(first, wide);
+    r.cl = qr_cluster(last, wide);
   }
   return S;
 }
@@ -368,7 +388,7 @@ struct FacSpans {
   }
 };
 
-// A device's largest-first tables and the schedule they were laid out for.
+// A device's tables of an operation and the schedule they were laid out for.
 struct FacDevice {
   SvdJob* jobs = nullptr;
   int64_t* off = nullptr;
@@ -379,7 +399,7 @@ struct tnt_fplan_s {
   std::shared_ptr<FactorPlan> p;
   std::mutex mu;
   std::map<int, std::pair<SvdJob*, int64_t*>> dev;  // jobs, work offsets (sector order)
-  std::map<int, FacDevice> lpt;                     // the same, in the order of the schedule
+  std::map<std::pair<int, int>, FacDevice> lpt;     // the same in a schedule's order, by device and operation
   std::map<int, FplanChunks> chunks;                // weighted-dot chunk tables
   std::unique_ptr<FacSpans> span;                   // made by the first SVD
   int64_t work_elems = 0;
@@ -391,11 +411,11 @@ struct tnt_fplan_s {
       cudaSetDevice(kv.first);
       cudaFree(kv.second.first);
       cudaFree(kv.second.second);
-      auto lt = lpt.find(kv.first);
-      if (lt != lpt.end()) {
-        cudaFree(lt->second.jobs);
-        cudaFree(lt->second.off);
-      }
+      for (auto& lt : lpt)
+        if (lt.first.first == kv.first) {
+          cudaFree(lt.second.jobs);
+          cudaFree(lt.second.off);
+        }
       auto it = chunks.find(kv.first);
       if (it != chunks.end()) {
         cudaFree(it->second.sector);
@@ -431,20 +451,20 @@ struct tnt_fplan_s {
     if (!span) span = std::make_unique<FacSpans>(p->tables.jobs);
     return *span;
   }
-  // Job and work-offset tables of the current device in the order of its schedule:
-  // each job carries its own output offsets, so the order only changes which CTA
+  // Job and work-offset tables of the current device in the order of an operation's
+  // schedule: each job carries its own output offsets, so the order only changes which CTA
   // starts first, and the largest sectors no longer start in the last wave.  An entry
   // is complete before it is published and never changes, so callers read it without
   // the lock while other threads add other devices (map nodes do not move).
-  const FacDevice& lpt_on_device() {
+  const FacDevice& lpt_on_device(FacOp op) {
     on_device();  // sector-order tables first (needed by truncation and dots)
-    int d = current_device();
+    const std::pair<int, int> at(current_device(), (int)op);
     std::lock_guard<std::mutex> g(mu);
-    auto it = lpt.find(d);
+    auto it = lpt.find(at);
     if (it != lpt.end()) return it->second;
     const auto& jobs = p->tables.jobs;
     FacDevice x;
-    x.sched = factor_schedule(jobs, svd_wide_cluster_size());
+    x.sched = factor_schedule(jobs, svd_wide_cluster_size(), op);
     std::vector<SvdJob> sj(jobs.size());
     std::vector<int64_t> sw(jobs.size());
     for (size_t i = 0; i < jobs.size(); ++i) {
@@ -453,8 +473,76 @@ struct tnt_fplan_s {
     }
     x.jobs = upload(sj);
     x.off = upload(sw);
-    return lpt.emplace(d, std::move(x)).first->second;
+    return lpt.emplace(at, std::move(x)).first->second;
   }
+};
+
+// The runs of a factorisation side by side, between two sets of events on the context's
+// side streams (a run is a chain of small launches that leaves most of the GPU idle; one
+// after the other they would add up).  Where the first run's sweeps take 16-CTA clusters,
+// it has a stream of the highest priority and the others wait for its gate: a shorter run
+// that took their place first would keep one of its sectors waiting (D = 2048: 25.6 ms
+// against 22.7).  While the caller's stream captures, all runs are on that stream
+// alone: side streams are shared by calls.
+class FacFork {
+ public:
+  FacFork(tnt_ctx_s* ctx, cudaStream_t st, size_t runs, bool first_wide = false) : ctx_(ctx), st_(st) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (runs < 2 || cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return;
+    std::lock_guard<std::recursive_mutex> g(ctx->mu);
+    if (ctx->side.empty()) {  // published whole, or not at all
+      int least = 0, greatest = 0;
+      cuda_check(cudaDeviceGetStreamPriorityRange(&least, &greatest), "cudaDeviceGetStreamPriorityRange");
+      std::vector<tnt_ctx_s::Side> made(4);
+      for (size_t i = 0; i < made.size(); ++i) {
+        cuda_check(cudaStreamCreateWithPriority(&made[i].stream, cudaStreamNonBlocking, i == 0 ? greatest : least),
+                   "cudaStreamCreate(side)");
+        cuda_check(cudaEventCreateWithFlags(&made[i].end, cudaEventDisableTiming), "cudaEventCreate(side)");
+      }
+      if (!ctx->side_begin)
+        cuda_check(cudaEventCreateWithFlags(&ctx->side_begin, cudaEventDisableTiming), "cudaEventCreate(fork)");
+      if (!ctx->side_gate)
+        cuda_check(cudaEventCreateWithFlags(&ctx->side_gate, cudaEventDisableTiming), "cudaEventCreate(gate)");
+      ctx->side = std::move(made);
+    }
+    wide_ = first_wide;
+    // run 0: the caller's stream, or the first side stream; the others from there on
+    for (size_t i = wide_ ? 0 : 1; i < 4 && used_.size() + 1 < runs; ++i) used_.push_back(&ctx->side[i]);
+    cuda_check(cudaEventRecord(ctx->side_begin, st), "cudaEventRecord(fork)");
+    for (tnt_ctx_s::Side* x : used_)
+      cuda_check(cudaStreamWaitEvent(x->stream, ctx->side_begin, 0), "cudaStreamWaitEvent(fork)");
+  }
+  FacFork(const FacFork&) = delete;
+  ~FacFork() { join(); }  // an error half way leaves nothing running beside the caller's stream
+  cudaStream_t stream(size_t run) const {
+    if (used_.empty()) return st_;
+    if (!wide_) return run == 0 ? st_ : used_[(run - 1) % used_.size()]->stream;
+    if (run == 0) return used_[0]->stream;
+    return run == 1 || used_.size() == 1 ? st_ : used_[1 + (run - 2) % (used_.size() - 1)]->stream;
+  }
+  // Before the first run's sweeps, and before another run (whose first kernels then give
+  // the sweeps time to take their place).
+  void gate(size_t run) {
+    if (!wide_ || used_.empty()) return;
+    if (run == 0)
+      cuda_check(cudaEventRecord(ctx_->side_gate, stream(0)), "cudaEventRecord(gate)");
+    else
+      cuda_check(cudaStreamWaitEvent(stream(run), ctx_->side_gate, 0), "cudaStreamWaitEvent(gate)");
+  }
+  void join() {
+    if (used_.empty()) return;
+    std::lock_guard<std::recursive_mutex> g(ctx_->mu);
+    for (tnt_ctx_s::Side* x : used_)
+      if (cudaEventRecord(x->end, x->stream) != cudaSuccess || cudaStreamWaitEvent(st_, x->end, 0) != cudaSuccess)
+        cudaStreamSynchronize(x->stream);
+    used_.clear();
+  }
+
+ private:
+  tnt_ctx_s* ctx_;
+  cudaStream_t st_;
+  std::vector<tnt_ctx_s::Side*> used_;
+  bool wide_ = false;
 };
 
 extern "C" {
@@ -1129,6 +1217,12 @@ void tnt_ctx_destroy(tnt_ctx* ctx) {
   cudaGetDevice(&prev);
   cudaSetDevice(ctx->device);
   if (ctx->cublas) cublasDestroy(ctx->cublas);
+  for (auto& x : ctx->side) {
+    cudaStreamDestroy(x.stream);
+    if (x.end) cudaEventDestroy(x.end);
+  }
+  if (ctx->side_begin) cudaEventDestroy(ctx->side_begin);
+  if (ctx->side_gate) cudaEventDestroy(ctx->side_gate);
   cudaFree(ctx->stage);
   cudaFree(ctx->svd_work);
   cudaFree(ctx->eigh_tmp);
@@ -1718,30 +1812,43 @@ namespace {
 // the cluster Jacobi engine, their factors taken back through the reflectors.  The engine
 // keeps reflectors in u and vh while others still read a, so factors written over a
 // (in place) come from the one-CTA kernels, which read a sector whole before they write.
-cudaError_t svd_launches(const FacSpans& spans, const FacDevice& dev, const double* a, double* u, double* s, double* vh,
-                         double* work, int32_t* status, cudaStream_t st) {
+void svd_launches(tnt_ctx_s* ctx, const FacSpans& spans, const FacDevice& dev, const double* a, double* u, double* s,
+                  double* vh, double* work, int32_t* status, cudaStream_t st) {
   const FacSchedule& q = dev.sched;
   const int32_t njobs = (int32_t)q.order.size();
-  if (q.few_svd) return launch_svd(dev.jobs, njobs, a, u, s, vh, work, dev.off, status, st, true);
-  cudaError_t e = cudaSuccess;
+  const bool in_place = spans.overlap(a, spans.a, u, spans.u) || spans.overlap(a, spans.a, vh, spans.v);
+  const bool first_wide = q.n_old == 0 && !in_place && !q.runs.empty() && !q.runs[0].one_cta &&
+                          jacobi_cluster(q.runs[0].max_k, 16) == 16;
+  FacFork fork(ctx, st, (q.n_old > 0 ? 1 : 0) + (in_place ? 1 : q.runs.size()), first_wide);
+  size_t at = 0;
+  auto check = [](cudaError_t e) { cuda_check(e, "svd kernel launch"); };
   if (q.n_old > 0)
-    e = launch_svd_split(dev.jobs, q.n_cluster, q.n_old, a, u, s, vh, work, dev.off, status, st, q.n_wide);
-  if (e == cudaSuccess && (spans.overlap(a, spans.a, u, spans.u) || spans.overlap(a, spans.a, vh, spans.v)))
-    return launch_svd(dev.jobs + q.n_old, njobs - q.n_old, a, u, s, vh, work, dev.off + q.n_old, status, st, true);
-  for (const FacRun& r : q.runs) {
-    const SvdJob* j = dev.jobs + r.first;
-    const int64_t* off = dev.off + r.first;
-    auto then = [&](cudaError_t x) { e = e == cudaSuccess ? x : e; };
-    if (e == cudaSuccess && r.rectangular)
-      then(launch_qr_factor(j, r.count, r.max_rows, r.max_k, kQrSvdFirst, a, u, vh, work, off, st));
-    if (e == cudaSuccess) then(launch_qr_factor(j, r.count, r.max_k, r.max_k, kQrSvdSecond, a, u, vh, work, off, st));
-    if (e == cudaSuccess) then(launch_jacobi(j, r.count, r.max_k, work, off, status, true, st));
-    if (e == cudaSuccess) then(launch_qr_apply(j, r.count, r.max_k, r.max_k, kQrSvdSecond, u, vh, work, off, st));
-    if (e == cudaSuccess && r.rectangular)
-      then(launch_qr_apply(j, r.count, r.max_rows, r.max_k, kQrSvdFirst, u, vh, work, off, st));
-    if (e == cudaSuccess) then(launch_svd_finish(j, r.count, r.max_k, u, s, vh, work, off, st));
+    check(launch_svd_split(dev.jobs, q.n_cluster, q.n_old, a, u, s, vh, work, dev.off, status, fork.stream(at++),
+                           q.n_wide));
+  if (in_place && njobs > q.n_old) {
+    check(launch_svd(dev.jobs + q.n_old, njobs - q.n_old, a, u, s, vh, work, dev.off + q.n_old, status,
+                     fork.stream(at++), true));
+  } else {
+    for (const FacRun& r : q.runs) {
+      const SvdJob* j = dev.jobs + r.first;
+      const int64_t* off = dev.off + r.first;
+      const size_t run = at++;
+      cudaStream_t x = fork.stream(run);
+      if (run > 0) fork.gate(run);
+      if (r.one_cta) {
+        check(launch_svd(j, r.count, a, u, s, vh, work, off, status, x, true));
+        continue;
+      }
+      if (r.rectangular) check(launch_qr_factor(j, r.count, r.max_rows, r.first_cl, kQrSvdFirst, a, u, vh, work, off, x));
+      check(launch_qr_factor(j, r.count, r.max_k, r.cl, kQrSvdSecond, a, u, vh, work, off, x));
+      if (run == 0) fork.gate(0);
+      check(launch_jacobi(j, r.count, r.max_k, work, off, status, true, x));
+      check(launch_qr_apply(j, r.count, r.max_k, r.max_k, kQrSvdSecond, u, vh, work, off, x));
+      if (r.rectangular) check(launch_qr_apply(j, r.count, r.max_rows, r.max_k, kQrSvdFirst, u, vh, work, off, x));
+      check(launch_svd_finish(j, r.count, r.max_k, u, s, vh, work, off, x));
+    }
   }
-  return e;
+  fork.join();
 }
 
 }  // namespace
@@ -1757,7 +1864,7 @@ tnt_status tnt_svd(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, double
     const SvdTables& t = plan->p->tables;
     if (t.jobs.empty()) return;
     need(a && u && s && vh, "null operand");
-    const FacDevice& dev = plan->lpt_on_device();
+    const FacDevice& dev = plan->lpt_on_device(kOpSvd);
     std::lock_guard<std::recursive_mutex> g(ctx->mu);
     if (ctx->svd_work_elems < (size_t)plan->work_elems) {
       cudaFree(ctx->svd_work);
@@ -1768,8 +1875,7 @@ tnt_status tnt_svd(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, double
     }
     cudaStream_t st = (cudaStream_t)stream;
     cuda_check(cudaMemsetAsync(ctx->status, 0, 2 * sizeof(int32_t), st), "memset status");
-    cuda_check(svd_launches(plan->spans(), dev, a, u, s, vh, ctx->svd_work, ctx->status, st),
-               "svd kernel launch");
+    svd_launches(ctx, plan->spans(), dev, a, u, s, vh, ctx->svd_work, ctx->status, st);
     int32_t hs[2] = {0, 0};
     cuda_check(cudaMemcpyAsync(hs, ctx->status, sizeof(hs), cudaMemcpyDeviceToHost, st), "read svd status");
     cuda_check(cudaStreamSynchronize(st), "stream synchronize");
@@ -1787,28 +1893,27 @@ tnt_status tnt_svd_ws_async(tnt_ctx* ctx, const tnt_fplan* fplan, const double* 
     const SvdTables& t = plan->p->tables;
     if (t.jobs.empty()) return;
     need(a && u && s && vh && work && status, "null operand");
-    const FacDevice& dev = plan->lpt_on_device();
+    const FacDevice& dev = plan->lpt_on_device(kOpSvd);
     cudaStream_t st = (cudaStream_t)stream;
     cuda_check(cudaMemsetAsync(status, 0, 2 * sizeof(int32_t), st), "memset status");
-    cuda_check(svd_launches(plan->spans(), dev, a, u, s, vh, work, status, st),
-               "svd kernel launch");
+    svd_launches(ctx, plan->spans(), dev, a, u, s, vh, work, status, st);
   });
 }
 
-tnt_status tnt_fplan_schedule(const tnt_fplan* plan, int32_t wide, int32_t* counts, int32_t* runs) {
+tnt_status tnt_fplan_schedule(const tnt_fplan* plan, int32_t op, int32_t wide, int32_t* counts, int32_t* runs) {
   return guarded([&] {
     need(plan && counts, "null argument");
+    need(op >= kOpSvd && op <= kOpEigh, "operation: 0 SVD, 1 QR, 2 eigh");
     need(wide == 0 || wide == 16, "the widest cluster is 16 CTAs, or 0 where only portable ones fit");
-    const FacSchedule s = factor_schedule(plan->p->tables.jobs, wide);
+    const FacSchedule s = factor_schedule(plan->p->tables.jobs, wide, (FacOp)op);
     counts[0] = s.n_old;
     counts[1] = s.n_cluster;
     counts[2] = s.n_wide;
     counts[3] = (int32_t)s.runs.size();
-    counts[4] = s.few_svd ? 1 : 0;
-    counts[5] = s.few_qr ? 1 : 0;
     for (size_t i = 0; runs && i < s.runs.size(); ++i) {
-      runs[2 * i] = s.runs[i].count;
-      runs[2 * i + 1] = jacobi_cluster(s.runs[i].max_k, wide);
+      const FacRun& r = s.runs[i];
+      runs[2 * i] = r.count;
+      runs[2 * i + 1] = r.one_cta ? 0 : op == kOpQr ? (int32_t)qr_class(r.max_rows) : (int32_t)jacobi_class(r.max_k, wide, op == kOpSvd);
     }
   });
 }
@@ -1829,12 +1934,11 @@ tnt_status tnt_svd_ws(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, dou
     const SvdTables& t = plan->p->tables;
     if (t.jobs.empty()) return;
     need(a && u && s && vh && work, "null operand");
-    const FacDevice& dev = plan->lpt_on_device();
+    const FacDevice& dev = plan->lpt_on_device(kOpSvd);
     cudaStream_t st = (cudaStream_t)stream;
     std::lock_guard<std::recursive_mutex> g(ctx->mu);  // the status words are the context's
     cuda_check(cudaMemsetAsync(ctx->status, 0, 2 * sizeof(int32_t), st), "memset status");
-    cuda_check(svd_launches(plan->spans(), dev, a, u, s, vh, work, ctx->status, st),
-               "svd kernel launch");
+    svd_launches(ctx, plan->spans(), dev, a, u, s, vh, work, ctx->status, st);
     int32_t hs[2] = {0, 0};
     cuda_check(cudaMemcpyAsync(hs, ctx->status, sizeof(hs), cudaMemcpyDeviceToHost, st), "read svd status");
     cuda_check(cudaStreamSynchronize(st), "stream synchronize");
@@ -1866,22 +1970,29 @@ tnt_status tnt_qr(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, double*
     const SvdTables& t = plan->p->tables;
     if (t.jobs.empty()) return;
     need(a && q && r, "null operand");
-    const FacDevice& dev = plan->lpt_on_device();
+    const FacDevice& dev = plan->lpt_on_device(kOpQr);
     std::lock_guard<std::recursive_mutex> g(ctx->mu);
     double* work = factor_work(ctx, plan);
     cudaStream_t st = (cudaStream_t)stream;
     const FacSchedule& sched = dev.sched;
-    const int32_t one_cta = sched.few_qr ? (int32_t)sched.order.size() : sched.n_old;
-    cuda_check(launch_qr(dev.jobs, one_cta, a, q, r, work, dev.off, st), "qr kernel launch");
+    FacFork fork(ctx, st, sched.runs.size() + (sched.n_old > 0 ? 1 : 0));
+    size_t at = 0;
+    if (sched.n_old > 0)
+      cuda_check(launch_qr(dev.jobs, sched.n_old, a, q, r, work, dev.off, fork.stream(at++)), "qr kernel launch");
     for (const FacRun& x : sched.runs) {
-      if (sched.few_qr) break;
       const SvdJob* j = dev.jobs + x.first;
       const int64_t* off = dev.off + x.first;
-      cuda_check(launch_qr_factor(j, x.count, x.max_rows, x.max_cols, kQrFactor, a, q, r, work, off, st),
+      cudaStream_t side = fork.stream(at++);
+      if (x.one_cta) {
+        cuda_check(launch_qr(j, x.count, a, q, r, work, off, side), "qr kernel launch");
+        continue;
+      }
+      cuda_check(launch_qr_factor(j, x.count, x.max_rows, x.cl, kQrFactor, a, q, r, work, off, side),
                  "cluster qr launch");
-      cuda_check(launch_qr_apply(j, x.count, x.max_rows, x.max_k, kQrFactor, q, r, work, off, st),
+      cuda_check(launch_qr_apply(j, x.count, x.max_rows, x.max_k, kQrFactor, q, r, work, off, side),
                  "qr accumulation launch");
     }
+    fork.join();
     cuda_check(cudaStreamSynchronize(st), "stream synchronize");
   });
 }
@@ -1897,7 +2008,7 @@ tnt_status tnt_eigh(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, doubl
     need(a && vecs && vals, "null operand");
     for (const SvdJob& j : t.jobs)
       need(j.m == j.n, "eigh requires an endomorphism (square coupled-sector blocks)");
-    const FacDevice& dev = plan->lpt_on_device();
+    const FacDevice& dev = plan->lpt_on_device(kOpEigh);
     std::lock_guard<std::recursive_mutex> g(ctx->mu);
     double* work = factor_work(ctx, plan);
     cudaStream_t st = (cudaStream_t)stream;
@@ -1908,12 +2019,19 @@ tnt_status tnt_eigh(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, doubl
     int32_t* bad = nullptr;
     // All sectors are checked and swept before any of them writes its outputs: a call
     // that fails leaves them as they were.
-    for (const FacRun& r : dev.sched.runs) {
+    FacFork sweeps(ctx, st, dev.sched.runs.size(),
+                   !dev.sched.runs.empty() && jacobi_cluster(dev.sched.runs[0].max_k, 16) == 16);
+    for (size_t i = 0; i < dev.sched.runs.size(); ++i) {
+      const FacRun& r = dev.sched.runs[i];
       const SvdJob* j = dev.jobs + r.first;
       const int64_t* off = dev.off + r.first;
-      cuda_check(launch_eigh_prepare(j, r.count, r.max_k, a, work, off, ctx->status, st), "eigh preparation launch");
-      cuda_check(launch_jacobi(j, r.count, r.max_k, work, off, ctx->status, false, st), "eigh sweeps launch");
+      cudaStream_t x = sweeps.stream(i);
+      if (i > 0) sweeps.gate(i);
+      cuda_check(launch_eigh_prepare(j, r.count, r.max_k, a, work, off, ctx->status, x), "eigh preparation launch");
+      if (i == 0) sweeps.gate(0);
+      cuda_check(launch_jacobi(j, r.count, r.max_k, work, off, ctx->status, false, x), "eigh sweeps launch");
     }
+    sweeps.join();
     if (dev.sched.n_old > 0) {
       // Sectors beyond the cluster engine go through the general SVD of the
       // shifted, positive semidefinite A + ||A||_F I.
@@ -1938,10 +2056,14 @@ tnt_status tnt_eigh(tnt_ctx* ctx, const tnt_fplan* fplan, const double* a, doubl
                  "eigh (shifted SVD) launch");
       cuda_check(cudaMemcpyAsync(&hs[1], bad, sizeof(int32_t), cudaMemcpyDeviceToHost, st), "read eigh flag");
     }
-    for (const FacRun& r : dev.sched.runs)
+    FacFork outputs(ctx, st, dev.sched.runs.size());
+    for (size_t i = 0; i < dev.sched.runs.size(); ++i) {
+      const FacRun& r = dev.sched.runs[i];
       cuda_check(launch_eigh_finish(dev.jobs + r.first, r.count, r.max_k, a, vecs, vals, mags, work, dev.off + r.first,
-                                    ctx->status, bad, st),
+                                    ctx->status, bad, outputs.stream(i)),
                  "eigh output launch");
+    }
+    outputs.join();
     cuda_check(cudaMemcpyAsync(&hs[0], ctx->status, sizeof(int32_t), cudaMemcpyDeviceToHost, st), "read eigh status");
     cuda_check(cudaStreamSynchronize(st), "stream synchronize");
     if (hs[1] != 0 || (hs[0] & 2)) throw std::invalid_argument("eigh requires Hermitian coupled-sector blocks");

@@ -238,10 +238,10 @@ __device__ __forceinline__ void rotate_within(double* base, int ls, int w, int n
 // product and both columns stand above the rounding noise k eps ||A||_F (columns of
 // the null space shrink to that level, and every rotation refills them with
 // noise whose cosine is O(1)).  Every warp leaves its columns' squared norms in
-// sv first; part: 32 doubles of shared memory.
-__device__ __forceinline__ double make_thresholds(const FacWork& f, int64_t ldw, int k, int rank, int cl, double* part,
+// sv first.
+__device__ __forceinline__ double make_thresholds(const FacWork& f, int64_t ldw, int k, int rank, int cl,
                                                   Thresholds& th) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   for (int c = rank * nwarps + warp; c < k; c += cl * nwarps) {
     double s = 0.0;
     for (int x = lane; x < k; x += 32) {
@@ -252,13 +252,9 @@ __device__ __forceinline__ double make_thresholds(const FacWork& f, int64_t ldw,
     if (lane == 0) f.sv[c] = s;
   }
   cluster_barrier(cl);
-  double fs = 0.0;
-  for (int c = tid; c < k; c += blockDim.x) fs += __ldcg(f.sv + c);
-  fs = warp_sum(fs);
-  if (lane == 0) part[warp] = fs;
-  __syncthreads();
-  double frob2 = 0.0;
-  for (int i = 0; i < nwarps; ++i) frob2 += part[i];
+  double frob2 = 0.0;  // every warp the same sum in the same order, whatever the CTA's size
+  for (int c = lane; c < k; c += 32) frob2 += __ldcg(f.sv + c);
+  frob2 = warp_sum(frob2);
   const double tol = 4.0 * sqrt((double)k) * DBL_EPSILON;
   th.tol = (float)tol;
   th.noise2 = (float)(((double)k * DBL_EPSILON) * ((double)k * DBL_EPSILON) * frob2);
@@ -335,7 +331,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
   if (k == 0) return;
   const FacWork f = fac_work(work + work_off[blockIdx.x / cl], ldw, k);
   extern __shared__ __align__(16) double sm[];
-  __shared__ double s_nrm[2][kSlots], s_d[kSlots], s_id[kSlots], part[32];
+  __shared__ double s_nrm[2][kSlots], s_d[kSlots], s_id[kSlots];
   __shared__ int s_max[2][16][2], s_cos, s_fill;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gl = lane % G, owner = warp * PP + lane / G;
@@ -348,7 +344,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
     return n < 0 ? 0 : n < w ? n : w;
   };
   Thresholds th;
-  const double tol = make_thresholds(f, ldw, k, rank, cl, part, th);
+  const double tol = make_thresholds(f, ldw, k, rank, cl, th);
 
   // The first round's pair of blocks from the scratch, J = I.
   int bi = 0, bj = 0;
@@ -598,7 +594,6 @@ __global__ void __launch_bounds__(NW * 32, 1)
   int* words = reinterpret_cast<int*>(f.meta + 4);  // per sweep parity: cosine, fill (float bits)
   extern __shared__ __align__(16) double sm[];
   __shared__ double nrm[ZR], s_d[ZR], s_id[ZR];
-  __shared__ double part[32];
   __shared__ int s_cos, s_fill;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int w, nb;
@@ -614,7 +609,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
       for (int x = lane; x < k; x += 32) J[(int64_t)c * k + x] = x == c ? 1.0 : 0.0;
   if (rank == 0 && tid < 4) words[tid] = 0;
   Thresholds th;
-  const double tol = make_thresholds(f, ldw, k, rank, cl, part, th);
+  const double tol = make_thresholds(f, ldw, k, rank, cl, th);
 
   int sweep = 0;
   for (; sweep < kMaxSweeps && k > 1; ++sweep) {
@@ -1253,6 +1248,15 @@ __global__ void __launch_bounds__(kSmallThreads)
 // a sweep takes k rounds plus an exchange per block pair, so wider clusters
 // add exchanges where they no longer shorten the rounds.
 int jacobi_cluster(int64_t k, int wide) { return k <= 64 ? 1 : k <= 128 ? 4 : wide > 0 ? 16 : 8; }
+
+int64_t jacobi_class(int64_t k, int wide, bool acc_j) {
+  if (k <= 64) return 64;    // 8 lanes a column
+  if (k <= 128) return 128;  // 16 lanes
+  if (wide > 0 && k <= (acc_j ? 320 : 448)) return acc_j ? 320 : 448;  // 32 lanes, columns resident
+  for (int64_t c : {384, 448, 512, 608, 768, 1024})
+    if (k <= c) return c;
+  return kJacobiMaxK;
+}
 
 cudaError_t launch_jacobi(const SvdJob* jobs, int32_t njobs, int64_t max_k, double* work, const int64_t* work_off,
                           int32_t* status, bool acc_j, cudaStream_t st) {

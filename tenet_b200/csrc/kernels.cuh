@@ -110,6 +110,9 @@ cudaError_t launch_svd(const SvdJob* jobs, int32_t njobs, const double* a, doubl
 // max_k (at most kJacobiMaxK) is the largest k of the jobs.
 constexpr int64_t kJacobiMaxK = 1536;
 int jacobi_cluster(int64_t k, int wide);  // wide: svd_wide_cluster_size() of the device
+// Largest k of the class whose kernels (lanes per column, blocks, cluster) a k takes: one
+// launch's sectors are of one class.
+int64_t jacobi_class(int64_t k, int wide, bool acc_j);
 cudaError_t launch_jacobi(const SvdJob* jobs, int32_t njobs, int64_t max_k, double* work, const int64_t* work_off,
                           int32_t* status, bool acc_j, cudaStream_t stream);
 cudaError_t launch_svd_finish(const SvdJob* jobs, int32_t njobs, int64_t max_k, double* u, double* s, double* vh,
@@ -121,16 +124,21 @@ cudaError_t launch_eigh_finish(const SvdJob* jobs, int32_t njobs, int64_t max_n,
                                const int32_t* status, const int32_t* bad, cudaStream_t stream);
 
 // Cluster Householder QR of sectors with at most kQrMaxRows rows (qr.cu), and
-// products with its Q; max_rows / max_cols / max_k over the jobs.
+// products with its Q; max_rows / max_k over the jobs, cl CTAs for each.
 constexpr int64_t kQrMaxRows = 1408;
+// Largest rows of the class of one panel width (32 reflectors, then 16).
+inline int64_t qr_class(int64_t rows) { return rows <= 640 ? 640 : kQrMaxRows; }
 enum : int {
   kQrFactor = 0,    // tnt_qr: X = A, R to vh, Q (launch_qr_apply) to u
   kQrSvdFirst = 1,  // rectangular sectors: the long side reduced, reflectors in its output region
   kQrSvdSecond = 2  // the square rest, transposed; reflectors in the short side's region, R^T to the scratch
 };
-cudaError_t launch_qr_factor(const SvdJob* jobs, int32_t njobs, int64_t max_rows, int64_t max_cols, int mode,
-                             const double* a, double* u, double* vh, double* work, const int64_t* work_off,
-                             cudaStream_t stream);
+struct QrSize {
+  int64_t rows, cols;
+};
+int qr_cluster(const std::vector<QrSize>& sizes, int wide);  // sizes of a launch, longest first
+cudaError_t launch_qr_factor(const SvdJob* jobs, int32_t njobs, int64_t max_rows, int cl, int mode, const double* a,
+                             double* u, double* vh, double* work, const int64_t* work_off, cudaStream_t stream);
 cudaError_t launch_qr_apply(const SvdJob* jobs, int32_t njobs, int64_t max_rows, int64_t max_k, int mode, double* u,
                             double* vh, double* work, const int64_t* work_off, cudaStream_t stream);
 

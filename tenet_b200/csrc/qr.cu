@@ -19,6 +19,7 @@
 // the Jacobi engine: its columns are graded and nearly orthogonal, which takes 9 to 10 sweeps where the sector's own columns
 // take 11 (N(0, 1)) to 18 (a spectrum over three decades) at 104 x 104.
 #include <algorithm>
+#include <functional>
 
 #include "panel.cuh"
 
@@ -30,6 +31,7 @@ using namespace panel;
 
 constexpr int kSlots = 16;   // partial products of the split first multiply
 constexpr int kGroups = 4;   // 8-column groups updated at once by a CTA
+constexpr int kSplits = kSlots / kGroups;  // of the rows, in every product: the order of its sum is the sector's own
 constexpr int kW2Stride = 12;
 
 // What a launch factors and where its reflectors, T and outputs live.
@@ -111,14 +113,16 @@ __device__ void apply_block(double* X, int64_t ldx, int c0, int ncols, int p0, i
   for (int base = first; base < ngroups; base += kGroups * step) {
     int gb = (ngroups - base + step - 1) / step;
     if (gb > kGroups) gb = kGroups;
-    const int avail = nwarps < kSlots ? nwarps : kSlots, splits = avail / gb;
     auto group_col = [&](int q) { return c0 + 8 * (base + q * step); };
-    if (warp < gb * splits) {  // W1 = V^T X, the rows split over `splits` warps per group
-      const int q = warp % gb, sp = warp / gb;
+    // Warps left over by fewer groups take fewer of the reflectors each.
+    const int parts = gb * kSplits * 4 <= nwarps && MT == 4 ? 4 : gb * kSplits * 2 <= nwarps ? 2 : 1;
+    if (warp < gb * kSplits * parts) {  // W1 = V^T X, the rows split over kSplits warps per group
+      const int q = warp % gb, sp = warp / gb % kSplits, part = warp / (gb * kSplits);
       const int col = group_col(q) + g;
       const double* x0 = X + p0 + (int64_t)col * ldx;
-      const int kst = (nrows + 3) / 4, per = (kst + splits - 1) / splits;
+      const int kst = (nrows + 3) / 4, per = (kst + kSplits - 1) / kSplits;
       const int k0 = sp * per, k1 = k0 + per < kst ? k0 + per : kst;
+      const int m0 = part * (MT / parts), m1 = m0 + MT / parts;
       double acc[MT][2];
 #pragma unroll
       for (int m = 0; m < MT; ++m) acc[m][0] = acc[m][1] = 0.0;
@@ -134,19 +138,21 @@ __device__ void apply_block(double* X, int64_t ldx, int c0, int ncols, int p0, i
         for (int u = 0; u < 4; ++u)
           if (st + u < k1)
 #pragma unroll
-            for (int m = 0; m < MT; ++m) dmma(acc[m][0], acc[m][1], s.V[(8 * m + g) * s.ldv + 4 * (st + u) + t4], b[u]);
+            for (int m = 0; m < MT; ++m)
+              if (m >= m0 && m < m1) dmma(acc[m][0], acc[m][1], s.V[(8 * m + g) * s.ldv + 4 * (st + u) + t4], b[u]);
       }
       double* o = s.part + (sp * gb + q) * s.slot;
 #pragma unroll
-      for (int m = 0; m < MT; ++m) {
-        o[(8 * m + g) * 8 + 2 * t4] = acc[m][0];
-        o[(8 * m + g) * 8 + 2 * t4 + 1] = acc[m][1];
-      }
+      for (int m = 0; m < MT; ++m)
+        if (m >= m0 && m < m1) {
+          o[(8 * m + g) * 8 + 2 * t4] = acc[m][0];
+          o[(8 * m + g) * 8 + 2 * t4 + 1] = acc[m][1];
+        }
     }
     __syncthreads();
     for (int e = tid; e < gb * s.slot; e += blockDim.x) {
       double w = s.part[e];
-      for (int sp = 1; sp < splits; ++sp) w += s.part[sp * gb * s.slot + e];
+      for (int sp = 1; sp < kSplits; ++sp) w += s.part[sp * gb * s.slot + e];
       s.part[e] = w;
     }
     __syncthreads();
@@ -529,27 +535,43 @@ cudaError_t apply_class(const SvdJob* jobs, int32_t njobs, int64_t max_k, double
   return cudaGetLastError();
 }
 
-// CTAs of a sector's cluster: one while the trailing update is a few column groups, up
-// to 16 where it is the larger part; but no wider than lets every cluster of the launch
-// run at once (a CTA fills its SM, and eight clusters of 16, 16 of 8, 36 of 4 or 74 of 2 fit
-// 148 SMs in their GPCs).  A second wave costs as much as the first, a narrower cluster
-// at most a third more: 300 x 300 sectors, 1 / 10 / 37 / 80 of them, in ms:
-//   16 CTAs 0.79 / 1.48 / 4.40 / 8.80, 8 0.82 / 0.82 / 2.42 / 4.83, 4 0.88 / 0.89 / 1.83 / 2.86,
-//   2 1.01 / 1.02 / 1.18 / 2.34, 1 1.27 / 1.27 / 1.44 / 1.75.
-int qr_cluster(int64_t max_cols, int32_t njobs) {
-  const int wide = svd_wide_cluster_size() > 0 ? 16 : 8;
-  const int most = max_cols <= 48 ? 1 : max_cols <= 128 ? 4 : max_cols <= 256 ? 8 : wide;
-  const int fits = njobs <= 8 ? 16 : njobs <= 16 ? 8 : njobs <= 36 ? 4 : njobs <= 74 ? 2 : 1;
-  return std::min(most, fits);
-}
-
 }  // namespace
 
-cudaError_t launch_qr_factor(const SvdJob* jobs, int32_t njobs, int64_t max_rows, int64_t max_cols, int mode,
-                             const double* a, double* u, double* vh, double* work, const int64_t* work_off,
-                             cudaStream_t st) {
+// A launch's cluster width, by a longest-first deal of its sectors.  A CTA fills its SM;
+// eight clusters of 16, 16 of 8, 36 of 4 or 74 of 2 fit 148 SMs in their GPCs.  A sector is a
+// chain of reflectors of about 2 us each, which no width shortens, and trailing updates,
+// which the width divides.  300 x 300 sectors, 1 / 10 / 37 / 80 of them, in ms: 16 CTAs
+// 0.79 / 1.48 / 4.40 / 8.80, 8 0.82 / 0.82 / 2.42 / 4.83, 4 0.88 / 0.89 / 1.83 / 2.86,
+// 2 1.01 / 1.02 / 1.18 / 2.34, 1 1.27 / 1.27 / 1.44 / 1.75.
+int qr_cluster(const std::vector<QrSize>& sizes, int wide) {
+  struct Width {
+    int cl, fits;
+  };
+  int best = 1;
+  double best_t = 0.0;
+  std::vector<double> load;
+  for (const Width& w : {Width{1, 148}, Width{2, 74}, Width{4, 36}, Width{8, 16}, Width{16, 8}}) {
+    if (w.cl > 8 && wide <= 0) break;
+    load.assign(w.fits, 0.0);  // a heap, the first cluster to be free in front
+    double top = 0.0;
+    for (const QrSize& z : sizes) {
+      const double r = (double)z.rows, n = (double)std::min(z.rows, z.cols);
+      const double t = 2.0 * n * (1.0 + r / 1500.0) + 1.9e-5 * r * (double)z.cols * n / w.cl;
+      std::pop_heap(load.begin(), load.end(), std::greater<double>());
+      top = std::max(top, load.back() += t);
+      std::push_heap(load.begin(), load.end(), std::greater<double>());
+    }
+    if (w.cl == 1 || top < 0.98 * best_t) {  // a wider cluster also pays for its barriers
+      best = w.cl;
+      best_t = top;
+    }
+  }
+  return best;
+}
+
+cudaError_t launch_qr_factor(const SvdJob* jobs, int32_t njobs, int64_t max_rows, int cl, int mode, const double* a,
+                             double* u, double* vh, double* work, const int64_t* work_off, cudaStream_t st) {
   if (njobs == 0) return cudaSuccess;
-  const int cl = qr_cluster(max_cols, njobs);
   if (max_rows <= 64) return factor_class<32, 2>(jobs, njobs, a, u, vh, work, work_off, cl, mode, st);
   if (max_rows <= 256) return factor_class<32, 8>(jobs, njobs, a, u, vh, work, work_off, cl, mode, st);
   if (max_rows <= 640) return factor_class<32, 20>(jobs, njobs, a, u, vh, work, work_off, cl, mode, st);

@@ -23,21 +23,42 @@ def plan_of(sectors):
     return typed.FactorPlan(typed.HomSpace(U1, [rows], [cols]))
 
 
-def schedule(plan, wide):
-    counts, runs = (C.c_int32 * 6)(), (C.c_int32 * (2 * plan.nsectors))()
-    _lib.call("tnt_fplan_schedule", plan._h, wide, counts, runs)
-    return list(counts[:4]), [tuple(runs[2 * i: 2 * i + 2]) for i in range(counts[3])]
+SVD, QR, EIGH = 0, 1, 2
 
 
-def test_grouping_follows_the_cluster_width():
+def schedule(plan, wide, op=SVD):
+    counts, runs = (C.c_int32 * 4)(), (C.c_int32 * (2 * plan.nsectors))()
+    _lib.call("tnt_fplan_schedule", plan._h, op, wide, counts, runs)
+    return list(counts), [tuple(runs[2 * i: 2 * i + 2]) for i in range(counts[3])]
+
+
+def test_grouping_follows_the_sizes_and_the_cluster_width():
     plan = plan_of(SECTORS)
     (old, clusters, wide, _), runs = schedule(plan, 16)
-    assert (old, clusters, wide) == (2, 1, 1) and runs == [(8, 16)]  # 8 x 16 CTAs fit the SMs at once
+    assert (old, clusters, wide) == (2, 1, 1) and runs == [(3, 320), (2, 128), (1, 64), (2, 0)]
     (old, clusters, wide, _), runs = schedule(plan, 0)
-    assert (old, clusters, wide) == (2, 1, 0) and runs == [(8, 8)]
-    many = plan_of([(200, 200)] * 20 + [(100, 100)] * 30 + [(3, 3)] * 150)
-    assert schedule(many, 16)[1] == [(20, 16), (30, 4), (150, 1)]
-    assert schedule(many, 0)[1] == [(20, 8), (30, 4), (150, 1)]
+    assert (old, clusters, wide) == (2, 1, 0) and runs == [(3, 384), (2, 128), (1, 64), (2, 0)]
+    assert schedule(plan, 16, QR)[1] == [(6, 640), (2, 0)]
+    square = plan_of([(n, n) for n, _ in SECTORS])
+    assert schedule(square, 16, EIGH)[1] == [(3, 448), (2, 128), (3, 64)]
+
+
+@pytest.mark.parametrize("op", [SVD, QR, EIGH])
+def test_a_sector_keeps_its_class_in_every_plan(op):
+    sizes = [1, 4, 5, 8, 9, 64, 65, 128, 129, 320, 321, 385, 448, 449, 513, 609, 640, 641, 769, 1025, 1408]
+    shapes = [(n, n) for n in sizes] + ([] if op == EIGH else [(2, 1408), (700, 8), (640, 8), (30, 641), (300, 900)])
+    alone = []
+    for s in shapes:
+        (old, _, _, n), runs = schedule(plan_of([s]), 16, op)
+        assert old == 0 and n == 1
+        alone.append(runs[0][1])
+    _, runs = schedule(plan_of(shapes), 16, op)
+    # every class of the joint plan holds exactly the sectors that have it alone (an SVD splits a
+    # class further by the panels of its QR passes)
+    joint = {}
+    for count, c in runs:
+        joint[c] = joint.get(c, 0) + count
+    assert joint == {c: alone.count(c) for c in set(alone)}
 
 
 def test_threads_on_different_devices_share_a_plan():

@@ -40,7 +40,7 @@ def run(kind, shapes, blocks):
     u, s, v = (torch.full((x,), np.nan, dtype=torch.float64, device="cuda") for x in (plan.u_size, plan.s_size,
                                                                                       plan.v_size))
     p = lambda t: C.c_void_p(t.data_ptr())
-    args = (p(a), p(u), p(s), p(v)) if kind == "svd" else (p(a), p(u), p(v))
+    args = {"svd": (p(a), p(u), p(s), p(v)), "qr": (p(a), p(u), p(v)), "eigh": (p(a), p(u), p(s), None)}[kind]
     _lib.call(f"tnt_{kind}", rt._h, plan._h, *args, rt.stream())
     u, s, v = (t.cpu().numpy() for t in (u, s, v))
     for (_, m, n, _), rec, i in zip(space.sectors(), plan.records.tolist(), index):

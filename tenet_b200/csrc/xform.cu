@@ -431,6 +431,7 @@ __device__ __forceinline__ void cp_async8(double* smem, const double* gmem) {
 // is written, positions step by additions (two divisions per tile and thread, not
 // two per element), and folded axes make the planes large.  0.6 GB U(1) tensor,
 // (a, b | c, d) -> (c, d | a, b): 186 -> 129 us, of 93 at the copy rate.
+template <bool kAdd>
 __global__ void __launch_bounds__(kXThreads, 3) xform_transpose_kernel(
     const XTrTile* __restrict__ tiles, int32_t ntiles, const XGroup* __restrict__ groups,
     const XEntry* __restrict__ src_e, const XEntry* __restrict__ dst_e, const double* __restrict__ coef,
@@ -522,34 +523,34 @@ __global__ void __launch_bounds__(kXThreads, 3) xform_transpose_kernel(
         });
       }
     };
-    if (beta == 0.0) {
+    if constexpr (!kAdd) {
       visit([](double* at, double x) { *at = x; });
-      return;
+    } else {
+      // Four elements are read before they are written: otherwise every load waits for
+      // the store before it (24 MB of ragged U(1) blocks 20 us, now 14).
+      double* at[4];
+      double v[4];
+      int have = 0;
+      auto flush = [&] {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (q < have) v[q] = fma(beta, *at[q], v[q]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (q < have) *at[q] = v[q];
+        have = 0;
+      };
+      visit([&](double* o, double x) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (q == have) {
+            at[q] = o;
+            v[q] = x;
+          }
+        if (++have == 4) flush();
+      });
+      flush();
     }
-    // Four elements are read before they are written: otherwise every load waits for
-    // the store before it (24 MB of ragged U(1) blocks 20 us, now 14).
-    double* at[4];
-    double v[4];
-    int have = 0;
-    auto flush = [&] {
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (q < have) v[q] = fma(beta, *at[q], v[q]);
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (q < have) *at[q] = v[q];
-      have = 0;
-    };
-    visit([&](double* o, double x) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (q == have) {
-          at[q] = o;
-          v[q] = x;
-        }
-      if (++have == 4) flush();
-    });
-    flush();
   };
 
   int32_t t = blockIdx.x;
@@ -599,16 +600,17 @@ cudaError_t launch_xform(const DevXform& x, double* dst, const double* src, doub
   }
   if (x.ntr > 0) {
     const int smem = 2 * x.tr_cap * (int)sizeof(double);
+    const auto kernel = beta != 0.0 ? xform_transpose_kernel<true> : xform_transpose_kernel<false>;
     if (smem > 40 * 1024) {  // beyond what a launch may ask for without it, next to the plane positions
       // Always the largest tile's need: the limit is the device's, and another thread's plan
       // may be launched between this call and the launch.
-      const cudaError_t e = cudaFuncSetAttribute(xform_transpose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  2 * kTrCap * (int)sizeof(double));
       if (e != cudaSuccess) return e;
     }
     const int grid = x.ntr < sms * 3 ? x.ntr : sms * 3;
-    xform_transpose_kernel<<<grid, kXThreads, smem, stream>>>(x.tr_tiles, x.ntr, x.groups, x.src, x.dst, x.coef, src,
-                                                             dst, alpha, beta, x.tr_cap);
+    kernel<<<grid, kXThreads, smem, stream>>>(x.tr_tiles, x.ntr, x.groups, x.src, x.dst, x.coef, src, dst, alpha, beta,
+                                              x.tr_cap);
   }
   return cudaGetLastError();
 }

@@ -949,9 +949,12 @@ static void split_tiles(XformTables& t) {
     target[k] = std::min<int64_t>(
         32768, std::max<int64_t>(512, total[k] / std::max<int64_t>(1, waves * slots - ngroups[k])));
   }
-  // Transposing tiles fill the staging buffer once a plan has a wave of such tiles;
-  // smaller plans spread over the slots.
-  const int64_t tr_cap = std::min<int64_t>(kTrCap, std::max<int64_t>(512, total[kXTransposing] / slots));
+  // Transposing tiles fill the staging buffer once a plan has two waves of such tiles.
+  // Plans of less than one wave get a tile per slot, those between two smaller ones: a
+  // second wave that is nearly empty costs a tile's latency (37 MB of U(1) blocks: 16.4
+  // us at one and a quarter waves of 4096, 14.4 at two).
+  const int64_t share = total[kXTransposing] / slots;
+  const int64_t tr_cap = std::min<int64_t>(kTrCap, std::max<int64_t>(512, share > kTrCap ? share / 2 : share));
   for (size_t gi = 0; gi < t.fgroups.size(); ++gi) {
     const XGroup& g = t.fgroups[gi];
     if (const int ks = axis_of(g)) {

@@ -855,10 +855,16 @@ static void fold_axes(XformTables& t) {
   t.fgroups.clear();
   t.fsrc.clear();
   t.fdst.clear();
-  int64_t total = 0;
+  int64_t total = 0, lanes = 0;  // elements, and the lanes that walk them as rows of the unfolded axis 0
   bool copies = true;
   for (auto& g : t.groups) {
+    int lead = 0;
+    while (lead + 1 < g.rank && g.dims[lead] == 1) ++lead;
+    const int64_t d0 = g.dims[lead];
+    int64_t w = 1;
+    while (w < 32 && w < d0) w *= 2;
     total += g.nelem;
+    lanes += g.nelem / std::max<int64_t>(1, d0) * ((d0 + w - 1) / w * w);
     copies &= g.nsrc == 1 && g.ndst == 1;
   }
   // Axis 0 where the copy is not transposing: rows no longer than a slot's share of the
@@ -867,8 +873,11 @@ static void fold_axes(XformTables& t) {
   // copies already keep eight columns' loads in flight, and rows of a few hundred walk a warp each
   // with fewer: up to 128 (Z2, 24-dimensional legs, 42 MB: 7.6 us, 11.3 at 576;
   // 32-dimensional, 134 MB: 28.2 us, 31.5 at 1024), and not below four columns a slot.
+  // Where a plan past 48 MB leaves a fifth of the lanes idle on its own rows, filling them is
+  // worth more (U(1), legs of ragged degeneracies, 288 MB: 77.9 us at 128, 63.6 at 1024).
   const int64_t group0 = std::min<int64_t>(1024, total / (148 * 3));
-  const int64_t copy0 = std::min<int64_t>(128, total / (148 * 3 * 4));
+  const bool idle = total > 3000000 && total < lanes * 4 / 5;
+  const int64_t copy0 = idle ? group0 : std::min<int64_t>(128, total / (148 * 3 * 4));
   std::vector<XEntry> src, dst;
   for (auto& g : t.groups) {
     int lead = 0;  // a source with stride 1 along the leading axis is not transposed

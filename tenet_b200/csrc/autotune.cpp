@@ -139,16 +139,10 @@ int choose_f64_cap(const std::vector<GemmJob>& jobs, int64_t nbatch, double g, d
       sizes[kinds++] = sizes[i];
   sizes.resize(kinds);
 
-  // Per cap: tiles by cost, and bounds on the time of a longest-first deal of them to
-  // the SMs: at least the SMs' mean load and the longest tile's chain (alone on its SM
-  // a tile still takes its latency, about six block times, per k-tile), at most the mean
-  // and one tile more.
-  struct Class {
-    double largest, cost;  // of the job's tiles (their place in the list), and of these
-    int64_t count;
-  };
+  // Per cap: bounds on the time of a longest-first deal of its tiles to the SMs: at least
+  // the SMs' mean load and the longest tile's chain (alone on its SM a tile still takes
+  // its latency, about six block times, per k-tile), at most the mean and one tile more.
   struct Option {
-    std::vector<Class> classes;
     double tiles = 0.0, mean = 0.0, chain = 0.0, least = 0.0, most = 0.0;
   };
   Option opt[kF64MaxBlocks + 1];
@@ -158,13 +152,11 @@ int choose_f64_cap(const std::vector<GemmJob>& jobs, int64_t nbatch, double g, d
     double top = 0.0;
     for (const Size& z : sizes) {
       const int mt = (z.mb + cap - 1) / cap, nt = (z.nb + cap - 1) / cap;
-      const double largest = (double)z.ks * (g + b * ceil_div(z.mb, mt) * ceil_div(z.nb, nt));
       for (int h = 1; h >= 0; --h)      // pieces one block taller than the others, then these
         for (int w = 1; w >= 0; --w) {  // and wider
           const int64_t n = z.count * (h ? z.mb % mt : mt - z.mb % mt) * (w ? z.nb % nt : nt - z.nb % nt);
           if (n == 0) continue;
           const double blocks = (double)(z.mb / mt + h) * (z.nb / nt + w), c = (double)z.ks * (g + b * blocks);
-          o.classes.push_back({largest, c, n});
           o.tiles += (double)n;
           o.mean += c * (double)n / sms;
           top = std::max(top, c);
@@ -176,44 +168,29 @@ int choose_f64_cap(const std::vector<GemmJob>& jobs, int64_t nbatch, double g, d
     o.most = deal ? std::max(o.mean + top, o.chain) : o.mean;
     bound = cap == kF64MaxBlocks ? o.most : std::min(bound, o.most);
   }
-  // Only caps that can still be the best are dealt out.
-  int best = 0, open = 0;
+  // Only caps that can still be the best, with other tiles than the next larger one, are dealt
+  // out, in the order of their lists (a deal by classes of equal tiles took another cap for an
+  // SU(2) map with sectors of 768 and 1024: 214 us, this one's 195).
+  std::vector<int> open;
   for (int cap = kF64MaxBlocks; cap >= 2; --cap)
-    if (opt[cap].least <= bound) {
-      best = open == 0 ? cap : best;
-      ++open;
-    }
-  if (open == 1) return best;
+    if (opt[cap].least <= bound && (cap == kF64MaxBlocks || opt[cap].tiles != opt[cap + 1].tiles)) open.push_back(cap);
+  int best = open.empty() ? kF64MaxBlocks : open[0];
+  if (open.size() < 2) return best;
   double best_t = 0.0;
-  for (int cap = kF64MaxBlocks; cap >= 2; --cap) {
-    Option& o = opt[cap];
-    if (o.least > bound) continue;
+  for (const int cap : open) {
+    const Option& o = opt[cap];
     double t = o.mean;
     if (o.tiles <= kDeal) {
-      std::sort(o.classes.begin(), o.classes.end(), [](const Class& x, const Class& y) {
-        return std::make_tuple(x.largest, x.cost) > std::make_tuple(y.largest, y.cost);
-      });
       std::vector<double> load(sms, 0.0);  // a heap, least loaded SM first
       double top = 0.0;
-      for (const Class& c : o.classes) {
-        int64_t n = c.count;
-        // Loads within one tile of each other: every SM takes one in each full round.
-        const double low = load.front();
-        if (n >= sms && top - low <= c.cost) {
-          const double add = (double)(n / sms) * c.cost;
-          for (double& l : load) l += add;
-          top += add;
-          n %= sms;
-        }
-        for (; n > 0; --n) {
-          std::pop_heap(load.begin(), load.end(), std::greater<double>());
-          top = std::max(top, load.back() += c.cost);
-          std::push_heap(load.begin(), load.end(), std::greater<double>());
-        }
+      for (const GemmTile& x : build_f64_tiles(jobs, nbatch, cap, g, b)) {
+        std::pop_heap(load.begin(), load.end(), std::greater<double>());
+        top = std::max(top, load.back() += (double)ksteps(jobs[x.job]) * (g + b * tile_blocks(x)));
+        std::push_heap(load.begin(), load.end(), std::greater<double>());
       }
       t = std::max(top, o.chain);
     }
-    if (cap == best || t < best_t) {
+    if (cap == open[0] || t < best_t) {
       best = cap;
       best_t = t;
     }

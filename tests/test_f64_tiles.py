@@ -1,6 +1,7 @@
 """The FP64 grouped GEMM's tiles and the rule that picks their size (host logic, no GPU)."""
 
 import ctypes as C
+import heapq
 import time
 
 import numpy as np
@@ -89,3 +90,41 @@ def test_the_choice_is_cheap_for_plans_of_many_sectors():
     _lib.lib().tnt_cplan_destroy(h)
     # these tiles are chosen and written in 0.2 ms; four candidate lists, sorted and dealt, took 10
     assert n.value > 10000 and best < 4e-3
+
+
+def deal(jobs, nbatch, cap, g=G, b=B, sms=SMS):
+    """Time of the cap's list, dealt longest first to the SMs."""
+    def pieces(n):
+        t = -(-n // cap)
+        return [n // t + (i < n % t) for i in range(t)] if n else []
+
+    rows = []
+    for q in range(nbatch):
+        for j, (m, n, k) in enumerate(jobs):
+            h, w = pieces(-(-m // 16)), pieces(-(-n // 16))
+            if h and w:
+                ks = float(-(-k // 16) + 1)
+                rows.append((-ks * (g + b * (h[0] * w[0])), q, j, ks, [x * y for x in h for y in w]))
+    rows.sort(key=lambda r: r[:3])
+    load, top, chain, total, count = [0.0] * sms, 0.0, 0.0, 0.0, 0
+    for *_, ks, blocks in rows:
+        for x in blocks:
+            c = ks * (g + b * x)
+            total, count, chain = total + c, count + 1, max(chain, ks * b * (6.0 + x))
+            top = max(top, heapq.heapreplace(load, load[0] + c) + c)
+    return max(top, chain) if count <= 20000 else total / sms
+
+
+SU2_16 = [(s, s, s) for s in (768, 1024, 1536, 512, 256)]  # the SU(2) rank-4 map of 16-dimensional legs
+CHOICES = [(SU2_16, 1), ([(768, 768, 768), (1024, 1024, 1024)], 2), (RAGGED, 7)]
+for _seed in range(40):
+    _r = np.random.default_rng(_seed)
+    _n, _most = int(_r.integers(1, 40)), int(_r.choice([40, 200, 700]))
+    CHOICES.append(([tuple(int(x) for x in _r.integers(1, _most, 3)) for _ in range(_n)], int(_r.integers(1, 9))))
+
+
+@pytest.mark.parametrize("jobs,nbatch", CHOICES)
+def test_the_choice_is_the_cap_whose_deal_ends_first(jobs, nbatch):
+    times = [deal(jobs, nbatch, cap) for cap in (5, 4, 3, 2)]
+    got = deal(jobs, nbatch, tiles(jobs, nbatch)[0])
+    assert got <= min(times) * (1 + 1e-12)  # the sums' order

@@ -46,9 +46,8 @@
 //
 // What bounds it (int8, S = 5): shared memory.  A 64-deep K block is 60 KB
 // written by the copies and 108 KB read by the MMAs, 1310 cycles at 128 bytes a
-// cycle against 960 of tensor work; 1170 - 1390 are measured, plus some 1700 per
-// tile to hand the accumulators over.  64 Hubbard composes (237 tiles of four K
-// blocks per SM): 1435 -> 1094 us; the effective-Hamiltonian products: 1395 ->
+// cycle against 960 of tensor work; and each tile hands the accumulators over.  64
+// Hubbard composes (237 tiles of four K blocks per SM): 1435 -> 1094 us; the effective-Hamiltonian products: 1395 ->
 // 1210 us, before and after 16 epilogue warps, their records laid out ahead, the
 // copies issued by 2 S lanes, and rows, columns and half K blocks of padding
 // left out.

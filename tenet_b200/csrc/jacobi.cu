@@ -41,8 +41,8 @@
 // their rounds instead of a CTA-wide barrier measured the same there.)
 // Measured on a B200 against the general kernels of svd.cu and a two-sided
 // Jacobi in shared memory: truncated SVD of the D = 2048 chain (six sectors of
-// 586, two of 293) 94.9 -> 21.8 ms, a whole two-site update at D = 224 (104 x 104)
-// 5.2 -> 1.15 ms, eigh at D = 224 6.4 -> 0.87 ms with eigenvalues to 4e-16 (1.4e-14).
+// 586, two of 293) 94.9 -> 22.6 ms, a whole two-site update at D = 224 (104 x 104)
+// 5.2 -> 1.13 ms, eigh at D = 224 6.4 -> 0.89 ms with eigenvalues to 4e-16 (1.4e-14).
 #include <algorithm>
 
 #include "panel.cuh"
@@ -1287,6 +1287,15 @@ cudaError_t launch_jacobi(const SvdJob* jobs, int32_t njobs, int64_t max_k, doub
     TNT_RING(32, 5, 5) TNT_RING(32, 6, 6) TNT_RING(32, 7, 7) TNT_RING(32, 8, 8) TNT_RING(32, 9, 9) TNT_RING(32, 10, 10)
     TNT_RING_EIGH(32, 12, 12) TNT_RING_EIGH(32, 14, 14)
   }
+  // Staged classes, on 16 CTAs: elements of a column per lane, accumulator rows, warps
+  // (columns of one block), passing column held.  To 608 columns a round is one block pair
+  // per CTA (block_split: 2 x 19 columns of 608 + 64 + 4 elements, 25688 of the 27648 doubles that
+  // fit; 2 x 20 of 640 do not), so a warp for each of ceil(k / 32) columns and the accumulator's 2 w
+  // rows rounded up to 32: 64 from 17 columns on.  Beyond, a CTA takes two pairs of 10 to 12
+  // columns a round up to 768, three of 9 to 11 up to 1024, then five or six of 7 or 8 (on 8
+  // CTAs 13 to 15, 10 to 12, 8): 15, 12 and 8 warps, within what shared memory (17, 13, 8) and the
+  // registers of a lane's part of a column (48, 64, 96 of 136, 170, 255) allow.
+  // From 17 elements a lane on a held column spills, so it is read again for its update.
   TNT_STAGED(12, 32, 16, true) TNT_STAGED(14, 32, 16, true) TNT_STAGED(16, 32, 16, true)
   TNT_STAGED(19, 64, 19, false) TNT_STAGED(24, 32, 15, false) TNT_STAGED(32, 32, 12, false) TNT_STAGED(48, 32, 8, false)
   return cudaErrorInvalidValue;

@@ -11,13 +11,14 @@
 // two.  Products with Q need no exchange: each CTA carries its own columns
 // through all panels.
 //
-// Measured: QR of the D = 1024 chain's bond matrix (six sectors of 293) 3.56 -> 0.75 ms
+// Measured: QR of the D = 1024 chain's bond matrix (six sectors of 293) 3.56 -> 0.79 ms
 // of kernels against one CTA per sector.
 //
 // The SVD factors X^T = Q R once (twice for a rectangular sector, whose first pass
-// makes it square; in the last pass the rows of X^T in falling order) and gives R^T to
-// the Jacobi engine: its columns are graded and nearly orthogonal, which takes 9 to 10 sweeps where the sector's own columns
-// take 11 (N(0, 1)) to 18 (a spectrum over three decades) at 104 x 104.
+// makes it square; in the last pass the rows of X^T in falling order) and gives R^T to the
+// Jacobi engine: its columns are graded and nearly orthogonal, which takes 9 to 10 sweeps
+// where the sector's own columns take 11 (N(0, 1)) to 18 (a spectrum over three decades)
+// at 104 x 104.
 #include <algorithm>
 #include <functional>
 
